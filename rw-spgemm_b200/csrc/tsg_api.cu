@@ -58,8 +58,6 @@ extern "C" int tsg_context_create(int device, tsg_context **out)
         e = cudaMalloc((void **)&ctx->d_status, sizeof(int));
     if (e == cudaSuccess)
         e = cudaMemset(ctx->d_status, 0, sizeof(int));
-    if (e == cudaSuccess && tsg_noalloc_prepare(device) != TSG_OK)
-        e = cudaErrorUnknown;
     if (e != cudaSuccess)
     {
         free(ctx);

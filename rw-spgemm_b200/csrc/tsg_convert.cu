@@ -153,6 +153,13 @@ int tsg_tiled_alloc_arrays(tsg_context *ctx, tsg_tiled *t, int with_csc)
     return TSG_OK;
 }
 
+static int alloc_row_view(tsg_context *ctx, tsg_tiled *mat)
+{
+    TSG_TRY(tsg_alloc(ctx, &mat->row_ptr, (size_t)mat->m + 1));
+    TSG_TRY(tsg_alloc(ctx, &mat->row_col, (size_t)mat->nnz));
+    return tsg_alloc(ctx, &mat->row_val, (size_t)mat->nnz);
+}
+
 extern "C" int tsg_csr_to_tiled(tsg_context *ctx, int m, int n, int nnz, const int *d_rowptr,
                                 const int *d_colidx, const double *d_val, int flags, tsg_tiled *out)
 {
@@ -195,7 +202,20 @@ extern "C" int tsg_csr_to_tiled(tsg_context *ctx, int m, int n, int nnz, const i
         TSG_CUDA(cudaMemsetAsync(out->tile_nnz, 0, sizeof(int), ctx->stream));
     }
     if (flags & TSG_TILED_CSC_VIEW)
+    {
+        // the row view is the input itself
+        TSG_TRY(alloc_row_view(ctx, out));
+        TSG_CUDA(cudaMemcpyAsync(out->row_ptr, d_rowptr, ((size_t)m + 1) * sizeof(int), cudaMemcpyDeviceToDevice,
+                                 ctx->stream));
+        if (nnz > 0)
+        {
+            TSG_CUDA(cudaMemcpyAsync(out->row_col, d_colidx, (size_t)nnz * sizeof(int), cudaMemcpyDeviceToDevice,
+                                     ctx->stream));
+            TSG_CUDA(cudaMemcpyAsync(out->row_val, d_val, (size_t)nnz * sizeof(double), cudaMemcpyDeviceToDevice,
+                                     ctx->stream));
+        }
         TSG_TRY(tsg_build_csc_view(ctx, out));
+    }
     return TSG_OK;
 }
 
@@ -267,18 +287,15 @@ int tsg_build_mask_t(tsg_context *ctx, tsg_tiled *mat)
 int tsg_build_row_view(tsg_context *ctx, tsg_tiled *mat)
 {
     if (!mat->row_ptr)
-    {
-        TSG_TRY(tsg_alloc(ctx, &mat->row_ptr, (size_t)mat->m + 1));
-        TSG_TRY(tsg_alloc(ctx, &mat->row_col, (size_t)mat->nnz));
-        TSG_TRY(tsg_alloc(ctx, &mat->row_val, (size_t)mat->nnz));
-    }
+        TSG_TRY(alloc_row_view(ctx, mat));
     return tsg_tiled_to_csr(ctx, mat, mat->row_ptr, mat->row_col, mat->row_val);
 }
 
 int tsg_build_csc_view(tsg_context *ctx, tsg_tiled *mat)
 {
     TSG_TRY(tsg_build_mask_t(ctx, mat));
-    TSG_TRY(tsg_build_row_view(ctx, mat));
+    if (!mat->row_ptr)
+        TSG_TRY(tsg_build_row_view(ctx, mat));
     const int T = mat->numtile, tilen = mat->tilen;
     if (!mat->csc_tile_ptr)
     {
@@ -341,60 +358,311 @@ __global__ void k_cm_gather(int T, const int *__restrict__ pos, const int *__res
 }
 
 // ---------------------------------------------------------------------------
-// Tiles -> CSR (src/tile2csr.h:8-137).  Half-warp per tile row, lane = row.
-// Row r of a tile spans [Ptr[r], Ptr[r+1]); the last real row of the tile
-// row ends at the tile nnz.
+// Tiles -> CSR (src/tile2csr.h:8-137), one CTA per tile row.  Row r of a tile
+// spans [Ptr[r], Ptr[r+1]); the last real row of the tile row ends at the
+// tile nnz.  A tile row's values are one range in both layouts, so its 16 row
+// offsets are the range's start plus a prefix of the 16 row lengths: no scan
+// over the matrix is needed and both passes run in one launch.
+//
+// Bound: bytes (16 of row offsets, 4 + 4 of value offset and column per tile,
+// 9 read and 12 written per value).  Pass 1 reads a tile's 16 row offsets as
+// one 16-byte word per thread and adds the byte differences.  Pass 2 takes NT
+// tiles at a time: their words go to shared memory, a ballot per row says
+// which tiles hold entries of it, and the row's warp walks those tiles only,
+// its entries flattened over the lanes: stores are consecutive, loads come
+// from runs of a row in a tile, and tiles empty in a row (nearly all of them
+// in a hypersparse product) cost one bit.
+// Measured on a B200 (before: a half-warp per tile row, its lanes walking a
+// row each, between a row-length pass and a scan): C of the 64^3 stencil,
+// 31.0 M values in 84 tiles a tile row, 0.874 -> 0.196 ms (3.5 TB/s); of an
+// R-MAT 16 graph, 164 M values in 3,075 tiles a row, 10.5 -> 1.47 ms; of
+// 65,536 random rows, 4.2 M values in 4,011 tiles a row, 2.67 -> 0.36 ms.
 // ---------------------------------------------------------------------------
-__global__ void k_t2c_rowlen(int m, int tilem, const int *__restrict__ tile_ptr,
-                             const int *__restrict__ tnnz, const unsigned char *__restrict__ Ptr,
-                             int *__restrict__ rowlen)
+enum
 {
-    const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int tr = (int)(gid >> 4);
-    const int lane = threadIdx.x & 15;
-    if (tr >= tilem)
-        return;
-    const int rows = tr == tilem - 1 ? m - (tilem - 1) * TSG_BS : TSG_BS;
-    if (lane >= rows)
-        return;
-    int sum = 0;
-    for (int t = tile_ptr[tr]; t < tile_ptr[tr + 1]; t++)
-    {
-        const int s = Ptr[(long long)t * TSG_BS + lane];
-        const int e = lane == rows - 1 ? tnnz[t + 1] - tnnz[t] : Ptr[(long long)t * TSG_BS + lane + 1];
-        sum += e - s;
-    }
-    rowlen[tr * TSG_BS + lane] = sum;
+    T2C_BOTH, // rowptr, colidx and val
+    T2C_ROWS, // rowptr alone
+    T2C_FILL  // colidx and val; rowptr is there
+};
+
+__device__ __forceinline__ uint4 t2c_ptr16(const unsigned char *Ptr, int t, bool aligned)
+{
+    const unsigned char *p = Ptr + (long long)t * TSG_BS;
+    if (aligned)
+        return *reinterpret_cast<const uint4 *>(p);
+    unsigned u[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        u[q] = p[4 * q] | (p[4 * q + 1] << 8) | (p[4 * q + 2] << 16) | ((unsigned)p[4 * q + 3] << 24);
+    return make_uint4(u[0], u[1], u[2], u[3]);
 }
 
-__global__ void k_t2c_fill(int m, int tilem, const int *__restrict__ tile_ptr,
-                           const int *__restrict__ tile_col, const int *__restrict__ tnnz,
-                           const unsigned char *__restrict__ Ptr, const unsigned char *__restrict__ Col,
-                           const double *__restrict__ Val, const int *__restrict__ rowptr,
-                           int *__restrict__ ccol, double *__restrict__ cval)
+// the 16 row lengths of a tile of cnt values, a byte each; rows real rows
+__device__ __forceinline__ void t2c_row_lens(uint4 w, int cnt, int rows, unsigned d[4])
 {
-    const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int tr = (int)(gid >> 4);
-    const int lane = threadIdx.x & 15;
-    if (tr >= tilem)
-        return;
-    const int rows = tr == tilem - 1 ? m - (tilem - 1) * TSG_BS : TSG_BS;
-    if (lane >= rows)
-        return;
-    int off = rowptr[tr * TSG_BS + lane];
-    for (int t = tile_ptr[tr]; t < tile_ptr[tr + 1]; t++)
+    const unsigned p[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int q = 0; q < 4; q++)
     {
-        const int s = Ptr[(long long)t * TSG_BS + lane];
-        const int e = lane == rows - 1 ? tnnz[t + 1] - tnnz[t] : Ptr[(long long)t * TSG_BS + lane + 1];
-        const int base = tnnz[t];
-        const int cb = tile_col[t] * TSG_BS;
-        for (int q = s; q < e; q++)
+        const unsigned nxt = (p[q] >> 8) | (q < 3 ? p[q < 3 ? q + 1 : 3] << 24 : (unsigned)cnt << 24);
+        d[q] = __vsub4(nxt, p[q]); // a full tile's 256 wraps to 0 and 0 - 240 to 16
+    }
+    if (rows < TSG_BS) // ragged last tile row
+#pragma unroll
+        for (int r = 0; r < TSG_BS; r++)
         {
-            ccol[off] = cb + Col[base + q];
-            cval[off] = Val[base + q];
-            off++;
+            const int sh = (r & 3) * 8;
+            if (r == rows - 1)
+                d[r >> 2] = (d[r >> 2] & ~(0xFFu << sh)) | (((unsigned)cnt - ((p[r >> 2] >> sh) & 0xFFu)) & 0xFFu) << sh;
+            else if (r >= rows)
+                d[r >> 2] &= ~(0xFFu << sh);
+        }
+}
+
+template <int NT>
+struct T2cSmem
+{
+    uint4 ptr[NT];               // row offsets of the step's tiles
+    int base[NT], col[NT];       // first value, first column
+    unsigned short cnt[NT];      // values
+    unsigned bits[TSG_BS][NT / 32]; // per row: tiles holding entries of it
+    unsigned short list[TSG_BS][NT]; // those tiles, in order
+    int len[TSG_BS], off[TSG_BS];    // row lengths; next output position of each row
+};
+
+template <int NT, int MODE>
+__global__ void __launch_bounds__(NT, 2048 / NT)
+    k_t2c(int m, int tr0, int tilem, const int *__restrict__ tile_ptr, const int *__restrict__ tile_col,
+          const int *__restrict__ tnnz, const unsigned char *__restrict__ Ptr, const unsigned char *__restrict__ Col,
+          const double *__restrict__ Val, int *__restrict__ rowptr, int *__restrict__ ccol, double *__restrict__ cval)
+{
+    __shared__ T2cSmem<NT> S;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tr = tr0 + blockIdx.x;
+    const int rows = tr == tilem - 1 ? m - (tilem - 1) * TSG_BS : TSG_BS;
+    const int t0 = tile_ptr[tr], t1 = tile_ptr[tr + 1];
+    const bool aligned = ((uintptr_t)Ptr & 15) == 0;
+    if (MODE != T2C_FILL)
+    {
+        if (tid < TSG_BS)
+            S.len[tid] = 0;
+        __syncthreads();
+        // 16-bit sums of the byte lengths, emptied into S.len before they can
+        // overflow (2048 tiles of at most 16)
+        unsigned lo[4] = {0u, 0u, 0u, 0u}, hi[4] = {0u, 0u, 0u, 0u};
+        int held = 0;
+        auto drain = [&]() {
+#pragma unroll
+            for (int r = 0; r < TSG_BS; r++)
+            {
+                const unsigned v = ((r & 1 ? hi[r >> 2] : lo[r >> 2]) >> ((r & 2) * 8)) & 0xFFFFu;
+                const unsigned sum = __reduce_add_sync(0xffffffffu, v);
+                if (lane == r && sum)
+                    atomicAdd(&S.len[r], (int)sum);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                lo[q] = hi[q] = 0u;
+        };
+        for (int tb = t0; tb < t1; tb += NT)
+        {
+            const int t = tb + tid;
+            if (t < t1)
+            {
+                unsigned d[4];
+                t2c_row_lens(t2c_ptr16(Ptr, t, aligned), tnnz[t + 1] - tnnz[t], rows, d);
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                {
+                    lo[q] += d[q] & 0x00FF00FFu;
+                    hi[q] += (d[q] >> 8) & 0x00FF00FFu;
+                }
+            }
+            if (++held == 2048)
+            {
+                drain();
+                held = 0;
+            }
+        }
+        if (t0 + warp * 32 < t1) // a warp that saw a tile
+            drain();
+        __syncthreads();
+        if (tid < 32)
+        {
+            const int n = lane < TSG_BS ? S.len[lane] : 0;
+            int incl = n;
+#pragma unroll
+            for (int d = 1; d < TSG_BS; d <<= 1)
+            {
+                const int o = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d)
+                    incl += o;
+            }
+            const int at = tnnz[t0] + incl - n;
+            if (lane < TSG_BS)
+                S.off[lane] = at;
+            if (lane < rows)
+                rowptr[tr * TSG_BS + lane] = at;
+            if (tr == tilem - 1 && lane == rows - 1)
+                rowptr[m] = at + n;
         }
     }
+    else if (tid < rows)
+        S.off[tid] = rowptr[tr * TSG_BS + tid];
+    if (MODE == T2C_ROWS)
+        return;
+    const unsigned char *pb = reinterpret_cast<const unsigned char *>(S.ptr);
+    for (int tb = t0; tb < t1; tb += NT)
+    {
+        const int t = tb + tid;
+        unsigned ne = 0; // rows the tile holds entries of
+        if (t < t1)
+        {
+            const uint4 w = t2c_ptr16(Ptr, t, aligned);
+            const int c0 = tnnz[t], cnt = tnnz[t + 1] - c0;
+            unsigned d[4];
+            t2c_row_lens(w, cnt, rows, d);
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+            {
+                // 0xFF per non-zero byte -> 4 bits
+                const unsigned f = __vcmpne4(d[q], 0u) & 0x08040201u;
+                ne |= ((f | (f >> 8) | (f >> 16) | (f >> 24)) & 15u) << (4 * q);
+            }
+            S.ptr[tid] = w;
+            S.base[tid] = c0;
+            S.cnt[tid] = (unsigned short)cnt;
+            S.col[tid] = tile_col[t] * TSG_BS;
+        }
+        unsigned mine = 0;
+#pragma unroll
+        for (int r = 0; r < TSG_BS; r++)
+        {
+            const unsigned b = __ballot_sync(0xffffffffu, (ne >> r) & 1u);
+            if (lane == r)
+                mine = b;
+        }
+        if (lane < TSG_BS)
+            S.bits[lane][warp] = mine;
+        __syncthreads();
+        for (int r = warp; r < rows; r += NT / 32)
+        {
+            // the row's tiles of this step, listed
+            unsigned word = lane < NT / 32 ? S.bits[r][lane] : 0u;
+            const int c = __popc(word);
+            int incl = c;
+#pragma unroll
+            for (int d = 1; d < NT / 32; d <<= 1)
+            {
+                const int o = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d)
+                    incl += o;
+            }
+            const int listed = __shfl_sync(0xffffffffu, incl, NT / 32 - 1);
+            for (int at = incl - c; word; word &= word - 1)
+                S.list[r][at++] = (unsigned short)(lane * 32 + __ffs(word) - 1);
+            __syncwarp();
+            int off = S.off[r];
+            for (int q0 = 0; q0 < listed; q0 += 32)
+            {
+                const int nv = min(32, listed - q0);
+                int src = 0, cb = 0, len = 0;
+                if (lane < nv)
+                {
+                    const int i = S.list[r][q0 + lane];
+                    const int s = pb[i * TSG_BS + r];
+                    len = (r == rows - 1 ? S.cnt[i] : pb[i * TSG_BS + r + 1]) - s;
+                    src = S.base[i] + s;
+                    cb = S.col[i];
+                }
+                int upto = len;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1)
+                {
+                    const int o = __shfl_up_sync(0xffffffffu, upto, d);
+                    if (lane >= d)
+                        upto += o;
+                }
+                const int n = __shfl_sync(0xffffffffu, upto, 31);
+                if (n == nv) // one entry per tile
+                {
+                    if (lane < nv)
+                    {
+                        ccol[off + lane] = cb + Col[src];
+                        cval[off + lane] = Val[src];
+                    }
+                }
+                else
+                {
+                    const int pre = upto - len;
+                    const int from = src - pre;
+                    for (int j0 = 0; j0 < n; j0 += 32)
+                    {
+                        const int j = j0 + lane;
+                        int l = 0; // the last listed tile starting at or before entry j
+#pragma unroll
+                        for (int sz = 16; sz > 0; sz >>= 1)
+                        {
+                            const int pc = __shfl_sync(0xffffffffu, pre, l + sz);
+                            if (l + sz < nv && pc <= j)
+                                l += sz;
+                        }
+                        const int fs = __shfl_sync(0xffffffffu, from, l);
+                        const int fc = __shfl_sync(0xffffffffu, cb, l);
+                        if (j < n)
+                        {
+                            ccol[off + j] = fc + Col[fs + j];
+                            cval[off + j] = Val[fs + j];
+                        }
+                    }
+                }
+                off += n;
+            }
+            if (lane == 0)
+                S.off[r] = off;
+        }
+        __syncthreads();
+    }
+}
+
+// Row pointers and / or entries of tile rows [tr0, tr1) of C; nothing is
+// allocated.  512 threads for wide tile rows (R-MAT 16, 3,075 tiles a row:
+// 1.47 ms, 1.80 with 256, 2.89 with 128; 8,192 rows of 366 tiles: 0.049, 0.052
+// and 0.079 ms).  For narrow ones the step's barriers cost more than its width
+// gives, so CTAs are small once there are enough of them to fill the GPU (64^3
+// stencil, 16,384 rows of 84 tiles: 0.196 ms with 128, 0.224 with 256, 0.297
+// with 512; 21^3, 579 rows of 36: 0.0215, 0.0177, 0.0176 ms).
+#define T2C_WIDE 256    // mean tiles per tile row
+#define T2C_MANY (148 * 16) // tile rows that fill every SM with 128-thread CTAs
+template <int MODE>
+static int t2c_launch(tsg_context *ctx, const tsg_tiled *C, int tr0, int tr1, int *rowptr, int *colidx, double *val)
+{
+    if (tr1 <= tr0)
+        return TSG_OK;
+    const unsigned grid = (unsigned)(tr1 - tr0);
+    const int nt = C->numtile / C->tilem >= T2C_WIDE ? 512 : tr1 - tr0 >= T2C_MANY ? 128 : 256;
+#define T2C_GO(NT)                                                                                                  \
+    k_t2c<NT, MODE><<<grid, NT, 0, ctx->stream>>>(C->m, tr0, C->tilem, C->tile_ptr, C->tile_columnidx, C->tile_nnz, \
+                                                  C->tile_csr_Ptr, C->tile_csr_Col, C->tile_csr_Value, rowptr, colidx, val)
+    if (nt == 512)
+        T2C_GO(512);
+    else if (nt == 256)
+        T2C_GO(256);
+    else
+        T2C_GO(128);
+#undef T2C_GO
+    TSG_LAUNCH_CHECK();
+    return TSG_OK;
+}
+
+int tsg_t2c_rows(tsg_context *ctx, const tsg_tiled *C, int *rowptr)
+{
+    return t2c_launch<T2C_ROWS>(ctx, C, 0, C->tilem, rowptr, nullptr, nullptr);
+}
+
+int tsg_t2c_fill(tsg_context *ctx, const tsg_tiled *C, int tr0, int tr1, int *rowptr, int *colidx, double *val)
+{
+    return t2c_launch<T2C_FILL>(ctx, C, tr0, tr1, rowptr, colidx, val);
 }
 
 extern "C" int tsg_tiled_to_csr(tsg_context *ctx, const tsg_tiled *C, int *d_rowptr, int *d_colidx,
@@ -402,21 +670,30 @@ extern "C" int tsg_tiled_to_csr(tsg_context *ctx, const tsg_tiled *C, int *d_row
 {
     if (!ctx || !C || !d_rowptr)
         return tsg_set_error(TSG_ERR_INVALID, "null argument");
-    const int m = C->m, tilem = C->tilem;
-    if (m == 0)
+    if (C->m == 0)
     {
         TSG_CUDA(cudaMemsetAsync(d_rowptr, 0, sizeof(int), ctx->stream));
         return TSG_OK;
     }
-    k_t2c_rowlen<<<tsg_blocks((long long)tilem * 16, 256), 256, 0, ctx->stream>>>(
-        m, tilem, C->tile_ptr, C->tile_nnz, C->tile_csr_Ptr, d_rowptr);
-    TSG_LAUNCH_CHECK();
-    TSG_TRY(tsg_scan_counts(ctx, d_rowptr, d_rowptr, m, nullptr));
-    k_t2c_fill<<<tsg_blocks((long long)tilem * 16, 256), 256, 0, ctx->stream>>>(
-        m, tilem, C->tile_ptr, C->tile_columnidx, C->tile_nnz, C->tile_csr_Ptr, C->tile_csr_Col,
-        C->tile_csr_Value, d_rowptr, d_colidx, d_val);
-    TSG_LAUNCH_CHECK();
-    return TSG_OK;
+    return t2c_launch<T2C_BOTH>(ctx, C, 0, C->tilem, d_rowptr, d_colidx, d_val);
+}
+
+// C's rows that tsg_tiled_to_csr_noalloc takes at most (its documented limit)
+#define NOALLOC_MAX_ROWS (4096LL * 8192)
+
+extern "C" int tsg_tiled_to_csr_noalloc(tsg_context *ctx, const tsg_tiled *C, int *d_rowptr, int *d_colidx,
+                                        double *d_val)
+{
+    if (!ctx || !C || !d_rowptr)
+        return tsg_set_error(TSG_ERR_INVALID, "null argument");
+    if (C->m < 0 || C->m > NOALLOC_MAX_ROWS)
+        return tsg_set_error(TSG_ERR_INVALID,
+                             "tsg_tiled_to_csr_noalloc: C has %d rows; without scratch memory at most %lld rows are "
+                             "taken (use tsg_tiled_to_csr)",
+                             C->m, NOALLOC_MAX_ROWS);
+    if (C->nnz > 0 && (!d_colidx || !d_val))
+        return tsg_set_error(TSG_ERR_INVALID, "null argument");
+    return tsg_tiled_to_csr(ctx, C, d_rowptr, d_colidx, d_val);
 }
 
 // Column-major download helper used by tsg_tiled_download (tsg_api.cu).

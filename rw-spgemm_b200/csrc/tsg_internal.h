@@ -35,10 +35,6 @@ struct tsg_context
     int last_step3;           // TSG_STEP3_* of the last numeric step launched
 };
 
-// Looks up the no-alloc conversion's scratch address on a device (that
-// device current); run at context creation.
-int tsg_noalloc_prepare(int device);
-
 // Reads and clears the context's device error word (synchronises the
 // context's stream); returns TSG_OK or the code a kernel recorded.
 int tsg_take_device_status(tsg_context *ctx);
@@ -135,6 +131,11 @@ int tsg_check_csr(tsg_context *ctx, int m, int n, int nnz, const int *rowptr, co
 
 // Column view of a row-major tiled matrix (csc_tile_ptr / rowidx / pos).
 int tsg_build_csc_view(tsg_context *ctx, tsg_tiled *mat);
+
+// Row pointers of C's CSR form (m > 0), and the entries of its tile rows
+// [tr0, tr1) given the row pointers; asynchronous, nothing is allocated.
+int tsg_t2c_rows(tsg_context *ctx, const tsg_tiled *C, int *rowptr);
+int tsg_t2c_fill(tsg_context *ctx, const tsg_tiled *C, int tr0, int tr1, int *rowptr, int *colidx, double *val);
 
 // Readback helper: copies one long long / int from device to host (syncs).
 int tsg_read_int(tsg_context *ctx, const int *dptr, long long *out);

@@ -672,13 +672,6 @@ extern "C" int tsg_spgemm(tsg_context *ctx, const tsg_tiled *A, const tsg_tiled 
     return spgemm_finish(ctx, R, info);
 }
 
-__global__ void k_t2c_rowlen(int m, int tilem, const int *__restrict__ tile_ptr, const int *__restrict__ tnnz,
-                             const unsigned char *__restrict__ Ptr, int *__restrict__ rowlen);
-__global__ void k_t2c_fill(int m, int tilem, const int *__restrict__ tile_ptr, const int *__restrict__ tile_col,
-                           const int *__restrict__ tnnz, const unsigned char *__restrict__ Ptr,
-                           const unsigned char *__restrict__ Col, const double *__restrict__ Val,
-                           const int *__restrict__ rowptr, int *__restrict__ ccol, double *__restrict__ cval);
-
 // C = A*B straight into host CSR buffers, the copy overlapping the numeric
 // step.  After step 2 the row pointer of C is final: it is computed and
 // copied first, so the host knows where every tile row's entries go.  Then
@@ -715,12 +708,7 @@ int tsg_spgemm_to_host(tsg_context *ctx, const tsg_tiled *A, const tsg_tiled *B,
         status = ([&]() -> int {
             // row pointer, to the host first
             if (m > 0)
-            {
-                k_t2c_rowlen<<<tsg_blocks((long long)tilem * 16, 256), 256, 0, st>>>(m, tilem, C.tile_ptr, C.tile_nnz,
-                                                                                   C.tile_csr_Ptr, d_rp);
-                TSG_LAUNCH_CHECK();
-                TSG_TRY(tsg_scan_counts(ctx, d_rp, d_rp, m, nullptr));
-            }
+                TSG_TRY(tsg_t2c_rows(ctx, &C, d_rp));
             else
                 TSG_CUDA(cudaMemsetAsync(d_rp, 0, sizeof(int), st));
             TSG_CUDA(cudaMemcpyAsync(h_rowptr, d_rp, ((size_t)m + 1) * sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -757,11 +745,7 @@ int tsg_spgemm_to_host(tsg_context *ctx, const tsg_tiled *A, const tsg_tiled *B,
                     continue;
                 if (spa)
                     TSG_TRY(launch_step3_spa_rows(ctx, P, R.nnzC, R.d_wide, r0, r1));
-                const int rows = std::min(m, r1 * TSG_BS) - r0 * TSG_BS;
-                k_t2c_fill<<<tsg_blocks((long long)(r1 - r0) * 16, 256), 256, 0, st>>>(
-                    rows, r1 - r0, C.tile_ptr + r0, C.tile_columnidx, C.tile_nnz, C.tile_csr_Ptr, C.tile_csr_Col,
-                    C.tile_csr_Value, d_rp + (long long)r0 * TSG_BS, d_ci, d_v);
-                TSG_LAUNCH_CHECK();
+                TSG_TRY(tsg_t2c_fill(ctx, &C, r0, r1, d_rp, d_ci, d_v));
                 TSG_CUDA(cudaEventRecord(ctx->copy_ev, st));
                 TSG_CUDA(cudaStreamWaitEvent(ctx->copy_stream, ctx->copy_ev, 0));
                 const long long e0 = h_rowptr[(long long)r0 * TSG_BS], e1 = h_rowptr[r1 * TSG_BS < m ? r1 * TSG_BS : m];

@@ -1,0 +1,54 @@
+"""Tiles -> CSR (k_t2c): a matrix that goes into tiles and out again is the
+matrix it was, bit for bit (copies: tolerance 0), at the sizes where the
+kernel's steps end: ragged last tile rows, full tiles (counts of 256), more
+tiles in a tile row than one step or one 16-bit sum holds, tile rows that
+choose each block size, and row offsets off their 16-byte boundary."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _matrix(kind, m, n, per_row, seed=3):
+    rng = np.random.default_rng(seed)
+    if kind == "full":
+        counts = np.full(m, n)
+    elif kind == "some":  # rows with nothing among them
+        counts = np.where(rng.random(m) < 0.3, 0, rng.integers(0, min(n, per_row) + 1, m))
+    else:
+        counts = np.full(m, min(n, per_row))
+    cols = [np.sort(rng.choice(n, c, replace=False)) if c < n else np.arange(n) for c in counts]
+    rp = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    ci = np.concatenate(cols).astype(np.int32) if rp[-1] else np.zeros(0, np.int32)
+    return m, n, rp, ci, rng.uniform(-1, 1, ci.size)
+
+
+SHAPES = [
+    ("full", 1, 1, 0), ("full", 17, 33, 0), ("full", 47, 16, 0), ("some", 31, 700, 40),
+    ("some", 5000, 600, 9),            # narrow tile rows, 256 threads
+    ("some", 16 * 2400 + 5, 300, 3),   # narrow and many, 128 threads
+    ("each", 33, 16 * 900, 400),       # wide, several steps of 512 tiles, most tiles empty in a row
+    ("each", 16, 16 * 1100000, 80000), # one tile row of > 2048 steps: the 16-bit sums are emptied
+]
+
+
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "-".join(map(str, s)))
+@pytest.mark.parametrize("off_boundary", [False, True])
+def test_tiles_and_back(tsg, ctx, shape, off_boundary):
+    import torch
+    m, n, rp, ci, v = _matrix(*shape)
+    d = torch.device("cuda", torch.cuda.current_device())
+    dev = [torch.from_numpy(x).to(d) for x in (rp, ci, v)]
+    T = tsg.csr_to_tiled(ctx, m, n, *dev, 0)
+    if off_boundary:
+        raw = torch.empty(16 * T.numtile + 1, dtype=torch.uint8, device=d)
+        tiles = T.download()
+        raw[1:] = torch.from_numpy(tiles["tile_csr_Ptr"]).to(d)
+        owned, T.s.tile_csr_Ptr = T.s.tile_csr_Ptr, raw.data_ptr() + 1
+    got = [x.cpu().numpy() for x in tsg.tiled_to_csr(ctx, T)]
+    if off_boundary:
+        T.s.tile_csr_Ptr = owned
+    T.free()
+    assert np.array_equal(got[0], rp)
+    assert np.array_equal(got[1], ci)
+    assert np.array_equal(got[2].view(np.uint64), v.view(np.uint64))
