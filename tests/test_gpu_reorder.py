@@ -167,3 +167,22 @@ def test_reorder_plan_ab_and_aat(tsg, ctx, oracle, gen, kind, algo, monkeypatch)
     np.testing.assert_array_equal(C[3], G[3])
     rel = np.abs(C[4] - G[4]) / np.maximum(np.abs(G[4]), 1e-300)
     assert rel.max(initial=0.0) <= 1e-12   # the inner index order changes with the ordering
+
+
+@pytest.mark.parametrize("leaves", [2047, 2048, 2049, 6000])
+def test_rcm_levels_with_large_buckets(tsg, ctx, oracle, leaves):
+    """RCM of a hub whose level has one bucket below, at and above the size
+    that the level kernel ranks by itself, with a path of narrow levels
+    behind it, equals the oracle's."""
+    import torch
+    n = leaves + 40
+    edges = [(0, i) for i in range(1, leaves + 1)] + [(leaves + i, leaves + i + 1) for i in range(39)]
+    r = np.array([e for a, b in edges for e in (a, b)])
+    c = np.array([e for a, b in edges for e in (b, a)])
+    key = np.sort(r.astype(np.int64) * n + c)
+    rp = np.searchsorted(key // n, np.arange(n + 1)).astype(np.int32)
+    ci = (key % n).astype(np.int32)
+    d = torch.device("cuda", torch.cuda.current_device())
+    got = tsg.order(ctx, "rcm", n, n, torch.from_numpy(rp).to(d), torch.from_numpy(ci).to(d)).cpu().numpy()
+    mat = (n, n, rp, ci, np.ones(ci.size))
+    assert np.array_equal(got, oracle.order("rcm", mat))
