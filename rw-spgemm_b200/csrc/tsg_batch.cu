@@ -537,13 +537,7 @@ __global__ void __launch_bounds__(NT)
     }
     else
     {
-        double *tacc = reinterpret_cast<double *>(s_raw) + hw * (TSG_BS * S3T_STRIDE);
-        if (!SCHED)
-        {
-            for (int q = lane; q < TSG_BS * S3T_STRIDE; q += 16)
-                tacc[q] = 0.0;
-            __syncwarp(hmask);
-        }
+        double *tA = reinterpret_cast<double *>(s_raw) + hw * S3T_WORDS;
         const long long total_items = itemoff[count];
         for (long long h = (long long)blockIdx.x * (NT / 16) + hw; h < total_items; h += nhw)
         {
@@ -555,7 +549,7 @@ __global__ void __launch_bounds__(NT)
             if (SCHED == 1)
                 step3_rows_item<W, CAP>(P, item, hmask, lane, reinterpret_cast<S3RowsSmem<W, CAP> *>(s_raw)[hw]);
             else
-                step3_tile(P, (int)item, hmask, lane, tacc);
+                step3_tile(P, (int)item, hmask, lane, tA);
         }
     }
     __syncthreads();
@@ -611,19 +605,15 @@ __global__ void __launch_bounds__(SPA_THREADS, 3)
 
 // ... and products with dense C tiles (>= `dense` values per tile on
 // average): the tile kernel, a half-warp per C tile.
-#define DENSE3_THREADS 256
+#define DENSE3_THREADS 128
 __global__ void __launch_bounds__(DENSE3_THREADS)
     k_batch_dense3(BatchProd *prods, int count, const long long *__restrict__ itemoff, const int *err, int dense)
 {
     if (*(volatile const int *)err)
         return;
-    __shared__ double s_acc[DENSE3_THREADS / 16][TSG_BS * S3T_STRIDE];
+    __shared__ __align__(16) double s_A[DENSE3_THREADS / 16][S3T_WORDS];
     const int lane = threadIdx.x & 15, hw = threadIdx.x >> 4;
     const unsigned hmask = TSG_HW_MASK(threadIdx.x);
-    double *tacc = s_acc[hw];
-    for (int q = lane; q < TSG_BS * S3T_STRIDE; q += 16)
-        tacc[q] = 0.0;
-    __syncwarp(hmask);
     const long long total_items = itemoff[count];
     const long long nhw = (long long)gridDim.x * (DENSE3_THREADS / 16);
     for (long long h = (long long)blockIdx.x * (DENSE3_THREADS / 16) + hw; h < total_items; h += nhw)
@@ -631,7 +621,7 @@ __global__ void __launch_bounds__(DENSE3_THREADS)
         const int p = find_product(itemoff, count, h);
         if (prods[p].status || prods[p].nnzC < (long long)dense * prods[p].numC)
             continue;
-        step3_tile(prods[p].P, (int)(h - itemoff[p]), hmask, lane, tacc);
+        step3_tile(prods[p].P, (int)(h - itemoff[p]), hmask, lane, s_A[hw]);
     }
     __syncthreads();
     if (threadIdx.x == 0)
@@ -785,7 +775,7 @@ static batch_kernel_t pick_kernel(const tsg_batch_params &p, size_t *smem, int *
     }
     if (p.schedule == TSG_SCHED_TILES)
     {
-        const size_t s3 = (size_t)(BATCH_THREADS / 16) * TSG_BS * S3T_STRIDE * 8;
+        const size_t s3 = (size_t)(BATCH_THREADS / 16) * S3T_WORDS * 8;
         *smem = s1 > s3 ? s1 : s3;
         return k_batch<0, 8, 256, BATCH_THREADS>;
     }

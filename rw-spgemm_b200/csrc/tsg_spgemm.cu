@@ -155,21 +155,15 @@ __global__ void __launch_bounds__(256) k_step2(ProdView P, int *__restrict__ bin
         atomicAdd(&bins[threadIdx.x], s_bins[threadIdx.x]);
 }
 
-#define S3_THREADS 256
+#define S3_THREADS 128
 #define S3_HW (S3_THREADS / 16)
 
-__global__ void __launch_bounds__(S3_THREADS) k_step3(ProdView P)
+__global__ void __launch_bounds__(S3_THREADS, 4) k_step3(ProdView P)
 {
-    __shared__ double s_acc[S3_HW][TSG_BS * S3T_STRIDE];
-    const int hw = threadIdx.x >> 4, lane = threadIdx.x & 15;
-    const unsigned hmask = TSG_HW_MASK(threadIdx.x);
-    double *acc = s_acc[hw];
-    for (int q = lane; q < TSG_BS * S3T_STRIDE; q += 16)
-        acc[q] = 0.0;
-    __syncwarp(hmask);
+    __shared__ __align__(16) double s_A[S3_HW][S3T_WORDS];
     const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
     if (t < P.numC)
-        step3_tile(P, (int)t, hmask, lane, acc);
+        step3_tile(P, (int)t, TSG_HW_MASK(threadIdx.x), threadIdx.x & 15, s_A[threadIdx.x >> 4]);
 }
 
 __global__ void __launch_bounds__(256) k_step3_elems(ProdView P)
