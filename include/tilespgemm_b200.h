@@ -311,6 +311,7 @@ typedef struct
 #define TSG_STEP3_SPA 5    /* k_step3_spa: SPA, CTA per tile-row segment      */
 #define TSG_STEP3_STAGED 6 /* k_step3_stg + k_step3_rest: SPA with operands
                             * staged in shared memory by bulk copies          */
+#define TSG_STEP3_WINDOWS 7 /* k_step3_win: warp per C row and column window */
 
 const char *tsg_status_string(int status);
 /* Message describing the last failure on the calling thread. */

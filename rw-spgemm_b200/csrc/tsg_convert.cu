@@ -434,7 +434,7 @@ template <int NT, int MODE>
 __global__ void __launch_bounds__(NT, 2048 / NT)
     k_t2c(int m, int tr0, int tilem, const int *__restrict__ tile_ptr, const int *__restrict__ tile_col,
           const int *__restrict__ tnnz, const unsigned char *__restrict__ Ptr, const unsigned char *__restrict__ Col,
-          const double *__restrict__ Val, int *__restrict__ rowptr, int *__restrict__ ccol, double *__restrict__ cval)
+          const double *__restrict__ Val, int *__restrict__ rowptr, int *__restrict__ ccol, double *__restrict__ cval, int colmask)
 {
     __shared__ T2cSmem<NT> S;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -588,7 +588,7 @@ __global__ void __launch_bounds__(NT, 2048 / NT)
                 {
                     if (lane < nv)
                     {
-                        ccol[off + lane] = cb + Col[src];
+                        ccol[off + lane] = cb + (Col[src] & colmask);
                         cval[off + lane] = Val[src];
                     }
                 }
@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(NT, 2048 / NT)
                         const int fc = __shfl_sync(0xffffffffu, cb, l);
                         if (j < n)
                         {
-                            ccol[off + j] = fc + Col[fs + j];
+                            ccol[off + j] = fc + (Col[fs + j] & colmask);
                             cval[off + j] = Val[fs + j];
                         }
                     }
@@ -635,7 +635,8 @@ __global__ void __launch_bounds__(NT, 2048 / NT)
 #define T2C_WIDE 256    // mean tiles per tile row
 #define T2C_MANY (148 * 16) // tile rows that fill every SM with 128-thread CTAs
 template <int MODE>
-static int t2c_launch(tsg_context *ctx, const tsg_tiled *C, int tr0, int tr1, int *rowptr, int *colidx, double *val)
+static int t2c_launch(tsg_context *ctx, const tsg_tiled *C, int tr0, int tr1, int *rowptr, int *colidx, double *val,
+                      int colmask = 0xFF)
 {
     if (tr1 <= tr0)
         return TSG_OK;
@@ -643,7 +644,7 @@ static int t2c_launch(tsg_context *ctx, const tsg_tiled *C, int tr0, int tr1, in
     const int nt = C->numtile / C->tilem >= T2C_WIDE ? 512 : tr1 - tr0 >= T2C_MANY ? 128 : 256;
 #define T2C_GO(NT)                                                                                                  \
     k_t2c<NT, MODE><<<grid, NT, 0, ctx->stream>>>(C->m, tr0, C->tilem, C->tile_ptr, C->tile_columnidx, C->tile_nnz, \
-                                                  C->tile_csr_Ptr, C->tile_csr_Col, C->tile_csr_Value, rowptr, colidx, val)
+                                                  C->tile_csr_Ptr, C->tile_csr_Col, C->tile_csr_Value, rowptr, colidx, val, colmask)
     if (nt == 512)
         T2C_GO(512);
     else if (nt == 256)
@@ -663,6 +664,12 @@ int tsg_t2c_rows(tsg_context *ctx, const tsg_tiled *C, int *rowptr)
 int tsg_t2c_fill(tsg_context *ctx, const tsg_tiled *C, int tr0, int tr1, int *rowptr, int *colidx, double *val)
 {
     return t2c_launch<T2C_FILL>(ctx, C, tr0, tr1, rowptr, colidx, val);
+}
+
+// A matrix's row view; packed column bytes are told apart from the row
+int tsg_t2c_view(tsg_context *ctx, const tsg_tiled *M, int *rowptr, int *colidx, double *val)
+{
+    return t2c_launch<T2C_BOTH>(ctx, M, 0, M->tilem, rowptr, colidx, val, 15);
 }
 
 extern "C" int tsg_tiled_to_csr(tsg_context *ctx, const tsg_tiled *C, int *d_rowptr, int *d_colidx,

@@ -34,6 +34,9 @@ struct ProdView
     const unsigned short *B_maskT;
     const int *B_rptr, *B_rcol; // row view of B (scalar CSR), may be null
     const double *B_rval;
+    const int *A_rptr, *A_rcol; // row view of A, may be null
+    const double *A_rval;
+    int mA, mB, nB;
     int browB; // mean entries per row of B (rounded down)
     int tilenB;
     int *C_ptr, *C_col, *C_row, *C_tnnz;
@@ -53,9 +56,21 @@ struct ProdView
 // ---------------------------------------------------------------------------
 #define S1_WORDS 1024
 
+// The count pass's bitmaps, kept for the emit pass, which then need not walk
+// the row's tile pairs again: tile row i's words at words + i * stride, its
+// first tile column and number of words in span[i] (no words: the row's
+// window is wider than stride words and is walked again).  words == null:
+// nothing is kept.
+struct StepOneBits
+{
+    unsigned *words;
+    int2 *span;
+    int stride;
+};
+
 template <bool EMIT>
 __device__ __forceinline__ int step1_row(const ProdView &P, int i, unsigned int *bm, int lane,
-                                         unsigned long long *pairs)
+                                         unsigned long long *pairs, const StepOneBits &K = {nullptr, nullptr, 0})
 {
     const int a0 = P.A_ptr[i], a1 = P.A_ptr[i + 1];
     int lo = INT_MAX, hi = -1;
@@ -155,11 +170,16 @@ __device__ __forceinline__ int step1_row(const ProdView &P, int i, unsigned int 
                 }
             }
             __syncwarp();
+            const bool keep = !EMIT && K.words && hi - (lo & ~31) < S1_WORDS * 32 && nw <= K.stride;
+            if (!EMIT && K.words && lane == 0)
+                K.span[i] = make_int2(c0, keep ? nw : 0);
             for (int wb = 0; wb < nw; wb += 32)
             {
                 const int w = wb + lane;
                 unsigned bits = w < nw ? bm[w] : 0u;
                 const int cnt = __popc(bits);
+                if (keep && w < nw)
+                    K.words[(long long)i * K.stride + w] = bits;
                 if (EMIT)
                 {
                     int incl = cnt;
@@ -192,6 +212,34 @@ __device__ __forceinline__ int step1_row(const ProdView &P, int i, unsigned int 
     return out;
 }
 
+// Emits tile row i's C tile columns from its kept words; false when none are
+// kept.  A lane per column: consecutive stores.
+__device__ __forceinline__ bool step1_emit_kept(const ProdView &P, int i, int lane, const StepOneBits &K)
+{
+    const int2 kept = K.words ? K.span[i] : make_int2(0, 0);
+    if (!kept.y)
+        return false;
+    const unsigned *words = K.words + (long long)i * K.stride;
+    int pos = P.C_ptr[i];
+    for (int wb = 0; wb < kept.y; wb += 32)
+    {
+        const unsigned mine = wb + lane < kept.y ? words[wb + lane] : 0u;
+        for (unsigned left = __ballot_sync(TSG_FULL_MASK, mine != 0u); left; left &= left - 1)
+        {
+            const int q = __ffs(left) - 1;
+            const unsigned bits = __shfl_sync(TSG_FULL_MASK, mine, q);
+            if ((bits >> lane) & 1u)
+            {
+                const int at = pos + __popc(bits & ((1u << lane) - 1u));
+                P.C_col[at] = kept.x + ((wb + q) << 5) + lane;
+                P.C_row[at] = i;
+            }
+            pos += __popc(bits);
+        }
+    }
+    return true;
+}
+
 // forward declarations of helpers defined below
 __device__ __forceinline__ unsigned bool_row(unsigned ma, uint4 q0, uint4 q1);
 __device__ __forceinline__ int hw_excl_scan(unsigned hmask, int lane, int cnt, int &total);
@@ -210,6 +258,9 @@ __device__ __forceinline__ int nnz_bin(int total);
 // ---------------------------------------------------------------------------
 #define S12_WORDS 256
 #define S12_MAXT 128
+// tile pairs from which a row is wide whatever its tiles: the warp takes them
+// 32 at a time (1,500 x 1,300 random, 3,775 pairs and 980 products a tile row)
+#define S12_MAXP 1024
 
 struct S12Smem
 {
@@ -218,41 +269,63 @@ struct S12Smem
     unsigned short acc[16][S12_MAXT + 2]; // [row][slot], padded: both access forms spread over banks
 };
 
-__device__ __forceinline__ int step12_row(const ProdView &P, int i, S12Smem &sm, int lane, int *s_bins)
+__device__ __forceinline__ int step12_row(const ProdView &P, int i, S12Smem &sm, int lane, int *s_bins,
+                                          const StepOneBits &K = {nullptr, nullptr, 0})
 {
     const int a0 = P.A_ptr[i], a1 = P.A_ptr[i + 1];
-    int lo = INT_MAX, hi = -1;
-    for (int pa = a0 + lane; pa < a1; pa += 32)
-    {
-        const int k = P.A_col[pa];
-        const int b0 = P.B_ptr[k], b1 = P.B_ptr[k + 1];
-        if (b1 > b0)
-        {
-            lo = min(lo, P.B_col[b0]);
-            hi = max(hi, P.B_col[b1 - 1]);
-        }
-    }
-    lo = __reduce_min_sync(TSG_FULL_MASK, lo);
-    hi = __reduce_max_sync(TSG_FULL_MASK, hi);
     const int cbase = P.C_ptr[i];
     const int ntiles = P.C_ptr[i + 1] - cbase;
-    if (hi < 0)
+    if (ntiles == 0)
         return 1;
-    const int c0 = lo & ~31;
-    const int nw = (hi - c0 + 32) >> 5;
-    if (nw > S12_WORDS || ntiles > S12_MAXT)
-        return 0; // wide row: the caller emits it with step1_row and runs step 2 per tile
-    for (int w = lane; w < nw; w += 32)
-        sm.bm[w] = 0;
-    __syncwarp();
-    for (int pa = a0; pa < a1; pa++)
+    if (ntiles > S12_MAXT)
+        return 0; // wide row: the caller emits it and runs step 2 on it
+    int pairs = 0;
+    for (int pa = a0 + lane; pa < a1; pa += 32)
+        pairs += P.B_ptr[P.A_col[pa] + 1] - P.B_ptr[P.A_col[pa]];
+    if (__reduce_add_sync(TSG_FULL_MASK, pairs) > S12_MAXP)
+        return 0;
+    int c0, nw;
+    const int2 kept = K.words ? K.span[i] : make_int2(0, 0);
+    if (kept.y)
     {
-        const int k = P.A_col[pa];
-        const int b0 = P.B_ptr[k], b1 = P.B_ptr[k + 1];
-        for (int pb = b0 + lane; pb < b1; pb += 32)
+        c0 = kept.x;
+        nw = kept.y;
+        if (nw > S12_WORDS)
+            return 0;
+        for (int w = lane; w < nw; w += 32)
+            sm.bm[w] = K.words[(long long)i * K.stride + w];
+    }
+    else
+    {
+        int lo = INT_MAX, hi = -1;
+        for (int pa = a0 + lane; pa < a1; pa += 32)
         {
-            const int j = P.B_col[pb] - c0;
-            atomicOr(&sm.bm[j >> 5], 1u << (j & 31));
+            const int k = P.A_col[pa];
+            const int b0 = P.B_ptr[k], b1 = P.B_ptr[k + 1];
+            if (b1 > b0)
+            {
+                lo = min(lo, P.B_col[b0]);
+                hi = max(hi, P.B_col[b1 - 1]);
+            }
+        }
+        lo = __reduce_min_sync(TSG_FULL_MASK, lo);
+        hi = __reduce_max_sync(TSG_FULL_MASK, hi);
+        c0 = lo & ~31;
+        nw = (hi - c0 + 32) >> 5;
+        if (nw > S12_WORDS)
+            return 0;
+        for (int w = lane; w < nw; w += 32)
+            sm.bm[w] = 0;
+        __syncwarp();
+        for (int pa = a0; pa < a1; pa++)
+        {
+            const int k = P.A_col[pa];
+            const int b0 = P.B_ptr[k], b1 = P.B_ptr[k + 1];
+            for (int pb = b0 + lane; pb < b1; pb += 32)
+            {
+                const int j = P.B_col[pb] - c0;
+                atomicOr(&sm.bm[j >> 5], 1u << (j & 31));
+            }
         }
     }
     __syncwarp();
@@ -559,7 +632,7 @@ __device__ __forceinline__ void step2_tile(const ProdView &P, int t, unsigned hm
 //
 // Bound: the FP64 pipe on dense tiles (32 instructions per k and two tiles).
 // Before, lane r walked row r's entries through a shared-memory row: a
-// load-add-store and a column byte per product: a band of 81 times a band of
+// load-add-store and a column byte per product.: a band of 81 times a band of
 // 81, 16,384 rows (107 M products), 0.345 -> 0.123 ms on a B200.
 #define S3T_DENSE 64
 #define S3T_STRIDE 18 // doubles per column of the spread A tile: 16-byte loads, stores spread over the banks

@@ -132,9 +132,11 @@ int tsg_check_csr(tsg_context *ctx, int m, int n, int nnz, const int *rowptr, co
 // Column view of a row-major tiled matrix (csc_tile_ptr / rowidx / pos).
 int tsg_build_csc_view(tsg_context *ctx, tsg_tiled *mat);
 
-// Row pointers of C's CSR form (m > 0), and the entries of its tile rows
-// [tr0, tr1) given the row pointers; asynchronous, nothing is allocated.
+// Row pointers of C's CSR form (m > 0), the whole row view of an operand, and
+// the entries of tile rows [tr0, tr1) given the row pointers; asynchronous,
+// nothing is allocated.
 int tsg_t2c_rows(tsg_context *ctx, const tsg_tiled *C, int *rowptr);
+int tsg_t2c_view(tsg_context *ctx, const tsg_tiled *M, int *rowptr, int *colidx, double *val);
 int tsg_t2c_fill(tsg_context *ctx, const tsg_tiled *C, int tr0, int tr1, int *rowptr, int *colidx, double *val);
 
 // Readback helper: copies one long long / int from device to host (syncs).

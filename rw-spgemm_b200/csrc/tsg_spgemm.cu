@@ -10,25 +10,47 @@
 // the tile schedule (half-warp per C tile, A-row x B-column intersection, as
 // the reference decomposes the work) or the row-segment schedule (half-warp
 // per run of C tiles in one tile row, tile-level Gustavson, no intersection).
+#include <limits.h>
+
 #include <algorithm>
 
 #include "tsg_device.cuh"
 #include "tsg_staged.cuh"
+#include "tsg_wide.cuh"
+#include "tsg_window.cuh"
 
 #define S1_WARPS 8
+// a CTA per tile row counts step 1's tiles from this many tile pairs per row
+// (mean tiles per row of A times B's): below it a warp per row keeps up
+#define S1_CTA_PAIRS 512
+// step 1's bitmaps are kept up to this many words per tile row, and in all
+#define S1_KEEP_WORDS 512
+#define S1_KEEP_TOTAL (1LL << 24)
+// tile columns of a CTA's shared memory in the wide-row step 2
+#define WIDE_SPAN 6144
 
 template <bool EMIT>
 __global__ void __launch_bounds__(S1_WARPS * 32) k_step1(ProdView P, int *__restrict__ C_cnt,
-                                                         unsigned long long *__restrict__ pairs)
+                                                         unsigned long long *__restrict__ pairs, StepOneBits K)
 {
     __shared__ unsigned int s_bm[S1_WARPS][S1_WORDS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int i = blockIdx.x * S1_WARPS + warp;
     if (i >= P.tilemA)
         return;
-    const int cnt = step1_row<EMIT>(P, i, s_bm[warp], lane, pairs);
+    const int cnt = step1_row<EMIT>(P, i, s_bm[warp], lane, pairs, K);
     if (!EMIT && lane == 0)
         C_cnt[i] = cnt;
+}
+
+// ... and a CTA per tile row (step1_row_cta)
+__global__ void __launch_bounds__(S1C_THREADS) k_step1_cta(ProdView P, int *__restrict__ C_cnt,
+                                                           unsigned long long *__restrict__ pairs, StepOneBits K)
+{
+    __shared__ S1cSmem S;
+    const int cnt = step1_row_cta(P, blockIdx.x, S, K, pairs);
+    if (threadIdx.x == 0)
+        C_cnt[blockIdx.x] = cnt;
 }
 
 // step 1's count pass summed over the block into one device word
@@ -52,9 +74,11 @@ __global__ void __launch_bounds__(S1_WARPS * 32) k_step1_total(ProdView P, unsig
     }
 }
 
-// fused step-1 emit + step 2 (warp per A tile row); wide rows are emitted by
-// step1_row and flagged for the wide-row step 2 (1, or 2 when hypersparse)
-__global__ void __launch_bounds__(256) k_step12(ProdView P, int *__restrict__ wide, int *__restrict__ bins)
+// fused step-1 emit + step 2 (warp per A tile row).  Wide rows are emitted
+// alone and left to the wide-row step 2: wide[i] says 1, or 2 when the row is
+// hypersparse (0 otherwise), and wide[tilemA ...] lists their units (wide_list).
+__global__ void __launch_bounds__(256) k_step12(ProdView P, StepOneBits K, int *__restrict__ wide,
+                                                int *__restrict__ bins)
 {
     __shared__ S12Smem sm[8];
     __shared__ int s_bins[4];
@@ -65,13 +89,14 @@ __global__ void __launch_bounds__(256) k_step12(ProdView P, int *__restrict__ wi
     const int i = blockIdx.x * 8 + warp;
     if (i < P.tilemA)
     {
-        const int done = step12_row(P, i, sm[warp], lane, s_bins);
+        const int done = step12_row(P, i, sm[warp], lane, s_bins, K);
         int kind = 0;
         if (!done)
         {
             static_assert(sizeof(S12Smem) >= S1_WORDS * sizeof(unsigned), "bitmap scratch");
             __syncwarp();
-            step1_row<true>(P, i, reinterpret_cast<unsigned *>(&sm[warp]), lane, nullptr);
+            if (!step1_emit_kept(P, i, lane, K))
+                step1_row<true>(P, i, reinterpret_cast<unsigned *>(&sm[warp]), lane, nullptr);
             __syncwarp(); // the row's C columns, emitted by all lanes
             kind = wide_kind(P, i, lane);
         }
@@ -79,9 +104,7 @@ __global__ void __launch_bounds__(256) k_step12(ProdView P, int *__restrict__ wi
         {
             wide[i] = kind;
             if (kind)
-                atomicAdd(&wide[P.tilemA], 1); // count of wide rows
-            if (kind == 2)
-                atomicAdd(&wide[P.tilemA + 1], 1); // count of hypersparse rows
+                wide_list(P, i, wide);
         }
     }
     __syncthreads();
@@ -104,39 +127,30 @@ __global__ void __launch_bounds__(256) k_step2_wide(ProdView P, const int *__res
         atomicAdd(&bins[threadIdx.x], s_bins[threadIdx.x]);
 }
 
-// scalar step 2 for the wide rows k_step12 left: CTAs take blocks of C tiles
-// from a device counter and run the wide rows' parts
-__global__ void __launch_bounds__(SPA_THREADS) k_step2_spa(ProdView P, const int *__restrict__ wide,
-                                                           unsigned *__restrict__ ctr, int *__restrict__ bins)
+// step 2 of the wide rows k_step12 listed, through B's row view: CTAs take
+// rows from a device counter
+template <int NT>
+__global__ void __launch_bounds__(NT, 1) k_step2_cta(ProdView P, int span, const int *__restrict__ wide,
+                                                  unsigned *__restrict__ ctr, int *__restrict__ bins)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
-    Spa2Smem &S = *reinterpret_cast<Spa2Smem *>(s_raw);
+    WideSmem<NT> &S = *reinterpret_cast<WideSmem<NT> *>(s_raw);
     __shared__ int s_bins[4];
-    __shared__ int s_blk;
-    if (wide[P.tilemA] == 0) // no wide row (k_step12 counted them)
+    const int units = wide[P.tilemA];
+    if (units == 0)
         return;
     if (threadIdx.x < 4)
         s_bins[threadIdx.x] = 0;
-    unsigned nxt = 0; // thread 0: the next block, claimed one block ahead
-    if (threadIdx.x == 0)
-        nxt = atomicAdd(ctr, 1u);
     for (;;)
     {
-        __syncthreads();
         if (threadIdx.x == 0)
-        {
-            s_blk = (int)nxt;
-            nxt = atomicAdd(ctr, 1u);
-        }
+            S.next = (int)atomicAdd(ctr, 1u);
         __syncthreads();
-        const long long tb = (long long)s_blk * SPA_BLK;
-        if (tb >= P.numC)
+        const int q = S.next;
+        if (q >= units)
             break;
-        if (threadIdx.x == 0)
-            spa_skip_hyper(P, wide, (int)tb, ctr, 0);
-        step2_spa_block(P, S, (int)tb, (int)min((long long)P.numC, tb + SPA_BLK), wide, s_bins);
+        step2_wide_row<NT>(P, S, span, wide[P.tilemA + 1 + 2 * q], wide[P.tilemA + 2 + 2 * q], s_bins);
     }
-    __syncthreads();
     if (threadIdx.x < 4 && s_bins[threadIdx.x])
         atomicAdd(&bins[threadIdx.x], s_bins[threadIdx.x]);
 }
@@ -270,6 +284,95 @@ __global__ void __launch_bounds__(SPA_THREADS, 2) k_step3_rest(ProdView P, const
     }
 }
 
+// warp per B row: its entry offset at every block boundary
+__global__ void __launch_bounds__(256) k_win_btab(int m, const int *__restrict__ rptr, const int *__restrict__ rcol,
+                                                  int blocks, int bits, int *__restrict__ tab)
+{
+    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (w >= m)
+        return;
+    const int e0 = rptr[w], e1 = rptr[w + 1];
+    int *t = tab + w * (blocks + 1);
+    // entry e opens the blocks after the previous entry's up to its own
+    for (int e = e0 + lane; e <= e1; e += 32)
+    {
+        const int prev = e > e0 ? rcol[e - 1] >> bits : -1;
+        const int cur = e < e1 ? rcol[e] >> bits : blocks;
+        for (int b = prev + 1; b <= cur; b++)
+            t[b] = e;
+    }
+}
+
+// thread per (tile row, window boundary): the first C tile at or after it;
+// thread per row of A: the list of heavy rows
+__global__ void __launch_bounds__(256) k_win_ctab(ProdView P, WinPlan Q)
+{
+    const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g < Q.mA && Q.A_rptr[g + 1] - Q.A_rptr[g] >= WIN_HEAVY)
+        Q.heavy[atomicAdd(&Q.count[1], 1u)] = (int)g;
+    if (g >= (long long)P.tilemA * (Q.windows + 1))
+        return;
+    const int I = (int)(g / (Q.windows + 1)), w = (int)(g % (Q.windows + 1));
+    const int c0 = P.C_ptr[I], c1 = P.C_ptr[I + 1];
+    Q.ctab[g] = c0 + lower_bound_int(P.C_col + c0, c1 - c0, w * WIN_TILES);
+}
+
+// tile rows [row0, row1); Q.count[0] zeroed.  The claims are the heavy rows'
+// (row, WIN_PART columns), then every other row's (tile row, window, WIN_ROWS
+// rows).
+__global__ void __launch_bounds__(WIN_THREADS, WIN_CTAS) k_step3_win(ProdView P, WinPlan Q, int row0, int row1)
+{
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    const int lane = threadIdx.x & 31;
+    WinTask &S = reinterpret_cast<WinTask *>(s_raw)[threadIdx.x >> 5];
+    for (int q = lane; q < WIN_COLS; q += 32)
+        S.acc[q] = 0.0;
+    __syncwarp();
+    const unsigned per = TSG_BS / WIN_ROWS; // claims of a (tile row, window)
+    const unsigned parts = (unsigned)Q.windows * WIN_PARTS;
+    const unsigned hclaims = Q.count[1] * parts;
+    const unsigned claims = hclaims + (unsigned)(row1 - row0) * Q.windows * per;
+    unsigned nxt = 0;
+    if (lane == 0)
+        nxt = atomicAdd(&Q.count[0], 1u);
+    for (;;)
+    {
+        const unsigned c = __shfl_sync(TSG_FULL_MASK, nxt, 0);
+        if (c >= claims)
+            break;
+        if (lane == 0)
+            nxt = atomicAdd(&Q.count[0], 1u);
+        if (c < hclaims)
+        {
+            const int row = Q.heavy[c / parts], part = (int)(c % parts);
+            const int I = row / TSG_BS, w = part / WIN_PARTS;
+            if (I < row0 || I >= row1 || part * WIN_PART >= P.nB)
+                continue;
+            const int *ct = Q.ctab + (long long)I * (Q.windows + 1) + w;
+            win_task(P, Q, S, I, row % TSG_BS, part * WIN_PART, (part + 1) * WIN_PART, Q.A_rptr[row],
+                     Q.A_rptr[row + 1], ct[0], ct[1], lane);
+            continue;
+        }
+        const int u = (c - hclaims) / per;
+        const int I = row0 + u / Q.windows, w = u % Q.windows;
+        const int r0 = ((c - hclaims) % per) * WIN_ROWS;
+        const int *ct = Q.ctab + (long long)I * (Q.windows + 1) + w;
+        const int t0 = ct[0], t1 = ct[1];
+        if (t0 == t1)
+            continue;
+        const int row = I * TSG_BS + r0;
+        const int e = lane <= WIN_ROWS ? Q.A_rptr[min(row + lane, Q.mA)] : 0;
+#pragma unroll 1
+        for (int k = 0; k < WIN_ROWS; k++)
+        {
+            const int e0 = __shfl_sync(TSG_FULL_MASK, e, k), e1 = __shfl_sync(TSG_FULL_MASK, e, k + 1);
+            if (e0 < e1 && e1 - e0 < WIN_HEAVY)
+                win_task(P, Q, S, I, r0 + k, w * WIN_COLS, (w + 1) * WIN_COLS, e0, e1, t0, t1, lane);
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Host orchestration.
 // ---------------------------------------------------------------------------
@@ -319,6 +422,12 @@ static ProdView make_view(const tsg_tiled *A, const tsg_tiled *B, tsg_tiled *C)
     P.B_rptr = B->row_ptr;
     P.B_rcol = B->row_col;
     P.B_rval = B->row_val;
+    P.A_rptr = A->row_ptr;
+    P.A_rcol = A->row_col;
+    P.A_rval = A->row_val;
+    P.mA = A->m;
+    P.mB = B->m;
+    P.nB = B->n;
     P.browB = B->m > 0 ? (int)(B->nnz / B->m) : 0;
     P.tilenB = B->tilen;
     P.C_ptr = C->tile_ptr;
@@ -388,17 +497,120 @@ static int spa_grid(tsg_context *ctx, K kern, int smem, unsigned *grid)
     return TSG_OK;
 }
 
-// step 2 for the rows k_step12 declined, through B's row view
-static int launch_step2_spa(tsg_context *ctx, const ProdView &P, const int *d_wide, int *d_bins)
+// step 2 for the rows k_step12 listed, through B's row view
+template <int NT>
+static int launch_step2_cta(tsg_context *ctx, const ProdView &P, int span, const int *d_wide, int *d_bins)
 {
-    unsigned *ctr = nullptr, grid = 0;
-    const int smem = (int)sizeof(Spa2Smem);
-    TSG_TRY(spa_grid(ctx, k_step2_spa, smem, &grid));
+    const int smem = (int)wide_smem<NT>(span);
+    TSG_CUDA(cudaFuncSetAttribute(k_step2_cta<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    int per_sm = 0;
+    TSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step2_cta<NT>, NT, smem));
+    unsigned *ctr = nullptr;
     TSG_TRY(tsg_alloc(ctx, &ctr, 1));
     TSG_CUDA(cudaMemsetAsync(ctr, 0, sizeof(unsigned), ctx->stream));
-    k_step2_spa<<<grid, SPA_THREADS, smem, ctx->stream>>>(P, d_wide, ctr, d_bins);
+    const int grid = std::min(P.tilemA, ctx->num_sms * std::max(per_sm, 1));
+    k_step2_cta<NT><<<grid, NT, smem, ctx->stream>>>(P, span, d_wide, ctr, d_bins);
     TSG_LAUNCH_CHECK();
     tsg_release(ctx, ctr);
+    return TSG_OK;
+}
+
+static int launch_step2_wide(tsg_context *ctx, const ProdView &P, const int *d_wide, int *d_bins)
+{
+    // the columns of C, or as many as a CTA's shared memory holds; narrow C
+    // leaves room for four CTAs of 512 threads on an SM (8,192 columns: 0.073
+    // ms, 0.083 with 1,024 threads; 16,384 columns of R-MAT 14: 0.45 and 0.38)
+    const int span = std::min(P.tilenB, WIDE_SPAN);
+    return span <= 512 ? launch_step2_cta<512>(ctx, P, span, d_wide, d_bins)
+                       : launch_step2_cta<1024>(ctx, P, span, d_wide, d_bins);
+}
+
+// What the window form of step 3 keeps for a product.
+struct WinScratch
+{
+    WinPlan Q;
+    int *rptr, *rcol; // A's row view, when A has none
+    double *rval;
+    bool ready;
+};
+
+// Whether a product runs step 3 by windows, and their table's shape
+static bool win_shape(const ProdView &P, long long nnzC, WinPlan &Q)
+{
+    if (!P.B_rptr || P.nB < 1 || P.mA < 1)
+        return false;
+    const long long windows = (P.nB + WIN_COLS - 1LL) / WIN_COLS;
+    // claims of every row as if it were heavy: 32-bit
+    if (nnzC < WIN_MIN_VALUES * windows * P.mA || windows * WIN_PARTS * (P.mA + TSG_BS) > INT_MAX)
+        return false;
+    int bits = WIN_PART_BITS;
+    while ((((P.nB - 1) >> bits) + 2LL) * P.mB > WIN_TABLE_WORDS && (P.nB - 1) >> bits)
+        bits++;
+    Q.windows = (int)windows;
+    Q.bits = bits;
+    Q.blocks = ((P.nB - 1) >> bits) + 1;
+    Q.mA = P.mA;
+    return true;
+}
+
+static void win_release(tsg_context *ctx, WinScratch &W)
+{
+    tsg_release(ctx, W.Q.btab);
+    tsg_release(ctx, W.Q.ctab);
+    tsg_release(ctx, W.rptr);
+    tsg_release(ctx, W.rcol);
+    tsg_release(ctx, W.rval);
+    tsg_release(ctx, W.Q.heavy);
+    tsg_release(ctx, W.Q.count);
+    W.ready = false;
+}
+
+// the tables of a product's windows, made once per product
+static int win_prepare(tsg_context *ctx, const ProdView &P, const tsg_tiled *A, WinScratch &W)
+{
+    if (W.ready)
+        return TSG_OK;
+    cudaStream_t st = ctx->stream;
+    WinPlan &Q = W.Q;
+    TSG_TRY(tsg_alloc(ctx, &Q.btab, (size_t)P.mB * (Q.blocks + 1)));
+    TSG_TRY(tsg_alloc(ctx, &Q.ctab, (size_t)P.tilemA * (Q.windows + 1)));
+    TSG_TRY(tsg_alloc(ctx, &Q.heavy, (size_t)P.mA));
+    TSG_TRY(tsg_alloc(ctx, &Q.count, 2));
+    TSG_CUDA(cudaMemsetAsync(Q.count, 0, 2 * sizeof(unsigned), st));
+    Q.A_rptr = P.A_rptr;
+    Q.A_rcol = P.A_rcol;
+    Q.A_rval = P.A_rval;
+    if (!P.A_rptr)
+    {
+        TSG_TRY(tsg_alloc(ctx, &W.rptr, (size_t)A->m + 1));
+        TSG_TRY(tsg_alloc(ctx, &W.rcol, (size_t)A->nnz));
+        TSG_TRY(tsg_alloc(ctx, &W.rval, (size_t)A->nnz));
+        TSG_TRY(tsg_t2c_view(ctx, A, W.rptr, W.rcol, W.rval));
+        Q.A_rptr = W.rptr;
+        Q.A_rcol = W.rcol;
+        Q.A_rval = W.rval;
+    }
+    k_win_btab<<<tsg_blocks((long long)P.mB * 32, 256), 256, 0, st>>>(P.mB, P.B_rptr, P.B_rcol, Q.blocks, Q.bits, Q.btab);
+    TSG_LAUNCH_CHECK();
+    k_win_ctab<<<tsg_blocks(std::max((long long)P.mA, (long long)P.tilemA * (Q.windows + 1)), 256), 256, 0, st>>>(P, Q);
+    TSG_LAUNCH_CHECK();
+    W.ready = true;
+    return TSG_OK;
+}
+
+// step 3 by windows for tile rows [row0, row1)
+static int launch_step3_win(tsg_context *ctx, const ProdView &P, const tsg_tiled *A, WinScratch &W, int row0, int row1)
+{
+    TSG_TRY(win_prepare(ctx, P, A, W));
+    const int smem = WIN_WARPS * (int)sizeof(WinTask);
+    TSG_CUDA(cudaFuncSetAttribute(k_step3_win, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    int per_sm = 0;
+    TSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step3_win, WIN_THREADS, smem));
+    TSG_CUDA(cudaMemsetAsync(W.Q.count, 0, sizeof(unsigned), ctx->stream));
+    const long long claims = (long long)(row1 - row0) * W.Q.windows * (TSG_BS / WIN_ROWS);
+    const long long grid = std::min((long long)ctx->num_sms * std::max(per_sm, 1), (claims + WIN_WARPS - 1) / WIN_WARPS);
+    k_step3_win<<<(unsigned)grid, WIN_THREADS, smem, ctx->stream>>>(P, W.Q, row0, row1);
+    TSG_LAUNCH_CHECK();
     return TSG_OK;
 }
 
@@ -459,12 +671,17 @@ static bool step3_by_spa(const tsg_context *ctx, const ProdView &P, long long nn
 }
 
 // the SPA numeric step for tile rows [row0, row1)
-static int launch_step3_spa_rows(tsg_context *ctx, const ProdView &P, long long nnzC, const int *d_kind, int row0,
-                                 int row1)
+static int launch_step3_spa_rows(tsg_context *ctx, const ProdView &P, const tsg_tiled *A, long long nnzC,
+                                 const int *d_kind, WinScratch &W, int row0, int row1)
 {
     const bool flat = spa_wants_flat(P.browB, P.numC, nnzC, P.tilemA);
     const bool whole = row0 == 0 && row1 == P.tilemA;
     ctx->last_step3 = flat ? TSG_STEP3_FLAT : P.padded ? TSG_STEP3_STAGED : TSG_STEP3_SPA;
+    if (flat && win_shape(P, nnzC, W.Q))
+    {
+        ctx->last_step3 = TSG_STEP3_WINDOWS;
+        return launch_step3_win(ctx, P, A, W, row0, row1);
+    }
     if (flat && nnzC >= (long long)SPA_BLK_NARROW_VALUES * P.numC)
         return whole ? launch_step3_spa<true, false, SPA_BLK_NARROW>(ctx, P, d_kind, 0, 0)
                      : launch_step3_spa<true, true, SPA_BLK_NARROW>(ctx, P, d_kind, row0, row1);
@@ -480,10 +697,11 @@ static int launch_step3_spa_rows(tsg_context *ctx, const ProdView &P, long long 
 
 // d_kind: the row kinds of the fused step 1/2 pass (0 narrow, 1 wide,
 // 2 hypersparse), or null
-static int launch_step3(tsg_context *ctx, const ProdView &P, long long nnzC, const int *d_kind)
+static int launch_step3(tsg_context *ctx, const ProdView &P, const tsg_tiled *A, long long nnzC, const int *d_kind,
+                        WinScratch &W)
 {
     if (step3_by_spa(ctx, P, nnzC))
-        return launch_step3_spa_rows(ctx, P, nnzC, d_kind, 0, P.tilemA);
+        return launch_step3_spa_rows(ctx, P, A, nnzC, d_kind, W, 0, P.tilemA);
     if (ctx->sched == TSG_SCHED_ROWS)
     {
         const int W = ctx->seg_tiles, cap = ctx->acc_cap;
@@ -516,6 +734,8 @@ struct SpgemmRun
     unsigned long long *d_pairs;
     int *d_bins;
     int *d_wide; // row kinds of the fused pass, or null
+    StepOneBits bits; // step 1's bitmaps, until the emit pass has read them
+    WinScratch win;
     long long numC, nnzC;
 };
 
@@ -547,7 +767,19 @@ static int spgemm_structure(tsg_context *ctx, const tsg_tiled *A, const tsg_tile
     if (tilem > 0)
     {
         ProdView P = make_view(A, B, C);
-        k_step1<false><<<tsg_blocks(tilem, S1_WARPS), S1_WARPS * 32, 0, st>>>(P, C->tile_ptr, R.d_pairs);
+        const int stride = std::min((B->tilen + 31) / 32, S1_KEEP_WORDS);
+        if ((long long)tilem * stride <= S1_KEEP_TOTAL)
+        {
+            R.bits.stride = stride;
+            TSG_TRY(tsg_alloc(ctx, &R.bits.words, (size_t)tilem * stride));
+            TSG_TRY(tsg_alloc(ctx, &R.bits.span, (size_t)tilem));
+            TSG_CUDA(cudaMemsetAsync(R.bits.span, 0, (size_t)tilem * sizeof(int2), st));
+        }
+        const long long pairs = (long long)(A->numtile / tilem) * (B->tilem ? B->numtile / B->tilem : 0);
+        if (pairs >= S1_CTA_PAIRS)
+            k_step1_cta<<<tilem, S1C_THREADS, 0, st>>>(P, C->tile_ptr, R.d_pairs, R.bits);
+        else
+            k_step1<false><<<tsg_blocks(tilem, S1_WARPS), S1_WARPS * 32, 0, st>>>(P, C->tile_ptr, R.d_pairs, R.bits);
         TSG_LAUNCH_CHECK();
         TSG_TRY(tsg_scan_counts(ctx, C->tile_ptr, C->tile_ptr, tilem, &numC));
     }
@@ -567,17 +799,19 @@ static int spgemm_structure(tsg_context *ctx, const tsg_tiled *A, const tsg_tile
         ProdView P = make_view(A, B, C);
         if (fused)
         {
-            TSG_TRY(tsg_alloc(ctx, &R.d_wide, (size_t)tilem + 2));
-            TSG_CUDA(cudaMemsetAsync(R.d_wide + tilem, 0, 2 * sizeof(int), st));
-            k_step12<<<tsg_blocks(tilem, 8), 256, 0, st>>>(P, R.d_wide, R.d_bins);
+            TSG_TRY(tsg_alloc(ctx, &R.d_wide, (size_t)tilem + 1 + 2 * wide_units(tilem, A->nnz)));
+            TSG_CUDA(cudaMemsetAsync(R.d_wide + tilem, 0, sizeof(int), st));
+            k_step12<<<tsg_blocks(tilem, 8), 256, 0, st>>>(P, R.bits, R.d_wide, R.d_bins);
             TSG_LAUNCH_CHECK();
         }
         else
         {
-            k_step1<true><<<tsg_blocks(tilem, S1_WARPS), S1_WARPS * 32, 0, st>>>(P, nullptr, nullptr);
+            k_step1<true><<<tsg_blocks(tilem, S1_WARPS), S1_WARPS * 32, 0, st>>>(P, nullptr, nullptr, StepOneBits{nullptr, nullptr, 0});
             TSG_LAUNCH_CHECK();
         }
     }
+    tsg_release(ctx, R.bits.words);
+    tsg_release(ctx, R.bits.span);
     if (timing)
         TSG_CUDA(cudaEventRecord(ctx->ev[1], st));
 
@@ -586,7 +820,7 @@ static int spgemm_structure(tsg_context *ctx, const tsg_tiled *A, const tsg_tile
     {
         ProdView P = make_view(A, B, C);
         if (fused && P.B_rptr)
-            TSG_TRY(launch_step2_spa(ctx, P, R.d_wide, R.d_bins));
+            TSG_TRY(launch_step2_wide(ctx, P, R.d_wide, R.d_bins));
         else if (fused)
         {
             k_step2_wide<<<tsg_blocks(numC * 16, 256), 256, 0, st>>>(P, R.d_wide, R.d_bins);
@@ -615,7 +849,7 @@ static int spgemm_finish(tsg_context *ctx, SpgemmRun &R, tsg_spgemm_info *info)
 {
     cudaStream_t st = ctx->stream;
     tsg_release(ctx, R.d_wide);
-    R.d_wide = nullptr;
+    win_release(ctx, R.win);
     {
         const int dev = tsg_take_device_status(ctx);
         if (dev != TSG_OK)
@@ -660,7 +894,7 @@ extern "C" int tsg_spgemm(tsg_context *ctx, const tsg_tiled *A, const tsg_tiled 
     TSG_TRY(spgemm_structure(ctx, A, B, C, R));
     // step 3: numeric
     if (R.nnzC > 0)
-        TSG_TRY(launch_step3(ctx, make_view(A, B, C), R.nnzC, R.d_wide));
+        TSG_TRY(launch_step3(ctx, make_view(A, B, C), A, R.nnzC, R.d_wide, R.win));
     if (ctx->timing)
         TSG_CUDA(cudaEventRecord(ctx->ev[3], ctx->stream));
     return spgemm_finish(ctx, R, info);
@@ -713,7 +947,7 @@ int tsg_spgemm_to_host(tsg_context *ctx, const tsg_tiled *A, const tsg_tiled *B,
             const ProdView P = make_view(A, B, &C);
             const bool spa = step3_by_spa(ctx, P, R.nnzC);
             if (!spa)
-                TSG_TRY(launch_step3(ctx, P, R.nnzC, R.d_wide));
+                TSG_TRY(launch_step3(ctx, P, A, R.nnzC, R.d_wide, R.win));
             // chunks of about equal nonzeros (>= TSG_CHUNK_NNZ each, at most TSG_MAX_CHUNKS)
             const long long nch = std::max(1LL, std::min((long long)TSG_MAX_CHUNKS, R.nnzC / TSG_CHUNK_NNZ));
             int r0 = 0;
@@ -738,7 +972,7 @@ int tsg_spgemm_to_host(tsg_context *ctx, const tsg_tiled *A, const tsg_tiled *B,
                 if (r1 <= r0)
                     continue;
                 if (spa)
-                    TSG_TRY(launch_step3_spa_rows(ctx, P, R.nnzC, R.d_wide, r0, r1));
+                    TSG_TRY(launch_step3_spa_rows(ctx, P, A, R.nnzC, R.d_wide, R.win, r0, r1));
                 TSG_TRY(tsg_t2c_fill(ctx, &C, r0, r1, d_rp, d_ci, d_v));
                 TSG_CUDA(cudaEventRecord(ctx->copy_ev, st));
                 TSG_CUDA(cudaStreamWaitEvent(ctx->copy_stream, ctx->copy_ev, 0));
@@ -768,6 +1002,7 @@ int tsg_spgemm_to_host(tsg_context *ctx, const tsg_tiled *A, const tsg_tiled *B,
     else
     {
         tsg_release(ctx, R.d_wide);
+        win_release(ctx, R.win);
         tsg_release(ctx, R.d_pairs);
         tsg_release(ctx, R.d_bins);
     }

@@ -1,10 +1,29 @@
-"""The dense tile kernel against the oracle: bands on both sides of the dense
-path, ragged tiles, infinite and NaN values.  Values bit for bit: the order of
-the sums is the oracle's."""
+"""Products whose rows are uneven or wide -- step 1 by a CTA per tile row with
+its bitmaps kept, step 2 of wide rows in parts, step 3 by column windows --
+and the dense tile kernel, against the oracle at the sizes where each changes:
+window and table-block edges, heavy rows around WIN_HEAVY (512) entries, tile
+rows around one part (2,048 entries), columns past one pass of step 2 (98,304)
+and past what step 1 keeps (262,144) or holds at once (1,048,576), an A with
+no row view.  Values bit for bit: the order of the sums is the oracle's."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
+
+
+def _rows(m, n, counts, seed, hub=0):
+    """Rows of counts[i] distinct random columns; hub: every row holds column 0 too."""
+    rng = np.random.default_rng(seed)
+    cols = []
+    for c in counts:
+        x = np.unique(rng.integers(0, n, int(c) * 2))
+        x = np.sort(rng.choice(x, min(int(c), x.size), replace=False)) if c else x[:0]
+        if hub and c:
+            x = np.unique(np.concatenate([[0], x]))
+        cols.append(x)
+    rp = np.concatenate([[0], np.cumsum([x.size for x in cols])]).astype(np.int32)
+    ci = np.concatenate(cols).astype(np.int32)
+    return m, n, rp, ci, rng.uniform(-1, 1, ci.size)
 
 
 def _tiled(tsg, ctx, mat, flags):
@@ -33,6 +52,46 @@ def _check(tsg, ctx, oracle, A, B, flagsA):
     for t in (tA, tB, C):
         t.free()
     return info
+
+
+def _case(name):
+    rng = np.random.default_rng(7)
+    if name.startswith("cols"):  # window and block edges
+        n = int(name[4:])
+        return _rows(70, 300, rng.integers(0, 60, 70), 1), _rows(300, n, rng.integers(0, min(n // 2, 26) + 1, 300), 2, hub=1)
+    if name == "heavy":  # rows around WIN_HEAVY entries among light ones, every B row holding column 0
+        counts = [511, 0, 513, 3, 512, 40, 700, 1, 2, 5, 0, 514, 9, 9, 9, 9, 600, 4]
+        return _rows(18, 1500, counts, 3), _rows(1500, 1300, rng.integers(0, 30, 1500), 4, hub=1)
+    if name == "parts":  # tile rows of about 1, 2 and 3 parts
+        counts = [127] * 16 + [128] * 16 + [129] * 16 + [257] * 16 + [3] * 5
+        return _rows(69, 4000, counts, 5), _rows(4000, 5000, rng.integers(0, 12, 4000), 6)
+    if name == "coarse table":  # 70,000 x 300,000: a table block wider than a heavy row's part; step 2 in passes
+        return _rows(40, 70000, [200] * 39 + [600], 8), _rows(70000, 300000, np.full(70000, 20), 9)
+    assert name == "step 1 in passes"
+    return _rows(33, 400, rng.integers(1, 40, 33), 10), _rows(400, 1100000, np.full(400, 300), 11)
+
+
+@pytest.mark.parametrize("name", ["cols15", "cols255", "cols256", "cols257", "cols1024", "cols1025", "cols2000", "heavy",
+                                  "parts", "coarse table", "step 1 in passes"])
+@pytest.mark.parametrize("view", [True, False])
+def test_uneven_products(tsg, ctx, oracle, name, view):
+    A, B = _case(name)
+    flags = tsg.TSG_TILED_CSC_VIEW if view else tsg.TSG_TILED_PACKED_COL
+    ctx.set_schedule("spa", dense=257)  # never the tile kernel
+    try:
+        info = _check(tsg, ctx, oracle, A, B, flags)
+    finally:
+        ctx.set_schedule("spa", dense=0)
+    assert (info["step3_name"] == "k_step3_win") == (name != "step 1 in passes")
+
+
+def test_window_step_on_tile_row_ranges(tsg, ctx, oracle, gen):
+    """The host call computes a skewed product in ranges of tile rows."""
+    mat = gen.rmat(12, 24, seed=5)
+    out = tsg.HostResultBuffers(mat[0], 1 << 24)
+    got, info = tsg.spgemm_csr_host_overlap(ctx, mat, None, out)
+    assert info["nnz_C"] > 2 << 20  # more than one chunk
+    _same(got[2:], oracle.gustavson(mat, mat, nthreads=8))
 
 
 @pytest.mark.parametrize("half", [7, 8, 20, 41])
