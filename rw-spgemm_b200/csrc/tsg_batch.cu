@@ -22,16 +22,22 @@
 #include <cooperative_groups.h>
 #include <stdlib.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "tsg_device.cuh"
+#include "tsg_wide.cuh"
+#include "tsg_window.cuh"
 
 int tsg_count_c_tiles_async(tsg_context *ctx, const tsg_tiled *A, const tsg_tiled *B, unsigned long long *total);
 
 struct BatchProd
 {
     ProdView P;
-    int *wide; // per A tile row: 1 when step 2 runs per tile (fused pass declined), 2 hypersparse
+    StepOneBits K; // step 1's bitmaps, kept in C's value range until step 3
+    int *wide;     // per A tile row: 1 when step 2 runs apart (fused pass declined), 2 hypersparse
+    WinPlan Q;     // step 3 by windows (win)
+    int win;
     long long capT, capN;
     int tilemA;
     int status; // 0 ok, 1 tile capacity, 2 value capacity
@@ -48,8 +54,9 @@ struct tsg_batch
     BatchProd *d_prod;
     long long *d_rowoff;
     long long *d_itemoff;
-    unsigned *d_bar; // [0] arrivals, [1] generation, [2] / [3] next tile block (SPA steps 3 / 2),
-                     // [4..5] the barrier's wait limit in ns (64-bit)
+    unsigned *d_bar; // [0] arrivals, [1] generation, [2] next tile block of the SPA step 3, [3] next
+                     // wide unit of step 2, [4..5] the barrier's wait limit in ns (64-bit), [6] wide
+                     // units, [7] parts of heavy rows, [8] next claim of the window step 3
     int *d_err;
     int *d_bins;
     void *arena;
@@ -63,11 +70,24 @@ struct tsg_batch
     std::vector<int> m, n, tilen; // per product C dimensions
     long long launches;
     unsigned long long wait_ns; // the grid barrier's wait limit
-    unsigned bar_init[8];       // host image of d_bar at creation (zeros, the wait limit at [4])
+    unsigned bar_init[16];       // host image of d_bar at creation (zeros, the wait limit at [4])
+    std::vector<long long> s1off;  // prefix of tilemA over the products whose step 1 takes a CTA per tile row, then the others'
+    std::vector<long long> winoff; // window step 3: prefixes of rows of B, ctab entries, rows of A, claims
+    long long *d_s1off, *d_winoff;
+    int4 *d_wlist, *d_hlist; // wide units of step 2; heavy rows' parts of the window step 3
+    int *win_tables;
+    int wins;    // products that take the windows
+    int gridw;   // persistent grid of k_batch_win
     int dense;                  // SPA schedule: values per C tile from which a product takes the tile kernel
 };
 
 #define BATCH_THREADS 128
+#define BATCH_SPAN 3072 // tile columns of step 2's wide rows in a CTA's shared memory (two CTAs an SM)
+// step 3 by windows: products with this many scalar products per (row,
+// window), up to this many words of table each and in all
+#define BATCH_WIN_MIN 16
+#define BATCH_WIN_WORDS (1LL << 22)
+#define BATCH_WIN_TOTAL (1LL << 26)
 // a barrier wait gives up after this floor plus a share of the batch's work
 // (a B200 does well over 10 scalar products per ns, so the bound is loose)
 #define BATCH_WAIT_FLOOR_NS 2000000000ULL
@@ -284,8 +304,8 @@ __device__ __forceinline__ unsigned long long gtimer() { return batch_clock_ns()
 
 template <int SCHED, int W, int CAP, int NT>
 __global__ void __launch_bounds__(NT)
-    k_batch(BatchProd *prods, int count, const long long *__restrict__ rowoff, long long *itemoff, unsigned *bar,
-            int *err, int *bins)
+    k_batch(BatchProd *prods, int count, const long long *__restrict__ rowoff, const long long *__restrict__ s1off,
+            int4 *wlist, long long *itemoff, unsigned *bar, int *err, int *bins)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
     __shared__ long long s_tmp[NT / 32 + 1];
@@ -300,15 +320,27 @@ __global__ void __launch_bounds__(NT)
     unsigned long long *stamp = reinterpret_cast<unsigned long long *>(itemoff + 2 * ((long long)count + 1));
     BATCH_STAMP(0)
 
-    // phase 1: step-1 counts
+    // phase 1: step-1 counts; the tile rows of products with many tile pairs
+    // (prefix s1off) a CTA each, the others' (prefix after it) a warp each
     {
-        unsigned *bm = reinterpret_cast<unsigned *>(s_raw) + warp * S1_WORDS;
-        for (long long w = (long long)blockIdx.x * (NT / 32) + warp; w < total_rows; w += nwarps)
+        S1cSmem<NT> &S1 = *reinterpret_cast<S1cSmem<NT> *>(s_raw);
+        for (long long u = blockIdx.x; u < s1off[count]; u += gridDim.x)
         {
-            const int p = find_product(rowoff, count, w);
+            const int p = find_product(s1off, count, u);
+            const int i = (int)(u - s1off[p]);
+            const int cnt = step1_row_cta<NT>(prods[p].P, i, S1, prods[p].K, nullptr);
+            if (threadIdx.x == 0)
+                prods[p].P.C_ptr[i] = cnt;
+            __syncthreads();
+        }
+        const long long *woff = s1off + count + 1;
+        unsigned *bm = reinterpret_cast<unsigned *>(s_raw) + warp * S1_WORDS;
+        for (long long w = (long long)blockIdx.x * (NT / 32) + warp; w < woff[count]; w += nwarps)
+        {
+            const int p = find_product(woff, count, w);
             const ProdView &P = prods[p].P;
-            const int i = (int)(w - rowoff[p]);
-            const int cnt = step1_row<false>(P, i, bm, lane32, nullptr);
+            const int i = (int)(w - woff[p]);
+            const int cnt = step1_row<false>(P, i, bm, lane32, nullptr, prods[p].K);
             if (lane32 == 0)
                 P.C_ptr[i] = cnt;
         }
@@ -370,8 +402,7 @@ __global__ void __launch_bounds__(NT)
                 run += ((long long)prods[p].numC + SCAN_CHUNK - 1) / SCAN_CHUNK;
             }
             chunkoff[count] = run;
-            bar[2] = 0;
-            bar[3] = 0;
+            bar[2] = bar[3] = bar[6] = bar[7] = bar[8] = 0;
         }
         if (threadIdx.x < 4)
             bins[threadIdx.x] = 0;
@@ -397,17 +428,27 @@ __global__ void __launch_bounds__(NT)
                 step1_row<true>(prods[p].P, i, bm, lane32, nullptr);
             else
             {
-                const int done = step12_row(prods[p].P, i, *s12, lane32, s_bins);
+                const int done = step12_row(prods[p].P, i, *s12, lane32, s_bins, prods[p].K);
                 int kind = 0;
                 if (!done)
                 {
                     __syncwarp();
-                    step1_row<true>(prods[p].P, i, reinterpret_cast<unsigned *>(s12), lane32, nullptr);
+                    if (!step1_emit_kept(prods[p].P, i, lane32, prods[p].K))
+                        step1_row<true>(prods[p].P, i, reinterpret_cast<unsigned *>(s12), lane32, nullptr);
                     __syncwarp(); // the row's C columns, emitted by all lanes
                     kind = SCHED == 3 ? wide_kind(prods[p].P, i, lane32) : 1;
                 }
                 if (lane32 == 0)
+                {
                     prods[p].wide[i] = kind;
+                    if (SCHED == 3 && kind)
+                    {
+                        const int parts = wide_parts(prods[p].P, i);
+                        int4 *at = wlist + atomicAdd(&bar[6], (unsigned)parts);
+                        for (int q = 0; q < parts; q++)
+                            at[q] = make_int4(p, i, q | parts << 16, 0);
+                    }
+                }
                 __syncwarp();
             }
         }
@@ -418,33 +459,18 @@ __global__ void __launch_bounds__(NT)
     // phase 5: step 2 (all tiles for the row schedule, tiles of wide rows otherwise)
     if (SCHED == 3)
     {
-        // wide rows through B's row view; CTAs take blocks of C tiles
-        Spa2Smem &S2 = *reinterpret_cast<Spa2Smem *>(s_raw);
-        const long long *blkoff = itemoff + count + 1;
-        unsigned nxt = 0; // thread 0: the next block, claimed one block ahead
-        if (threadIdx.x == 0)
-            nxt = atomicAdd(&bar[3], 1u);
-        int p = 0;
+        // wide rows through B's row view; CTAs take units of the list
+        WideSmem<NT> &S2 = *reinterpret_cast<WideSmem<NT> *>(s_raw);
         for (;;)
         {
-            __syncthreads();
             if (threadIdx.x == 0)
-            {
-                s_row = (int)nxt;
-                nxt = atomicAdd(&bar[3], 1u);
-            }
+                s_row = (int)atomicAdd(&bar[3], 1u);
             __syncthreads();
-            const long long blk = s_row;
-            if (blk >= blkoff[count])
+            const int u = s_row;
+            if (u >= (int)*(volatile unsigned *)&bar[6])
                 break;
-            p = find_product_from(blkoff, count, blk, p);
-            if (prods[p].status)
-                continue;
-            const ProdView &P = prods[p].P;
-            const long long tb = (blk - blkoff[p]) * SPA_BLK;
-            if (threadIdx.x == 0)
-                spa_skip_hyper(P, prods[p].wide, (int)tb, &bar[3], blkoff[p]);
-            step2_spa_block(P, S2, (int)tb, (int)min((long long)P.numC, tb + SPA_BLK), prods[p].wide, s_bins);
+            const int4 w = __ldcg(wlist + u);
+            step2_wide_row<NT>(prods[w.x].P, S2, BATCH_SPAN, w.y, w.z, s_bins);
         }
     }
     else
@@ -588,13 +614,99 @@ __global__ void __launch_bounds__(SPA_THREADS, 3)
         if (blk >= blkoff[count])
             break;
         p = find_product_from(blkoff, count, blk, p);
-        if (prods[p].status || prods[p].nnzC >= (long long)dense * prods[p].numC)
+        if (prods[p].win || prods[p].status || prods[p].nnzC >= (long long)dense * prods[p].numC)
             continue;
         const ProdView &P = prods[p].P;
         const long long tb = (blk - blkoff[p]) * SPA_BLK;
         if (threadIdx.x == 0)
             spa_skip_hyper(P, prods[p].wide, (int)tb, &bar[2], blkoff[p]);
         step3_spa_block<true>(P, S, (int)tb, (int)min((long long)P.numC, tb + SPA_BLK), prods[p].wide);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        atomicMax(reinterpret_cast<unsigned long long *>(const_cast<long long *>(itemoff)) + 2 * ((long long)count + 1) +
+                      7,
+                  gtimer());
+}
+
+// ... the tables of the products that take the windows (prefixes over the
+// products of their rows of B, entries of ctab and rows of A), and their
+// heavy rows' parts ...
+__device__ __forceinline__ bool batch_win_on(const BatchProd &b, int dense)
+{
+    return b.win && !b.status && b.nnzC > 0 && b.nnzC < (long long)dense * b.numC;
+}
+
+__global__ void __launch_bounds__(256)
+    k_batch_wtab(const BatchProd *prods, int count, const long long *__restrict__ winoff, int4 *hlist, unsigned *bar,
+                 const int *err, int dense)
+{
+    if (*(volatile const int *)err)
+        return;
+    const long long *boff = winoff, *toff = boff + count + 1, *aoff = toff + count + 1;
+    const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
+    for (long long w = gt >> 5; w < boff[count]; w += nt >> 5)
+    {
+        const BatchProd &b = prods[find_product(boff, count, w)];
+        if (batch_win_on(b, dense))
+            win_btab_row((int)(w - boff[&b - prods]), b.P.B_rptr, b.P.B_rcol, b.Q.blocks, b.Q.bits, b.Q.btab);
+    }
+    for (long long g = gt; g < toff[count]; g += nt)
+    {
+        const BatchProd &b = prods[find_product(toff, count, g)];
+        if (batch_win_on(b, dense))
+            win_ctab_entry(b.P, b.Q, g - toff[&b - prods]);
+    }
+    for (long long g = gt; g < aoff[count]; g += nt)
+    {
+        const int p = find_product(aoff, count, g);
+        const BatchProd &b = prods[p];
+        const int row = (int)(g - aoff[p]);
+        if (batch_win_on(b, dense) && b.Q.A_rptr[row + 1] - b.Q.A_rptr[row] >= WIN_HEAVY)
+        {
+            const int parts = (b.P.nB + WIN_PART - 1) / WIN_PART;
+            int4 *at = hlist + atomicAdd(&bar[7], (unsigned)parts);
+            for (int q = 0; q < parts; q++)
+                at[q] = make_int4(p, row, q, 0);
+        }
+    }
+}
+
+// ... their numeric step ...
+__global__ void __launch_bounds__(WIN_THREADS, WIN_CTAS)
+    k_batch_win(const BatchProd *prods, int count, const long long *__restrict__ winoff, const int4 *__restrict__ hlist,
+                const long long *itemoff, unsigned *bar, const int *err, int dense)
+{
+    if (*(volatile const int *)err)
+        return;
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    const int lane = threadIdx.x & 31;
+    WinTask &S = reinterpret_cast<WinTask *>(s_raw)[threadIdx.x >> 5];
+    for (int q = lane; q < WIN_COLS; q += 32)
+        S.acc[q] = 0.0;
+    __syncwarp();
+    const long long *coff = winoff + 3 * ((long long)count + 1);
+    const unsigned hclaims = bar[7], claims = hclaims + (unsigned)coff[count];
+    unsigned nxt = 0;
+    int p = 0;
+    if (lane == 0)
+        nxt = atomicAdd(&bar[8], 1u);
+    for (;;)
+    {
+        const unsigned c = __shfl_sync(TSG_FULL_MASK, nxt, 0);
+        if (c >= claims)
+            break;
+        if (lane == 0)
+            nxt = atomicAdd(&bar[8], 1u);
+        if (c < hclaims)
+        {
+            const int4 h = hlist[c];
+            win_claim_heavy(prods[h.x].P, prods[h.x].Q, S, h.y, h.z, lane);
+            continue;
+        }
+        p = find_product_from(coff, count, c - hclaims, p);
+        if (batch_win_on(prods[p], dense))
+            win_claim_rows(prods[p].P, prods[p].Q, S, 0, (unsigned)(c - hclaims - coff[p]), lane);
     }
     __syncthreads();
     if (threadIdx.x == 0)
@@ -749,7 +861,8 @@ extern "C" int tsg_product_bounds(tsg_context *ctx, const tsg_tiled *A, const ts
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-typedef void (*batch_kernel_t)(BatchProd *, int, const long long *, long long *, unsigned *, int *, int *);
+typedef void (*batch_kernel_t)(BatchProd *, int, const long long *, const long long *, int4 *, long long *, unsigned *,
+                               int *, int *);
 
 // Kernel, dynamic shared memory and block size of a batch schedule.
 static batch_kernel_t pick_kernel(const tsg_batch_params &p, size_t *smem, int *threads)
@@ -757,14 +870,13 @@ static batch_kernel_t pick_kernel(const tsg_batch_params &p, size_t *smem, int *
     *threads = BATCH_THREADS;
     const size_t s1a = (size_t)(BATCH_THREADS / 32) * S1_WORDS * 4;
     const size_t s12 = (size_t)(BATCH_THREADS / 32) * sizeof(S12Smem);
-    const size_t s1 = s1a > s12 ? s1a : s12;
+    const size_t s1 = std::max(std::max(s1a, s12), sizeof(S1cSmem<BATCH_THREADS>));
     if (p.schedule == TSG_SCHED_SPA)
     {
         *threads = SPA_THREADS;
         const size_t t1a = (size_t)(SPA_THREADS / 32) * S1_WORDS * 4;
         const size_t t12 = (size_t)(SPA_THREADS / 32) * sizeof(S12Smem);
-        const size_t t1 = t1a > t12 ? t1a : t12;
-        *smem = t1 > sizeof(Spa2Smem) ? t1 : sizeof(Spa2Smem);
+        *smem = std::max(std::max(t1a, t12), std::max(wide_smem<SPA_THREADS>(BATCH_SPAN), sizeof(S1cSmem<SPA_THREADS>)));
         return k_batch<3, 8, 256, SPA_THREADS>;
     }
     if (p.schedule == TSG_SCHED_ELEMS)
@@ -814,8 +926,18 @@ static int record_run(tsg_batch *b, cudaStream_t st)
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    TSG_CUDA(cudaLaunchKernelEx(&cfg, kern, b->d_prod, b->count, (const long long *)b->d_rowoff, b->d_itemoff,
+    TSG_CUDA(cudaLaunchKernelEx(&cfg, kern, b->d_prod, b->count, (const long long *)b->d_rowoff,
+                                (const long long *)b->d_s1off, b->d_wlist, b->d_itemoff,
                                 b->d_bar, b->d_err, b->d_bins));
+    if (b->wins)
+    {
+        k_batch_wtab<<<b->ctx->num_sms * 8, 256, 0, st>>>(b->d_prod, b->count, b->d_winoff, b->d_hlist, b->d_bar, b->d_err,
+                                                          b->dense);
+        TSG_CUDA(cudaGetLastError());
+        k_batch_win<<<b->gridw, WIN_THREADS, WIN_WARPS * sizeof(WinTask), st>>>(
+            b->d_prod, b->count, b->d_winoff, b->d_hlist, b->d_itemoff, b->d_bar, b->d_err, b->dense);
+        TSG_CUDA(cudaGetLastError());
+    }
     if (b->params.schedule == TSG_SCHED_SPA)
     {
         k_batch_spa3<<<b->grid3, SPA_THREADS, sizeof(SpaSmem), st>>>(b->d_prod, b->count, b->d_itemoff, b->d_bar,
@@ -903,9 +1025,17 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
             return st;
         }
     }
+    b->s1off.assign(2 * ((size_t)count + 1), 0);
+    b->winoff.assign(4 * ((size_t)count + 1), 0);
+    std::vector<long long> tables(count, 0); // words of each product's window tables
+    long long wunits = 0, hparts = 0, words = 0;
     for (int p = 0; p < count; p++)
     {
         const long long prods = v_prods[p], capT = v_tiles[p];
+        const bool cta = step1_by_cta(&A[p], &B[p]);
+        b->s1off[p + 1] = b->s1off[p] + (cta ? A[p].tilem : 0);
+        b->s1off[count + 2 + p] = b->s1off[count + 1 + p] + (cta ? 0 : A[p].tilem);
+        wunits += (long long)wide_units(A[p].tilem, A[p].nnz);
         total_prods += prods;
         long long capN = prods < 256 * capT ? prods : 256 * capT;
         if (capN > 2147483647LL || capT > 2147483647LL / 16)
@@ -919,6 +1049,30 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
         h.capN = capN;
         chunk_cap += (capT + SCAN_CHUNK - 1) / SCAN_CHUNK;
         h.tilemA = A[p].tilem;
+        if (prm.schedule == TSG_SCHED_SPA && A[p].row_ptr && A[p].m > 0 && B[p].n > 0)
+        {
+            const long long windows = (B[p].n + WIN_COLS - 1LL) / WIN_COLS;
+            const long long parts = (long long)(A[p].nnz / WIN_HEAVY) * ((B[p].n + WIN_PART - 1) / WIN_PART);
+            const long long claims = (long long)A[p].tilem * windows * WIN_PER, centries = A[p].tilem * (windows + 1);
+            int bits, blocks;
+            if (prods >= BATCH_WIN_MIN * windows * A[p].m &&
+                win_table(B[p].m, B[p].n, std::min(BATCH_WIN_WORDS, BATCH_WIN_TOTAL - words), bits, blocks) &&
+                b->winoff[3 * ((size_t)count + 1) + p] + claims + hparts + parts < 2147483647LL)
+            {
+                h.win = 1;
+                h.Q.windows = (int)windows;
+                h.Q.bits = bits;
+                h.Q.blocks = blocks;
+                h.Q.mA = A[p].m;
+                hparts += parts;
+                tables[p] = (blocks + 1LL) * B[p].m + centries;
+                words += (blocks + 1LL) * B[p].m;
+                b->wins++;
+            }
+            const long long add[4] = {B[p].m, centries, A[p].m, claims};
+            for (int q = 0; q < 4; q++)
+                b->winoff[q * ((size_t)count + 1) + p + 1] = b->winoff[q * ((size_t)count + 1) + p] + (h.win ? add[q] : 0);
+        }
         b->rowoff[p] = run;
         run += A[p].tilem;
         b->m[p] = A[p].m;
@@ -931,13 +1085,26 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
                  align256((size_t)capN * 8);
     }
     b->rowoff[count] = run;
-    b->arena_bytes = bytes;
+    long long table_words = 0;
+    for (long long t : tables)
+        table_words += t;
+    b->arena_bytes = bytes + (b->wins ? 4 * (size_t)table_words + sizeof(int4) * (size_t)hparts : 0);
     int st = TSG_OK;
     if ((st = tsg_alloc(ctx, (char **)&b->arena, bytes ? bytes : 256)) != TSG_OK)
     {
         delete b;
         return st;
     }
+    if ((b->wins && ((st = tsg_alloc(ctx, &b->win_tables, (size_t)table_words)) != TSG_OK ||
+                     (st = tsg_alloc(ctx, &b->d_hlist, (size_t)hparts)) != TSG_OK ||
+                     (st = tsg_alloc(ctx, &b->d_winoff, b->winoff.size())) != TSG_OK)) ||
+        (st = tsg_alloc(ctx, &b->d_s1off, b->s1off.size())) != TSG_OK ||
+        (st = tsg_alloc(ctx, &b->d_wlist, (size_t)wunits)) != TSG_OK)
+    {
+        tsg_batch_destroy(b);
+        return st;
+    }
+    table_words = 0;
     for (int p = 0; p < count; p++)
     {
         BatchProd &h = b->host[p];
@@ -970,6 +1137,12 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
         P.B_rptr = B[p].row_ptr;
         P.B_rcol = B[p].row_col;
         P.B_rval = B[p].row_val;
+        P.A_rptr = A[p].row_ptr;
+        P.A_rcol = A[p].row_col;
+        P.A_rval = A[p].row_val;
+        P.mA = A[p].m;
+        P.mB = B[p].m;
+        P.nB = B[p].n;
         P.browB = B[p].m > 0 ? (int)(B[p].nnz / B[p].m) : 0;
         P.tilenB = B[p].tilen;
         P.C_ptr = (int *)take(((size_t)A[p].tilem + 1) * 4);
@@ -984,9 +1157,27 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
         P.numC = 0;
         P.padded = 0;
         P.status = nullptr; // the batch's error word, set once it is allocated
+        // step 1's bitmaps stay in the value range, which step 3 is the first to write
+        const int stride = std::min((B[p].tilen + 31) / 32, S1_KEEP_WORDS);
+        const size_t kept = ((size_t)A[p].tilem * stride * 4 + 15) & ~(size_t)15;
+        if (prm.schedule != TSG_SCHED_ROWS && kept + (size_t)A[p].tilem * sizeof(int2) <= (size_t)h.capN * 8)
+        {
+            h.K.words = (unsigned *)P.C_Val;
+            h.K.span = (int2 *)((char *)P.C_Val + kept);
+            h.K.stride = stride;
+        }
+        if (h.win)
+        {
+            h.Q.A_rptr = P.A_rptr;
+            h.Q.A_rcol = P.A_rcol;
+            h.Q.A_rval = P.A_rval;
+            h.Q.btab = b->win_tables + table_words;
+            h.Q.ctab = h.Q.btab + (h.Q.blocks + 1LL) * P.mB;
+            table_words += tables[p];
+        }
     }
     if ((st = tsg_alloc(ctx, &b->d_prod, (size_t)count)) != TSG_OK || (st = tsg_alloc(ctx, &b->d_rowoff, (size_t)count + 1)) ||
-        (st = tsg_alloc(ctx, &b->d_itemoff, 3 * ((size_t)count + 1) + 8 + (size_t)chunk_cap)) || (st = tsg_alloc(ctx, &b->d_bar, 8)) ||
+        (st = tsg_alloc(ctx, &b->d_itemoff, 3 * ((size_t)count + 1) + 8 + (size_t)chunk_cap)) || (st = tsg_alloc(ctx, &b->d_bar, 16)) ||
         (st = tsg_alloc(ctx, &b->d_err, 1)) || (st = tsg_alloc(ctx, &b->d_bins, 4)))
     {
         tsg_batch_destroy(b);
@@ -1003,6 +1194,9 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
     memcpy(&b->bar_init[4], &b->wait_ns, sizeof(unsigned long long));
     cudaMemcpyAsync(b->d_prod, b->host.data(), sizeof(BatchProd) * count, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(b->d_rowoff, b->rowoff.data(), sizeof(long long) * (count + 1), cudaMemcpyHostToDevice, s);
+    cudaMemcpyAsync(b->d_s1off, b->s1off.data(), sizeof(long long) * b->s1off.size(), cudaMemcpyHostToDevice, s);
+    if (b->wins)
+        cudaMemcpyAsync(b->d_winoff, b->winoff.data(), sizeof(long long) * b->winoff.size(), cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(b->d_bar, b->bar_init, sizeof(b->bar_init), cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(b->d_err, &b->bar_init[0], sizeof(int), cudaMemcpyHostToDevice, s);
     // co-resident grid
@@ -1033,6 +1227,18 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
             return tsg_set_error(TSG_ERR_CUDA, "batch numeric kernel cannot be resident");
         }
         b->grid3 = per3 * ctx->num_sms;
+    }
+    if (b->wins)
+    {
+        int perw = 0;
+        const int wsmem = WIN_WARPS * (int)sizeof(WinTask);
+        if (cudaFuncSetAttribute(k_batch_win, cudaFuncAttributeMaxDynamicSharedMemorySize, wsmem) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perw, k_batch_win, WIN_THREADS, wsmem) != cudaSuccess || perw < 1)
+        {
+            tsg_batch_destroy(b);
+            return tsg_set_error(TSG_ERR_CUDA, "batch window kernel cannot be resident");
+        }
+        b->gridw = perw * ctx->num_sms;
     }
     b->block = threads;
     b->smem = smem;
@@ -1206,6 +1412,11 @@ extern "C" int tsg_batch_destroy(tsg_batch *b)
     tsg_release(ctx, b->d_bar);
     tsg_release(ctx, b->d_err);
     tsg_release(ctx, b->d_bins);
+    tsg_release(ctx, b->d_s1off);
+    tsg_release(ctx, b->d_winoff);
+    tsg_release(ctx, b->d_wlist);
+    tsg_release(ctx, b->d_hlist);
+    tsg_release(ctx, b->win_tables);
     char *a = (char *)b->arena;
     tsg_release(ctx, a);
     cudaStreamSynchronize(ctx->stream);

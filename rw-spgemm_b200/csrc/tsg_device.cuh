@@ -370,46 +370,39 @@ __device__ __forceinline__ int step12_row(const ProdView &P, int i, S12Smem &sm,
         const int b0 = P.B_ptr[k], b1 = P.B_ptr[k + 1];
         if (b1 - b0 >= 8)
         {
-            // lane per B tile; the A tile's row masks are the same for all
-            // lanes, so the walk over its set bits does not diverge
-            const uint4 *amq = reinterpret_cast<const uint4 *>(P.A_mask + (long long)pa * TSG_BS);
-            const uint4 aq0 = __ldg(amq), aq1 = __ldg(amq + 1);
-            const unsigned aw[8] = {aq0.x, aq0.y, aq0.z, aq0.w, aq1.x, aq1.y, aq1.z, aq1.w};
-            // A tile with a dense row: B's masks as two 16-byte loads
-            const bool adense = __popc(aq0.x) + __popc(aq0.y) + __popc(aq0.z) + __popc(aq0.w) + __popc(aq1.x) +
-                                    __popc(aq1.y) + __popc(aq1.z) + __popc(aq1.w) > 64;
+            // lane per B tile, its 16 row masks in registers.  A sparse A tile
+            // is taken column by column: the rows with an entry in column k
+            // (a ballot over the row masks, the same for all lanes) get B's
+            // row k; a tile with many entries row by row, all of B at once
+            const unsigned am = lane < TSG_BS ? P.A_mask[(long long)pa * TSG_BS + lane] : 0u;
+            const bool adense = __reduce_add_sync(TSG_FULL_MASK, __popc(am)) > 64;
+            unsigned rows[TSG_BS]; // sparse: rows of A with an entry in column k
+#pragma unroll
+            for (int k = 0; k < TSG_BS; k++)
+                rows[k] = adense ? __shfl_sync(TSG_FULL_MASK, am, k)
+                                 : __ballot_sync(TSG_FULL_MASK, (am >> (15 - k)) & 1u);
             for (int pb = b0 + lane; pb < b1; pb += 32)
             {
                 const int j = P.B_col[pb] - c0;
                 const int slot = sm.pre[j >> 5] + __popc(sm.bm[j >> 5] & ((1u << (j & 31)) - 1u));
-                const unsigned short *mbk = P.B_mask + (long long)pb * TSG_BS;
+                const uint4 *mb = reinterpret_cast<const uint4 *>(P.B_mask + (long long)pb * TSG_BS);
+                const uint4 q0 = __ldg(mb), q1 = __ldg(mb + 1);
                 if (adense)
                 {
-                    const uint4 *mb = reinterpret_cast<const uint4 *>(mbk);
-                    const uint4 q0 = __ldg(mb), q1 = __ldg(mb + 1);
 #pragma unroll
-                    for (int rr = 0; rr < 16; rr++)
-                    {
-                        const unsigned mrow = (rr & 1) ? (aw[rr >> 1] >> 16) : (aw[rr >> 1] & 0xFFFFu);
-                        if (mrow)
-                            sm.acc[rr][slot] |= (unsigned short)bool_row(mrow, q0, q1);
-                    }
+                    for (int rr = 0; rr < TSG_BS; rr++)
+                        if (rows[rr])
+                            sm.acc[rr][slot] |= (unsigned short)bool_row(rows[rr], q0, q1);
                     continue;
                 }
+                const unsigned w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
 #pragma unroll
-                for (int rr = 0; rr < 16; rr++)
+                for (int k = 0; k < TSG_BS; k++)
                 {
-                    const unsigned mrow = (rr & 1) ? (aw[rr >> 1] >> 16) : (aw[rr >> 1] & 0xFFFFu);
-                    if (!mrow)
-                        continue;
-                    unsigned acc = 0, bits = mrow;
-                    do
-                    {
-                        const int bit = 31 - __clz(bits);
-                        bits ^= 1u << bit;
-                        acc |= __ldg(mbk + (15 - bit));
-                    } while (bits);
-                    sm.acc[rr][slot] |= (unsigned short)acc;
+                    const unsigned brow = (k & 1) ? (w[k >> 1] >> 16) : (w[k >> 1] & 0xFFFFu);
+                    if (brow)
+                        for (unsigned left = rows[k]; left; left &= left - 1)
+                            sm.acc[__ffs(left) - 1][slot] |= (unsigned short)brow;
                 }
             }
             __syncwarp();
@@ -1439,179 +1432,6 @@ __device__ __forceinline__ void step3_spa_segment(const ProdView &P, SpaSmem &S,
 }
 
 // ---------------------------------------------------------------------------
-// Step 2 for wide tile rows (more C tiles or a wider column window than the
-// fused row pass holds), through B's row view.  One CTA owns a segment of
-// consecutive C tiles of tile row I (at most SP2_SEGT tiles, a SP2_WIN
-// tile-column window); warp r walks A's row r and, for every A(r, k), B's
-// row k: each entry's column sets its bit in the 32-bit row-r mask word of
-// its C tile (shared-memory atomicOr; the order does not matter for an OR).
-// The masks then go out through step2_store like every other step-2 path.
-// ---------------------------------------------------------------------------
-#define SP2_SEGT 1024
-#define SP2_MS (SP2_SEGT + 1) // row stride of the [row][tile] mask words (a tile's rows in distinct banks)
-#define SP2_WIN 4096
-
-#define SP2_CO_CHUNK 1024 // A entries the CTA stages per pass
-
-struct Spa2Coop
-{
-    int bs[SP2_CO_CHUNK];          // B row start (cut to the segment) of each staged A entry
-    int off[SP2_CO_CHUNK + 1];     // its first item (B entry) in the chunk; off[n] = items
-    unsigned char row[SP2_CO_CHUNK];
-    int tile0[SP2_CO_CHUNK + 1];   // value offset of each A tile the chunk can touch
-    int wsum[SPA_WARPS];
-    int ptile;                     // the chunk's first A tile
-};
-
-struct Spa2Smem
-{
-    unsigned m[TSG_BS * SP2_MS]; // [row][tile] mask words
-    unsigned short map[SP2_WIN];
-    Spa2Coop co;
-};
-
-// exclusive prefix of v over the CTA's SPA_THREADS threads (thread order)
-// and the total; wsum holds SPA_WARPS ints
-__device__ __forceinline__ int block_excl_scan(int v, int *wsum, int *total, int tid, int lane)
-{
-    int incl = v;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1)
-    {
-        const int o = __shfl_up_sync(TSG_FULL_MASK, incl, d);
-        if (lane >= d)
-            incl += o;
-    }
-    const int warp = tid >> 5;
-    if (lane == 31)
-        wsum[warp] = incl;
-    __syncthreads();
-    int base = 0, tot = 0;
-#pragma unroll
-    for (int w = 0; w < SPA_WARPS; w++)
-    {
-        const int x = wsum[w];
-        base += w < warp ? x : 0;
-        tot += x;
-    }
-    __syncthreads();
-    *total = tot;
-    return base + incl - v;
-}
-
-
-// The CTA (SPA_THREADS threads) computes the masks of C tiles [t0, t1).
-__device__ __forceinline__ void step2_spa_segment(const ProdView &P, Spa2Smem &S, int t0, int t1, int *s_bins)
-{
-    const int tid = threadIdx.x, lane = tid & 31, r = tid >> 5;
-    const int I = P.C_row[t0];
-    const int J0 = P.C_col[t0], J1 = P.C_col[t1 - 1] + 1;
-    const int nt = min(t1 - t0, SP2_SEGT);
-    const int win = min(J1 - J0, SP2_WIN);
-    const bool full = t0 == P.C_ptr[I] && t1 == P.C_ptr[I + 1];
-    __syncthreads();
-    for (int q = tid; q < nt * TSG_BS; q += SPA_THREADS)
-        S.m[(q & 15) * SP2_MS + (q >> 4)] = 0u;
-    for (int q = tid; q < win; q += SPA_THREADS)
-        S.map[q] = 0xFFFF;
-    __syncthreads();
-    for (int jl = tid; jl < nt; jl += SPA_THREADS)
-    {
-        const int w = P.C_col[t0 + jl] - J0;
-        if (w < win)
-            S.map[w] = (unsigned short)jl;
-    }
-    __syncthreads();
-    // A's entries of the tile row, SP2_CO_CHUNK at a time: every thread
-    // stages entries (row, B's row cut to the segment's columns), then the
-    // chunk's B entries are split evenly over the warps, each setting its
-    // entry's column bit in the row's mask word (an OR: any order)
-    Spa2Coop &C = S.co;
-    const bool ptr16 = (reinterpret_cast<unsigned long long>(P.A_Ptr) & 15ULL) == 0;
-    const int pa_beg = P.A_ptr[I], pa_end = P.A_ptr[I + 1];
-    const int v_beg = P.A_tnnz[pa_beg], v_end = P.A_tnnz[pa_end];
-    for (int c0 = v_beg; c0 < v_end; c0 += SP2_CO_CHUNK)
-    {
-        const int ne = min(SP2_CO_CHUNK, v_end - c0);
-        if (tid == 0)
-            C.ptile = a_tile_of(P, pa_beg, pa_end, c0);
-        __syncthreads();
-        const int p0 = C.ptile;
-        const int ntl = min(ne, pa_end - p0); // tiles that can hold the chunk's entries
-        for (int q = tid; q <= ntl; q += SPA_THREADS)
-            C.tile0[q] = P.A_tnnz[p0 + q];
-        __syncthreads();
-        int len[2];
-#pragma unroll
-        for (int h = 0; h < 2; h++)
-        {
-            const int j = tid + h * SPA_THREADS;
-            len[h] = 0;
-            if (j < ne)
-            {
-                int row, k;
-                a_entry(P, C.tile0, ntl, p0, ptr16, c0 + j, row, k);
-                int b0 = P.B_rptr[k], b1 = P.B_rptr[k + 1];
-                if (!full)
-                {
-                    b0 += lower_bound_int(P.B_rcol + b0, b1 - b0, J0 * TSG_BS);
-                    b1 = b0 + lower_bound_int(P.B_rcol + b0, b1 - b0, J1 * TSG_BS);
-                }
-                C.bs[j] = b0;
-                C.row[j] = (unsigned char)row;
-                len[h] = b1 - b0;
-            }
-        }
-        int tot0, tot1;
-        const int x0 = block_excl_scan(len[0], C.wsum, &tot0, tid, lane);
-        const int x1 = block_excl_scan(len[1], C.wsum, &tot1, tid, lane);
-        if (tid < ne)
-            C.off[tid] = x0;
-        if (tid + SPA_THREADS < ne)
-            C.off[tid + SPA_THREADS] = tot0 + x1;
-        if (tid == 0)
-            C.off[ne] = tot0 + tot1;
-        __syncthreads();
-        const int items = tot0 + tot1;
-        const int per = (items + SPA_WARPS - 1) / SPA_WARPS;
-        const int w0 = r * per, w1 = min(items, w0 + per);
-        if (w0 + lane < w1)
-        {
-            // the entry of this lane's first item: the last entry starting at or before it
-            const int first = w0 + lane;
-            int lo = 0, hi = ne - 1;
-            while (lo < hi)
-            {
-                const int mid = (lo + hi + 1) >> 1;
-                if (C.off[mid] <= first)
-                    lo = mid;
-                else
-                    hi = mid - 1;
-            }
-            int ent = lo;
-            for (int item = first; item < w1; item += 32)
-            {
-                while (C.off[ent + 1] <= item)
-                    ent++;
-                const int col = P.B_rcol[C.bs[ent] + (item - C.off[ent])];
-                const int J = col >> 4;
-                if (J < J0 || J - J0 >= win)
-                    continue;
-                const int slot = S.map[J - J0];
-                if (slot < nt)
-                    atomicOr(&S.m[C.row[ent] * SP2_MS + slot], 1u << (15 - (col & 15)));
-            }
-        }
-        __syncthreads();
-    }
-    __syncthreads();
-    // half-warp per C tile: row offsets, masks, tile count, bin
-    const unsigned hmask = TSG_HW_MASK(tid);
-    for (int jl = tid >> 4; jl < nt; jl += SPA_THREADS / 16)
-        step2_store(P, t0 + jl, hmask, tid & 15, S.m[(tid & 15) * SP2_MS + jl], s_bins);
-}
-
-// ---------------------------------------------------------------------------
 // Hypersparse tile rows.  With very sparse, unstructured operands step 1's
 // tile structure of a C tile row holds nearly every tile column while the
 // row's scalar products reach only a few of those tiles (n = 65,536 with 8
@@ -1619,13 +1439,9 @@ __device__ __forceinline__ void step2_spa_segment(const ProdView &P, Spa2Smem &S
 // row).  The SPA segments would spend their time on empty tiles, segment
 // after segment, each re-walking A's row.  A wide row whose scalar products
 // (counted by the fused step-1/2 pass, wide_kind) are below HYP_RATIO per C
-// tile is therefore done whole by one CTA:
-//  - step 2 zero-fills the row's masks, row offsets and tile counts with
-//    16-byte stores, ORs every product's bit into C's mask word in global
-//    memory (two rows' 16-bit masks share a 32-bit word), notes the tiles
-//    hit in a shared bitmap and finishes only those tiles, a thread per tile
-//    (row offsets, count and bin from its 16 masks);
-//  - step 3 zero-fills the row's values and adds every product into its
+// tile therefore has its numeric step done whole by one CTA (its symbolic step
+// is any wide row's):
+//  - it zero-fills the row's values and adds every product into its
 //    value slot -- the tile's value offset + the row offset + the popcount
 //    of the row mask left of the column -- in global memory.  Warp r takes
 //    row r's products in generation order (A's entries in column order, each
@@ -1640,7 +1456,6 @@ __device__ __forceinline__ void step2_spa_segment(const ProdView &P, Spa2Smem &S
 // ---------------------------------------------------------------------------
 #define HYP_WIN 16384
 #define HYP_RATIO 4
-static_assert(HYP_WIN / 32 <= SPA_THREADS, "one hit-bitmap word per thread");
 
 struct HypStage
 {
@@ -1652,41 +1467,10 @@ struct HypStage
 
 struct HypSmem
 {
-    unsigned short map[HYP_WIN]; // tile column - W0 -> tile - s0 (only C's columns are read);
-                                 // step 2 then lists the window's hit tiles here
-    unsigned hit[HYP_WIN / 32];  // tiles of the window that received a product (step 2)
-    int wsum[SPA_WARPS];
+    unsigned short map[HYP_WIN]; // tile column - W0 -> tile - s0 (only C's columns are read)
     int win_end;
     HypStage stage[SPA_WARPS];
 };
-
-// Exclusive scan of v over the CTA (SPA_THREADS threads); total = the sum.
-__device__ __forceinline__ int hyp_cta_scan(int v, int *wsum, int &total)
-{
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int incl = v;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1)
-    {
-        const int o = __shfl_up_sync(TSG_FULL_MASK, incl, d);
-        if (lane >= d)
-            incl += o;
-    }
-    if (lane == 31)
-        wsum[w] = incl;
-    __syncthreads();
-    int off = 0, tot = 0;
-#pragma unroll
-    for (int q = 0; q < SPA_WARPS; q++)
-    {
-        const int x = wsum[q];
-        off += q < w ? x : 0;
-        tot += x;
-    }
-    total = tot;
-    __syncthreads();
-    return off + incl - v;
-}
 
 // 2 when the wide A tile row i is hypersparse, else 1: B has a row view,
 // the row's C tiles span less than one map window (HYP_WIN tile columns), and
@@ -1730,9 +1514,9 @@ __device__ __forceinline__ int wide_kind(const ProdView &P, int i, int lane)
 // Warp r enumerates the products of C row 16 I + r: A's entries of the row in
 // column order, each with its B row (row view), flattened 32 products at a
 // time.  f(valid, e, bi) is called with the whole warp converged; e is the
-// staged entry (G.a[e] its A value when VAL), bi the product's index in B's
+// staged entry (G.a[e] its A value), bi the product's index in B's
 // row view.  Lane order within a batch, and batch order, follow k.
-template <bool VAL, typename F>
+template <typename F>
 __device__ __forceinline__ void hyp_walk(const ProdView &P, HypStage &G, int I, int r, int lane, F f)
 {
     const int pa_beg = P.A_ptr[I], pa_end = P.A_ptr[I + 1];
@@ -1747,8 +1531,7 @@ __device__ __forceinline__ void hyp_walk(const ProdView &P, HypStage &G, int I, 
             if (mr)
             {
                 kb = P.A_col[pa] * TSG_BS;
-                if (VAL)
-                    st = P.A_tnnz[pa] + P.A_Ptr[(long long)pa * TSG_BS + r];
+                st = P.A_tnnz[pa] + P.A_Ptr[(long long)pa * TSG_BS + r];
             }
         }
         const int cnt = __popc(mr);
@@ -1775,8 +1558,7 @@ __device__ __forceinline__ void hyp_walk(const ProdView &P, HypStage &G, int I, 
                     const int k = kb + (15 - bit);
                     const int b0 = P.B_rptr[k];
                     G.bl[e] = make_int2(b0, P.B_rptr[k + 1] - b0);
-                    if (VAL)
-                        G.a[e] = P.A_Val[st + x];
+                    G.a[e] = P.A_Val[st + x];
                 }
             }
             __syncwarp();
@@ -1834,84 +1616,6 @@ __device__ __forceinline__ int hyp_window(const ProdView &P, HypSmem &S, int s0,
     return s1;
 }
 
-// Step 2 of hypersparse tile row I by the CTA (SPA_THREADS threads).
-__device__ __forceinline__ void step2_hyper_row(const ProdView &P, HypSmem &S, int I, int *s_bins)
-{
-    const int tid = threadIdx.x, lane = tid & 31, r = tid >> 5;
-    const int rs = P.C_ptr[I], re = P.C_ptr[I + 1];
-    __syncthreads();
-    {
-        const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-        uint4 *mk = reinterpret_cast<uint4 *>(P.C_mask + (long long)rs * TSG_BS);
-        uint4 *pt = reinterpret_cast<uint4 *>(P.C_Ptr + (long long)rs * TSG_BS);
-        for (int q = tid; q < 2 * (re - rs); q += SPA_THREADS)
-            mk[q] = z;
-        for (int q = tid; q < re - rs; q += SPA_THREADS)
-        {
-            pt[q] = z;
-            P.C_tnnz[rs + q] = 0;
-        }
-    }
-    __threadfence_block();
-    for (int s0 = rs; s0 < re;)
-    {
-        __syncthreads();
-        const int W0 = P.C_col[s0];
-        for (int q = tid; q < HYP_WIN / 32; q += SPA_THREADS)
-            S.hit[q] = 0u;
-        const int s1 = hyp_window(P, S, s0, re, W0);
-        const int nw = s1 - s0;
-        hyp_walk<false>(P, S.stage[r], I, r, lane, [&](bool valid, int, int bi) {
-            if (!valid)
-                return;
-            const int col = P.B_rcol[bi];
-            const int w = (col >> 4) - W0;
-            if (w < 0 || w >= HYP_WIN)
-                return; // another window's product
-            const int sl = S.map[w];
-            if (sl >= nw)
-                return;
-            const long long t = (long long)s0 + sl;
-            unsigned *word = reinterpret_cast<unsigned *>(P.C_mask + t * TSG_BS + (r & ~1));
-            atomicOr(word, 1u << ((15 - (col & 15)) + ((r & 1) << 4)));
-            const unsigned hb = 1u << (sl & 31);
-            if (!(S.hit[sl >> 5] & hb))
-                atomicOr(&S.hit[sl >> 5], hb);
-        });
-        __threadfence_block();
-        __syncthreads();
-        // list the tiles that received a product (over the map), then a
-        // thread per listed tile: its 16 row masks (two 16-byte loads from
-        // L2), row offsets, count and bin
-        const unsigned hw = tid < ((nw + 31) >> 5) ? S.hit[tid] : 0u;
-        int nh;
-        int at = hyp_cta_scan(__popc(hw), S.wsum, nh);
-        for (unsigned b = hw; b; b &= b - 1)
-            S.map[at++] = (unsigned short)(tid * 32 + __ffs(b) - 1);
-        __syncthreads();
-        for (int j = tid; j < nh; j += SPA_THREADS)
-        {
-            const long long t = (long long)s0 + S.map[j];
-            const uint4 *mp = reinterpret_cast<const uint4 *>(P.C_mask + t * TSG_BS);
-            const uint4 m0 = __ldcg(mp), m1 = __ldcg(mp + 1);
-            const unsigned w2[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
-            unsigned pk[4] = {0u, 0u, 0u, 0u};
-            int run = 0;
-#pragma unroll
-            for (int rr = 0; rr < TSG_BS; rr++)
-            {
-                pk[rr >> 2] |= (unsigned)run << ((rr & 3) * 8);
-                run += __popc((w2[rr >> 1] >> ((rr & 1) * 16)) & 0xFFFFu);
-            }
-            *reinterpret_cast<uint4 *>(P.C_Ptr + t * TSG_BS) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-            P.C_tnnz[t] = run;
-            if (s_bins)
-                atomicAdd(&s_bins[nnz_bin(run)], 1);
-        }
-        s0 = s1;
-    }
-}
-
 // Step 3 of hypersparse tile row I by the CTA.
 __device__ __forceinline__ void step3_hyper_row(const ProdView &P, HypSmem &S, int I)
 {
@@ -1931,7 +1635,7 @@ __device__ __forceinline__ void step3_hyper_row(const ProdView &P, HypSmem &S, i
         const int W0 = P.C_col[s0];
         const int s1 = hyp_window(P, S, s0, re, W0);
         const int nw = s1 - s0;
-        hyp_walk<true>(P, G, I, r, lane, [&](bool valid, int e, int bi) {
+        hyp_walk(P, G, I, r, lane, [&](bool valid, int e, int bi) {
             int pos = -1 - lane; // distinct keys for lanes without a slot
             double prod = 0.0;
             if (valid)
@@ -2044,7 +1748,7 @@ __device__ __forceinline__ void spa_skip_hyper(const ProdView &P, const int *__r
 
 // Hypersparse rows (kind[I] == 2, kind may be null) are done whole by the
 // block owning their first tile.
-static_assert(sizeof(HypSmem) <= sizeof(SpaSmem) && sizeof(HypSmem) <= sizeof(Spa2Smem), "hyper scratch");
+static_assert(sizeof(HypSmem) <= sizeof(SpaSmem), "hyper scratch");
 
 // only (may be null): only the tile rows I with only[I] != 0 (the rows the
 // staged numeric step left).
@@ -2069,35 +1773,6 @@ __device__ __forceinline__ void step3_spa_block(const ProdView &P, SpaSmem &S, i
             const int n = __syncthreads_count(ok);
             const int t1 = t0 + (n > 0 ? n : 1);
             step3_spa_segment<FLAT>(P, S, t0, t1);
-            t0 = t1;
-        }
-    });
-}
-
-// Symbolic counterpart, for the pieces of wide rows only (wide[I] != 0;
-// 2 marks a hypersparse row).  Long rows go in chunks of SP2_SEGT tiles, one
-// segment's worth: each segment walks A's whole row, so shorter chunks would
-// repeat that walk.
-__device__ __forceinline__ void step2_spa_block(const ProdView &P, Spa2Smem &S, int tb, int te,
-                                                const int *__restrict__ wide, int *s_bins)
-{
-    spa_block_pieces<SP2_SEGT>(P, tb, te, [&](int I, int ps, int pe) {
-        const int kind = wide[I];
-        if (!kind)
-            return;
-        if (kind == 2)
-        {
-            if (ps == P.C_ptr[I])
-                step2_hyper_row(P, reinterpret_cast<HypSmem &>(S), I, s_bins);
-            return;
-        }
-        for (int t0 = ps; t0 < pe;)
-        {
-            const int cand = t0 + 1 + (int)threadIdx.x;
-            const bool ok = threadIdx.x < SP2_SEGT && cand <= pe && P.C_col[cand - 1] - P.C_col[t0] < SP2_WIN;
-            const int n = __syncthreads_count(ok);
-            const int t1 = t0 + (n > 0 ? n : 1);
-            step2_spa_segment(P, S, t0, t1, s_bins);
             t0 = t1;
         }
     });

@@ -20,11 +20,8 @@
 #include "tsg_window.cuh"
 
 #define S1_WARPS 8
-// a CTA per tile row counts step 1's tiles from this many tile pairs per row
-// (mean tiles per row of A times B's): below it a warp per row keeps up
-#define S1_CTA_PAIRS 512
-// step 1's bitmaps are kept up to this many words per tile row, and in all
-#define S1_KEEP_WORDS 512
+#define S1C_THREADS 256
+// step 1's bitmaps are kept up to this many words in all
 #define S1_KEEP_TOTAL (1LL << 24)
 // tile columns of a CTA's shared memory in the wide-row step 2
 #define WIDE_SPAN 6144
@@ -47,8 +44,8 @@ __global__ void __launch_bounds__(S1_WARPS * 32) k_step1(ProdView P, int *__rest
 __global__ void __launch_bounds__(S1C_THREADS) k_step1_cta(ProdView P, int *__restrict__ C_cnt,
                                                            unsigned long long *__restrict__ pairs, StepOneBits K)
 {
-    __shared__ S1cSmem S;
-    const int cnt = step1_row_cta(P, blockIdx.x, S, K, pairs);
+    __shared__ S1cSmem<S1C_THREADS> S;
+    const int cnt = step1_row_cta<S1C_THREADS>(P, blockIdx.x, S, K, pairs);
     if (threadIdx.x == 0)
         C_cnt[blockIdx.x] = cnt;
 }
@@ -284,41 +281,26 @@ __global__ void __launch_bounds__(SPA_THREADS, 2) k_step3_rest(ProdView P, const
     }
 }
 
-// warp per B row: its entry offset at every block boundary
+// The windows' tables of one product (a warp per row of B)
 __global__ void __launch_bounds__(256) k_win_btab(int m, const int *__restrict__ rptr, const int *__restrict__ rcol,
                                                   int blocks, int bits, int *__restrict__ tab)
 {
     const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (w >= m)
-        return;
-    const int e0 = rptr[w], e1 = rptr[w + 1];
-    int *t = tab + w * (blocks + 1);
-    // entry e opens the blocks after the previous entry's up to its own
-    for (int e = e0 + lane; e <= e1; e += 32)
-    {
-        const int prev = e > e0 ? rcol[e - 1] >> bits : -1;
-        const int cur = e < e1 ? rcol[e] >> bits : blocks;
-        for (int b = prev + 1; b <= cur; b++)
-            t[b] = e;
-    }
+    if (w < m)
+        win_btab_row((int)w, rptr, rcol, blocks, bits, tab);
 }
 
-// thread per (tile row, window boundary): the first C tile at or after it;
-// thread per row of A: the list of heavy rows
+// ctab, and the list of heavy rows
 __global__ void __launch_bounds__(256) k_win_ctab(ProdView P, WinPlan Q)
 {
     const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (g < Q.mA && Q.A_rptr[g + 1] - Q.A_rptr[g] >= WIN_HEAVY)
         Q.heavy[atomicAdd(&Q.count[1], 1u)] = (int)g;
-    if (g >= (long long)P.tilemA * (Q.windows + 1))
-        return;
-    const int I = (int)(g / (Q.windows + 1)), w = (int)(g % (Q.windows + 1));
-    const int c0 = P.C_ptr[I], c1 = P.C_ptr[I + 1];
-    Q.ctab[g] = c0 + lower_bound_int(P.C_col + c0, c1 - c0, w * WIN_TILES);
+    if (g < (long long)P.tilemA * (Q.windows + 1))
+        win_ctab_entry(P, Q, g);
 }
 
-// tile rows [row0, row1); Q.count[0] zeroed.  The claims are the heavy rows'
+// Step 3 by windows, tile rows [row0, row1); Q.count[0] zeroed.  The claims are the heavy rows'
 // (row, WIN_PART columns), then every other row's (tile row, window, WIN_ROWS
 // rows).
 __global__ void __launch_bounds__(WIN_THREADS, WIN_CTAS) k_step3_win(ProdView P, WinPlan Q, int row0, int row1)
@@ -329,10 +311,9 @@ __global__ void __launch_bounds__(WIN_THREADS, WIN_CTAS) k_step3_win(ProdView P,
     for (int q = lane; q < WIN_COLS; q += 32)
         S.acc[q] = 0.0;
     __syncwarp();
-    const unsigned per = TSG_BS / WIN_ROWS; // claims of a (tile row, window)
-    const unsigned parts = (unsigned)Q.windows * WIN_PARTS;
+    const unsigned parts = (unsigned)(P.nB + WIN_PART - 1) / WIN_PART;
     const unsigned hclaims = Q.count[1] * parts;
-    const unsigned claims = hclaims + (unsigned)(row1 - row0) * Q.windows * per;
+    const unsigned claims = hclaims + (unsigned)(row1 - row0) * Q.windows * WIN_PER;
     unsigned nxt = 0;
     if (lane == 0)
         nxt = atomicAdd(&Q.count[0], 1u);
@@ -343,32 +324,13 @@ __global__ void __launch_bounds__(WIN_THREADS, WIN_CTAS) k_step3_win(ProdView P,
             break;
         if (lane == 0)
             nxt = atomicAdd(&Q.count[0], 1u);
-        if (c < hclaims)
+        if (c >= hclaims)
+            win_claim_rows(P, Q, S, row0, c - hclaims, lane);
+        else
         {
-            const int row = Q.heavy[c / parts], part = (int)(c % parts);
-            const int I = row / TSG_BS, w = part / WIN_PARTS;
-            if (I < row0 || I >= row1 || part * WIN_PART >= P.nB)
-                continue;
-            const int *ct = Q.ctab + (long long)I * (Q.windows + 1) + w;
-            win_task(P, Q, S, I, row % TSG_BS, part * WIN_PART, (part + 1) * WIN_PART, Q.A_rptr[row],
-                     Q.A_rptr[row + 1], ct[0], ct[1], lane);
-            continue;
-        }
-        const int u = (c - hclaims) / per;
-        const int I = row0 + u / Q.windows, w = u % Q.windows;
-        const int r0 = ((c - hclaims) % per) * WIN_ROWS;
-        const int *ct = Q.ctab + (long long)I * (Q.windows + 1) + w;
-        const int t0 = ct[0], t1 = ct[1];
-        if (t0 == t1)
-            continue;
-        const int row = I * TSG_BS + r0;
-        const int e = lane <= WIN_ROWS ? Q.A_rptr[min(row + lane, Q.mA)] : 0;
-#pragma unroll 1
-        for (int k = 0; k < WIN_ROWS; k++)
-        {
-            const int e0 = __shfl_sync(TSG_FULL_MASK, e, k), e1 = __shfl_sync(TSG_FULL_MASK, e, k + 1);
-            if (e0 < e1 && e1 - e0 < WIN_HEAVY)
-                win_task(P, Q, S, I, r0 + k, w * WIN_COLS, (w + 1) * WIN_COLS, e0, e1, t0, t1, lane);
+            const int row = Q.heavy[c / parts], I = row / TSG_BS;
+            if (I >= row0 && I < row1)
+                win_claim_heavy(P, Q, S, row, (int)(c % parts), lane);
         }
     }
 }
@@ -543,12 +505,9 @@ static bool win_shape(const ProdView &P, long long nnzC, WinPlan &Q)
     // claims of every row as if it were heavy: 32-bit
     if (nnzC < WIN_MIN_VALUES * windows * P.mA || windows * WIN_PARTS * (P.mA + TSG_BS) > INT_MAX)
         return false;
-    int bits = WIN_PART_BITS;
-    while ((((P.nB - 1) >> bits) + 2LL) * P.mB > WIN_TABLE_WORDS && (P.nB - 1) >> bits)
-        bits++;
+    if (!win_table(P.mB, P.nB, WIN_TABLE_WORDS, Q.bits, Q.blocks))
+        return false;
     Q.windows = (int)windows;
-    Q.bits = bits;
-    Q.blocks = ((P.nB - 1) >> bits) + 1;
     Q.mA = P.mA;
     return true;
 }
@@ -773,10 +732,8 @@ static int spgemm_structure(tsg_context *ctx, const tsg_tiled *A, const tsg_tile
             R.bits.stride = stride;
             TSG_TRY(tsg_alloc(ctx, &R.bits.words, (size_t)tilem * stride));
             TSG_TRY(tsg_alloc(ctx, &R.bits.span, (size_t)tilem));
-            TSG_CUDA(cudaMemsetAsync(R.bits.span, 0, (size_t)tilem * sizeof(int2), st));
         }
-        const long long pairs = (long long)(A->numtile / tilem) * (B->tilem ? B->numtile / B->tilem : 0);
-        if (pairs >= S1_CTA_PAIRS)
+        if (step1_by_cta(A, B))
             k_step1_cta<<<tilem, S1C_THREADS, 0, st>>>(P, C->tile_ptr, R.d_pairs, R.bits);
         else
             k_step1<false><<<tsg_blocks(tilem, S1_WARPS), S1_WARPS * 32, 0, st>>>(P, C->tile_ptr, R.d_pairs, R.bits);

@@ -17,16 +17,26 @@
 // meet a bit already set, which a load tells cheaper than an atomic.  The
 // bitmap words are kept (`words`, see StepOneBits) for the emit pass.
 // ---------------------------------------------------------------------------
-#define S1C_THREADS 256
-#define S1C_WARPS (S1C_THREADS / 32)
 #define S1C_WORDS 2048
+// a CTA per tile row from this many tile pairs per row (mean tiles per row of
+// A times B's): below it a warp per row keeps up
+#define S1_CTA_PAIRS 512
+// a row's words are kept up to this many (16,384 tile columns)
+#define S1_KEEP_WORDS 512
 
+static inline bool step1_by_cta(const tsg_tiled *A, const tsg_tiled *B)
+{
+    return A->tilem > 0 && B->tilem > 0 &&
+           (long long)(A->numtile / A->tilem) * (B->numtile / B->tilem) >= S1_CTA_PAIRS;
+}
+
+template <int NT>
 struct S1cSmem
 {
     unsigned bm[S1C_WORDS];
-    int b0[S1C_THREADS];      // per A tile of the chunk: its B tile row's first tile ...
-    int off[S1C_THREADS + 1]; // ... and its first pair
-    int wsum[S1C_WARPS];
+    int b0[NT];      // per A tile of the chunk: its B tile row's first tile less its first pair ...
+    int off[NT + 1]; // ... and its first pair
+    int wsum[NT / 32];
     int lo, hi, cnt;
 };
 
@@ -68,8 +78,9 @@ __device__ __forceinline__ int last_at_or_before(const int *off, int n, int x)
     return lo;
 }
 
-// C tiles of tile row i, counted by the CTA; thread 0 gets the count
-__device__ __forceinline__ int step1_row_cta(const ProdView &P, int i, S1cSmem &S, const StepOneBits &K,
+// C tiles of tile row i, counted by the CTA (NT threads); thread 0 gets the count
+template <int NT>
+__device__ __forceinline__ int step1_row_cta(const ProdView &P, int i, S1cSmem<NT> &S, const StepOneBits &K,
                                              unsigned long long *pairs)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -83,7 +94,7 @@ __device__ __forceinline__ int step1_row_cta(const ProdView &P, int i, S1cSmem &
     __syncthreads();
     int lo = INT_MAX, hi = -1;
     unsigned long long np = 0;
-    for (int pa = a0 + tid; pa < a1; pa += S1C_THREADS)
+    for (int pa = a0 + tid; pa < a1; pa += NT)
     {
         const int k = P.A_col[pa];
         const int b0 = P.B_ptr[k], b1 = P.B_ptr[k + 1];
@@ -116,11 +127,11 @@ __device__ __forceinline__ int step1_row_cta(const ProdView &P, int i, S1cSmem &
     {
         const int c1 = min(hi + 1, c0 + S1C_WORDS * 32);
         const int nw = (c1 - c0 + 31) >> 5;
-        for (int w = tid; w < nw; w += S1C_THREADS)
+        for (int w = tid; w < nw; w += NT)
             S.bm[w] = 0u;
-        for (int g = a0; g < a1; g += S1C_THREADS)
+        for (int g = a0; g < a1; g += NT)
         {
-            const int n = min(S1C_THREADS, a1 - g);
+            const int n = min(NT, a1 - g);
             int b0 = 0, len = 0;
             if (tid < n)
             {
@@ -129,13 +140,13 @@ __device__ __forceinline__ int step1_row_cta(const ProdView &P, int i, S1cSmem &
                 len = P.B_ptr[k + 1] - b0;
             }
             int total;
-            const int pre = cta_excl_scan<S1C_WARPS>(len, S.wsum, total);
+            const int pre = cta_excl_scan<NT / 32>(len, S.wsum, total);
             S.b0[tid] = b0 - pre;
             S.off[tid] = pre;
             if (tid == n - 1)
                 S.off[n] = total;
             __syncthreads();
-            const int per = (total + S1C_WARPS - 1) / S1C_WARPS;
+            const int per = (total + (NT / 32) - 1) / (NT / 32);
             const int w1 = min(total, (warp + 1) * per);
             int item = warp * per + lane;
             if (item < w1)
@@ -159,7 +170,7 @@ __device__ __forceinline__ int step1_row_cta(const ProdView &P, int i, S1cSmem &
         }
         int cnt = 0;
         const bool keep = K.words && once && nw <= K.stride;
-        for (int w = tid; w < nw; w += S1C_THREADS)
+        for (int w = tid; w < nw; w += NT)
         {
             const unsigned bits = S.bm[w];
             cnt += __popc(bits);
@@ -231,10 +242,15 @@ static inline size_t wide_units(int tilem, int nnzA)
     return (size_t)tilem + nnzA / WIDE_SPLIT;
 }
 
-__device__ __forceinline__ void wide_list(const ProdView &P, int i, int *wide)
+__device__ __forceinline__ int wide_parts(const ProdView &P, int i)
 {
     const int entries = P.A_tnnz[P.A_ptr[i + 1]] - P.A_tnnz[P.A_ptr[i]];
-    const int parts = min(WIDE_PARTS, 1 + entries / WIDE_SPLIT);
+    return min(WIDE_PARTS, 1 + entries / WIDE_SPLIT);
+}
+
+__device__ __forceinline__ void wide_list(const ProdView &P, int i, int *wide)
+{
+    const int parts = wide_parts(P, i);
     int *at = wide + P.tilemA + 1 + 2 * atomicAdd(&wide[P.tilemA], parts);
     for (int q = 0; q < parts; q++)
     {

@@ -78,6 +78,45 @@ struct WinPlan
     int mA;
 };
 
+// B row w's entry offset at every block boundary, by a warp
+__device__ __forceinline__ void win_btab_row(int w, const int *__restrict__ rptr, const int *__restrict__ rcol,
+                                             int blocks, int bits, int *__restrict__ tab)
+{
+    const int lane = threadIdx.x & 31;
+    const int e0 = rptr[w], e1 = rptr[w + 1];
+    int *t = tab + (long long)w * (blocks + 1);
+    // entry e opens the blocks after the previous entry's up to its own
+    for (int e = e0 + lane; e <= e1; e += 32)
+    {
+        const int prev = e > e0 ? rcol[e - 1] >> bits : -1;
+        const int cur = e < e1 ? rcol[e] >> bits : blocks;
+        for (int b = prev + 1; b <= cur; b++)
+            t[b] = e;
+    }
+}
+
+// entry g of ctab, (tile row, window boundary): the first C tile at or after it
+__device__ __forceinline__ void win_ctab_entry(const ProdView &P, const WinPlan &Q, long long g)
+{
+    const int I = (int)(g / (Q.windows + 1)), w = (int)(g % (Q.windows + 1));
+    const int c0 = P.C_ptr[I], c1 = P.C_ptr[I + 1];
+    Q.ctab[g] = c0 + lower_bound_int(P.C_col + c0, c1 - c0, w * WIN_TILES);
+}
+
+// The table's shape for m x n rows of B and at most `words` of table; false
+// when even one block per row is too many.
+static inline bool win_table(int mB, int nB, long long words, int &bits, int &blocks)
+{
+    for (bits = WIN_PART_BITS;; bits++)
+    {
+        blocks = ((nB - 1) >> bits) + 1;
+        if ((blocks + 1LL) * mB <= words)
+            return true;
+        if (blocks == 1)
+            return false;
+    }
+}
+
 // an A entry's value and its part of B's row inside columns [c0, c1)
 struct WinEntry
 {
@@ -85,12 +124,13 @@ struct WinEntry
     int b0, len;
 };
 
-__device__ __forceinline__ WinEntry win_entry(const ProdView &P, const WinPlan &Q, int x, int e1, int c0, int c1)
+// entry x (none when x >= e1), column k of A
+__device__ __forceinline__ WinEntry win_entry(const ProdView &P, const WinPlan &Q, int x, int e1, int k, int c0, int c1)
 {
     WinEntry E = {0.0, 0, 0};
     if (x < e1)
     {
-        const int *t = Q.btab + (long long)Q.A_rcol[x] * (Q.blocks + 1);
+        const int *t = Q.btab + (long long)k * (Q.blocks + 1);
         const int blk = c0 >> Q.bits;
         E.a = Q.A_rval[x];
         E.b0 = t[blk];
@@ -106,22 +146,45 @@ __device__ __forceinline__ WinEntry win_entry(const ProdView &P, const WinPlan &
 }
 
 // C row r of tile row I, columns [c0, c1); its A entries are [e0, e1) of the
-// row view, its C tiles [t0, t1).  All lanes of the warp call it.
+// row view (E: this lane's of the first 32, loaded by the caller), its C tiles
+// [t0, t1), at most 64.  All lanes of the warp call it.
+//
+// Loads go ahead of their use, since a warp of short rows would wait on one
+// chain of them after another: the entries' columns two groups of 32 ahead,
+// their parts of B one group, B's entries two batches, the row's masks and
+// value offsets from the start.
 __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, WinTask &S, int I, int r, int c0, int c1,
-                                         int e0, int e1, int t0, int t1, int lane)
+                                         int e0, int e1, WinEntry E, int t0, int t1, int lane)
 {
     const unsigned upto = 0xffffffffu >> (31 - lane); // lanes up to this one
+    unsigned mk[2];
+    int at[2], base[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+    {
+        const int t = t0 + 32 * h + lane;
+        mk[h] = 0u;
+        at[h] = base[h] = 0;
+        if (t < t1)
+        {
+            base[h] = P.C_col[t] * TSG_BS - c0;
+            mk[h] = P.C_mask[(long long)t * TSG_BS + r];
+            at[h] = P.C_tnnz[t] + P.C_Ptr[(long long)t * TSG_BS + r];
+        }
+    }
     bool any = false;
-    WinEntry nxt = win_entry(P, Q, e0 + lane, e1, c0, c1);
+    int k = e0 + 32 + lane < e1 ? Q.A_rcol[e0 + 32 + lane] : 0;
     for (int g = e0; g < e1; g += 32)
     {
-        const WinEntry E = nxt;
-        if (g + 32 < e1)
-            nxt = win_entry(P, Q, g + 32 + lane, e1, c0, c1);
+        const WinEntry nxt = win_entry(P, Q, g + 32 + lane, e1, k, c0, c1);
+        k = g + 64 + lane < e1 ? Q.A_rcol[g + 64 + lane] : 0;
         const int len = E.len;
         const unsigned full = __ballot_sync(TSG_FULL_MASK, len > 0);
         if (!full)
+        {
+            E = nxt;
             continue;
+        }
         any = true;
         int incl = len;
 #pragma unroll
@@ -214,27 +277,76 @@ __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, Wi
             p0 = np0;
             p1 = np1;
         }
+        E = nxt;
     }
     if (!any)
         return;
-    for (int t = t0 + lane; t < t1; t += 32)
+#pragma unroll
+    for (int h = 0; h < 2; h++)
     {
-        const int base = P.C_col[t] * TSG_BS - c0;
-        const long long tt = (long long)t * TSG_BS + r;
-        unsigned mk = P.C_mask[tt];
-        if (!mk || base < 0 || base >= c1 - c0)
-            continue;
-        int q = P.C_tnnz[t] + P.C_Ptr[tt];
-        double *acc = S.acc + base;
-        do
+        unsigned m = base[h] >= 0 && base[h] < c1 - c0 ? mk[h] : 0u; // a heavy row's part holds some of the tiles
+        double *acc = S.acc + base[h];
+        int q = at[h];
+        while (m)
         {
-            const int bit = 31 - __clz(mk);
-            mk ^= 1u << bit;
+            const int bit = 31 - __clz(m);
+            m ^= 1u << bit;
             P.C_Val[q] = acc[15 - bit];
             acc[15 - bit] = 0.0;
             P.C_Colb[q] = (unsigned char)(15 - bit);
             q++;
-        } while (mk);
+        }
     }
     __syncwarp();
 }
+static_assert(WIN_TILES <= 64, "C tiles of a window");
+
+// columns [part * WIN_PART, ...) of heavy row `row`
+__device__ __forceinline__ void win_claim_heavy(const ProdView &P, const WinPlan &Q, WinTask &S, int row, int part,
+                                                int lane)
+{
+    const int *ct = Q.ctab + (long long)(row / TSG_BS) * (Q.windows + 1) + part / WIN_PARTS;
+    const int e0 = Q.A_rptr[row], e1 = Q.A_rptr[row + 1], c0 = part * WIN_PART, c1 = c0 + WIN_PART;
+    const int k = e0 + lane < e1 ? Q.A_rcol[e0 + lane] : 0;
+    win_task(P, Q, S, row / TSG_BS, row % TSG_BS, c0, c1, e0, e1, win_entry(P, Q, e0 + lane, e1, k, c0, c1), ct[0],
+             ct[1], lane);
+}
+
+// claim c of the tile rows from row0 on: WIN_ROWS rows of a (tile row, window)
+#define WIN_PER (TSG_BS / WIN_ROWS) // claims of a (tile row, window)
+__device__ __forceinline__ void win_claim_rows(const ProdView &P, const WinPlan &Q, WinTask &S, int row0, unsigned c,
+                                               int lane)
+{
+    const int u = c / WIN_PER;
+    const int I = row0 + u / Q.windows, w = u % Q.windows;
+    const int r0 = (c % WIN_PER) * WIN_ROWS;
+    const int *ct = Q.ctab + (long long)I * (Q.windows + 1) + w;
+    const int t0 = ct[0], t1 = ct[1];
+    if (t0 == t1)
+        return;
+    const int row = I * TSG_BS + r0;
+    const int c0 = w * WIN_COLS, c1 = c0 + WIN_COLS;
+    const int e = lane <= WIN_ROWS ? Q.A_rptr[min(row + lane, Q.mA)] : 0;
+    // first entries of the rows: columns two rows ahead, parts of B one
+    auto col = [&](int i) {
+        const int x0 = __shfl_sync(TSG_FULL_MASK, e, i), x1 = __shfl_sync(TSG_FULL_MASK, e, i + 1);
+        return i < WIN_ROWS && x0 + lane < x1 ? Q.A_rcol[x0 + lane] : 0;
+    };
+    int k1 = col(0);
+    int k2 = col(1);
+    int e0 = __shfl_sync(TSG_FULL_MASK, e, 0), e1 = __shfl_sync(TSG_FULL_MASK, e, 1);
+    WinEntry E = win_entry(P, Q, e0 + lane, e1, k1, c0, c1);
+#pragma unroll 1
+    for (int i = 0; i < WIN_ROWS; i++)
+    {
+        const int e2 = __shfl_sync(TSG_FULL_MASK, e, min(i + 2, WIN_ROWS));
+        const WinEntry nxt = win_entry(P, Q, e1 + lane, e2, k2, c0, c1);
+        k2 = col(i + 2);
+        if (e0 < e1 && e1 - e0 < WIN_HEAVY)
+            win_task(P, Q, S, I, r0 + i, c0, c1, e0, e1, E, t0, t1, lane);
+        e0 = e1;
+        e1 = e2;
+        E = nxt;
+    }
+}
+

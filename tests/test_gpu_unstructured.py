@@ -94,6 +94,23 @@ def test_window_step_on_tile_row_ranges(tsg, ctx, oracle, gen):
     _same(got[2:], oracle.gustavson(mat, mat, nthreads=8))
 
 
+def test_batch_of_uneven_products(tsg, ctx, oracle, gen):
+    """All routes of a batch's steps in one: windows with heavy rows, the SPA
+    kernel, hypersparse rows, dense tiles, an empty product."""
+    empty = (20, 300, np.zeros(21, np.int32), np.zeros(0, np.int32), np.zeros(0))
+    mats = [_case("heavy"), _case("cols257"), _case("parts"), (gen.rmat(11, 12, seed=2), gen.rmat(11, 12, seed=3)),
+            (gen.random_poisson(8192, 8192, 4.0, seed=10), gen.random_poisson(8192, 8192, 4.0, seed=11)),
+            (gen.banded(400, 40, seed=1), gen.banded(400, 30, seed=2)), (empty, _case("cols257")[1])]
+    pairs = [tuple(_tiled(tsg, ctx, x, tsg.TSG_TILED_CSC_VIEW) for x in ab) for ab in mats]
+    batch = tsg.Batch(ctx, pairs)
+    for _ in range(2):
+        batch.run()
+        batch.sync()
+        for p, (a, b) in enumerate(mats):
+            _same([x.cpu().numpy() for x in tsg.tiled_to_csr(ctx, batch.product(p))], oracle.gustavson(a, b, nthreads=8))
+    batch.close()
+
+
 @pytest.mark.parametrize("half", [7, 8, 20, 41])
 @pytest.mark.parametrize("special", [None, np.inf, -np.inf, np.nan])
 def test_dense_tiles_with_values_that_zero_does_not_absorb(tsg, ctx, oracle, gen, half, special):
