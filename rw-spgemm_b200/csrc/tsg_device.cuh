@@ -1751,17 +1751,18 @@ __device__ __forceinline__ void spa_skip_hyper(const ProdView &P, const int *__r
 static_assert(sizeof(HypSmem) <= sizeof(SpaSmem), "hyper scratch");
 
 // only (may be null): only the tile rows I with only[I] != 0 (the rows the
-// staged numeric step left).
+// staged numeric step left); hyper: hypersparse rows too.
 template <bool FLAT, int BLK = SPA_BLK>
 __device__ __forceinline__ void step3_spa_block(const ProdView &P, SpaSmem &S, int tb, int te,
-                                                const int *__restrict__ kind, const int *__restrict__ only = nullptr)
+                                                const int *__restrict__ kind, const int *__restrict__ only = nullptr,
+                                                bool hyper = true)
 {
     spa_block_pieces<BLK>(P, tb, te, [&](int I, int ps, int pe) {
         if (only && !only[I])
             return;
         if (kind && kind[I] == 2)
         {
-            if (ps == P.C_ptr[I])
+            if (hyper && ps == P.C_ptr[I])
                 step3_hyper_row(P, reinterpret_cast<HypSmem &>(S), I);
             return;
         }

@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(256) k_step12(ProdView P, StepOneBits K, int *
         {
             wide[i] = kind;
             if (kind)
-                wide_list(P, i, wide);
+                wide_list(P, i, kind, wide);
         }
     }
     __syncthreads();
@@ -146,7 +146,8 @@ __global__ void __launch_bounds__(NT, 1) k_step2_cta(ProdView P, int span, const
         const int q = S.next;
         if (q >= units)
             break;
-        step2_wide_row<NT>(P, S, span, wide[P.tilemA + 1 + 2 * q], wide[P.tilemA + 2 + 2 * q], s_bins);
+        const int2 u = wide_units_of(P, wide)[q];
+        step2_wide_row<NT>(P, S, span, u.x, u.y, s_bins);
     }
     if (threadIdx.x < 4 && s_bins[threadIdx.x])
         atomicAdd(&bins[threadIdx.x], s_bins[threadIdx.x]);
@@ -215,12 +216,14 @@ __global__ void __launch_bounds__(128) k_step3_rows(ProdView P)
 // clamped to those tiles (a separate instantiation keeps the whole-product
 // form's registers).
 template <bool FLAT, bool RANGED, int BLK>
-__global__ void __launch_bounds__(SPA_THREADS, 3) k_step3_spa(ProdView P, const int *__restrict__ kind, int row0,
-                                                              int row1, unsigned *__restrict__ ctr)
+__global__ void __launch_bounds__(SPA_THREADS, 3) k_step3_spa(ProdView P, const int *__restrict__ kind, int hyper,
+                                                              int row0, int row1, unsigned *__restrict__ ctr)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
     SpaSmem &S = *reinterpret_cast<SpaSmem *>(s_raw);
     __shared__ int s_blk;
+    if (!hyper && kind[P.tilemA + 1] == P.numC) // every row was done by k_step3_hyper
+        return;
     unsigned nxt = 0; // thread 0: the next block, claimed one block ahead
     if (threadIdx.x == 0)
         nxt = atomicAdd(ctr, 1u);
@@ -241,7 +244,39 @@ __global__ void __launch_bounds__(SPA_THREADS, 3) k_step3_spa(ProdView P, const 
         if (threadIdx.x == 0)
             spa_skip_hyper<BLK>(P, kind, (int)tb, ctr, -blk0);
         // the block, clamped to the tiles of rows [row0, row1)
-        step3_spa_block<FLAT, BLK>(P, S, max((int)tb, t_beg), (int)min((long long)t_end, tb + BLK), kind);
+        step3_spa_block<FLAT, BLK>(P, S, max((int)tb, t_beg), (int)min((long long)t_end, tb + BLK), kind, nullptr, hyper);
+    }
+}
+
+// The hypersparse rows of tile rows [row0, row1), a CTA each, from step 2's
+// list of wide rows.  Found through the blocks of C tiles they took longer to
+// find than to compute: 65,536 rows of 64 products, 16 blocks to a tile row,
+// 0.759 -> 0.391 ms.
+__global__ void __launch_bounds__(SPA_THREADS, 3) k_step3_hyper(ProdView P, const int *__restrict__ wide, int row0,
+                                                                int row1, unsigned *__restrict__ ctr)
+{
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    HypSmem &S = *reinterpret_cast<HypSmem *>(s_raw);
+    __shared__ int s_unit;
+    const int units = wide[P.tilemA];
+    const int2 *list = wide_units_of(P, wide);
+    unsigned nxt = 0; // thread 0: the next unit, claimed one ahead
+    if (threadIdx.x == 0)
+        nxt = atomicAdd(ctr, 1u);
+    for (;;)
+    {
+        __syncthreads();
+        if (threadIdx.x == 0)
+        {
+            s_unit = (int)nxt;
+            nxt = atomicAdd(ctr, 1u);
+        }
+        __syncthreads();
+        if (s_unit >= units)
+            break;
+        const int2 u = list[s_unit];
+        if ((u.y & 0xFFFF) == 0 && u.x >= row0 && u.x < row1 && wide[u.x] == 2)
+            step3_hyper_row(P, S, u.x);
     }
 }
 
@@ -574,16 +609,25 @@ static int launch_step3_win(tsg_context *ctx, const ProdView &P, const tsg_tiled
 }
 
 template <bool FLAT, bool RANGED, int BLK = SPA_BLK>
-static int launch_step3_spa(tsg_context *ctx, const ProdView &P0, const int *d_kind, int row0, int row1)
+static int launch_step3_spa(tsg_context *ctx, const ProdView &P0, const int *d_kind, bool hyper_apart, int row0, int row1)
 {
     ProdView P = P0;
     P.status = ctx->d_status;
     unsigned *ctr = nullptr, grid = 0;
     const int smem = (int)sizeof(SpaSmem);
     TSG_TRY(spa_grid(ctx, k_step3_spa<FLAT, RANGED, BLK>, smem, &grid));
-    TSG_TRY(tsg_alloc(ctx, &ctr, 1));
-    TSG_CUDA(cudaMemsetAsync(ctr, 0, sizeof(unsigned), ctx->stream));
-    k_step3_spa<FLAT, RANGED, BLK><<<grid, SPA_THREADS, smem, ctx->stream>>>(P, d_kind, row0, row1, ctr);
+    TSG_TRY(tsg_alloc(ctx, &ctr, 2));
+    TSG_CUDA(cudaMemsetAsync(ctr, 0, 2 * sizeof(unsigned), ctx->stream));
+    if (hyper_apart)
+    {
+        const int hsmem = (int)sizeof(HypSmem);
+        unsigned hgrid = 0;
+        TSG_TRY(spa_grid(ctx, k_step3_hyper, hsmem, &hgrid));
+        k_step3_hyper<<<hgrid, SPA_THREADS, hsmem, ctx->stream>>>(P, d_kind, RANGED ? row0 : 0, RANGED ? row1 : P.tilemA,
+                                                                  ctr + 1);
+        TSG_LAUNCH_CHECK();
+    }
+    k_step3_spa<FLAT, RANGED, BLK><<<grid, SPA_THREADS, smem, ctx->stream>>>(P, d_kind, !hyper_apart, row0, row1, ctr);
     TSG_LAUNCH_CHECK();
     tsg_release(ctx, ctr);
     return TSG_OK;
@@ -642,16 +686,18 @@ static int launch_step3_spa_rows(tsg_context *ctx, const ProdView &P, const tsg_
         return launch_step3_win(ctx, P, A, W, row0, row1);
     }
     if (flat && nnzC >= (long long)SPA_BLK_NARROW_VALUES * P.numC)
-        return whole ? launch_step3_spa<true, false, SPA_BLK_NARROW>(ctx, P, d_kind, 0, 0)
-                     : launch_step3_spa<true, true, SPA_BLK_NARROW>(ctx, P, d_kind, row0, row1);
+        return whole ? launch_step3_spa<true, false, SPA_BLK_NARROW>(ctx, P, d_kind, false, 0, 0)
+                     : launch_step3_spa<true, true, SPA_BLK_NARROW>(ctx, P, d_kind, false, row0, row1);
+    // mostly hypersparse rows (few values in many tiles): those by themselves
+    const bool hyper = d_kind && nnzC < (long long)HYP_RATIO * P.numC && P.numC > (long long)S12_MAXT * P.tilemA;
     if (flat)
-        return whole ? launch_step3_spa<true, false>(ctx, P, d_kind, 0, 0)
-                     : launch_step3_spa<true, true>(ctx, P, d_kind, row0, row1);
+        return whole ? launch_step3_spa<true, false>(ctx, P, d_kind, hyper, 0, 0)
+                     : launch_step3_spa<true, true>(ctx, P, d_kind, hyper, row0, row1);
     if (P.padded)
         return whole ? launch_step3_stg<false>(ctx, P, d_kind, 0, 0) : launch_step3_stg<true>(ctx, P, d_kind, row0, row1);
     // operands viewing a batch arena: not padded for the bulk copies' rounding
-    return whole ? launch_step3_spa<false, false>(ctx, P, d_kind, 0, 0)
-                 : launch_step3_spa<false, true>(ctx, P, d_kind, row0, row1);
+    return whole ? launch_step3_spa<false, false>(ctx, P, d_kind, false, 0, 0)
+                 : launch_step3_spa<false, true>(ctx, P, d_kind, false, row0, row1);
 }
 
 // d_kind: the row kinds of the fused step 1/2 pass (0 narrow, 1 wide,
@@ -756,8 +802,8 @@ static int spgemm_structure(tsg_context *ctx, const tsg_tiled *A, const tsg_tile
         ProdView P = make_view(A, B, C);
         if (fused)
         {
-            TSG_TRY(tsg_alloc(ctx, &R.d_wide, (size_t)tilem + 1 + 2 * wide_units(tilem, A->nnz)));
-            TSG_CUDA(cudaMemsetAsync(R.d_wide + tilem, 0, sizeof(int), st));
+            TSG_TRY(tsg_alloc(ctx, &R.d_wide, (size_t)tilem + 3 + 2 * wide_units(tilem, A->nnz)));
+            TSG_CUDA(cudaMemsetAsync(R.d_wide + tilem, 0, 2 * sizeof(int), st));
             k_step12<<<tsg_blocks(tilem, 8), 256, 0, st>>>(P, R.bits, R.d_wide, R.d_bins);
             TSG_LAUNCH_CHECK();
         }

@@ -232,8 +232,9 @@ __device__ __forceinline__ int wide_word(int w, int h)
 
 // A wide row is one unit of work, or one for every WIDE_SPLIT entries of A in
 // it, each a part of its columns: the CTA that took an R-MAT hub row whole
-// would finish last.  Units are listed as (row, part | parts << 16) at
-// wide[tilemA + 1 ...], wide[tilemA] of them.
+// would finish last.  Units are listed as (row, part | parts << 16) in
+// wide_units_of, wide[tilemA] of them; wide[tilemA + 1] counts the C tiles of
+// hypersparse rows.
 #define WIDE_SPLIT 2048
 #define WIDE_PARTS 16
 
@@ -248,15 +249,19 @@ __device__ __forceinline__ int wide_parts(const ProdView &P, int i)
     return min(WIDE_PARTS, 1 + entries / WIDE_SPLIT);
 }
 
-__device__ __forceinline__ void wide_list(const ProdView &P, int i, int *wide)
+__device__ __forceinline__ const int2 *wide_units_of(const ProdView &P, const int *wide)
+{
+    return reinterpret_cast<const int2 *>(wide + ((P.tilemA + 3) & ~1));
+}
+
+__device__ __forceinline__ void wide_list(const ProdView &P, int i, int kind, int *wide)
 {
     const int parts = wide_parts(P, i);
-    int *at = wide + P.tilemA + 1 + 2 * atomicAdd(&wide[P.tilemA], parts);
+    int2 *at = const_cast<int2 *>(wide_units_of(P, wide)) + atomicAdd(&wide[P.tilemA], parts);
     for (int q = 0; q < parts; q++)
-    {
-        at[2 * q] = i;
-        at[2 * q + 1] = q | parts << 16;
-    }
+        at[q] = make_int2(i, q | parts << 16);
+    if (kind == 2)
+        atomicAdd(&wide[P.tilemA + 1], P.C_ptr[i + 1] - P.C_ptr[i]);
 }
 
 // A unit by the CTA (NT threads); span: tile columns the launch's shared
