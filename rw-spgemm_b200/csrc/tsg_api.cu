@@ -55,14 +55,15 @@ extern "C" int tsg_context_create(int device, tsg_context **out)
     for (int i = 0; i < 8 && e == cudaSuccess; i++)
         e = cudaEventCreate(&ctx->ev[i]);
     if (e == cudaSuccess)
-        e = cudaMalloc((void **)&ctx->d_status, sizeof(int));
+        e = cudaMalloc((void **)&ctx->d_ctl, sizeof(TsgControl));
     if (e == cudaSuccess)
-        e = cudaMemset(ctx->d_status, 0, sizeof(int));
+        e = cudaMemset(ctx->d_ctl, 0, sizeof(TsgControl));
     if (e != cudaSuccess)
     {
         free(ctx);
         return tsg_set_error(TSG_ERR_CUDA, "context creation failed: %s", cudaGetErrorString(e));
     }
+    ctx->d_status = &ctx->d_ctl->status;
     ctx->own_stream = 1;
     ctx->sched = TSG_SCHED_SPA;
     ctx->seg_tiles = 8;
@@ -97,7 +98,7 @@ extern "C" int tsg_context_destroy(tsg_context *ctx)
     if (ctx->own_stream)
         cudaStreamDestroy(ctx->stream);
     cudaFreeHost(ctx->h_pinned);
-    cudaFree(ctx->d_status);
+    cudaFree(ctx->d_ctl);
     free(ctx);
     return TSG_OK;
 }
@@ -107,7 +108,11 @@ int tsg_take_device_status(tsg_context *ctx)
     int *h = (int *)(ctx->h_pinned + 63);
     TSG_CUDA(cudaMemcpyAsync(h, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     TSG_CUDA(cudaStreamSynchronize(ctx->stream));
-    const int code = *h;
+    return tsg_check_device_status(ctx, *h);
+}
+
+int tsg_check_device_status(tsg_context *ctx, int code)
+{
     if (code == TSG_OK)
         return TSG_OK;
     TSG_CUDA(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
@@ -195,7 +200,6 @@ extern "C" int tsg_context_synchronize(tsg_context *ctx)
 {
     if (!ctx)
         return tsg_set_error(TSG_ERR_INVALID, "null context");
-    TSG_CUDA(cudaStreamSynchronize(ctx->stream));
     return tsg_take_device_status(ctx);
 }
 

@@ -13,6 +13,34 @@
 // tile kernel is faster than the sparse accumulator (the default threshold)
 #define TSG_SPA_DENSE_DEFAULT 64
 
+// What a product's kernels count, in one block of device memory the context
+// keeps: cleared by one memset and read back by one copy per product.
+struct TsgControl
+{
+    unsigned long long pairs; // matched tile pairs
+    int bins[4];              // C tiles by size
+    unsigned ctr[8];          // work counters: TSG_CTR_*
+    int status;               // error word kernels set (TSG_ERR_TIMEOUT, TSG_ERR_OVERFLOW); outlives the clearing
+};
+enum
+{
+    TSG_CTR_STEP2,
+    TSG_CTR_STEP3,
+    TSG_CTR_REST,  // rows another step-3 kernel left, hypersparse rows
+    TSG_CTR_HEAVY, // heavy rows of the window step 3: kept over the ranges of a product
+};
+
+// kernels whose resident CTAs per SM the context remembers
+enum
+{
+    TSG_OCC_SPA = 0, // + FLAT, RANGED, narrow blocks
+    TSG_OCC_STG = 8, // + RANGED
+    TSG_OCC_REST = 10,
+    TSG_OCC_WIN = 12,
+    TSG_OCC_HYPER,
+    TSG_OCC_COUNT
+};
+
 struct tsg_context
 {
     int device;
@@ -29,7 +57,9 @@ struct tsg_context
     int fuse12;          // step-1 emit fused with step 2 for narrow tile rows
     cudaStream_t copy_stream; // device-to-host copies overlapping compute (created on first use)
     cudaEvent_t copy_ev;      // orders a chunk's copy after its fill
-    int *d_status;            // device error word kernels set (TSG_ERR_TIMEOUT, TSG_ERR_OVERFLOW), 0 when clear
+    TsgControl *d_ctl;        // device block of counters and the error word
+    int *d_status;            // its error word, 0 when clear
+    int occ[TSG_OCC_COUNT];   // resident CTAs per SM, 0: not asked yet
     long long allocs;         // device allocations tsg_alloc made on the context
     int spa_dense;            // SPA schedule: C values per tile from which a product takes the tile kernel
     int last_step3;           // TSG_STEP3_* of the last numeric step launched
@@ -38,6 +68,8 @@ struct tsg_context
 // Reads and clears the context's device error word (synchronises the
 // context's stream); returns TSG_OK or the code a kernel recorded.
 int tsg_take_device_status(tsg_context *ctx);
+// ... the same for a word that has been read back: clears it unless TSG_OK
+int tsg_check_device_status(tsg_context *ctx, int code);
 
 // C tile rows are copied to the host in at most TSG_MAX_CHUNKS chunks of at
 // least TSG_CHUNK_NNZ nonzeros (tsg_spgemm_to_host).

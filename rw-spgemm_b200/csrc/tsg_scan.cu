@@ -143,9 +143,8 @@ static int scan_partials(tsg_context *ctx, long long *p, long long nb)
 
 int tsg_scan_counts(tsg_context *ctx, const int *in, int *out, long long n, long long *total)
 {
-    long long *d_total = nullptr;
-    if (total)
-        TSG_TRY(tsg_alloc(ctx, &d_total, 1));
+    // the last block writes the total straight to page-locked host memory
+    long long *d_total = total ? ctx->h_pinned : nullptr;
     if (n <= SCAN_TILE)
     {
         k_scan_apply<int, int><<<1, SCAN_THREADS, 0, ctx->stream>>>(in, n, nullptr, out, d_total);
@@ -165,8 +164,6 @@ int tsg_scan_counts(tsg_context *ctx, const int *in, int *out, long long n, long
     }
     if (total)
     {
-        TSG_CUDA(cudaMemcpyAsync(ctx->h_pinned, d_total, sizeof(long long), cudaMemcpyDeviceToHost, ctx->stream));
-        tsg_release(ctx, d_total);
         TSG_CUDA(cudaStreamSynchronize(ctx->stream));
         *total = ctx->h_pinned[0];
         if (*total > 2147483647LL)

@@ -11,6 +11,7 @@
 // the reference decomposes the work) or the row-segment schedule (half-warp
 // per run of C tiles in one tile row, tile-level Gustavson, no intersection).
 #include <limits.h>
+#include <stddef.h>
 
 #include <algorithm>
 
@@ -330,12 +331,12 @@ __global__ void __launch_bounds__(256) k_win_ctab(ProdView P, WinPlan Q)
 {
     const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (g < Q.mA && Q.A_rptr[g + 1] - Q.A_rptr[g] >= WIN_HEAVY)
-        Q.heavy[atomicAdd(&Q.count[1], 1u)] = (int)g;
+        Q.heavy[atomicAdd(Q.nheavy, 1u)] = (int)g;
     if (g < (long long)P.tilemA * (Q.windows + 1))
         win_ctab_entry(P, Q, g);
 }
 
-// Step 3 by windows, tile rows [row0, row1); Q.count[0] zeroed.  The claims are the heavy rows'
+// Step 3 by windows, tile rows [row0, row1); *Q.claim zeroed.  The claims are the heavy rows'
 // (row, WIN_PART columns), then every other row's (tile row, window, WIN_ROWS
 // rows).
 __global__ void __launch_bounds__(WIN_THREADS, WIN_CTAS) k_step3_win(ProdView P, WinPlan Q, int row0, int row1)
@@ -347,18 +348,18 @@ __global__ void __launch_bounds__(WIN_THREADS, WIN_CTAS) k_step3_win(ProdView P,
         S.acc[q] = 0.0;
     __syncwarp();
     const unsigned parts = (unsigned)(P.nB + WIN_PART - 1) / WIN_PART;
-    const unsigned hclaims = Q.count[1] * parts;
+    const unsigned hclaims = *Q.nheavy * parts;
     const unsigned claims = hclaims + (unsigned)(row1 - row0) * Q.windows * WIN_PER;
     unsigned nxt = 0;
     if (lane == 0)
-        nxt = atomicAdd(&Q.count[0], 1u);
+        nxt = atomicAdd(Q.claim, 1u);
     for (;;)
     {
         const unsigned c = __shfl_sync(TSG_FULL_MASK, nxt, 0);
         if (c >= claims)
             break;
         if (lane == 0)
-            nxt = atomicAdd(&Q.count[0], 1u);
+            nxt = atomicAdd(Q.claim, 1u);
         if (c >= hclaims)
             win_claim_rows(P, Q, S, row0, c - hclaims, lane);
         else
@@ -483,14 +484,30 @@ static int launch_step2(tsg_context *ctx, const ProdView &P, int *d_bins)
     return TSG_OK;
 }
 
-// persistent grid of a SPA kernel: resident CTAs on every SM
+// resident CTAs per SM of a kernel with smem bytes of dynamic shared memory,
+// asked once per context
 template <typename K>
-static int spa_grid(tsg_context *ctx, K kern, int smem, unsigned *grid)
+static int resident_ctas(tsg_context *ctx, int slot, K kern, int threads, int smem, int *per_sm)
 {
-    TSG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    int per_sm = 0;
-    TSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, SPA_THREADS, smem));
-    *grid = (unsigned)(ctx->num_sms * (per_sm > 0 ? per_sm : 1));
+    if (!ctx->occ[slot])
+    {
+        int n = 0;
+        TSG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        TSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem));
+        if (n < 1)
+            return tsg_set_error(TSG_ERR_CUDA, "a persistent kernel does not fit an SM");
+        ctx->occ[slot] = n;
+    }
+    *per_sm = ctx->occ[slot];
+    return TSG_OK;
+}
+
+// clears a step-3 kernel's counter for a range of tile rows after the first
+// (the product's start cleared it before)
+static int clear_counters(tsg_context *ctx, int row0, int first, int count)
+{
+    if (row0 > 0)
+        TSG_CUDA(cudaMemsetAsync(&ctx->d_ctl->ctr[first], 0, count * sizeof(unsigned), ctx->stream));
     return TSG_OK;
 }
 
@@ -502,13 +519,9 @@ static int launch_step2_cta(tsg_context *ctx, const ProdView &P, int span, const
     TSG_CUDA(cudaFuncSetAttribute(k_step2_cta<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     int per_sm = 0;
     TSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step2_cta<NT>, NT, smem));
-    unsigned *ctr = nullptr;
-    TSG_TRY(tsg_alloc(ctx, &ctr, 1));
-    TSG_CUDA(cudaMemsetAsync(ctr, 0, sizeof(unsigned), ctx->stream));
     const int grid = std::min(P.tilemA, ctx->num_sms * std::max(per_sm, 1));
-    k_step2_cta<NT><<<grid, NT, smem, ctx->stream>>>(P, span, d_wide, ctr, d_bins);
+    k_step2_cta<NT><<<grid, NT, smem, ctx->stream>>>(P, span, d_wide, &ctx->d_ctl->ctr[TSG_CTR_STEP2], d_bins);
     TSG_LAUNCH_CHECK();
-    tsg_release(ctx, ctr);
     return TSG_OK;
 }
 
@@ -555,7 +568,6 @@ static void win_release(tsg_context *ctx, WinScratch &W)
     tsg_release(ctx, W.rcol);
     tsg_release(ctx, W.rval);
     tsg_release(ctx, W.Q.heavy);
-    tsg_release(ctx, W.Q.count);
     W.ready = false;
 }
 
@@ -569,8 +581,8 @@ static int win_prepare(tsg_context *ctx, const ProdView &P, const tsg_tiled *A, 
     TSG_TRY(tsg_alloc(ctx, &Q.btab, (size_t)P.mB * (Q.blocks + 1)));
     TSG_TRY(tsg_alloc(ctx, &Q.ctab, (size_t)P.tilemA * (Q.windows + 1)));
     TSG_TRY(tsg_alloc(ctx, &Q.heavy, (size_t)P.mA));
-    TSG_TRY(tsg_alloc(ctx, &Q.count, 2));
-    TSG_CUDA(cudaMemsetAsync(Q.count, 0, 2 * sizeof(unsigned), st));
+    Q.claim = &ctx->d_ctl->ctr[TSG_CTR_STEP3];
+    Q.nheavy = &ctx->d_ctl->ctr[TSG_CTR_HEAVY];
     Q.A_rptr = P.A_rptr;
     Q.A_rcol = P.A_rcol;
     Q.A_rval = P.A_rval;
@@ -597,12 +609,11 @@ static int launch_step3_win(tsg_context *ctx, const ProdView &P, const tsg_tiled
 {
     TSG_TRY(win_prepare(ctx, P, A, W));
     const int smem = WIN_WARPS * (int)sizeof(WinTask);
-    TSG_CUDA(cudaFuncSetAttribute(k_step3_win, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     int per_sm = 0;
-    TSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step3_win, WIN_THREADS, smem));
-    TSG_CUDA(cudaMemsetAsync(W.Q.count, 0, sizeof(unsigned), ctx->stream));
+    TSG_TRY(resident_ctas(ctx, TSG_OCC_WIN, k_step3_win, WIN_THREADS, smem, &per_sm));
+    TSG_TRY(clear_counters(ctx, row0, TSG_CTR_STEP3, 1));
     const long long claims = (long long)(row1 - row0) * W.Q.windows * (TSG_BS / WIN_ROWS);
-    const long long grid = std::min((long long)ctx->num_sms * std::max(per_sm, 1), (claims + WIN_WARPS - 1) / WIN_WARPS);
+    const long long grid = std::min((long long)ctx->num_sms * per_sm, (claims + WIN_WARPS - 1) / WIN_WARPS);
     k_step3_win<<<(unsigned)grid, WIN_THREADS, smem, ctx->stream>>>(P, W.Q, row0, row1);
     TSG_LAUNCH_CHECK();
     return TSG_OK;
@@ -613,23 +624,23 @@ static int launch_step3_spa(tsg_context *ctx, const ProdView &P0, const int *d_k
 {
     ProdView P = P0;
     P.status = ctx->d_status;
-    unsigned *ctr = nullptr, grid = 0;
+    unsigned *ctr = ctx->d_ctl->ctr;
     const int smem = (int)sizeof(SpaSmem);
-    TSG_TRY(spa_grid(ctx, k_step3_spa<FLAT, RANGED, BLK>, smem, &grid));
-    TSG_TRY(tsg_alloc(ctx, &ctr, 2));
-    TSG_CUDA(cudaMemsetAsync(ctr, 0, 2 * sizeof(unsigned), ctx->stream));
+    int per_sm = 0;
+    TSG_TRY(resident_ctas(ctx, TSG_OCC_SPA + (FLAT ? 1 : 0) + (RANGED ? 2 : 0) + (BLK == SPA_BLK ? 0 : 4),
+                          k_step3_spa<FLAT, RANGED, BLK>, SPA_THREADS, smem, &per_sm));
+    TSG_TRY(clear_counters(ctx, row0, TSG_CTR_STEP3, 2));
     if (hyper_apart)
     {
-        const int hsmem = (int)sizeof(HypSmem);
-        unsigned hgrid = 0;
-        TSG_TRY(spa_grid(ctx, k_step3_hyper, hsmem, &hgrid));
-        k_step3_hyper<<<hgrid, SPA_THREADS, hsmem, ctx->stream>>>(P, d_kind, RANGED ? row0 : 0, RANGED ? row1 : P.tilemA,
-                                                                  ctr + 1);
+        int hper_sm = 0;
+        TSG_TRY(resident_ctas(ctx, TSG_OCC_HYPER, k_step3_hyper, SPA_THREADS, (int)sizeof(HypSmem), &hper_sm));
+        k_step3_hyper<<<ctx->num_sms * hper_sm, SPA_THREADS, sizeof(HypSmem), ctx->stream>>>(
+            P, d_kind, RANGED ? row0 : 0, RANGED ? row1 : P.tilemA, &ctr[TSG_CTR_REST]);
         TSG_LAUNCH_CHECK();
     }
-    k_step3_spa<FLAT, RANGED, BLK><<<grid, SPA_THREADS, smem, ctx->stream>>>(P, d_kind, !hyper_apart, row0, row1, ctr);
+    k_step3_spa<FLAT, RANGED, BLK><<<ctx->num_sms * per_sm, SPA_THREADS, smem, ctx->stream>>>(
+        P, d_kind, !hyper_apart, row0, row1, &ctr[TSG_CTR_STEP3]);
     TSG_LAUNCH_CHECK();
-    tsg_release(ctx, ctr);
     return TSG_OK;
 }
 
@@ -640,26 +651,21 @@ static int launch_step3_stg(tsg_context *ctx, const ProdView &P0, const int *d_k
 {
     ProdView P = P0;
     P.status = ctx->d_status;
-    unsigned *ctr = nullptr, grid = 0;
+    unsigned *ctr = ctx->d_ctl->ctr;
     int *left = nullptr;
-    const int smem = (int)sizeof(StgSmem);
-    TSG_CUDA(cudaFuncSetAttribute(k_step3_stg<RANGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    int per_sm = 0;
-    TSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step3_stg<RANGED>, STG_THREADS, smem));
-    if (per_sm < 1)
-        return tsg_set_error(TSG_ERR_CUDA, "the staged numeric step does not fit an SM");
-    TSG_TRY(tsg_alloc(ctx, &ctr, 2));
+    const int smem = (int)sizeof(StgSmem), rsmem = (int)sizeof(SpaSmem);
+    int per_sm = 0, rest_per_sm = 0;
+    TSG_TRY(resident_ctas(ctx, TSG_OCC_STG + (RANGED ? 1 : 0), k_step3_stg<RANGED>, STG_THREADS, smem, &per_sm));
+    TSG_TRY(resident_ctas(ctx, TSG_OCC_REST + (RANGED ? 1 : 0), k_step3_rest<RANGED>, SPA_THREADS, rsmem, &rest_per_sm));
+    TSG_TRY(clear_counters(ctx, row0, TSG_CTR_STEP3, 2));
     TSG_TRY(tsg_alloc(ctx, &left, (size_t)P.tilemA + 1));
-    TSG_CUDA(cudaMemsetAsync(ctr, 0, 2 * sizeof(unsigned), ctx->stream));
     TSG_CUDA(cudaMemsetAsync(left, 0, ((size_t)P.tilemA + 1) * sizeof(int), ctx->stream));
-    k_step3_stg<RANGED><<<ctx->num_sms * per_sm, STG_THREADS, smem, ctx->stream>>>(P, d_kind, row0, row1, ctr, left,
-                                                                                 ctx->d_status);
+    k_step3_stg<RANGED><<<ctx->num_sms * per_sm, STG_THREADS, smem, ctx->stream>>>(P, d_kind, row0, row1,
+                                                                                 &ctr[TSG_CTR_STEP3], left, ctx->d_status);
     TSG_LAUNCH_CHECK();
-    const int rsmem = (int)sizeof(SpaSmem);
-    TSG_TRY(spa_grid(ctx, k_step3_rest<RANGED>, rsmem, &grid));
-    k_step3_rest<RANGED><<<grid, SPA_THREADS, rsmem, ctx->stream>>>(P, d_kind, left, row0, row1, ctr + 1);
+    k_step3_rest<RANGED><<<ctx->num_sms * rest_per_sm, SPA_THREADS, rsmem, ctx->stream>>>(P, d_kind, left, row0, row1,
+                                                                                       &ctr[TSG_CTR_REST]);
     TSG_LAUNCH_CHECK();
-    tsg_release(ctx, ctr);
     tsg_release(ctx, left);
     return TSG_OK;
 }
@@ -736,8 +742,6 @@ static int launch_step3(tsg_context *ctx, const ProdView &P, const tsg_tiled *A,
 // What steps 1-2 leave for step 3 and the statistics.
 struct SpgemmRun
 {
-    unsigned long long *d_pairs;
-    int *d_bins;
     int *d_wide; // row kinds of the fused pass, or null
     StepOneBits bits; // step 1's bitmaps, until the emit pass has read them
     WinScratch win;
@@ -763,10 +767,9 @@ static int spgemm_structure(tsg_context *ctx, const tsg_tiled *A, const tsg_tile
         TSG_CUDA(cudaEventRecord(ctx->ev[0], st));
 
     // step 1: structure
-    TSG_TRY(tsg_alloc(ctx, &R.d_pairs, 1));
-    TSG_TRY(tsg_alloc(ctx, &R.d_bins, 4));
-    TSG_CUDA(cudaMemsetAsync(R.d_pairs, 0, sizeof(unsigned long long), st));
-    TSG_CUDA(cudaMemsetAsync(R.d_bins, 0, 4 * sizeof(int), st));
+    unsigned long long *d_pairs = &ctx->d_ctl->pairs;
+    int *d_bins = ctx->d_ctl->bins;
+    TSG_CUDA(cudaMemsetAsync(ctx->d_ctl, 0, offsetof(TsgControl, status), st));
     TSG_TRY(tsg_alloc(ctx, &C->tile_ptr, (size_t)tilem + 1));
     long long numC = 0;
     if (tilem > 0)
@@ -780,9 +783,9 @@ static int spgemm_structure(tsg_context *ctx, const tsg_tiled *A, const tsg_tile
             TSG_TRY(tsg_alloc(ctx, &R.bits.span, (size_t)tilem));
         }
         if (step1_by_cta(A, B))
-            k_step1_cta<<<tilem, S1C_THREADS, 0, st>>>(P, C->tile_ptr, R.d_pairs, R.bits);
+            k_step1_cta<<<tilem, S1C_THREADS, 0, st>>>(P, C->tile_ptr, d_pairs, R.bits);
         else
-            k_step1<false><<<tsg_blocks(tilem, S1_WARPS), S1_WARPS * 32, 0, st>>>(P, C->tile_ptr, R.d_pairs, R.bits);
+            k_step1<false><<<tsg_blocks(tilem, S1_WARPS), S1_WARPS * 32, 0, st>>>(P, C->tile_ptr, d_pairs, R.bits);
         TSG_LAUNCH_CHECK();
         TSG_TRY(tsg_scan_counts(ctx, C->tile_ptr, C->tile_ptr, tilem, &numC));
     }
@@ -804,7 +807,7 @@ static int spgemm_structure(tsg_context *ctx, const tsg_tiled *A, const tsg_tile
         {
             TSG_TRY(tsg_alloc(ctx, &R.d_wide, (size_t)tilem + 3 + 2 * wide_units(tilem, A->nnz)));
             TSG_CUDA(cudaMemsetAsync(R.d_wide + tilem, 0, 2 * sizeof(int), st));
-            k_step12<<<tsg_blocks(tilem, 8), 256, 0, st>>>(P, R.bits, R.d_wide, R.d_bins);
+            k_step12<<<tsg_blocks(tilem, 8), 256, 0, st>>>(P, R.bits, R.d_wide, d_bins);
             TSG_LAUNCH_CHECK();
         }
         else
@@ -823,14 +826,14 @@ static int spgemm_structure(tsg_context *ctx, const tsg_tiled *A, const tsg_tile
     {
         ProdView P = make_view(A, B, C);
         if (fused && P.B_rptr)
-            TSG_TRY(launch_step2_wide(ctx, P, R.d_wide, R.d_bins));
+            TSG_TRY(launch_step2_wide(ctx, P, R.d_wide, d_bins));
         else if (fused)
         {
-            k_step2_wide<<<tsg_blocks(numC * 16, 256), 256, 0, st>>>(P, R.d_wide, R.d_bins);
+            k_step2_wide<<<tsg_blocks(numC * 16, 256), 256, 0, st>>>(P, R.d_wide, d_bins);
             TSG_LAUNCH_CHECK();
         }
         else
-            TSG_TRY(launch_step2(ctx, P, R.d_bins));
+            TSG_TRY(launch_step2(ctx, P, d_bins));
         TSG_TRY(tsg_scan_counts(ctx, C->tile_nnz, C->tile_nnz, numC, &nnzC));
     }
     else
@@ -853,26 +856,18 @@ static int spgemm_finish(tsg_context *ctx, SpgemmRun &R, tsg_spgemm_info *info)
     cudaStream_t st = ctx->stream;
     tsg_release(ctx, R.d_wide);
     win_release(ctx, R.win);
-    {
-        const int dev = tsg_take_device_status(ctx);
-        if (dev != TSG_OK)
-        {
-            tsg_release(ctx, R.d_pairs);
-            tsg_release(ctx, R.d_bins);
-            return dev;
-        }
-    }
+    // the counters and the error word in one read-back
+    TsgControl *h = (TsgControl *)ctx->h_pinned;
+    TSG_CUDA(cudaMemcpyAsync(h, ctx->d_ctl, sizeof(TsgControl), cudaMemcpyDeviceToHost, st));
+    TSG_CUDA(cudaStreamSynchronize(st));
+    TSG_TRY(tsg_check_device_status(ctx, h->status));
     if (info)
     {
         memset(info, 0, sizeof(*info));
         info->numtile_C = R.numC;
         info->nnz_C = R.nnzC;
-        long long *h = ctx->h_pinned;
-        TSG_CUDA(cudaMemcpyAsync(h, R.d_pairs, sizeof(long long), cudaMemcpyDeviceToHost, st));
-        TSG_CUDA(cudaMemcpyAsync(h + 1, R.d_bins, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
-        TSG_CUDA(cudaStreamSynchronize(st));
-        info->tile_pairs = h[0];
-        memcpy(info->bins, h + 1, 4 * sizeof(int));
+        info->tile_pairs = (long long)h->pairs;
+        memcpy(info->bins, h->bins, sizeof(info->bins));
         info->step3_kernel = R.nnzC > 0 ? ctx->last_step3 : TSG_STEP3_NONE;
         if (ctx->timing)
         {
@@ -882,8 +877,6 @@ static int spgemm_finish(tsg_context *ctx, SpgemmRun &R, tsg_spgemm_info *info)
             info->ms_total = ev_ms(ctx->ev[0], ctx->ev[3]);
         }
     }
-    tsg_release(ctx, R.d_pairs);
-    tsg_release(ctx, R.d_bins);
     return TSG_OK;
 }
 
@@ -1006,8 +999,6 @@ int tsg_spgemm_to_host(tsg_context *ctx, const tsg_tiled *A, const tsg_tiled *B,
     {
         tsg_release(ctx, R.d_wide);
         win_release(ctx, R.win);
-        tsg_release(ctx, R.d_pairs);
-        tsg_release(ctx, R.d_bins);
     }
     tsg_tiled_free(ctx, &C);
     if (status == TSG_OK)

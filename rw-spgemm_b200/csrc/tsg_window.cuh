@@ -73,7 +73,7 @@ struct WinPlan
     int *btab;          // [B row][blocks + 1]: B's row pointer at every block of 1 << bits columns
     int *ctab;          // [tile row][windows + 1]: first C tile of every window
     int *heavy;         // heavy rows of A
-    unsigned *count;    // [0] claims, [1] heavy rows
+    unsigned *claim, *nheavy; // counters: claims, heavy rows
     int blocks, bits, windows;
     int mA;
 };
