@@ -186,3 +186,49 @@ def test_rcm_levels_with_large_buckets(tsg, ctx, oracle, leaves):
     got = tsg.order(ctx, "rcm", n, n, torch.from_numpy(rp).to(d), torch.from_numpy(ci).to(d)).cpu().numpy()
     mat = (n, n, rp, ci, np.ones(ci.size))
     assert np.array_equal(got, oracle.order("rcm", mat))
+
+
+@pytest.mark.parametrize("longest", [1, 33, 255, 256, 257, 900])
+def test_permute_rows_up_to_and_past_the_ranked_length(tsg, ctx, longest):
+    """Rows ranked in place (up to 256 entries) and whole-matrix sorts, repeated
+    columns among them, against a stable numpy sort (copies: tolerance 0)."""
+    import torch
+    rng = np.random.default_rng(longest)
+    m, n = 70, 1200
+    counts = rng.integers(0, longest + 1, m)
+    counts[11] = longest
+    rp = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    ci = np.concatenate([np.sort(rng.choice(n, c, replace=bool(i % 3 == 0))) for i, c in enumerate(counts)]).astype(np.int32)
+    v = rng.uniform(-1, 1, ci.size)
+    row_old, col_new = rng.permutation(m).astype(np.int32), rng.permutation(n).astype(np.int32)
+    d = torch.device("cuda", torch.cuda.current_device())
+    got = tsg.permute_csr(ctx, m, n, *[torch.from_numpy(x).to(d) for x in (rp, ci, v, row_old, col_new)])
+    rows = [np.arange(rp[o], rp[o + 1]) for o in row_old]
+    at = np.concatenate([e[np.argsort(col_new[ci[e]], kind="stable")] for e in rows])
+    np.testing.assert_array_equal(got[0].cpu().numpy(), np.concatenate([[0], np.cumsum(counts[row_old])]))
+    np.testing.assert_array_equal(got[1].cpu().numpy(), col_new[ci[at]])
+    np.testing.assert_array_equal(got[2].cpu().numpy(), v[at])
+
+
+def test_rcm_of_patterns_that_are_not_symmetric_or_not_in_order(tsg, ctx, oracle, gen):
+    """One entry without its mirror, a repeated one, rows out of order: the
+    pattern is symmetrised by a sort, as before."""
+    import torch
+    d = torch.device("cuda", torch.cuda.current_device())
+    m, n, rp, ci, v = gen.laplacian_2d(20)
+    want = oracle.order("rcm", (m, n, rp, ci, v))
+
+    def rcm(rp, ci):
+        return tsg.order(ctx, "rcm", m, n, torch.from_numpy(rp).to(d), torch.from_numpy(ci).to(d)).cpu().numpy()
+
+    assert np.array_equal(rcm(rp, ci), want)
+    at = int(np.flatnonzero(ci[rp[50]:rp[51]] > 50)[0] + rp[50])  # drop (50, j): (j, 50) stays
+    rp1 = rp.copy()
+    rp1[51:] -= 1
+    assert np.array_equal(rcm(rp1, np.delete(ci, at)), want)
+    rp2 = rp.copy()
+    rp2[51:] += 1
+    assert np.array_equal(rcm(rp2, np.insert(ci, at, ci[at])), want)
+    ci3 = ci.copy()
+    ci3[rp[50]:rp[51]] = ci3[rp[50]:rp[51]][::-1]
+    assert np.array_equal(rcm(rp, ci3), want)
