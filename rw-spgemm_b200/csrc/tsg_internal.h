@@ -20,6 +20,7 @@ struct TsgControl
     unsigned long long pairs; // matched tile pairs
     int bins[4];              // C tiles by size
     unsigned ctr[8];          // work counters: TSG_CTR_*
+    int input;                // what the check of a CSR input found
     int status;               // error word kernels set (TSG_ERR_TIMEOUT, TSG_ERR_OVERFLOW); outlives the clearing
 };
 enum
@@ -158,8 +159,13 @@ int tsg_sort_pairs_u64(tsg_context *ctx, unsigned long long *keys, int *vals, lo
 int tsg_sort_pairs_u32(tsg_context *ctx, unsigned int *keys, int *vals, long long n, int end_bit);
 
 // Validates a device CSR (ptr monotone, rowptr[0]=0, rowptr[m]=nnz, columns
-// in range and strictly increasing per row).
-int tsg_check_csr(tsg_context *ctx, int m, int n, int nnz, const int *rowptr, const int *colidx);
+// in range and strictly increasing per row).  The first queues the check, for
+// kernels that follow to look at *d_err (nonzero: the arrays are not to be
+// used); the second gives its result once the stream has been waited for
+// (m > 0).
+int tsg_check_csr_start(tsg_context *ctx, int m, int n, int nnz, const int *rowptr, const int *colidx,
+                        const int **d_err);
+int tsg_check_csr_result(tsg_context *ctx, int n);
 
 // Column view of a row-major tiled matrix (csc_tile_ptr / rowidx / pos).
 int tsg_build_csc_view(tsg_context *ctx, tsg_tiled *mat);

@@ -255,20 +255,25 @@ __global__ void k_check_csr(int m, int n, int nnz, const int *__restrict__ rowpt
         atomicOr(err, bad);
 }
 
-int tsg_check_csr(tsg_context *ctx, int m, int n, int nnz, const int *rowptr, const int *colidx)
+int tsg_check_csr_start(tsg_context *ctx, int m, int n, int nnz, const int *rowptr, const int *colidx,
+                        const int **d_err)
 {
+    *d_err = &ctx->d_ctl->input;
     if (m < 0 || n < 0 || nnz < 0)
         return tsg_set_error(TSG_ERR_INVALID, "negative CSR dimension");
     if (m == 0)
         return nnz == 0 ? TSG_OK : tsg_set_error(TSG_ERR_INPUT, "m = 0 with nnz > 0");
-    int *d_err;
-    TSG_TRY(tsg_alloc(ctx, &d_err, 1));
-    TSG_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), ctx->stream));
-    k_check_csr<<<tsg_blocks((long long)m * 32, 256), 256, 0, ctx->stream>>>(m, n, nnz, rowptr, colidx, d_err);
+    int *err = &ctx->d_ctl->input;
+    TSG_CUDA(cudaMemsetAsync(err, 0, sizeof(int), ctx->stream));
+    k_check_csr<<<tsg_blocks((long long)m * 32, 256), 256, 0, ctx->stream>>>(m, n, nnz, rowptr, colidx, err);
     TSG_LAUNCH_CHECK();
-    long long err;
-    TSG_TRY(tsg_read_int(ctx, d_err, &err));
-    tsg_release(ctx, d_err);
+    TSG_CUDA(cudaMemcpyAsync(ctx->h_pinned + 62, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    return TSG_OK;
+}
+
+int tsg_check_csr_result(tsg_context *ctx, int n)
+{
+    const int err = *(const int *)(ctx->h_pinned + 62);
     if (err & 1)
         return tsg_set_error(TSG_ERR_INPUT, "CSR row pointer malformed (rowptr[0]=0, monotone, rowptr[m]=nnz)");
     if (err & 2)

@@ -29,17 +29,24 @@ SHAPES = [
     ("some", 16 * 2400 + 5, 300, 3),   # narrow and many, 128 threads
     ("each", 33, 16 * 900, 400),       # wide, several steps of 512 tiles, most tiles empty in a row
     ("each", 16, 16 * 1100000, 80000), # one tile row of > 2048 steps: the 16-bit sums are emptied
+    ("each", 48, 900, 31), ("each", 48, 900, 32), ("each", 37, 16 * 1024 + 5, 33),  # around 512 entries a tile row
+    ("full", 37, 700, 0),              # a CTA each, full tiles, ragged
 ]
 
 
 @pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "-".join(map(str, s)))
 @pytest.mark.parametrize("off_boundary", [False, True])
-def test_tiles_and_back(tsg, ctx, shape, off_boundary):
+def test_tiles_and_back(tsg, ctx, oracle, shape, off_boundary):
     import torch
     m, n, rp, ci, v = _matrix(*shape)
     d = torch.device("cuda", torch.cuda.current_device())
     dev = [torch.from_numpy(x).to(d) for x in (rp, ci, v)]
     T = tsg.csr_to_tiled(ctx, m, n, *dev, 0)
+    if n < 100000:  # and the tiles are the oracle's
+        tiles, want = T.download(), oracle.csr2tile_row_major((m, n, rp, ci, v))
+        for k in ("tile_ptr", "tile_columnidx", "tile_rowidx", "tile_nnz", "tile_csr_Ptr", "tile_csr_Value", "mask"):
+            np.testing.assert_array_equal(tiles[k], want[k], err_msg=k)
+        np.testing.assert_array_equal(tiles["tile_csr_Col"], want["tile_csr_Col"] & 15)
     if off_boundary:
         raw = torch.empty(16 * T.numtile + 1, dtype=torch.uint8, device=d)
         tiles = T.download()
@@ -52,3 +59,27 @@ def test_tiles_and_back(tsg, ctx, shape, off_boundary):
     assert np.array_equal(got[0], rp)
     assert np.array_equal(got[1], ci)
     assert np.array_equal(got[2].view(np.uint64), v.view(np.uint64))
+
+
+@pytest.mark.parametrize("m,n,tiles", [(16 * 300, 70, 255), (16 * 300, 70, 256), (16 * 300, 70, 257),
+                                       (16 * 5000 + 3, 40, 4000), (16 * 262150, 33, 262149)])
+def test_column_view_of_columns_short_and_long(tsg, ctx, m, n, tiles):
+    """Tile columns around the 256 tiles that a warp ranks, past them, and over
+    more tile rows (262,144) than one bitmap pass: tiles ascending by row in
+    every column."""
+    import torch
+    rng = np.random.default_rng(tiles)
+    rows = 16 * np.sort(rng.choice((m + 15) // 16, tiles, replace=False)).astype(np.int64)  # one entry a tile row
+    cols = rng.integers(0, 16, tiles)
+    extra = rng.integers(0, m, 2000)
+    key = np.unique(np.concatenate([rows * n + cols, extra * n + rng.integers(16, n, 2000)]))
+    r, ci = key // n, (key % n).astype(np.int32)
+    rp = np.searchsorted(r, np.arange(m + 1)).astype(np.int32)
+    d = torch.device("cuda", torch.cuda.current_device())
+    T = tsg.csr_to_tiled(ctx, m, n, *[torch.from_numpy(x).to(d) for x in (rp, ci, rng.uniform(-1, 1, ci.size))],
+                         tsg.TSG_TILED_CSC_VIEW)
+    got = T.download(colmajor=True)
+    T.free()
+    tc = np.unique((ci // 16).astype(np.int64) * ((m + 15) // 16) + r // 16)  # (tile column, tile row)
+    np.testing.assert_array_equal(got["csc_tile_rowidx"], tc % ((m + 15) // 16))
+    np.testing.assert_array_equal(np.diff(got["csc_tile_ptr"]), np.bincount(tc // ((m + 15) // 16), minlength=(n + 15) // 16))
