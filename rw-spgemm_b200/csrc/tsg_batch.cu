@@ -86,7 +86,7 @@ struct tsg_batch
 // step 3 by windows: products with this many scalar products per (row,
 // window), up to this many words of table each and in all
 #define BATCH_WIN_MIN 16
-#define BATCH_WIN_WORDS (1LL << 22)
+#define BATCH_WIN_WORDS (1LL << 22) // (btab; wtab holds two words a window beside it)
 #define BATCH_WIN_TOTAL (1LL << 26)
 // a barrier wait gives up after this floor plus a share of the batch's work
 // (a B200 does well over 10 scalar products per ns, so the bound is loose)
@@ -649,7 +649,8 @@ __global__ void __launch_bounds__(256)
     {
         const BatchProd &b = prods[find_product(boff, count, w)];
         if (batch_win_on(b, dense))
-            win_btab_row((int)(w - boff[&b - prods]), b.P.B_rptr, b.P.B_rcol, b.Q.blocks, b.Q.bits, b.Q.btab);
+            win_btab_row((int)(w - boff[&b - prods]), b.P.B_rptr, b.P.B_rcol, b.Q.blocks, b.Q.bits, b.Q.btab,
+                         b.Q.windows, b.Q.wtab);
     }
     for (long long g = gt; g < toff[count]; g += nt)
     {
@@ -1065,8 +1066,8 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
                 h.Q.blocks = blocks;
                 h.Q.mA = A[p].m;
                 hparts += parts;
-                tables[p] = (blocks + 1LL) * B[p].m + centries;
-                words += (blocks + 1LL) * B[p].m;
+                tables[p] = (blocks + 1LL) * B[p].m + centries + 2 * windows * B[p].m + 1;
+                words += (blocks + 1LL + 2 * windows) * B[p].m;
                 b->wins++;
             }
             const long long add[4] = {B[p].m, centries, A[p].m, claims};
@@ -1171,7 +1172,8 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
             h.Q.A_rptr = P.A_rptr;
             h.Q.A_rcol = P.A_rcol;
             h.Q.A_rval = P.A_rval;
-            h.Q.btab = b->win_tables + table_words;
+            h.Q.wtab = (int2 *)(b->win_tables + ((table_words + 1) & ~1LL));
+            h.Q.btab = (int *)(h.Q.wtab + (long long)h.Q.windows * P.mB);
             h.Q.ctab = h.Q.btab + (h.Q.blocks + 1LL) * P.mB;
             table_words += tables[p];
         }

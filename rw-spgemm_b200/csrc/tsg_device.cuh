@@ -466,6 +466,36 @@ __device__ __forceinline__ int step12_row(const ProdView &P, int i, S12Smem &sm,
 // ---------------------------------------------------------------------------
 // Helpers
 // ---------------------------------------------------------------------------
+// The lane's place among the valid lanes with its key, lowest lane first, and
+// the largest place of the warp.  Lanes that share a key are found through a
+// byte per (hashed) key that every lane writes and reads back: 7 cycles of an
+// SM's issue where __match_any_sync, a loop over the distinct keys on this
+// architecture, takes 70 for 32 of them (measured).  Only columns that are
+// met twice cost more, a ballot each.  tag: TSG_TAGS bytes of this warp; the
+// caller has a warp barrier between calls.
+#define TSG_TAGS 256
+__device__ __forceinline__ int same_key_rank(int key, bool valid, unsigned char *tag, int lane, int &last)
+{
+    if (valid)
+        tag[key & (TSG_TAGS - 1)] = (unsigned char)lane;
+    __syncwarp();
+    unsigned left = __ballot_sync(TSG_FULL_MASK, valid && tag[key & (TSG_TAGS - 1)] != lane);
+    last = 0;
+    if (!left)
+        return 0;
+    int rank = 0;
+    do
+    {
+        const int k = __shfl_sync(TSG_FULL_MASK, key, __ffs(left) - 1);
+        const unsigned same = __ballot_sync(TSG_FULL_MASK, valid && key == k);
+        if (valid && key == k)
+            rank = __popc(same & ((1u << lane) - 1u));
+        last = max(last, __popc(same) - 1);
+        left &= ~same;
+    } while (left);
+    return rank;
+}
+
 __device__ __forceinline__ int lower_bound_int(const int *__restrict__ a, int n, int key)
 {
     int lo = 0;
@@ -996,6 +1026,7 @@ struct SpaSmem
     unsigned cm[TSG_BS * SPA_CMS];  // [row][tile]: (entries of the row in earlier tiles << 16) | C row mask
     int rstart[TSG_BS];             // first accumulator slot of each row's private, column-sorted run
     unsigned short map[SPA_WIN];    // tile column - J0 -> segment tile, 0xFFFF none
+    unsigned char tag[SPA_WARPS][TSG_TAGS];
     union
     {
         SpaStage stage[SPA_WARPS]; // per-row form
@@ -1047,8 +1078,8 @@ __host__ __device__ __forceinline__ bool spa_wants_flat(int browB, long long num
 // bl (cut to the segment) and values a, in k order -- to the row's
 // accumulator run.  FLATTEN: when their B rows hold fewer than SPA_FLAT
 // entries on average, the products are flattened, 32 per batch in k order;
-// lanes of a batch meeting the same slot are folded by the lowest of them in
-// lane order and batches follow one another behind warp barriers, so every
+// lanes of a batch meeting the same slot add one after another in lane order
+// and batches follow one another behind warp barriers, so every
 // slot still sums its products in k order.  Otherwise (or !FLATTEN) a warp
 // pass per entry streams its B row, the next row's first 32 entries
 // prefetched.  bl is overwritten.
@@ -1086,37 +1117,25 @@ __device__ __forceinline__ void spa_apply_stage(const ProdView &P, SpaSmem &S, c
             for (int ib = 0; ib < ni; ib += 32)
             {
                 const int item = ib + lane;
-                int pos = -1 - lane; // distinct keys for lanes without a slot
+                int pos = -1;
                 double prod = 0.0;
                 if (item < ni)
                 {
                     while (ent + 1 < ne && bl[ent + 1].y <= item)
                         ent++;
                     const int bi = bl[ent].x + item;
-                    const int p = spa_slot(S, cmr, rs, J0, J1, full, P.B_rcol[bi]);
-                    if (p >= 0)
-                    {
-                        pos = p;
+                    pos = spa_slot(S, cmr, rs, J0, J1, full, P.B_rcol[bi]);
+                    if (pos >= 0)
                         prod = __dmul_rn(a[ent], P.B_rval[bi]);
-                    }
                 }
-                const unsigned grp = __match_any_sync(TSG_FULL_MASK, pos);
-                const bool lead = pos >= 0 && lane == __ffs(grp) - 1;
-                const int rounds = __reduce_max_sync(TSG_FULL_MASK, pos >= 0 ? __popc(grp) : 0);
-                double acc = lead ? S.acc[pos] : 0.0;
-                unsigned gl = grp;
-                for (int q = 0; q < rounds; q++)
+                int last;
+                const int rank = same_key_rank(pos, pos >= 0, S.tag[threadIdx.x >> 5], lane, last);
+                for (int q = 0; q <= last; q++)
                 {
-                    const double v = __shfl_sync(TSG_FULL_MASK, prod, gl ? __ffs(gl) - 1 : lane);
-                    if (gl)
-                    {
-                        acc = __dadd_rn(acc, v);
-                        gl &= gl - 1;
-                    }
+                    if (pos >= 0 && rank == q)
+                        S.acc[pos] = __dadd_rn(S.acc[pos], prod);
+                    __syncwarp();
                 }
-                if (lead)
-                    S.acc[pos] = acc;
-                __syncwarp();
             }
             return;
         }
@@ -1210,7 +1229,13 @@ __device__ __forceinline__ void spa_coop_apply(const ProdView &P, SpaSmem &S, in
                 if (len == 0)
                     row = TSG_BS; // adds nothing to this segment
             }
-            const unsigned peers = __match_any_sync(TSG_FULL_MASK, row);
+            unsigned peers = TSG_FULL_MASK; // lanes with this lane's row (0..16)
+#pragma unroll
+            for (int b = 0; b < 5; b++)
+            {
+                const unsigned one = __ballot_sync(TSG_FULL_MASK, (row >> b) & 1);
+                peers &= (row >> b) & 1 ? one : ~one;
+            }
             er[h] = row;
             eb[h] = b0;
             el[h] = len;
@@ -1446,7 +1471,7 @@ __device__ __forceinline__ void step3_spa_segment(const ProdView &P, SpaSmem &S,
 //    of the row mask left of the column -- in global memory.  Warp r takes
 //    row r's products in generation order (A's entries in column order, each
 //    with its B row), 32 at a time; lanes of one batch that meet the same
-//    slot are summed by the lowest of them in lane order, and batches follow
+//    slot add one after another in lane order, and batches follow
 //    one another behind warp barriers, so every C entry sums its products in
 //    k order, each product rounded before the add, as the reference does.
 // The tile column -> tile map covers HYP_WIN tile columns.  Rows are marked
@@ -1462,7 +1487,7 @@ struct HypStage
     int2 bl[SPA_STAGE];      // B row: first entry, length
     int off[SPA_STAGE + 1];  // first product of each staged entry
     double a[SPA_STAGE];     // A value of each staged entry
-    double prod[32];         // products of the current batch, by lane
+    unsigned char tag[TSG_TAGS];
 };
 
 struct HypSmem
@@ -1636,7 +1661,7 @@ __device__ __forceinline__ void step3_hyper_row(const ProdView &P, HypSmem &S, i
         const int s1 = hyp_window(P, S, s0, re, W0);
         const int nw = s1 - s0;
         hyp_walk(P, G, I, r, lane, [&](bool valid, int e, int bi) {
-            int pos = -1 - lane; // distinct keys for lanes without a slot
+            int pos = -1;
             double prod = 0.0;
             if (valid)
             {
@@ -1659,22 +1684,14 @@ __device__ __forceinline__ void step3_hyper_row(const ProdView &P, HypSmem &S, i
                     }
                 }
             }
-            const unsigned grp = __match_any_sync(TSG_FULL_MASK, pos);
-            G.prod[lane] = prod;
-            __syncwarp();
-            if (pos >= 0 && lane == __ffs(grp) - 1)
+            int last;
+            const int rank = same_key_rank(pos, pos >= 0, G.tag, lane, last);
+            for (int q = 0; q <= last; q++)
             {
-                double acc = __ldcg(P.C_Val + pos);
-                unsigned gl = grp;
-                while (gl)
-                {
-                    const int l = __ffs(gl) - 1;
-                    gl &= gl - 1;
-                    acc = __dadd_rn(acc, G.prod[l]);
-                }
-                P.C_Val[pos] = acc;
+                if (pos >= 0 && rank == q)
+                    P.C_Val[pos] = __dadd_rn(__ldcg(P.C_Val + pos), prod);
+                __syncwarp();
             }
-            __syncwarp();
         });
         s0 = s1;
     }

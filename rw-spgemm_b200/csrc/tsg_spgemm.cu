@@ -319,11 +319,12 @@ __global__ void __launch_bounds__(SPA_THREADS, 2) k_step3_rest(ProdView P, const
 
 // The windows' tables of one product (a warp per row of B)
 __global__ void __launch_bounds__(256) k_win_btab(int m, const int *__restrict__ rptr, const int *__restrict__ rcol,
-                                                  int blocks, int bits, int *__restrict__ tab)
+                                                  int blocks, int bits, int *__restrict__ tab, int windows,
+                                                  int2 *__restrict__ wtab)
 {
     const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (w < m)
-        win_btab_row((int)w, rptr, rcol, blocks, bits, tab);
+        win_btab_row((int)w, rptr, rcol, blocks, bits, tab, windows, wtab);
 }
 
 // ctab, and the list of heavy rows
@@ -562,6 +563,7 @@ static bool win_shape(const ProdView &P, long long nnzC, WinPlan &Q)
 
 static void win_release(tsg_context *ctx, WinScratch &W)
 {
+    tsg_release(ctx, W.Q.wtab);
     tsg_release(ctx, W.Q.btab);
     tsg_release(ctx, W.Q.ctab);
     tsg_release(ctx, W.rptr);
@@ -579,6 +581,9 @@ static int win_prepare(tsg_context *ctx, const ProdView &P, const tsg_tiled *A, 
     cudaStream_t st = ctx->stream;
     WinPlan &Q = W.Q;
     TSG_TRY(tsg_alloc(ctx, &Q.btab, (size_t)P.mB * (Q.blocks + 1)));
+    Q.wtab = nullptr;
+    if ((long long)P.mB * Q.windows <= WIN_TABLE_WORDS / 2)
+        TSG_TRY(tsg_alloc(ctx, &Q.wtab, (size_t)P.mB * Q.windows));
     TSG_TRY(tsg_alloc(ctx, &Q.ctab, (size_t)P.tilemA * (Q.windows + 1)));
     TSG_TRY(tsg_alloc(ctx, &Q.heavy, (size_t)P.mA));
     Q.claim = &ctx->d_ctl->ctr[TSG_CTR_STEP3];
@@ -596,7 +601,7 @@ static int win_prepare(tsg_context *ctx, const ProdView &P, const tsg_tiled *A, 
         Q.A_rcol = W.rcol;
         Q.A_rval = W.rval;
     }
-    k_win_btab<<<tsg_blocks((long long)P.mB * 32, 256), 256, 0, st>>>(P.mB, P.B_rptr, P.B_rcol, Q.blocks, Q.bits, Q.btab);
+    k_win_btab<<<tsg_blocks((long long)P.mB * 32, 256), 256, 0, st>>>(P.mB, P.B_rptr, P.B_rcol, Q.blocks, Q.bits, Q.btab, Q.windows, Q.wtab);
     TSG_LAUNCH_CHECK();
     k_win_ctab<<<tsg_blocks(std::max((long long)P.mA, (long long)P.tilemA * (Q.windows + 1)), 256), 256, 0, st>>>(P, Q);
     TSG_LAUNCH_CHECK();

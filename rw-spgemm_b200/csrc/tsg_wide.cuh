@@ -235,8 +235,10 @@ __device__ __forceinline__ int wide_word(int w, int h)
 // would finish last.  Units are listed as (row, part | parts << 16) in
 // wide_units_of, wide[tilemA] of them; wide[tilemA + 1] counts the C tiles of
 // hypersparse rows.
-#define WIDE_SPLIT 2048
-#define WIDE_PARTS 16
+#ifndef WIDE_SPLIT
+#define WIDE_SPLIT 1024
+#endif
+#define WIDE_PARTS 32
 
 static inline size_t wide_units(int tilem, int nnzA)
 {
@@ -277,10 +279,19 @@ __device__ __forceinline__ void step2_wide_row(const ProdView &P, WideSmem<NT> &
     const bool whole = parts == 1;
     if (!whole)
     {
-        // the C tiles of this part of the row's columns
-        const int first = P.C_col[rs], width = (P.C_col[re - 1] - first + parts) / parts, n = re - rs;
-        rb = rs + lower_bound_int(P.C_col + rs, n, first + part * width);
-        re = rs + lower_bound_int(P.C_col + rs, n, first + (part + 1) * width);
+        // the C tiles of this part of the row's columns: parts of about equal
+        // counts of B's tiles (a skewed graph's first columns hold most of its
+        // entries)
+        const int first = P.C_col[rs], last = P.C_col[re - 1] + 1, n = re - rs;
+        const int *bc = P.B_cptr + first;
+        const long long all = bc[last - first] - bc[0];
+        auto bound = [&](int q) {
+            const int c = q == 0 ? 0 : q == parts ? last - first
+                                                  : lower_bound_int(bc, last - first, bc[0] + (int)(all * q / parts));
+            return rs + lower_bound_int(P.C_col + rs, n, first + c);
+        };
+        rb = bound(part);
+        re = bound(part + 1);
     }
     const bool ptr16 = (reinterpret_cast<unsigned long long>(P.A_Ptr) & 15ULL) == 0;
     const int pa_beg = P.A_ptr[I], pa_end = P.A_ptr[I + 1];

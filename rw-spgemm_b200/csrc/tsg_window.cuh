@@ -53,6 +53,9 @@
 #define WIN_PARTS (WIN_COLS / WIN_PART)
 #define WIN_WARPS 8
 #define WIN_THREADS (WIN_WARPS * 32)
+#ifndef WIN_ROUNDS
+#define WIN_ROUNDS 3 // entries after the first that a batch adds entry by entry
+#endif
 // a product takes the windows when C holds at least this many values per (row, window)
 #define WIN_MIN_VALUES 8
 #define WIN_TABLE_WORDS (1LL << 26) // most words of the table of B's row pointers
@@ -62,7 +65,9 @@ struct WinTask
     double acc[WIN_COLS]; // all zero between tasks
     double a[32];         // staged A entries of the group: value,
     int b[32];            // B index less the entry's first product,
-    int end[32];          // and the product after its last
+    int end[32];          // and the product after its last; at the end of a task, per C tile of
+    int pre[32];          // the row: its column and mask, its value offset and its first value
+    unsigned char tag[TSG_TAGS];
 };
 
 // Where the windows of a product lie.
@@ -70,6 +75,7 @@ struct WinPlan
 {
     const int *A_rptr, *A_rcol; // A's row view
     const double *A_rval;
+    int2 *wtab;         // [B row][windows]: the row's entries in the window (null: B too large, btab)
     int *btab;          // [B row][blocks + 1]: B's row pointer at every block of 1 << bits columns
     int *ctab;          // [tile row][windows + 1]: first C tile of every window
     int *heavy;         // heavy rows of A
@@ -80,7 +86,8 @@ struct WinPlan
 
 // B row w's entry offset at every block boundary, by a warp
 __device__ __forceinline__ void win_btab_row(int w, const int *__restrict__ rptr, const int *__restrict__ rcol,
-                                             int blocks, int bits, int *__restrict__ tab)
+                                             int blocks, int bits, int *__restrict__ tab, int windows,
+                                             int2 *__restrict__ wtab)
 {
     const int lane = threadIdx.x & 31;
     const int e0 = rptr[w], e1 = rptr[w + 1];
@@ -92,6 +99,18 @@ __device__ __forceinline__ void win_btab_row(int w, const int *__restrict__ rptr
         const int cur = e < e1 ? rcol[e] >> bits : blocks;
         for (int b = prev + 1; b <= cur; b++)
             t[b] = e;
+        if (wtab)
+        {
+            // ... and ends the window before it, which the entry before it was in
+            int2 *u = wtab + (long long)w * windows;
+            const int pw = e > e0 ? rcol[e - 1] / WIN_COLS : -1, cw = e < e1 ? rcol[e] / WIN_COLS : windows;
+            if (pw >= 0 && cw > pw)
+                u[pw].y = e;
+            for (int b = pw + 1; b < cw; b++)
+                u[b] = make_int2(e, e);
+            if (cw > pw && cw < windows)
+                u[cw].x = e;
+        }
     }
 }
 
@@ -125,10 +144,19 @@ struct WinEntry
 };
 
 // entry x (none when x >= e1), column k of A
+// (WHOLE: [c0, c1) is a window)
+template <bool WHOLE>
 __device__ __forceinline__ WinEntry win_entry(const ProdView &P, const WinPlan &Q, int x, int e1, int k, int c0, int c1)
 {
     WinEntry E = {0.0, 0, 0};
-    if (x < e1)
+    if (x < e1 && WHOLE && Q.wtab)
+    {
+        const int2 t = Q.wtab[(long long)k * Q.windows + c0 / WIN_COLS];
+        E.a = Q.A_rval[x];
+        E.b0 = t.x;
+        E.len = t.y - t.x;
+    }
+    else if (x < e1)
     {
         const int *t = Q.btab + (long long)k * (Q.blocks + 1);
         const int blk = c0 >> Q.bits;
@@ -145,6 +173,23 @@ __device__ __forceinline__ WinEntry win_entry(const ProdView &P, const WinPlan &
     return E;
 }
 
+// column of the n-th entry (from 0) of a row mask, bit 15 - c for column c
+__device__ __forceinline__ int win_nth_column(unsigned mask, int n)
+{
+    int c = 0;
+#pragma unroll
+    for (int half = 8; half > 0; half >>= 1)
+    {
+        // the mask's upper `half` of its lowest 2 * half bits
+        const int t = __popc(mask >> half);
+        const bool low = n >= t;
+        n -= low ? t : 0;
+        c += low ? half : 0;
+        mask = low ? mask & ((1u << half) - 1u) : mask >> half;
+    }
+    return c;
+}
+
 // C row r of tile row I, columns [c0, c1); its A entries are [e0, e1) of the
 // row view (E: this lane's of the first 32, loaded by the caller), its C tiles
 // [t0, t1), at most 64.  All lanes of the warp call it.
@@ -153,6 +198,7 @@ __device__ __forceinline__ WinEntry win_entry(const ProdView &P, const WinPlan &
 // chain of them after another: the entries' columns two groups of 32 ahead,
 // their parts of B one group, B's entries two batches, the row's masks and
 // value offsets from the start.
+template <bool WHOLE>
 __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, WinTask &S, int I, int r, int c0, int c1,
                                          int e0, int e1, WinEntry E, int t0, int t1, int lane)
 {
@@ -176,7 +222,7 @@ __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, Wi
     int k = e0 + 32 + lane < e1 ? Q.A_rcol[e0 + 32 + lane] : 0;
     for (int g = e0; g < e1; g += 32)
     {
-        const WinEntry nxt = win_entry(P, Q, g + 32 + lane, e1, k, c0, c1);
+        const WinEntry nxt = win_entry<WHOLE>(P, Q, g + 32 + lane, e1, k, c0, c1);
         k = g + 64 + lane < e1 ? Q.A_rcol[g + 64 + lane] : 0;
         const int len = E.len;
         const unsigned full = __ballot_sync(TSG_FULL_MASK, len > 0);
@@ -205,10 +251,10 @@ __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, Wi
         }
         __syncwarp();
         // batches of 32 products, the next two batches' loads issued before
-        // this pair's additions.  one: the batch holds one entry's products
+        // this pair's additions.  rel: the lane's entry, from the batch's first
         int cur = 0, until = S.end[0]; // the entry at the last loaded batch's end, and its end
-        auto load = [&](int ib, bool &one, int &col, double &p) {
-            one = true;
+        auto load = [&](int ib, int &rel, int &col, double &p) {
+            rel = 0;
             col = -1;
             p = 0.0;
             if (ib >= total)
@@ -222,8 +268,8 @@ __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, Wi
                 const bool mine = len > 0 && pre > ib && pre < ib + 32;
                 const unsigned starts = __reduce_or_sync(TSG_FULL_MASK, mine ? 1u << (pre - ib) : 0u);
                 const int before = __popc(__ballot_sync(TSG_FULL_MASK, len > 0 && pre <= ib)) - 1;
-                e = before + __popc(starts & upto);
-                one = starts == 0u;
+                rel = __popc(starts & upto);
+                e = before + rel;
                 cur = before + __popc(starts);
                 until = S.end[cur];
             }
@@ -234,35 +280,28 @@ __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, Wi
                 p = __dmul_rn(S.a[e], P.B_rval[bi]);
             }
         };
-        auto add = [&](bool one, int col, double p) {
-            if (one) // distinct columns
+        // products of one entry meet distinct columns; those of a few entries
+        // are added entry by entry, others in lane order where columns meet
+        auto add = [&](int rel, int col, double p) {
+            const int more = __reduce_max_sync(TSG_FULL_MASK, rel); // entries after the batch's first
+            int last = more, rank = rel;
+            if (more > WIN_ROUNDS)
+                rank = same_key_rank(col, col >= 0, S.tag, lane, last);
+            for (int q = 0; q <= last; q++)
             {
-                if (col >= 0)
+                if (col >= 0 && rank == q)
                     S.acc[col] = __dadd_rn(S.acc[col], p);
+                __syncwarp();
             }
-            else
-            {
-                const unsigned same = __match_any_sync(TSG_FULL_MASK, col);
-                const int rank = col >= 0 ? __popc(same & upto) - 1 : 0;
-                const int last = __reduce_max_sync(TSG_FULL_MASK, rank);
-                for (int q = 0; q <= last; q++)
-                {
-                    if (q)
-                        __syncwarp();
-                    if (col >= 0 && rank == q)
-                        S.acc[col] = __dadd_rn(S.acc[col], p);
-                }
-            }
-            __syncwarp();
         };
-        bool s0, s1;
+        int s0, s1;
         int col0, col1;
         double p0, p1;
         load(0, s0, col0, p0);
         load(32, s1, col1, p1);
         for (int ib = 0; ib < total; ib += 64)
         {
-            bool n0, n1;
+            int n0, n1;
             int ncol0, ncol1;
             double np0, np1;
             load(ib + 64, n0, ncol0, np0);
@@ -281,24 +320,80 @@ __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, Wi
     }
     if (!any)
         return;
+#ifndef WIN_OUT_LANE
+    // the row's values out, 32 tiles at a time, flattened over the lanes:
+    // consecutive lanes store consecutive values of a tile's row (a lane per
+    // tile would touch a line per value, and read a bank 32 ways)
 #pragma unroll
     for (int h = 0; h < 2; h++)
     {
-        unsigned m = base[h] >= 0 && base[h] < c1 - c0 ? mk[h] : 0u; // a heavy row's part holds some of the tiles
-        double *acc = S.acc + base[h];
-        int q = at[h];
-        while (m)
+        const unsigned m = base[h] >= 0 && base[h] < c1 - c0 ? mk[h] : 0u; // a heavy row's part holds some of the tiles
+        const int len = __popc(m);
+        const unsigned full = __ballot_sync(TSG_FULL_MASK, len > 0);
+        if (!full)
+            continue;
+        int incl = len;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1)
         {
-            const int bit = 31 - __clz(m);
-            m ^= 1u << bit;
-            P.C_Val[q] = acc[15 - bit];
-            acc[15 - bit] = 0.0;
-            P.C_Colb[q] = (unsigned char)(15 - bit);
-            q++;
+            const int o = __shfl_up_sync(TSG_FULL_MASK, incl, d);
+            if (lane >= d)
+                incl += o;
+        }
+        const int total = __shfl_sync(TSG_FULL_MASK, incl, 31);
+        const int pre = incl - len;
+        if (len > 0)
+        {
+            const int e = __popc(full & upto) - 1;
+            S.b[e] = base[h] << 16 | (int)m;
+            S.end[e] = at[h] - pre;
+            S.pre[e] = pre;
+        }
+        __syncwarp();
+        for (int ib = 0; ib < total; ib += 32)
+        {
+            const bool mine = len > 0 && pre > ib && pre < ib + 32;
+            const unsigned starts = __reduce_or_sync(TSG_FULL_MASK, mine ? 1u << (pre - ib) : 0u);
+            const int e = __popc(__ballot_sync(TSG_FULL_MASK, len > 0 && pre <= ib)) - 1 + __popc(starts & upto);
+            const int j = ib + lane;
+            if (j < total)
+            {
+                const int w = S.b[e];
+                const int c = win_nth_column((unsigned)w & 0xFFFFu, j - S.pre[e]);
+                double *acc = S.acc + (w >> 16) + c;
+                const int q = S.end[e] + j;
+                P.C_Val[q] = *acc;
+                *acc = 0.0;
+                P.C_Colb[q] = (unsigned char)c;
+            }
+        }
+        __syncwarp();
+    }
+}
+#else
+    // the row's values out, a lane per C tile of the row, each starting at a
+    // column of its own (all at once would read one bank)
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+    {
+        const unsigned m = base[h] >= 0 && base[h] < c1 - c0 ? mk[h] : 0u; // a heavy row's part holds some of the tiles
+        const int turn = lane & 15;
+        unsigned left = ((m << turn) | (m >> (16 - turn))) & 0xFFFFu;
+        double *acc = S.acc + base[h];
+        while (left)
+        {
+            const int bit = 31 - __clz(left);
+            left ^= 1u << bit;
+            const int c = 15 - ((bit - turn) & 15);
+            const int q = at[h] + __popc(m >> (16 - c));
+            P.C_Val[q] = acc[c];
+            acc[c] = 0.0;
+            P.C_Colb[q] = (unsigned char)c;
         }
     }
     __syncwarp();
 }
+#endif
 static_assert(WIN_TILES <= 64, "C tiles of a window");
 
 // columns [part * WIN_PART, ...) of heavy row `row`
@@ -308,7 +403,7 @@ __device__ __forceinline__ void win_claim_heavy(const ProdView &P, const WinPlan
     const int *ct = Q.ctab + (long long)(row / TSG_BS) * (Q.windows + 1) + part / WIN_PARTS;
     const int e0 = Q.A_rptr[row], e1 = Q.A_rptr[row + 1], c0 = part * WIN_PART, c1 = c0 + WIN_PART;
     const int k = e0 + lane < e1 ? Q.A_rcol[e0 + lane] : 0;
-    win_task(P, Q, S, row / TSG_BS, row % TSG_BS, c0, c1, e0, e1, win_entry(P, Q, e0 + lane, e1, k, c0, c1), ct[0],
+    win_task<false>(P, Q, S, row / TSG_BS, row % TSG_BS, c0, c1, e0, e1, win_entry<false>(P, Q, e0 + lane, e1, k, c0, c1), ct[0],
              ct[1], lane);
 }
 
@@ -335,15 +430,15 @@ __device__ __forceinline__ void win_claim_rows(const ProdView &P, const WinPlan 
     int k1 = col(0);
     int k2 = col(1);
     int e0 = __shfl_sync(TSG_FULL_MASK, e, 0), e1 = __shfl_sync(TSG_FULL_MASK, e, 1);
-    WinEntry E = win_entry(P, Q, e0 + lane, e1, k1, c0, c1);
+    WinEntry E = win_entry<true>(P, Q, e0 + lane, e1, k1, c0, c1);
 #pragma unroll 1
     for (int i = 0; i < WIN_ROWS; i++)
     {
         const int e2 = __shfl_sync(TSG_FULL_MASK, e, min(i + 2, WIN_ROWS));
-        const WinEntry nxt = win_entry(P, Q, e1 + lane, e2, k2, c0, c1);
+        const WinEntry nxt = win_entry<true>(P, Q, e1 + lane, e2, k2, c0, c1);
         k2 = col(i + 2);
         if (e0 < e1 && e1 - e0 < WIN_HEAVY)
-            win_task(P, Q, S, I, r0 + i, c0, c1, e0, e1, E, t0, t1, lane);
+            win_task<true>(P, Q, S, I, r0 + i, c0, c1, e0, e1, E, t0, t1, lane);
         e0 = e1;
         e1 = e2;
         E = nxt;

@@ -1,8 +1,8 @@
 """Products whose rows are uneven or wide -- step 1 by a CTA per tile row with
 its bitmaps kept, step 2 of wide rows in parts, step 3 by column windows --
 and the dense tile kernel, against the oracle at the sizes where each changes:
-window and table-block edges, heavy rows around WIN_HEAVY (512) entries, tile
-rows around one part (2,048 entries), columns past one pass of step 2 (98,304)
+window and table-block edges, heavy rows around WIN_HEAVY (256) entries, tile
+rows around one part (1,024 entries), columns past one pass of step 2 (98,304)
 and past what step 1 keeps (262,144) or holds at once (1,048,576), an A with
 no row view.  Values bit for bit: the order of the sums is the oracle's."""
 import numpy as np
@@ -60,10 +60,10 @@ def _case(name):
         n = int(name[4:])
         return _rows(70, 300, rng.integers(0, 60, 70), 1), _rows(300, n, rng.integers(0, min(n // 2, 26) + 1, 300), 2, hub=1)
     if name == "heavy":  # rows around WIN_HEAVY entries among light ones, every B row holding column 0
-        counts = [511, 0, 513, 3, 512, 40, 700, 1, 2, 5, 0, 514, 9, 9, 9, 9, 600, 4]
+        counts = [255, 0, 257, 3, 256, 40, 700, 1, 2, 5, 0, 258, 9, 9, 9, 9, 600, 4]
         return _rows(18, 1500, counts, 3), _rows(1500, 1300, rng.integers(0, 30, 1500), 4, hub=1)
-    if name == "parts":  # tile rows of about 1, 2 and 3 parts
-        counts = [127] * 16 + [128] * 16 + [129] * 16 + [257] * 16 + [3] * 5
+    if name == "parts":  # tile rows of 1, 2 and 5 parts
+        counts = [63] * 16 + [64] * 16 + [65] * 16 + [257] * 16 + [3] * 5
         return _rows(69, 4000, counts, 5), _rows(4000, 5000, rng.integers(0, 12, 4000), 6)
     if name == "coarse table":  # 70,000 x 300,000: a table block wider than a heavy row's part; step 2 in passes
         return _rows(40, 70000, [200] * 39 + [600], 8), _rows(70000, 300000, np.full(70000, 20), 9)
