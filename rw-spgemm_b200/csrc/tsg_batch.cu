@@ -76,6 +76,7 @@ struct tsg_batch
     long long *d_s1off, *d_winoff;
     int4 *d_wlist, *d_hlist; // wide units of step 2; heavy rows' parts of the window step 3
     int *win_tables;
+    int split;   // A entries of a unit of step 2's wide rows
     int wins;    // products that take the windows
     int gridw;   // persistent grid of k_batch_win
     int dense;                  // SPA schedule: values per C tile from which a product takes the tile kernel
@@ -305,7 +306,7 @@ __device__ __forceinline__ unsigned long long gtimer() { return batch_clock_ns()
 template <int SCHED, int W, int CAP, int NT>
 __global__ void __launch_bounds__(NT)
     k_batch(BatchProd *prods, int count, const long long *__restrict__ rowoff, const long long *__restrict__ s1off,
-            int4 *wlist, long long *itemoff, unsigned *bar, int *err, int *bins)
+            int4 *wlist, int split, long long *itemoff, unsigned *bar, int *err, int *bins)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
     __shared__ long long s_tmp[NT / 32 + 1];
@@ -443,7 +444,7 @@ __global__ void __launch_bounds__(NT)
                     prods[p].wide[i] = kind;
                     if (SCHED == 3 && kind)
                     {
-                        const int parts = wide_parts(prods[p].P, i);
+                        const int parts = wide_parts(prods[p].P, i, split);
                         int4 *at = wlist + atomicAdd(&bar[6], (unsigned)parts);
                         for (int q = 0; q < parts; q++)
                             at[q] = make_int4(p, i, q | parts << 16, 0);
@@ -862,8 +863,8 @@ extern "C" int tsg_product_bounds(tsg_context *ctx, const tsg_tiled *A, const ts
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-typedef void (*batch_kernel_t)(BatchProd *, int, const long long *, const long long *, int4 *, long long *, unsigned *,
-                               int *, int *);
+typedef void (*batch_kernel_t)(BatchProd *, int, const long long *, const long long *, int4 *, int, long long *,
+                               unsigned *, int *, int *);
 
 // Kernel, dynamic shared memory and block size of a batch schedule.
 static batch_kernel_t pick_kernel(const tsg_batch_params &p, size_t *smem, int *threads)
@@ -928,7 +929,7 @@ static int record_run(tsg_batch *b, cudaStream_t st)
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     TSG_CUDA(cudaLaunchKernelEx(&cfg, kern, b->d_prod, b->count, (const long long *)b->d_rowoff,
-                                (const long long *)b->d_s1off, b->d_wlist, b->d_itemoff,
+                                (const long long *)b->d_s1off, b->d_wlist, b->split, b->d_itemoff,
                                 b->d_bar, b->d_err, b->d_bins));
     if (b->wins)
     {
@@ -1029,14 +1030,17 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
     b->s1off.assign(2 * ((size_t)count + 1), 0);
     b->winoff.assign(4 * ((size_t)count + 1), 0);
     std::vector<long long> tables(count, 0); // words of each product's window tables
-    long long wunits = 0, hparts = 0, words = 0;
+    long long wunits = 0, hparts = 0, words = 0, entries = 0;
+    for (int p = 0; p < count; p++)
+        entries += A[p].nnz;
+    b->split = wide_split(entries, ctx->num_sms);
     for (int p = 0; p < count; p++)
     {
         const long long prods = v_prods[p], capT = v_tiles[p];
         const bool cta = step1_by_cta(&A[p], &B[p]);
         b->s1off[p + 1] = b->s1off[p] + (cta ? A[p].tilem : 0);
         b->s1off[count + 2 + p] = b->s1off[count + 1 + p] + (cta ? 0 : A[p].tilem);
-        wunits += (long long)wide_units(A[p].tilem, A[p].nnz);
+        wunits += (long long)wide_units(A[p].tilem, A[p].nnz, b->split);
         total_prods += prods;
         long long capN = prods < 256 * capT ? prods : 256 * capT;
         if (capN > 2147483647LL || capT > 2147483647LL / 16)

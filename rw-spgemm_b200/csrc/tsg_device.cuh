@@ -66,11 +66,18 @@ struct StepOneBits
     unsigned *words;
     int2 *span;
     int stride;
+    int *widest; // raised to the widest window, in tile columns (or null)
 };
+
+__device__ __forceinline__ void step1_widest(const StepOneBits &K, int lo, int hi)
+{
+    if (K.widest && hi - lo + 1 > *(volatile int *)K.widest)
+        atomicMax(K.widest, hi - lo + 1);
+}
 
 template <bool EMIT>
 __device__ __forceinline__ int step1_row(const ProdView &P, int i, unsigned int *bm, int lane,
-                                         unsigned long long *pairs, const StepOneBits &K = {nullptr, nullptr, 0})
+                                         unsigned long long *pairs, const StepOneBits &K = {nullptr, nullptr, 0, nullptr})
 {
     const int a0 = P.A_ptr[i], a1 = P.A_ptr[i + 1];
     int lo = INT_MAX, hi = -1;
@@ -171,8 +178,12 @@ __device__ __forceinline__ int step1_row(const ProdView &P, int i, unsigned int 
             }
             __syncwarp();
             const bool keep = !EMIT && K.words && hi - (lo & ~31) < S1_WORDS * 32 && nw <= K.stride;
-            if (!EMIT && K.words && lane == 0)
-                K.span[i] = make_int2(c0, keep ? nw : 0);
+            if (!EMIT && lane == 0)
+            {
+                step1_widest(K, lo, hi);
+                if (K.words)
+                    K.span[i] = make_int2(c0, keep ? nw : 0);
+            }
             for (int wb = 0; wb < nw; wb += 32)
             {
                 const int w = wb + lane;
@@ -260,7 +271,9 @@ __device__ __forceinline__ int nnz_bin(int total);
 #define S12_MAXT 128
 // tile pairs from which a row is wide whatever its tiles: the warp takes them
 // 32 at a time (1,500 x 1,300 random, 3,775 pairs and 980 products a tile row)
+#ifndef S12_MAXP
 #define S12_MAXP 1024
+#endif
 
 struct S12Smem
 {
@@ -270,7 +283,7 @@ struct S12Smem
 };
 
 __device__ __forceinline__ int step12_row(const ProdView &P, int i, S12Smem &sm, int lane, int *s_bins,
-                                          const StepOneBits &K = {nullptr, nullptr, 0})
+                                          const StepOneBits &K = {nullptr, nullptr, 0, nullptr})
 {
     const int a0 = P.A_ptr[i], a1 = P.A_ptr[i + 1];
     const int cbase = P.C_ptr[i];

@@ -19,6 +19,7 @@ struct TsgControl
 {
     unsigned long long pairs; // matched tile pairs
     int bins[4];              // C tiles by size
+    int widest;               // widest column window of a C tile row, in tile columns
     unsigned ctr[8];          // work counters: TSG_CTR_*
     int input;                // what the check of a CSR input found
     int status;               // error word kernels set (TSG_ERR_TIMEOUT, TSG_ERR_OVERFLOW); outlives the clearing

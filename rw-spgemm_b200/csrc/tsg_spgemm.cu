@@ -12,6 +12,7 @@
 // per run of C tiles in one tile row, tile-level Gustavson, no intersection).
 #include <limits.h>
 #include <stddef.h>
+#include <stdlib.h>
 
 #include <algorithm>
 
@@ -75,7 +76,7 @@ __global__ void __launch_bounds__(S1_WARPS * 32) k_step1_total(ProdView P, unsig
 // fused step-1 emit + step 2 (warp per A tile row).  Wide rows are emitted
 // alone and left to the wide-row step 2: wide[i] says 1, or 2 when the row is
 // hypersparse (0 otherwise), and wide[tilemA ...] lists their units (wide_list).
-__global__ void __launch_bounds__(256) k_step12(ProdView P, StepOneBits K, int *__restrict__ wide,
+__global__ void __launch_bounds__(256) k_step12(ProdView P, StepOneBits K, int split, int *__restrict__ wide,
                                                 int *__restrict__ bins)
 {
     __shared__ S12Smem sm[8];
@@ -102,7 +103,7 @@ __global__ void __launch_bounds__(256) k_step12(ProdView P, StepOneBits K, int *
         {
             wide[i] = kind;
             if (kind)
-                wide_list(P, i, kind, wide);
+                wide_list(P, i, kind, split, wide);
         }
     }
     __syncthreads();
@@ -526,13 +527,14 @@ static int launch_step2_cta(tsg_context *ctx, const ProdView &P, int span, const
     return TSG_OK;
 }
 
-static int launch_step2_wide(tsg_context *ctx, const ProdView &P, const int *d_wide, int *d_bins)
+static int launch_step2_wide(tsg_context *ctx, const ProdView &P, int widest, const int *d_wide, int *d_bins)
 {
-    // the columns of C, or as many as a CTA's shared memory holds; narrow C
-    // leaves room for four CTAs of 512 threads on an SM (8,192 columns: 0.073
-    // ms, 0.083 with 1,024 threads; 16,384 columns of R-MAT 14: 0.45 and 0.38)
-    const int span = std::min(P.tilenB, WIDE_SPAN);
-    return span <= 512 ? launch_step2_cta<512>(ctx, P, span, d_wide, d_bins)
+    // the widest row of C, or as many columns as a CTA's shared memory holds
+    const int span = std::max(1, std::min(widest, WIDE_SPAN));
+    static int force = getenv("S2_NT") ? atoi(getenv("S2_NT")) : 0;
+    const int nt = force ? force : span <= 512 ? 512 : 1024;
+    return nt == 256 ? launch_step2_cta<256>(ctx, P, span, d_wide, d_bins)
+           : nt == 512 ? launch_step2_cta<512>(ctx, P, span, d_wide, d_bins)
                        : launch_step2_cta<1024>(ctx, P, span, d_wide, d_bins);
 }
 
@@ -748,6 +750,7 @@ static int launch_step3(tsg_context *ctx, const ProdView &P, const tsg_tiled *A,
 struct SpgemmRun
 {
     int *d_wide; // row kinds of the fused pass, or null
+    int widest;       // widest window of a C tile row, in tile columns
     StepOneBits bits; // step 1's bitmaps, until the emit pass has read them
     WinScratch win;
     long long numC, nnzC;
@@ -787,12 +790,15 @@ static int spgemm_structure(tsg_context *ctx, const tsg_tiled *A, const tsg_tile
             TSG_TRY(tsg_alloc(ctx, &R.bits.words, (size_t)tilem * stride));
             TSG_TRY(tsg_alloc(ctx, &R.bits.span, (size_t)tilem));
         }
+        R.bits.widest = &ctx->d_ctl->widest;
         if (step1_by_cta(A, B))
             k_step1_cta<<<tilem, S1C_THREADS, 0, st>>>(P, C->tile_ptr, d_pairs, R.bits);
         else
             k_step1<false><<<tsg_blocks(tilem, S1_WARPS), S1_WARPS * 32, 0, st>>>(P, C->tile_ptr, d_pairs, R.bits);
         TSG_LAUNCH_CHECK();
+        TSG_CUDA(cudaMemcpyAsync(ctx->h_pinned + 2, &ctx->d_ctl->widest, sizeof(int), cudaMemcpyDeviceToHost, st));
         TSG_TRY(tsg_scan_counts(ctx, C->tile_ptr, C->tile_ptr, tilem, &numC));
+        R.widest = *(const int *)(ctx->h_pinned + 2);
     }
     else
         TSG_CUDA(cudaMemsetAsync(C->tile_ptr, 0, sizeof(int), st));
@@ -810,14 +816,15 @@ static int spgemm_structure(tsg_context *ctx, const tsg_tiled *A, const tsg_tile
         ProdView P = make_view(A, B, C);
         if (fused)
         {
-            TSG_TRY(tsg_alloc(ctx, &R.d_wide, (size_t)tilem + 3 + 2 * wide_units(tilem, A->nnz)));
+            const int split = wide_split(A->nnz, ctx->num_sms);
+            TSG_TRY(tsg_alloc(ctx, &R.d_wide, (size_t)tilem + 3 + 2 * wide_units(tilem, A->nnz, split)));
             TSG_CUDA(cudaMemsetAsync(R.d_wide + tilem, 0, 2 * sizeof(int), st));
-            k_step12<<<tsg_blocks(tilem, 8), 256, 0, st>>>(P, R.bits, R.d_wide, d_bins);
+            k_step12<<<tsg_blocks(tilem, 8), 256, 0, st>>>(P, R.bits, split, R.d_wide, d_bins);
             TSG_LAUNCH_CHECK();
         }
         else
         {
-            k_step1<true><<<tsg_blocks(tilem, S1_WARPS), S1_WARPS * 32, 0, st>>>(P, nullptr, nullptr, StepOneBits{nullptr, nullptr, 0});
+            k_step1<true><<<tsg_blocks(tilem, S1_WARPS), S1_WARPS * 32, 0, st>>>(P, nullptr, nullptr, StepOneBits{nullptr, nullptr, 0, nullptr});
             TSG_LAUNCH_CHECK();
         }
     }
@@ -831,7 +838,7 @@ static int spgemm_structure(tsg_context *ctx, const tsg_tiled *A, const tsg_tile
     {
         ProdView P = make_view(A, B, C);
         if (fused && P.B_rptr)
-            TSG_TRY(launch_step2_wide(ctx, P, R.d_wide, d_bins));
+            TSG_TRY(launch_step2_wide(ctx, P, R.widest, R.d_wide, d_bins));
         else if (fused)
         {
             k_step2_wide<<<tsg_blocks(numC * 16, 256), 256, 0, st>>>(P, R.d_wide, d_bins);

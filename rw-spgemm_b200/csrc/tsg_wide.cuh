@@ -122,6 +122,8 @@ __device__ __forceinline__ int step1_row_cta(const ProdView &P, int i, S1cSmem<N
     hi = S.hi;
     if (hi < 0)
         return 0;
+    if (tid == 0)
+        step1_widest(K, lo, hi);
     const bool once = hi - (lo & ~31) < S1C_WORDS * 32;
     for (int c0 = lo & ~31; c0 <= hi; c0 += S1C_WORDS * 32)
     {
@@ -230,25 +232,32 @@ __device__ __forceinline__ int wide_word(int w, int h)
     return w * 8 + (h ^ ((w >> 2) & 7));
 }
 
-// A wide row is one unit of work, or one for every WIDE_SPLIT entries of A in
-// it, each a part of its columns: the CTA that took an R-MAT hub row whole
-// would finish last.  Units are listed as (row, part | parts << 16) in
+// A wide row is one unit of work, or one for every `split` entries of A in it,
+// each a part of its columns: the CTA that took an R-MAT hub row whole would
+// finish last.  Every part stages all the row's entries, so rows are split
+// only once they are half an SM's share of A (wide_split): R-MAT 14,
+// step 2: 0.38 ms unsplit, 0.295 split; a band times random rows 0.062 unsplit,
+// 0.103 split from 1,024 entries on.
+// Units are listed as (row, part | parts << 16) in
 // wide_units_of, wide[tilemA] of them; wide[tilemA + 1] counts the C tiles of
 // hypersparse rows.
-#ifndef WIDE_SPLIT
-#define WIDE_SPLIT 1024
-#endif
 #define WIDE_PARTS 32
 
-static inline size_t wide_units(int tilem, int nnzA)
+static inline int wide_split(long long nnzA, int num_sms)
 {
-    return (size_t)tilem + nnzA / WIDE_SPLIT;
+    const long long share = nnzA / (2 * num_sms);
+    return share < 1024 ? 1024 : (int)share;
 }
 
-__device__ __forceinline__ int wide_parts(const ProdView &P, int i)
+static inline size_t wide_units(int tilem, int nnzA, int split)
+{
+    return (size_t)tilem + nnzA / split;
+}
+
+__device__ __forceinline__ int wide_parts(const ProdView &P, int i, int split)
 {
     const int entries = P.A_tnnz[P.A_ptr[i + 1]] - P.A_tnnz[P.A_ptr[i]];
-    return min(WIDE_PARTS, 1 + entries / WIDE_SPLIT);
+    return min(WIDE_PARTS, 1 + entries / split);
 }
 
 __device__ __forceinline__ const int2 *wide_units_of(const ProdView &P, const int *wide)
@@ -256,9 +265,9 @@ __device__ __forceinline__ const int2 *wide_units_of(const ProdView &P, const in
     return reinterpret_cast<const int2 *>(wide + ((P.tilemA + 3) & ~1));
 }
 
-__device__ __forceinline__ void wide_list(const ProdView &P, int i, int kind, int *wide)
+__device__ __forceinline__ void wide_list(const ProdView &P, int i, int kind, int split, int *wide)
 {
-    const int parts = wide_parts(P, i);
+    const int parts = wide_parts(P, i, split);
     int2 *at = const_cast<int2 *>(wide_units_of(P, wide)) + atomicAdd(&wide[P.tilemA], parts);
     for (int q = 0; q < parts; q++)
         at[q] = make_int2(i, q | parts << 16);

@@ -53,8 +53,11 @@
 #define WIN_PARTS (WIN_COLS / WIN_PART)
 #define WIN_WARPS 8
 #define WIN_THREADS (WIN_WARPS * 32)
+#ifndef WIN_FEW
+#define WIN_FEW 3 // values of a tile's row up to which a lane stores its tile's own
+#endif
 #ifndef WIN_ROUNDS
-#define WIN_ROUNDS 3 // entries after the first that a batch adds entry by entry
+#define WIN_ROUNDS 6 // entries after the first that a batch adds entry by entry
 #endif
 // a product takes the windows when C holds at least this many values per (row, window)
 #define WIN_MIN_VALUES 8
@@ -250,8 +253,8 @@ __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, Wi
             S.end[at] = incl;
         }
         __syncwarp();
-        // batches of 32 products, the next two batches' loads issued before
-        // this pair's additions.  rel: the lane's entry, from the batch's first
+        // batches of 32 products, a batch's loads issued two batches before its
+        // additions.  rel: the lane's entry, from the batch's first
         int cur = 0, until = S.end[0]; // the entry at the last loaded batch's end, and its end
         auto load = [&](int ib, int &rel, int &col, double &p) {
             rel = 0;
@@ -282,39 +285,37 @@ __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, Wi
         };
         // products of one entry meet distinct columns; those of a few entries
         // are added entry by entry, others in lane order where columns meet
+        // products of one entry meet distinct columns; those of a few entries
+        // are added entry by entry, others in lane order where columns meet
         auto add = [&](int rel, int col, double p) {
-            const int more = __reduce_max_sync(TSG_FULL_MASK, rel); // entries after the batch's first
-            int last = more, rank = rel;
-            if (more > WIN_ROUNDS)
+            int last = rel >> 8, rank = rel & 0xFF;
+            if (last > WIN_ROUNDS)
                 rank = same_key_rank(col, col >= 0, S.tag, lane, last);
-            for (int q = 0; q <= last; q++)
+            rank = col >= 0 ? rank : -1;
+            double *acc = S.acc + max(col, 0);
+            if (rank == 0)
+                *acc = __dadd_rn(*acc, p);
+            __syncwarp();
+            for (int q = 1; q <= last; q++)
             {
-                if (col >= 0 && rank == q)
-                    S.acc[col] = __dadd_rn(S.acc[col], p);
+                if (rank == q)
+                    *acc = __dadd_rn(*acc, p);
                 __syncwarp();
             }
         };
-        int s0, s1;
-        int col0, col1;
+        int s0, s1, col0, col1;
         double p0, p1;
         load(0, s0, col0, p0);
         load(32, s1, col1, p1);
         for (int ib = 0; ib < total; ib += 64)
         {
-            int n0, n1;
-            int ncol0, ncol1;
-            double np0, np1;
-            load(ib + 64, n0, ncol0, np0);
-            load(ib + 96, n1, ncol1, np1);
             add(s0, col0, p0);
+            load(ib + 64, s0, col0, p0);
             if (ib + 32 < total)
+            {
                 add(s1, col1, p1);
-            s0 = n0;
-            s1 = n1;
-            col0 = ncol0;
-            col1 = ncol1;
-            p0 = np0;
-            p1 = np1;
+                load(ib + 96, s1, col1, p1);
+            }
         }
         E = nxt;
     }
@@ -332,6 +333,20 @@ __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, Wi
         const unsigned full = __ballot_sync(TSG_FULL_MASK, len > 0);
         if (!full)
             continue;
+        if (__reduce_max_sync(TSG_FULL_MASK, len) <= WIN_FEW)
+        {
+            double *acc = S.acc + base[h];
+            int q = at[h];
+            for (unsigned left = m; left;)
+            {
+                const int bit = 31 - __clz(left);
+                left ^= 1u << bit;
+                P.C_Val[q] = acc[15 - bit];
+                acc[15 - bit] = 0.0;
+                P.C_Colb[q++] = (unsigned char)(15 - bit);
+            }
+            continue;
+        }
         int incl = len;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1)
