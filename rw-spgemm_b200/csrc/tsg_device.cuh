@@ -262,8 +262,7 @@ __device__ __forceinline__ int nnz_bin(int total);
 // one pass of S12_WORDS words and the row has at most S12_MAXT C tiles, the
 // bitmap's word-prefix popcounts give each B tile's C slot in O(1), and the
 // warp ORs the 16x16 boolean products of every (A tile, B tile) pair of the
-// row into per-slot row masks in shared memory (two B tiles at a time, one
-// per half-warp, lane = row), then writes masks, row offsets and tile counts.
+// row into per-slot row masks in shared memory, then writes masks, row offsets and tile counts.
 // No intersection is searched.  Returns 1 if the row was completed, 0 if it
 // needs the tile-schedule step 2 (C columns are emitted either way).
 // ---------------------------------------------------------------------------
@@ -280,6 +279,7 @@ struct S12Smem
     unsigned bm[S12_WORDS];
     unsigned short pre[S12_WORDS];
     unsigned short acc[16][S12_MAXT + 2]; // [row][slot], padded: both access forms spread over banks
+    unsigned b[8][32];                    // [two rows][lane]: the lane's B tile
 };
 
 __device__ __forceinline__ int step12_row(const ProdView &P, int i, S12Smem &sm, int lane, int *s_bins,
@@ -374,82 +374,98 @@ __device__ __forceinline__ int step12_row(const ProdView &P, int i, S12Smem &sm,
     for (int q = half; q < ntiles; q += 2)
         sm.acc[r][q] = 0;
     __syncwarp();
-    // OR the boolean products of all (A tile, B tile) pairs of the row: unit
-    // (row r, B tile) ORs the B rows its A row meets -- one 16-bit load per
-    // set bit of a sparse A row, two 16-byte loads for a dense one
-    for (int pa = a0; pa < a1; pa++)
+    // OR the boolean products of all (A tile, B tile) pairs of the row: A's
+    // tiles one after another, a lane per B tile, the next A tile's loads
+    // issued before this one's products.  A's row masks are the same for all
+    // lanes, so the walk over its entries does not diverge; the B row of an
+    // entry is a word of the lane's B tile in shared memory, two rows to a
+    // word, lanes in distinct banks (read where B holds its masks, 32 bytes
+    // apart, it took a load of five to eight wavefronts; selected from
+    // registers, twice the instructions).  64^3 stencil, 22 tiles of A and of
+    // B a row: a 64^3 grid's matrix 0.40 -> 0.385 ms.
+    for (int g = a0; g < a1; g += 32)
     {
-        const int k = P.A_col[pa];
-        const int b0 = P.B_ptr[k], b1 = P.B_ptr[k + 1];
-        if (b1 - b0 >= 8)
+        const int cnt = min(32, a1 - g);
+        int gb = 0, gl = 0;
+        if (lane < cnt)
         {
-            // lane per B tile, its 16 row masks in registers.  A sparse A tile
-            // is taken column by column: the rows with an entry in column k
-            // (a ballot over the row masks, the same for all lanes) get B's
-            // row k; a tile with many entries row by row, all of B at once
-            const unsigned am = lane < TSG_BS ? P.A_mask[(long long)pa * TSG_BS + lane] : 0u;
-            const bool adense = __reduce_add_sync(TSG_FULL_MASK, __popc(am)) > 64;
-            unsigned rows[TSG_BS]; // sparse: rows of A with an entry in column k
-#pragma unroll
-            for (int k = 0; k < TSG_BS; k++)
-                rows[k] = adense ? __shfl_sync(TSG_FULL_MASK, am, k)
-                                 : __ballot_sync(TSG_FULL_MASK, (am >> (15 - k)) & 1u);
-            for (int pb = b0 + lane; pb < b1; pb += 32)
+            const int k = P.A_col[g + lane];
+            gb = P.B_ptr[k];
+            gl = P.B_ptr[k + 1] - gb;
+        }
+        unsigned nam = 0u;
+        int nj = c0;
+        uint4 nq0 = make_uint4(0u, 0u, 0u, 0u), nq1 = nq0;
+        auto fetch = [&](int t) {
+            const int tb = __shfl_sync(TSG_FULL_MASK, gb, t), tl = __shfl_sync(TSG_FULL_MASK, gl, t);
+            nam = lane < TSG_BS ? P.A_mask[(long long)(g + t) * TSG_BS + lane] : 0u;
+            if (lane < tl)
             {
-                const int j = P.B_col[pb] - c0;
-                const int slot = sm.pre[j >> 5] + __popc(sm.bm[j >> 5] & ((1u << (j & 31)) - 1u));
-                const uint4 *mb = reinterpret_cast<const uint4 *>(P.B_mask + (long long)pb * TSG_BS);
-                const uint4 q0 = __ldg(mb), q1 = __ldg(mb + 1);
-                if (adense)
+                nj = P.B_col[tb + lane];
+                const uint4 *mb = reinterpret_cast<const uint4 *>(P.B_mask + (long long)(tb + lane) * TSG_BS);
+                nq0 = __ldg(mb);
+                nq1 = __ldg(mb + 1);
+            }
+        };
+        fetch(0);
+        for (int t = 0; t < cnt; t++)
+        {
+            const int b0 = __shfl_sync(TSG_FULL_MASK, gb, t), len = __shfl_sync(TSG_FULL_MASK, gl, t);
+            const unsigned am = nam;
+            int j = nj - c0;
+            uint4 q0 = nq0, q1 = nq1;
+            if (t + 1 < cnt)
+                fetch(t + 1);
+            const bool adense = __reduce_add_sync(TSG_FULL_MASK, __popc(am)) > 64;
+            for (int p0 = 0; p0 < len; p0 += 32)
+            {
+                const bool mine = p0 + lane < len;
+                if (p0 && mine) // B tile rows of more than a warp
+                {
+                    j = P.B_col[b0 + p0 + lane] - c0;
+                    const uint4 *mb = reinterpret_cast<const uint4 *>(P.B_mask + (long long)(b0 + p0 + lane) * TSG_BS);
+                    q0 = __ldg(mb);
+                    q1 = __ldg(mb + 1);
+                }
+                const int slot = mine ? sm.pre[j >> 5] + __popc(sm.bm[j >> 5] & ((1u << (j & 31)) - 1u)) : 0;
+                if (adense) // all of B's rows at once
                 {
 #pragma unroll
-                    for (int rr = 0; rr < TSG_BS; rr++)
-                        if (rows[rr])
-                            sm.acc[rr][slot] |= (unsigned short)bool_row(rows[rr], q0, q1);
+                    for (int r = 0; r < TSG_BS; r++)
+                    {
+                        const unsigned mrow = __shfl_sync(TSG_FULL_MASK, am, r);
+                        if (mrow && mine)
+                            sm.acc[r][slot] |= (unsigned short)bool_row(mrow, q0, q1);
+                    }
                     continue;
                 }
-                const unsigned w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+                sm.b[0][lane] = q0.x;
+                sm.b[1][lane] = q0.y;
+                sm.b[2][lane] = q0.z;
+                sm.b[3][lane] = q0.w;
+                sm.b[4][lane] = q1.x;
+                sm.b[5][lane] = q1.y;
+                sm.b[6][lane] = q1.z;
+                sm.b[7][lane] = q1.w;
 #pragma unroll
-                for (int k = 0; k < TSG_BS; k++)
+                for (int r = 0; r < TSG_BS; r++)
                 {
-                    const unsigned brow = (k & 1) ? (w[k >> 1] >> 16) : (w[k >> 1] & 0xFFFFu);
-                    if (brow)
-                        for (unsigned left = rows[k]; left; left &= left - 1)
-                            sm.acc[__ffs(left) - 1][slot] |= (unsigned short)brow;
+                    unsigned left = __shfl_sync(TSG_FULL_MASK, am, r);
+                    if (!left)
+                        continue;
+                    unsigned acc = 0;
+                    do
+                    {
+                        const int k = __clz(left) - 16; // highest bit first: column ascending
+                        left &= 0x7FFFu >> k;
+                        acc |= sm.b[k >> 1][lane] >> ((k & 1) * 16);
+                    } while (left);
+                    if (mine)
+                        sm.acc[r][slot] |= (unsigned short)acc;
                 }
             }
             __syncwarp();
-            continue;
         }
-        const unsigned ma = P.A_mask[(long long)pa * TSG_BS + r];
-        if (ma)
-        {
-            const bool dense_row = __popc(ma) > 4;
-            for (int pb = b0 + half; pb < b1; pb += 2)
-            {
-                const int j = P.B_col[pb] - c0;
-                const int slot = sm.pre[j >> 5] + __popc(sm.bm[j >> 5] & ((1u << (j & 31)) - 1u));
-                const unsigned short *mbk = P.B_mask + (long long)pb * TSG_BS;
-                unsigned acc = 0;
-                if (dense_row)
-                {
-                    const uint4 *mb = reinterpret_cast<const uint4 *>(mbk);
-                    acc = bool_row(ma, __ldg(mb), __ldg(mb + 1));
-                }
-                else
-                {
-                    unsigned bits = ma;
-                    do
-                    {
-                        const int bit = 31 - __clz(bits);
-                        bits ^= 1u << bit;
-                        acc |= __ldg(mbk + (15 - bit));
-                    } while (bits);
-                }
-                sm.acc[r][slot] |= (unsigned short)acc;
-            }
-        }
-        __syncwarp();
     }
     // row offsets, masks and counts, one C tile per half-warp
     const unsigned hmask = TSG_HW_MASK(threadIdx.x);

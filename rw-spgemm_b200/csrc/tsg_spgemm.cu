@@ -76,16 +76,17 @@ __global__ void __launch_bounds__(S1_WARPS * 32) k_step1_total(ProdView P, unsig
 // fused step-1 emit + step 2 (warp per A tile row).  Wide rows are emitted
 // alone and left to the wide-row step 2: wide[i] says 1, or 2 when the row is
 // hypersparse (0 otherwise), and wide[tilemA ...] lists their units (wide_list).
-__global__ void __launch_bounds__(256) k_step12(ProdView P, StepOneBits K, int split, int *__restrict__ wide,
+#define S12_WARPS 4
+__global__ void __launch_bounds__(S12_WARPS * 32) k_step12(ProdView P, StepOneBits K, int split, int *__restrict__ wide,
                                                 int *__restrict__ bins)
 {
-    __shared__ S12Smem sm[8];
+    __shared__ S12Smem sm[S12_WARPS];
     __shared__ int s_bins[4];
     if (threadIdx.x < 4)
         s_bins[threadIdx.x] = 0;
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int i = blockIdx.x * 8 + warp;
+    const int i = blockIdx.x * S12_WARPS + warp;
     if (i < P.tilemA)
     {
         const int done = step12_row(P, i, sm[warp], lane, s_bins, K);
@@ -332,7 +333,7 @@ __global__ void __launch_bounds__(256) k_win_btab(int m, const int *__restrict__
 __global__ void __launch_bounds__(256) k_win_ctab(ProdView P, WinPlan Q)
 {
     const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g < Q.mA && Q.A_rptr[g + 1] - Q.A_rptr[g] >= WIN_HEAVY)
+    if (g < Q.mA && Q.A_rptr[g + 1] - Q.A_rptr[g] >= Q.heavy_min)
         Q.heavy[atomicAdd(Q.nheavy, 1u)] = (int)g;
     if (g < (long long)P.tilemA * (Q.windows + 1))
         win_ctab_entry(P, Q, g);
@@ -548,7 +549,7 @@ struct WinScratch
 };
 
 // Whether a product runs step 3 by windows, and their table's shape
-static bool win_shape(const ProdView &P, long long nnzC, WinPlan &Q)
+static bool win_shape(const ProdView &P, long long nnzA, long long nnzC, WinPlan &Q)
 {
     if (!P.B_rptr || P.nB < 1 || P.mA < 1)
         return false;
@@ -560,6 +561,7 @@ static bool win_shape(const ProdView &P, long long nnzC, WinPlan &Q)
         return false;
     Q.windows = (int)windows;
     Q.mA = P.mA;
+    Q.heavy_min = win_heavy(nnzA);
     return true;
 }
 
@@ -693,7 +695,7 @@ static int launch_step3_spa_rows(tsg_context *ctx, const ProdView &P, const tsg_
     const bool flat = spa_wants_flat(P.browB, P.numC, nnzC, P.tilemA);
     const bool whole = row0 == 0 && row1 == P.tilemA;
     ctx->last_step3 = flat ? TSG_STEP3_FLAT : P.padded ? TSG_STEP3_STAGED : TSG_STEP3_SPA;
-    if (flat && win_shape(P, nnzC, W.Q))
+    if (flat && win_shape(P, A->nnz, nnzC, W.Q))
     {
         ctx->last_step3 = TSG_STEP3_WINDOWS;
         return launch_step3_win(ctx, P, A, W, row0, row1);
@@ -819,7 +821,7 @@ static int spgemm_structure(tsg_context *ctx, const tsg_tiled *A, const tsg_tile
             const int split = wide_split(A->nnz, ctx->num_sms);
             TSG_TRY(tsg_alloc(ctx, &R.d_wide, (size_t)tilem + 3 + 2 * wide_units(tilem, A->nnz, split)));
             TSG_CUDA(cudaMemsetAsync(R.d_wide + tilem, 0, 2 * sizeof(int), st));
-            k_step12<<<tsg_blocks(tilem, 8), 256, 0, st>>>(P, R.bits, split, R.d_wide, d_bins);
+            k_step12<<<tsg_blocks(tilem, S12_WARPS), S12_WARPS * 32, 0, st>>>(P, R.bits, split, R.d_wide, d_bins);
             TSG_LAUNCH_CHECK();
         }
         else

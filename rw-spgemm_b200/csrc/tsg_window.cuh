@@ -40,7 +40,10 @@
 #define WIN_PART_BITS 8
 #endif
 #ifndef WIN_HEAVY
-#define WIN_HEAVY 512 // A entries that make a row heavy
+#define WIN_HEAVY 256 // fewest A entries that make a row heavy
+#endif
+#ifndef WIN_HEAVY_SHARE
+#define WIN_HEAVY_SHARE 2048
 #endif
 #ifndef WIN_ROWS
 #define WIN_ROWS 4 // rows per claim
@@ -85,7 +88,18 @@ struct WinPlan
     unsigned *claim, *nheavy; // counters: claims, heavy rows
     int blocks, bits, windows;
     int mA;
+    int heavy_min;      // A entries that make a row heavy (win_heavy)
 };
+
+// A row is heavy when it would hold up the others: a task of 256 columns
+// meets shorter parts of B's rows, so only then is it worth cutting.  R-MAT 14
+// (228 K entries of A): 0.72 ms from 256 entries on, 0.81 from 512; R-MAT 16
+// (955 K): 5.99 and 5.52 ms.
+static inline int win_heavy(long long nnzA)
+{
+    const long long share = nnzA / WIN_HEAVY_SHARE;
+    return share < WIN_HEAVY ? WIN_HEAVY : (int)share;
+}
 
 // B row w's entry offset at every block boundary, by a warp
 __device__ __forceinline__ void win_btab_row(int w, const int *__restrict__ rptr, const int *__restrict__ rcol,
@@ -452,7 +466,7 @@ __device__ __forceinline__ void win_claim_rows(const ProdView &P, const WinPlan 
         const int e2 = __shfl_sync(TSG_FULL_MASK, e, min(i + 2, WIN_ROWS));
         const WinEntry nxt = win_entry<true>(P, Q, e1 + lane, e2, k2, c0, c1);
         k2 = col(i + 2);
-        if (e0 < e1 && e1 - e0 < WIN_HEAVY)
+        if (e0 < e1 && e1 - e0 < Q.heavy_min)
             win_task<true>(P, Q, S, I, r0 + i, c0, c1, e0, e1, E, t0, t1, lane);
         e0 = e1;
         e1 = e2;
