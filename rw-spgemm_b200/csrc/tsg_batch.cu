@@ -40,6 +40,7 @@ struct BatchProd
     int win;
     long long capT, capN;
     int tilemA;
+    int hypT;   // C tiles of hypersparse rows
     int status; // 0 ok, 1 tile capacity, 2 value capacity
     int numC, nnzC;
 };
@@ -56,14 +57,15 @@ struct tsg_batch
     long long *d_itemoff;
     unsigned *d_bar; // [0] arrivals, [1] generation, [2] next tile block of the SPA step 3, [3] next
                      // wide unit of step 2, [4..5] the barrier's wait limit in ns (64-bit), [6] wide
-                     // units, [7] parts of heavy rows, [8] next claim of the window step 3
+                     // units, [7] parts of heavy rows, [8] next claim of the window step 3, [9] next
+                     // unit of the hypersparse step 3
     int *d_err;
     int *d_bins;
     void *arena;
     size_t arena_bytes;
     int grid, block;
     size_t smem;
-    int grid3; // persistent grid of k_batch_spa3 (SPA schedule)
+    int grid3, gridh; // persistent grids of k_batch_spa3 and k_batch_hyper (SPA schedule)
     cudaGraph_t graph;
     cudaGraphExec_t exec;
     int graph_ok;
@@ -76,6 +78,9 @@ struct tsg_batch
     long long *d_s1off, *d_winoff;
     int4 *d_wlist, *d_hlist; // wide units of step 2; heavy rows' parts of the window step 3
     int *win_tables;
+    long long *d_denseoff;      // C tiles of the products with dense tiles, prefix
+    cudaStream_t side[2];       // step 3's kernels run beside one another
+    cudaEvent_t fork, join[2];
     int split;   // A entries of a unit of step 2's wide rows
     int wins;    // products that take the windows
     int gridw;   // persistent grid of k_batch_win
@@ -306,7 +311,7 @@ __device__ __forceinline__ unsigned long long gtimer() { return batch_clock_ns()
 template <int SCHED, int W, int CAP, int NT>
 __global__ void __launch_bounds__(NT)
     k_batch(BatchProd *prods, int count, const long long *__restrict__ rowoff, const long long *__restrict__ s1off,
-            int4 *wlist, int split, long long *itemoff, unsigned *bar, int *err, int *bins)
+            int4 *wlist, int split, long long *denseoff, int dense, long long *itemoff, unsigned *bar, int *err, int *bins)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
     __shared__ long long s_tmp[NT / 32 + 1];
@@ -367,6 +372,7 @@ __global__ void __launch_bounds__(NT)
                 bp.numC = (int)tot;
             }
             bp.P.numC = bp.numC;
+            bp.hypT = 0;
         }
     }
     if (!grid_barrier(bar, err))
@@ -403,7 +409,7 @@ __global__ void __launch_bounds__(NT)
                 run += ((long long)prods[p].numC + SCAN_CHUNK - 1) / SCAN_CHUNK;
             }
             chunkoff[count] = run;
-            bar[2] = bar[3] = bar[6] = bar[7] = bar[8] = 0;
+            bar[2] = bar[3] = bar[6] = bar[7] = bar[8] = bar[9] = 0;
         }
         if (threadIdx.x < 4)
             bins[threadIdx.x] = 0;
@@ -448,6 +454,8 @@ __global__ void __launch_bounds__(NT)
                         int4 *at = wlist + atomicAdd(&bar[6], (unsigned)parts);
                         for (int q = 0; q < parts; q++)
                             at[q] = make_int4(p, i, q | parts << 16, 0);
+                        if (kind == 2)
+                            atomicAdd(&prods[p].hypT, prods[p].P.C_ptr[i + 1] - prods[p].P.C_ptr[i]);
                     }
                 }
                 __syncwarp();
@@ -549,7 +557,22 @@ __global__ void __launch_bounds__(NT)
     // phase 7: step 3 (the SPA schedule runs it as two kernels after this one:
     // k_batch_spa3 and k_batch_dense3, each at its own occupancy)
     if (SCHED == 3)
+    {
+        // C tiles of the products that take the tile kernel, prefix
+        if (blockIdx.x == 0)
+        {
+            for (int p = threadIdx.x; p < count; p += NT)
+            {
+                const BatchProd &bp = prods[p];
+                denseoff[p] = !bp.status && bp.numC > 0 && bp.nnzC >= (long long)dense * bp.numC ? bp.numC : 0;
+            }
+            __syncthreads();
+            const long long all = block_scan_ll<NT>(denseoff, count, s_tmp);
+            if (threadIdx.x == 0)
+                denseoff[count] = all;
+        }
         return;
+    }
     if (SCHED == 2)
     {
         int2 *pairs = reinterpret_cast<int2 *>(s_raw) + warp * S3E_PAIRS;
@@ -615,19 +638,55 @@ __global__ void __launch_bounds__(SPA_THREADS, 3)
         if (blk >= blkoff[count])
             break;
         p = find_product_from(blkoff, count, blk, p);
-        if (prods[p].win || prods[p].status || prods[p].nnzC >= (long long)dense * prods[p].numC)
+        if (prods[p].win || prods[p].status || prods[p].nnzC >= (long long)dense * prods[p].numC ||
+            prods[p].hypT == prods[p].numC)
+        {
+            if (threadIdx.x == 0) // nothing of this product is left to take
+                atomicMax(&bar[2], (unsigned)blkoff[p + 1]);
             continue;
+        }
         const ProdView &P = prods[p].P;
         const long long tb = (blk - blkoff[p]) * SPA_BLK;
         if (threadIdx.x == 0)
             spa_skip_hyper(P, prods[p].wide, (int)tb, &bar[2], blkoff[p]);
-        step3_spa_block<true>(P, S, (int)tb, (int)min((long long)P.numC, tb + SPA_BLK), prods[p].wide);
+        step3_spa_block<true>(P, S, (int)tb, (int)min((long long)P.numC, tb + SPA_BLK), prods[p].wide, nullptr, false);
     }
     __syncthreads();
     if (threadIdx.x == 0)
         atomicMax(reinterpret_cast<unsigned long long *>(const_cast<long long *>(itemoff)) + 2 * ((long long)count + 1) +
                       7,
                   gtimer());
+}
+
+// ... the hypersparse rows of those products, a CTA each, from step 2's list ...
+__global__ void __launch_bounds__(SPA_THREADS, 3)
+    k_batch_hyper(const BatchProd *prods, const int4 *__restrict__ wlist, unsigned *bar, const int *err, int dense)
+{
+    if (*(volatile const int *)err)
+        return;
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    HypSmem &S = *reinterpret_cast<HypSmem *>(s_raw);
+    __shared__ int s_unit;
+    const int units = (int)bar[6];
+    unsigned nxt = 0; // thread 0: the next unit, claimed one ahead
+    if (threadIdx.x == 0)
+        nxt = atomicAdd(&bar[9], 1u);
+    for (;;)
+    {
+        __syncthreads();
+        if (threadIdx.x == 0)
+        {
+            s_unit = (int)nxt;
+            nxt = atomicAdd(&bar[9], 1u);
+        }
+        __syncthreads();
+        if (s_unit >= units)
+            break;
+        const int4 u = wlist[s_unit];
+        const BatchProd &b = prods[u.x];
+        if ((u.z & 0xFFFF) == 0 && b.wide[u.y] == 2 && !b.win && !b.status && b.nnzC < (long long)dense * b.numC)
+            step3_hyper_row(b.P, S, u.y);
+    }
 }
 
 // ... the tables of the products that take the windows (prefixes over the
@@ -717,25 +776,28 @@ __global__ void __launch_bounds__(WIN_THREADS, WIN_CTAS)
                   gtimer());
 }
 
-// ... and products with dense C tiles (>= `dense` values per tile on
-// average): the tile kernel, a half-warp per C tile.
+// ... and products with dense C tiles (>= the batch's threshold of values per
+// tile on average): the tile kernel, a half-warp per C tile of theirs
+// (denseoff: their tiles, prefix; walked among the tiles of all products,
+// finding out cost four times the work).
 #define DENSE3_THREADS 128
-__global__ void __launch_bounds__(DENSE3_THREADS)
-    k_batch_dense3(BatchProd *prods, int count, const long long *__restrict__ itemoff, const int *err, int dense)
+__global__ void __launch_bounds__(DENSE3_THREADS, 4)
+    k_batch_dense3(BatchProd *prods, int count, const long long *__restrict__ denseoff, const long long *__restrict__ itemoff,
+                   const int *err)
 {
     if (*(volatile const int *)err)
         return;
     __shared__ __align__(16) double s_A[DENSE3_THREADS / 16][S3T_WORDS];
     const int lane = threadIdx.x & 15, hw = threadIdx.x >> 4;
     const unsigned hmask = TSG_HW_MASK(threadIdx.x);
-    const long long total_items = itemoff[count];
+    const long long total_items = denseoff[count];
+    if (total_items == 0)
+        return;
     const long long nhw = (long long)gridDim.x * (DENSE3_THREADS / 16);
     for (long long h = (long long)blockIdx.x * (DENSE3_THREADS / 16) + hw; h < total_items; h += nhw)
     {
-        const int p = find_product(itemoff, count, h);
-        if (prods[p].status || prods[p].nnzC < (long long)dense * prods[p].numC)
-            continue;
-        step3_tile(prods[p].P, (int)(h - itemoff[p]), hmask, lane, s_A[hw]);
+        const int p = find_product(denseoff, count, h);
+        step3_tile(prods[p].P, (int)(h - denseoff[p]), hmask, lane, s_A[hw]);
     }
     __syncthreads();
     if (threadIdx.x == 0)
@@ -864,7 +926,7 @@ extern "C" int tsg_product_bounds(tsg_context *ctx, const tsg_tiled *A, const ts
 // host side
 // ---------------------------------------------------------------------------
 typedef void (*batch_kernel_t)(BatchProd *, int, const long long *, const long long *, int4 *, int, long long *,
-                               unsigned *, int *, int *);
+                               int, long long *, unsigned *, int *, int *);
 
 // Kernel, dynamic shared memory and block size of a batch schedule.
 static batch_kernel_t pick_kernel(const tsg_batch_params &p, size_t *smem, int *threads)
@@ -929,8 +991,16 @@ static int record_run(tsg_batch *b, cudaStream_t st)
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     TSG_CUDA(cudaLaunchKernelEx(&cfg, kern, b->d_prod, b->count, (const long long *)b->d_rowoff,
-                                (const long long *)b->d_s1off, b->d_wlist, b->split, b->d_itemoff,
+                                (const long long *)b->d_s1off, b->d_wlist, b->split, b->d_denseoff, b->dense,
+                                b->d_itemoff,
                                 b->d_bar, b->d_err, b->d_bins));
+    if (b->params.schedule != TSG_SCHED_SPA)
+        return TSG_OK;
+    // step 3's kernels share no product: side by side, so that none waits for
+    // another's last rows
+    TSG_CUDA(cudaEventRecord(b->fork, st));
+    for (int q = 0; q < 2; q++)
+        TSG_CUDA(cudaStreamWaitEvent(b->side[q], b->fork, 0));
     if (b->wins)
     {
         k_batch_wtab<<<b->ctx->num_sms * 8, 256, 0, st>>>(b->d_prod, b->count, b->d_winoff, b->d_hlist, b->d_bar, b->d_err,
@@ -940,14 +1010,19 @@ static int record_run(tsg_batch *b, cudaStream_t st)
             b->d_prod, b->count, b->d_winoff, b->d_hlist, b->d_itemoff, b->d_bar, b->d_err, b->dense);
         TSG_CUDA(cudaGetLastError());
     }
-    if (b->params.schedule == TSG_SCHED_SPA)
-    {
-        k_batch_spa3<<<b->grid3, SPA_THREADS, sizeof(SpaSmem), st>>>(b->d_prod, b->count, b->d_itemoff, b->d_bar,
-                                                                     b->d_err, b->dense);
-        TSG_CUDA(cudaGetLastError());
-        k_batch_dense3<<<b->ctx->num_sms * 8, DENSE3_THREADS, 0, st>>>(b->d_prod, b->count, b->d_itemoff, b->d_err,
+    k_batch_hyper<<<b->gridh, SPA_THREADS, sizeof(HypSmem), b->side[0]>>>(b->d_prod, b->d_wlist, b->d_bar, b->d_err,
                                                                         b->dense);
-        TSG_CUDA(cudaGetLastError());
+    TSG_CUDA(cudaGetLastError());
+    k_batch_spa3<<<b->grid3, SPA_THREADS, sizeof(SpaSmem), b->side[0]>>>(b->d_prod, b->count, b->d_itemoff, b->d_bar,
+                                                                       b->d_err, b->dense);
+    TSG_CUDA(cudaGetLastError());
+    k_batch_dense3<<<b->ctx->num_sms * 4, DENSE3_THREADS, 0, b->side[1]>>>(b->d_prod, b->count, b->d_denseoff,
+                                                                         b->d_itemoff, b->d_err);
+    TSG_CUDA(cudaGetLastError());
+    for (int q = 0; q < 2; q++)
+    {
+        TSG_CUDA(cudaEventRecord(b->join[q], b->side[q]));
+        TSG_CUDA(cudaStreamWaitEvent(st, b->join[q], 0));
     }
     return TSG_OK;
 }
@@ -1101,7 +1176,17 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
         delete b;
         return st;
     }
-    if ((b->wins && ((st = tsg_alloc(ctx, &b->win_tables, (size_t)table_words)) != TSG_OK ||
+    cudaError_t se = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
+    for (int q = 0; q < 2 && se == cudaSuccess; q++)
+        if ((se = cudaEventCreateWithFlags(&b->join[q], cudaEventDisableTiming)) == cudaSuccess)
+            se = cudaStreamCreateWithFlags(&b->side[q], cudaStreamNonBlocking);
+    if (se != cudaSuccess)
+    {
+        tsg_batch_destroy(b);
+        return tsg_set_error(TSG_ERR_CUDA, "batch streams: %s", cudaGetErrorString(se));
+    }
+    if ((st = tsg_alloc(ctx, &b->d_denseoff, (size_t)count + 1)) != TSG_OK ||
+        (b->wins && ((st = tsg_alloc(ctx, &b->win_tables, (size_t)table_words)) != TSG_OK ||
                      (st = tsg_alloc(ctx, &b->d_hlist, (size_t)hparts)) != TSG_OK ||
                      (st = tsg_alloc(ctx, &b->d_winoff, b->winoff.size())) != TSG_OK)) ||
         (st = tsg_alloc(ctx, &b->d_s1off, b->s1off.size())) != TSG_OK ||
@@ -1223,8 +1308,13 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
     b->grid3 = 0;
     if (prm.schedule == TSG_SCHED_SPA)
     {
-        int per3 = 0;
-        if (cudaFuncSetAttribute(k_batch_spa3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SpaSmem)) !=
+        int per3 = 0, perh = 0;
+        if (cudaFuncSetAttribute(k_batch_hyper, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(HypSmem)) !=
+                cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perh, k_batch_hyper, SPA_THREADS, sizeof(HypSmem)) !=
+                cudaSuccess ||
+            perh < 1 ||
+            cudaFuncSetAttribute(k_batch_spa3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SpaSmem)) !=
                 cudaSuccess ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per3, k_batch_spa3, SPA_THREADS, sizeof(SpaSmem)) !=
                 cudaSuccess ||
@@ -1234,6 +1324,7 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
             return tsg_set_error(TSG_ERR_CUDA, "batch numeric kernel cannot be resident");
         }
         b->grid3 = per3 * ctx->num_sms;
+        b->gridh = perh * ctx->num_sms;
     }
     if (b->wins)
     {
@@ -1420,6 +1511,7 @@ extern "C" int tsg_batch_destroy(tsg_batch *b)
     tsg_release(ctx, b->d_err);
     tsg_release(ctx, b->d_bins);
     tsg_release(ctx, b->d_s1off);
+    tsg_release(ctx, b->d_denseoff);
     tsg_release(ctx, b->d_winoff);
     tsg_release(ctx, b->d_wlist);
     tsg_release(ctx, b->d_hlist);
@@ -1427,6 +1519,15 @@ extern "C" int tsg_batch_destroy(tsg_batch *b)
     char *a = (char *)b->arena;
     tsg_release(ctx, a);
     cudaStreamSynchronize(ctx->stream);
+    for (int q = 0; q < 2; q++)
+    {
+        if (b->side[q])
+            cudaStreamDestroy(b->side[q]);
+        if (b->join[q])
+            cudaEventDestroy(b->join[q]);
+    }
+    if (b->fork)
+        cudaEventDestroy(b->fork);
     delete b;
     return TSG_OK;
 }

@@ -270,9 +270,7 @@ __device__ __forceinline__ int nnz_bin(int total);
 #define S12_MAXT 128
 // tile pairs from which a row is wide whatever its tiles: the warp takes them
 // 32 at a time (1,500 x 1,300 random, 3,775 pairs and 980 products a tile row)
-#ifndef S12_MAXP
 #define S12_MAXP 1024
-#endif
 
 struct S12Smem
 {
@@ -1740,6 +1738,8 @@ __device__ __forceinline__ void step3_hyper_row(const ProdView &P, HypSmem &S, i
 // SPA_BLK_NARROW_VALUES values (wide rows of skewed products such as R-MAT):
 // twice the blocks, so a hub row's segments spread over more CTAs
 #define SPA_BLK_NARROW 128
+// and for narrow rows of a product that would not fill the GPU with blocks
+#define SPA_BLK_SMALL 32
 #define SPA_BLK_NARROW_VALUES 4
 
 // calls piece(I, t0, t1) for the pieces [t0, t1) owned by block [tb, te),

@@ -12,7 +12,6 @@
 // per run of C tiles in one tile row, tile-level Gustavson, no intersection).
 #include <limits.h>
 #include <stddef.h>
-#include <stdlib.h>
 
 #include <algorithm>
 
@@ -530,12 +529,12 @@ static int launch_step2_cta(tsg_context *ctx, const ProdView &P, int span, const
 
 static int launch_step2_wide(tsg_context *ctx, const ProdView &P, int widest, const int *d_wide, int *d_bins)
 {
-    // the widest row of C, or as many columns as a CTA's shared memory holds
+    // the widest row of C, or as many columns as a CTA's shared memory holds;
+    // narrow C leaves room for four CTAs of 512 threads on an SM (8,192 columns:
+    // 0.073 ms, 0.083 with 1,024 threads; 16,384 columns of R-MAT 14: 0.45 and
+    // 0.38)
     const int span = std::max(1, std::min(widest, WIDE_SPAN));
-    static int force = getenv("S2_NT") ? atoi(getenv("S2_NT")) : 0;
-    const int nt = force ? force : span <= 512 ? 512 : 1024;
-    return nt == 256 ? launch_step2_cta<256>(ctx, P, span, d_wide, d_bins)
-           : nt == 512 ? launch_step2_cta<512>(ctx, P, span, d_wide, d_bins)
+    return span <= 512 ? launch_step2_cta<512>(ctx, P, span, d_wide, d_bins)
                        : launch_step2_cta<1024>(ctx, P, span, d_wide, d_bins);
 }
 
@@ -636,7 +635,7 @@ static int launch_step3_spa(tsg_context *ctx, const ProdView &P0, const int *d_k
     unsigned *ctr = ctx->d_ctl->ctr;
     const int smem = (int)sizeof(SpaSmem);
     int per_sm = 0;
-    TSG_TRY(resident_ctas(ctx, TSG_OCC_SPA + (FLAT ? 1 : 0) + (RANGED ? 2 : 0) + (BLK == SPA_BLK ? 0 : 4),
+    TSG_TRY(resident_ctas(ctx, TSG_OCC_SPA + (FLAT ? 1 : 0) + (RANGED ? 2 : 0) + (BLK == SPA_BLK ? 0 : BLK == SPA_BLK_NARROW ? 4 : 8),
                           k_step3_spa<FLAT, RANGED, BLK>, SPA_THREADS, smem, &per_sm));
     TSG_TRY(clear_counters(ctx, row0, TSG_CTR_STEP3, 2));
     if (hyper_apart)
@@ -700,9 +699,15 @@ static int launch_step3_spa_rows(tsg_context *ctx, const ProdView &P, const tsg_
         ctx->last_step3 = TSG_STEP3_WINDOWS;
         return launch_step3_win(ctx, P, A, W, row0, row1);
     }
-    if (flat && nnzC >= (long long)SPA_BLK_NARROW_VALUES * P.numC)
+    const bool small = flat && P.numC <= (long long)SPA_BLK_SMALL * P.tilemA && P.numC < (long long)SPA_BLK * 6 * ctx->num_sms;
+    if (flat && !small && nnzC >= (long long)SPA_BLK_NARROW_VALUES * P.numC)
         return whole ? launch_step3_spa<true, false, SPA_BLK_NARROW>(ctx, P, d_kind, false, 0, 0)
                      : launch_step3_spa<true, true, SPA_BLK_NARROW>(ctx, P, d_kind, false, row0, row1);
+    // narrow rows in too few blocks to go round (squares of grids' matrices: 64^2,
+    // 11 blocks of 256 tiles, 0.121 -> 0.043 ms; 256^2, 198 blocks, 0.123 -> 0.107)
+    if (small)
+        return whole ? launch_step3_spa<true, false, SPA_BLK_SMALL>(ctx, P, d_kind, false, 0, 0)
+                     : launch_step3_spa<true, true, SPA_BLK_SMALL>(ctx, P, d_kind, false, row0, row1);
     // mostly hypersparse rows (few values in many tiles): those by themselves
     const bool hyper = d_kind && nnzC < (long long)HYP_RATIO * P.numC && P.numC > (long long)S12_MAXT * P.tilemA;
     if (flat)

@@ -201,9 +201,9 @@ __device__ __forceinline__ int step1_row_cta(const ProdView &P, int i, S1cSmem<N
 // 65,536 columns, and a hypersparse row is no special case.
 //
 // Bound: instructions of the walk and, for hypersparse rows, the 52 bytes
-// written per C tile.  On a B200: R-MAT 16 (402 M products)
-// 3.09 -> 1.71 ms, R-MAT 14 (53 M) 1.03 -> 0.38 ms, 65,536 random rows (16.4 M
-// C tiles, 4.2 M products) 0.875 -> 0.55 ms, the scan of the counts included.
+// written per C tile.  On a B200, with the scan of the counts: R-MAT 16 (402 M
+// products) 3.09 -> 1.51 ms, R-MAT 14 (53 M) 1.03 -> 0.295 ms, 65,536 random rows
+// (16.4 M C tiles, 4.2 M products) 0.875 -> 0.545 ms.
 // ---------------------------------------------------------------------------
 #define WIDE_UNROLL 4
 

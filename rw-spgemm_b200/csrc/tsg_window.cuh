@@ -17,51 +17,35 @@
 //    at every window (or block of windows) boundary, made once per product,
 //    instead of two binary searches per entry;
 //  - the products of 32 A entries are flattened over the lanes in k order;
-//    lanes of one batch that meet the same column add one after another in
-//    lane order, batches follow one another behind warp barriers;
+//    a batch's entries, or the lanes that meet the same column, add one after
+//    another, batches follow one another behind warp barriers;
 //  - the values leave through C's masks, which hold exactly the columns that
 //    were written; what is read is cleared for the next task.
 // Warps claim WIN_ROWS rows of a (tile row, window) at a time from a device
 // counter, one claim ahead.
 //
-// Bound: the latency of B's entries from L2 and the shared-memory
-// read-modify-write, hidden by as many warps as their accumulators fit.
-// On a B200, k_step3_spa<flat> before: R-MAT 16 (402 M products) 14.9 -> 5.8 ms,
-// R-MAT 14 (53 M) 3.70 -> 1.10 ms, a band of 65 times 8,192 random rows (4.2 M)
-// 0.169 -> 0.147 ms.
+// Bound: instructions, about 200 per batch of 32 products (issue slots 60 %
+// busy, shared memory 52 %); the latency of B's entries from L2 is hidden by
+// as many warps as their accumulators fit.  On a B200, k_step3_spa<flat>
+// before: R-MAT 16 (402 M products) 14.9 -> 5.5 ms, R-MAT 14 (53 M) 3.70 ->
+// 0.72 ms, a band of 65 times 8,192 random rows (4.2 M) 0.169 -> 0.136 ms.
 #pragma once
 
 #include "tsg_device.cuh"
 
-#ifndef WIN_COLS
-#define WIN_COLS 1024
-#endif
-#ifndef WIN_PART_BITS
+#define WIN_COLS 1024 // (512: as many warps again, R-MAT 16 no faster)
 #define WIN_PART_BITS 8
-#endif
-#ifndef WIN_HEAVY
 #define WIN_HEAVY 256 // fewest A entries that make a row heavy
-#endif
-#ifndef WIN_HEAVY_SHARE
-#define WIN_HEAVY_SHARE 2048
-#endif
-#ifndef WIN_ROWS
-#define WIN_ROWS 4 // rows per claim
-#endif
-#ifndef WIN_CTAS
+#define WIN_HEAVY_SHARE 2048 // and the share of A's entries
+#define WIN_ROWS 2 // rows per claim
 #define WIN_CTAS 3
-#endif
 #define WIN_TILES (WIN_COLS / TSG_BS)
 #define WIN_PART (1 << WIN_PART_BITS) // columns of a task of a heavy row
 #define WIN_PARTS (WIN_COLS / WIN_PART)
 #define WIN_WARPS 8
 #define WIN_THREADS (WIN_WARPS * 32)
-#ifndef WIN_FEW
 #define WIN_FEW 3 // values of a tile's row up to which a lane stores its tile's own
-#endif
-#ifndef WIN_ROUNDS
 #define WIN_ROUNDS 6 // entries after the first that a batch adds entry by entry
-#endif
 // a product takes the windows when C holds at least this many values per (row, window)
 #define WIN_MIN_VALUES 8
 #define WIN_TABLE_WORDS (1LL << 26) // most words of the table of B's row pointers
@@ -268,7 +252,8 @@ __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, Wi
         }
         __syncwarp();
         // batches of 32 products, a batch's loads issued two batches before its
-        // additions.  rel: the lane's entry, from the batch's first
+        // additions.  rel: the lane's entry, counted from the batch's
+        // first, and the batch's last (<< 8)
         int cur = 0, until = S.end[0]; // the entry at the last loaded batch's end, and its end
         auto load = [&](int ib, int &rel, int &col, double &p) {
             rel = 0;
@@ -285,8 +270,8 @@ __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, Wi
                 const bool mine = len > 0 && pre > ib && pre < ib + 32;
                 const unsigned starts = __reduce_or_sync(TSG_FULL_MASK, mine ? 1u << (pre - ib) : 0u);
                 const int before = __popc(__ballot_sync(TSG_FULL_MASK, len > 0 && pre <= ib)) - 1;
-                rel = __popc(starts & upto);
-                e = before + rel;
+                rel = __popc(starts & upto) | __popc(starts) << 8;
+                e = before + (rel & 0xFF);
                 cur = before + __popc(starts);
                 until = S.end[cur];
             }
@@ -297,8 +282,6 @@ __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, Wi
                 p = __dmul_rn(S.a[e], P.B_rval[bi]);
             }
         };
-        // products of one entry meet distinct columns; those of a few entries
-        // are added entry by entry, others in lane order where columns meet
         // products of one entry meet distinct columns; those of a few entries
         // are added entry by entry, others in lane order where columns meet
         auto add = [&](int rel, int col, double p) {
@@ -335,7 +318,6 @@ __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, Wi
     }
     if (!any)
         return;
-#ifndef WIN_OUT_LANE
     // the row's values out, 32 tiles at a time, flattened over the lanes:
     // consecutive lanes store consecutive values of a tile's row (a lane per
     // tile would touch a line per value, and read a bank 32 ways)
@@ -399,30 +381,6 @@ __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, Wi
         __syncwarp();
     }
 }
-#else
-    // the row's values out, a lane per C tile of the row, each starting at a
-    // column of its own (all at once would read one bank)
-#pragma unroll
-    for (int h = 0; h < 2; h++)
-    {
-        const unsigned m = base[h] >= 0 && base[h] < c1 - c0 ? mk[h] : 0u; // a heavy row's part holds some of the tiles
-        const int turn = lane & 15;
-        unsigned left = ((m << turn) | (m >> (16 - turn))) & 0xFFFFu;
-        double *acc = S.acc + base[h];
-        while (left)
-        {
-            const int bit = 31 - __clz(left);
-            left ^= 1u << bit;
-            const int c = 15 - ((bit - turn) & 15);
-            const int q = at[h] + __popc(m >> (16 - c));
-            P.C_Val[q] = acc[c];
-            acc[c] = 0.0;
-            P.C_Colb[q] = (unsigned char)c;
-        }
-    }
-    __syncwarp();
-}
-#endif
 static_assert(WIN_TILES <= 64, "C tiles of a window");
 
 // columns [part * WIN_PART, ...) of heavy row `row`
