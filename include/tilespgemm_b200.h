@@ -312,6 +312,8 @@ typedef struct
 #define TSG_STEP3_STAGED 6 /* k_step3_stg + k_step3_rest: SPA with operands
                             * staged in shared memory by bulk copies          */
 #define TSG_STEP3_WINDOWS 7 /* k_step3_win: warp per C row and column window */
+#define TSG_STEP3_NARROW 8 /* k_step3_nar: warp per C rows of few tiles, then
+                              k_step3_rest                                   */
 
 const char *tsg_status_string(int status);
 /* Message describing the last failure on the calling thread. */

@@ -1738,8 +1738,6 @@ __device__ __forceinline__ void step3_hyper_row(const ProdView &P, HypSmem &S, i
 // SPA_BLK_NARROW_VALUES values (wide rows of skewed products such as R-MAT):
 // twice the blocks, so a hub row's segments spread over more CTAs
 #define SPA_BLK_NARROW 128
-// and for narrow rows of a product that would not fill the GPU with blocks
-#define SPA_BLK_SMALL 32
 #define SPA_BLK_NARROW_VALUES 4
 
 // calls piece(I, t0, t1) for the pieces [t0, t1) owned by block [tb, te),

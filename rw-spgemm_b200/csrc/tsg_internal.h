@@ -35,10 +35,11 @@ enum
 // kernels whose resident CTAs per SM the context remembers
 enum
 {
-    TSG_OCC_SPA = 0,  // + FLAT, RANGED, narrow or small blocks
-    TSG_OCC_STG = 12, // + RANGED
-    TSG_OCC_REST = 14,
-    TSG_OCC_WIN = 16,
+    TSG_OCC_SPA = 0, // + FLAT, RANGED, narrow blocks
+    TSG_OCC_STG = 8, // + RANGED
+    TSG_OCC_REST = 10, // + RANGED, FLAT
+    TSG_OCC_WIN = 14,
+    TSG_OCC_NAR,
     TSG_OCC_HYPER,
     TSG_OCC_COUNT
 };

@@ -285,7 +285,8 @@ __global__ void __launch_bounds__(SPA_THREADS, 3) k_step3_hyper(ProdView P, cons
 // The tile rows the staged numeric step left (left[I] != 0: its stage would
 // not fit, or the row is hypersparse), by the SPA kernel; nothing unless it
 // left some (left[tilemA]).
-template <bool RANGED>
+// FLAT: a product of short B rows.
+template <bool RANGED, bool FLAT>
 __global__ void __launch_bounds__(SPA_THREADS, 2) k_step3_rest(ProdView P, const int *__restrict__ kind,
                                                                const int *__restrict__ left, int row0, int row1,
                                                                unsigned *__restrict__ ctr)
@@ -314,7 +315,7 @@ __global__ void __launch_bounds__(SPA_THREADS, 2) k_step3_rest(ProdView P, const
             break;
         if (threadIdx.x == 0)
             spa_skip_hyper(P, kind, (int)tb, ctr, -blk0);
-        step3_spa_block<false>(P, S, max((int)tb, t_beg), (int)min((long long)t_end, tb + SPA_BLK), kind, left);
+        step3_spa_block<FLAT>(P, S, max((int)tb, t_beg), (int)min((long long)t_end, tb + SPA_BLK), kind, left);
     }
 }
 
@@ -370,6 +371,31 @@ __global__ void __launch_bounds__(WIN_THREADS, WIN_CTAS) k_step3_win(ProdView P,
             if (I >= row0 && I < row1)
                 win_claim_heavy(P, Q, S, row, (int)(c % parts), lane);
         }
+    }
+}
+
+// Step 3 of narrow rows, tile rows [row0, row1); *Q.claim zeroed.
+__global__ void __launch_bounds__(WIN_THREADS, WIN_CTAS)
+    k_step3_nar(ProdView P, WinPlan Q, int row0, int row1, const int *__restrict__ kind, int *__restrict__ left)
+{
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    const int lane = threadIdx.x & 31;
+    NarTask &S = reinterpret_cast<NarTask *>(s_raw)[threadIdx.x >> 5];
+    for (int q = lane; q < WIN_COLS; q += 32)
+        S.acc[q] = 0.0;
+    __syncwarp();
+    const unsigned claims = (unsigned)(row1 - row0) * NAR_PER;
+    unsigned nxt = 0;
+    if (lane == 0)
+        nxt = atomicAdd(Q.claim, 1u);
+    for (;;)
+    {
+        const unsigned c = __shfl_sync(TSG_FULL_MASK, nxt, 0);
+        if (c >= claims)
+            break;
+        if (lane == 0)
+            nxt = atomicAdd(Q.claim, 1u);
+        nar_claim(P, Q, S, row0, c, kind, left, lane);
     }
 }
 
@@ -576,6 +602,31 @@ static void win_release(tsg_context *ctx, WinScratch &W)
     W.ready = false;
 }
 
+// A's row view, made once per product when A has none
+static int win_rows(tsg_context *ctx, const ProdView &P, const tsg_tiled *A, WinScratch &W)
+{
+    WinPlan &Q = W.Q;
+    Q.claim = &ctx->d_ctl->ctr[TSG_CTR_STEP3];
+    Q.nheavy = &ctx->d_ctl->ctr[TSG_CTR_HEAVY];
+    Q.mA = P.mA;
+    Q.A_rptr = P.A_rptr;
+    Q.A_rcol = P.A_rcol;
+    Q.A_rval = P.A_rval;
+    if (P.A_rptr)
+        return TSG_OK;
+    if (!W.rptr)
+    {
+        TSG_TRY(tsg_alloc(ctx, &W.rptr, (size_t)A->m + 1));
+        TSG_TRY(tsg_alloc(ctx, &W.rcol, (size_t)A->nnz));
+        TSG_TRY(tsg_alloc(ctx, &W.rval, (size_t)A->nnz));
+        TSG_TRY(tsg_t2c_view(ctx, A, W.rptr, W.rcol, W.rval));
+    }
+    Q.A_rptr = W.rptr;
+    Q.A_rcol = W.rcol;
+    Q.A_rval = W.rval;
+    return TSG_OK;
+}
+
 // the tables of a product's windows, made once per product
 static int win_prepare(tsg_context *ctx, const ProdView &P, const tsg_tiled *A, WinScratch &W)
 {
@@ -589,21 +640,7 @@ static int win_prepare(tsg_context *ctx, const ProdView &P, const tsg_tiled *A, 
         TSG_TRY(tsg_alloc(ctx, &Q.wtab, (size_t)P.mB * Q.windows));
     TSG_TRY(tsg_alloc(ctx, &Q.ctab, (size_t)P.tilemA * (Q.windows + 1)));
     TSG_TRY(tsg_alloc(ctx, &Q.heavy, (size_t)P.mA));
-    Q.claim = &ctx->d_ctl->ctr[TSG_CTR_STEP3];
-    Q.nheavy = &ctx->d_ctl->ctr[TSG_CTR_HEAVY];
-    Q.A_rptr = P.A_rptr;
-    Q.A_rcol = P.A_rcol;
-    Q.A_rval = P.A_rval;
-    if (!P.A_rptr)
-    {
-        TSG_TRY(tsg_alloc(ctx, &W.rptr, (size_t)A->m + 1));
-        TSG_TRY(tsg_alloc(ctx, &W.rcol, (size_t)A->nnz));
-        TSG_TRY(tsg_alloc(ctx, &W.rval, (size_t)A->nnz));
-        TSG_TRY(tsg_t2c_view(ctx, A, W.rptr, W.rcol, W.rval));
-        Q.A_rptr = W.rptr;
-        Q.A_rcol = W.rcol;
-        Q.A_rval = W.rval;
-    }
+    TSG_TRY(win_rows(ctx, P, A, W));
     k_win_btab<<<tsg_blocks((long long)P.mB * 32, 256), 256, 0, st>>>(P.mB, P.B_rptr, P.B_rcol, Q.blocks, Q.bits, Q.btab, Q.windows, Q.wtab);
     TSG_LAUNCH_CHECK();
     k_win_ctab<<<tsg_blocks(std::max((long long)P.mA, (long long)P.tilemA * (Q.windows + 1)), 256), 256, 0, st>>>(P, Q);
@@ -635,7 +672,7 @@ static int launch_step3_spa(tsg_context *ctx, const ProdView &P0, const int *d_k
     unsigned *ctr = ctx->d_ctl->ctr;
     const int smem = (int)sizeof(SpaSmem);
     int per_sm = 0;
-    TSG_TRY(resident_ctas(ctx, TSG_OCC_SPA + (FLAT ? 1 : 0) + (RANGED ? 2 : 0) + (BLK == SPA_BLK ? 0 : BLK == SPA_BLK_NARROW ? 4 : 8),
+    TSG_TRY(resident_ctas(ctx, TSG_OCC_SPA + (FLAT ? 1 : 0) + (RANGED ? 2 : 0) + (BLK == SPA_BLK ? 0 : 4),
                           k_step3_spa<FLAT, RANGED, BLK>, SPA_THREADS, smem, &per_sm));
     TSG_TRY(clear_counters(ctx, row0, TSG_CTR_STEP3, 2));
     if (hyper_apart)
@@ -664,15 +701,44 @@ static int launch_step3_stg(tsg_context *ctx, const ProdView &P0, const int *d_k
     const int smem = (int)sizeof(StgSmem), rsmem = (int)sizeof(SpaSmem);
     int per_sm = 0, rest_per_sm = 0;
     TSG_TRY(resident_ctas(ctx, TSG_OCC_STG + (RANGED ? 1 : 0), k_step3_stg<RANGED>, STG_THREADS, smem, &per_sm));
-    TSG_TRY(resident_ctas(ctx, TSG_OCC_REST + (RANGED ? 1 : 0), k_step3_rest<RANGED>, SPA_THREADS, rsmem, &rest_per_sm));
+    TSG_TRY(resident_ctas(ctx, TSG_OCC_REST + (RANGED ? 1 : 0), k_step3_rest<RANGED, false>, SPA_THREADS, rsmem, &rest_per_sm));
     TSG_TRY(clear_counters(ctx, row0, TSG_CTR_STEP3, 2));
     TSG_TRY(tsg_alloc(ctx, &left, (size_t)P.tilemA + 1));
     TSG_CUDA(cudaMemsetAsync(left, 0, ((size_t)P.tilemA + 1) * sizeof(int), ctx->stream));
     k_step3_stg<RANGED><<<ctx->num_sms * per_sm, STG_THREADS, smem, ctx->stream>>>(P, d_kind, row0, row1,
                                                                                  &ctr[TSG_CTR_STEP3], left, ctx->d_status);
     TSG_LAUNCH_CHECK();
-    k_step3_rest<RANGED><<<ctx->num_sms * rest_per_sm, SPA_THREADS, rsmem, ctx->stream>>>(P, d_kind, left, row0, row1,
+    k_step3_rest<RANGED, false><<<ctx->num_sms * rest_per_sm, SPA_THREADS, rsmem, ctx->stream>>>(P, d_kind, left, row0, row1,
                                                                                        &ctr[TSG_CTR_REST]);
+    TSG_LAUNCH_CHECK();
+    tsg_release(ctx, left);
+    return TSG_OK;
+}
+
+// step 3 of narrow rows for tile rows [row0, row1), then the SPA kernel for the
+// rows it left
+template <bool RANGED>
+static int launch_step3_nar(tsg_context *ctx, const ProdView &P0, const tsg_tiled *A, WinScratch &W, const int *d_kind,
+                            int row0, int row1)
+{
+    ProdView P = P0;
+    P.status = ctx->d_status;
+    TSG_TRY(win_rows(ctx, P, A, W));
+    int *left = nullptr;
+    const int smem = WIN_WARPS * (int)sizeof(NarTask), rsmem = (int)sizeof(SpaSmem);
+    int per_sm = 0, rest_per_sm = 0;
+    TSG_TRY(resident_ctas(ctx, TSG_OCC_NAR, k_step3_nar, WIN_THREADS, smem, &per_sm));
+    TSG_TRY(resident_ctas(ctx, TSG_OCC_REST + (RANGED ? 1 : 0) + 2, k_step3_rest<RANGED, true>, SPA_THREADS, rsmem,
+                          &rest_per_sm));
+    TSG_TRY(clear_counters(ctx, row0, TSG_CTR_STEP3, 2));
+    TSG_TRY(tsg_alloc(ctx, &left, (size_t)P.tilemA + 1));
+    TSG_CUDA(cudaMemsetAsync(left, 0, ((size_t)P.tilemA + 1) * sizeof(int), ctx->stream));
+    const long long claims = (long long)(row1 - row0) * NAR_PER;
+    const long long grid = std::min((long long)ctx->num_sms * per_sm, (claims + WIN_WARPS - 1) / WIN_WARPS);
+    k_step3_nar<<<(unsigned)grid, WIN_THREADS, smem, ctx->stream>>>(P, W.Q, row0, row1, d_kind, left);
+    TSG_LAUNCH_CHECK();
+    k_step3_rest<RANGED, true><<<ctx->num_sms * rest_per_sm, SPA_THREADS, rsmem, ctx->stream>>>(
+        P, d_kind, left, row0, row1, &ctx->d_ctl->ctr[TSG_CTR_REST]);
     TSG_LAUNCH_CHECK();
     tsg_release(ctx, left);
     return TSG_OK;
@@ -699,15 +765,15 @@ static int launch_step3_spa_rows(tsg_context *ctx, const ProdView &P, const tsg_
         ctx->last_step3 = TSG_STEP3_WINDOWS;
         return launch_step3_win(ctx, P, A, W, row0, row1);
     }
-    const bool small = flat && P.numC <= (long long)SPA_BLK_SMALL * P.tilemA && P.numC < (long long)SPA_BLK * 6 * ctx->num_sms;
-    if (flat && !small && nnzC >= (long long)SPA_BLK_NARROW_VALUES * P.numC)
+    if (flat && P.numC <= (long long)NAR_MEAN * P.tilemA)
+    {
+        ctx->last_step3 = TSG_STEP3_NARROW;
+        return whole ? launch_step3_nar<false>(ctx, P, A, W, d_kind, row0, row1)
+                     : launch_step3_nar<true>(ctx, P, A, W, d_kind, row0, row1);
+    }
+    if (flat && nnzC >= (long long)SPA_BLK_NARROW_VALUES * P.numC)
         return whole ? launch_step3_spa<true, false, SPA_BLK_NARROW>(ctx, P, d_kind, false, 0, 0)
                      : launch_step3_spa<true, true, SPA_BLK_NARROW>(ctx, P, d_kind, false, row0, row1);
-    // narrow rows in too few blocks to go round (squares of grids' matrices: 64^2,
-    // 11 blocks of 256 tiles, 0.121 -> 0.043 ms; 256^2, 198 blocks, 0.123 -> 0.107)
-    if (small)
-        return whole ? launch_step3_spa<true, false, SPA_BLK_SMALL>(ctx, P, d_kind, false, 0, 0)
-                     : launch_step3_spa<true, true, SPA_BLK_SMALL>(ctx, P, d_kind, false, row0, row1);
     // mostly hypersparse rows (few values in many tiles): those by themselves
     const bool hyper = d_kind && nnzC < (long long)HYP_RATIO * P.numC && P.numC > (long long)S12_MAXT * P.tilemA;
     if (flat)

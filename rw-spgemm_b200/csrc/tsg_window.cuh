@@ -60,6 +60,26 @@ struct WinTask
     unsigned char tag[TSG_TAGS];
 };
 
+// Rows of few C tiles (grid matrices, thin bands): a row's 25 products leave
+// most of a CTA's 256 threads at its barriers, so a warp takes NAR_ROWS rows as
+// above, a batch holding the products of several.  A slot for every tile (of
+// NAR_ROWS rows, or fewer rows of more tiles) takes the place of the window,
+// found through a table by tile column.  Only the table's entries at C tiles
+// are set, and only those are read.
+#define NAR_ROWS 4   // rows per claim
+#define NAR_TILES 64 // (row, C tile) slots of the accumulator
+#define NAR_SPAN 384 // tile columns of the table
+// C tiles a tile row has on average, at most, in a product that takes this
+// form.  k_step3_spa<flat> and this one on a B200: 10 tiles (64^2 grid) 0.044 and
+// 0.024 ms, 12 (512^2) 0.364 and 0.137, 5 (65,536 rows, 3 entries) 0.114 and
+// 0.039; 48 (32,768 rows of 17 times one entry a row) 0.074 and 0.088.
+#define NAR_MEAN 32
+struct NarTask : WinTask
+{
+    unsigned char map[NAR_SPAN]; // tile column less the first -> C tile
+};
+static_assert(NAR_TILES * TSG_BS == WIN_COLS, "slots of a task");
+
 // Where the windows of a product lie.
 struct WinPlan
 {
@@ -144,13 +164,31 @@ struct WinEntry
     int b0, len;
 };
 
+// What a task covers: a part of a heavy row, a row's window, or whole rows
+// with a slot per C tile (NarTask).
+enum
+{
+    WIN_HEAVY_PART,
+    WIN_WINDOW,
+    WIN_WHOLE_ROWS
+};
+
 // entry x (none when x >= e1), column k of A
-// (WHOLE: [c0, c1) is a window)
-template <bool WHOLE>
+template <int FORM>
 __device__ __forceinline__ WinEntry win_entry(const ProdView &P, const WinPlan &Q, int x, int e1, int k, int c0, int c1)
 {
     WinEntry E = {0.0, 0, 0};
-    if (x < e1 && WHOLE && Q.wtab)
+    if (FORM == WIN_WHOLE_ROWS)
+    {
+        if (x < e1)
+        {
+            E.a = Q.A_rval[x];
+            E.b0 = P.B_rptr[k];
+            E.len = P.B_rptr[k + 1] - E.b0;
+        }
+        return E;
+    }
+    if (x < e1 && FORM == WIN_WINDOW && Q.wtab)
     {
         const int2 t = Q.wtab[(long long)k * Q.windows + c0 / WIN_COLS];
         E.a = Q.A_rval[x];
@@ -194,14 +232,17 @@ __device__ __forceinline__ int win_nth_column(unsigned mask, int n)
 // C row r of tile row I, columns [c0, c1); its A entries are [e0, e1) of the
 // row view (E: this lane's of the first 32, loaded by the caller), its C tiles
 // [t0, t1), at most 64.  All lanes of the warp call it.
+// WIN_WHOLE_ROWS: nr rows from r on, whose entries begin at `ends` of lanes 0
+// to nr - 1; c0 the first tile's column and c1 the tile columns to the last;
+// nr * (t1 - t0) at most 64.
 //
 // Loads go ahead of their use, since a warp of short rows would wait on one
 // chain of them after another: the entries' columns two groups of 32 ahead,
 // their parts of B one group, B's entries two batches, the row's masks and
 // value offsets from the start.
-template <bool WHOLE>
-__device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, WinTask &S, int I, int r, int c0, int c1,
-                                         int e0, int e1, WinEntry E, int t0, int t1, int lane)
+template <int FORM, class Task>
+__device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, Task &S, int I, int r, int c0, int c1,
+                                         int e0, int e1, WinEntry E, int t0, int t1, int lane, int nr = 1, int ends = 0)
 {
     const unsigned upto = 0xffffffffu >> (31 - lane); // lanes up to this one
     unsigned mk[2];
@@ -212,7 +253,18 @@ __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, Wi
         const int t = t0 + 32 * h + lane;
         mk[h] = 0u;
         at[h] = base[h] = 0;
-        if (t < t1)
+        if (FORM == WIN_WHOLE_ROWS)
+        {
+            const int q = 32 * h + lane, row = q / (t1 - t0);
+            if (row < nr)
+            {
+                const long long w = (long long)(t - row * (t1 - t0)) * TSG_BS + r + row;
+                base[h] = q * TSG_BS;
+                mk[h] = P.C_mask[w];
+                at[h] = P.C_tnnz[t - row * (t1 - t0)] + P.C_Ptr[w];
+            }
+        }
+        else if (t < t1)
         {
             base[h] = P.C_col[t] * TSG_BS - c0;
             mk[h] = P.C_mask[(long long)t * TSG_BS + r];
@@ -223,7 +275,7 @@ __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, Wi
     int k = e0 + 32 + lane < e1 ? Q.A_rcol[e0 + 32 + lane] : 0;
     for (int g = e0; g < e1; g += 32)
     {
-        const WinEntry nxt = win_entry<WHOLE>(P, Q, g + 32 + lane, e1, k, c0, c1);
+        const WinEntry nxt = win_entry<FORM>(P, Q, g + 32 + lane, e1, k, c0, c1);
         k = g + 64 + lane < e1 ? Q.A_rcol[g + 64 + lane] : 0;
         const int len = E.len;
         const unsigned full = __ballot_sync(TSG_FULL_MASK, len > 0);
@@ -249,6 +301,16 @@ __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, Wi
             S.a[at] = E.a;
             S.b[at] = E.b0 - pre;
             S.end[at] = incl;
+        }
+        if constexpr (FORM == WIN_WHOLE_ROWS)
+        {
+            // the slots of the entry's row
+            int row = 0;
+#pragma unroll
+            for (int q = 1; q < NAR_ROWS; q++)
+                row += g + lane >= __shfl_sync(TSG_FULL_MASK, ends, q) && q < nr ? 1 : 0;
+            if (len > 0)
+                S.pre[__popc(full & upto) - 1] = row * (t1 - t0) * TSG_BS;
         }
         __syncwarp();
         // batches of 32 products, a batch's loads issued two batches before its
@@ -278,7 +340,14 @@ __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, Wi
             if (item < total)
             {
                 const int bi = S.b[e] + item;
-                col = P.B_rcol[bi] - c0;
+                if constexpr (FORM == WIN_WHOLE_ROWS)
+                {
+                    const int c = P.B_rcol[bi], w = (c >> 4) - c0;
+                    if ((unsigned)w < (unsigned)c1)
+                        col = S.map[w] * TSG_BS + (c & 15) + S.pre[e];
+                }
+                else
+                    col = P.B_rcol[bi] - c0;
                 p = __dmul_rn(S.a[e], P.B_rval[bi]);
             }
         };
@@ -324,7 +393,7 @@ __device__ __forceinline__ void win_task(const ProdView &P, const WinPlan &Q, Wi
 #pragma unroll
     for (int h = 0; h < 2; h++)
     {
-        const unsigned m = base[h] >= 0 && base[h] < c1 - c0 ? mk[h] : 0u; // a heavy row's part holds some of the tiles
+        const unsigned m = FORM == WIN_WHOLE_ROWS || (base[h] >= 0 && base[h] < c1 - c0) ? mk[h] : 0u; // a heavy row's part holds some of the tiles
         const int len = __popc(m);
         const unsigned full = __ballot_sync(TSG_FULL_MASK, len > 0);
         if (!full)
@@ -390,7 +459,7 @@ __device__ __forceinline__ void win_claim_heavy(const ProdView &P, const WinPlan
     const int *ct = Q.ctab + (long long)(row / TSG_BS) * (Q.windows + 1) + part / WIN_PARTS;
     const int e0 = Q.A_rptr[row], e1 = Q.A_rptr[row + 1], c0 = part * WIN_PART, c1 = c0 + WIN_PART;
     const int k = e0 + lane < e1 ? Q.A_rcol[e0 + lane] : 0;
-    win_task<false>(P, Q, S, row / TSG_BS, row % TSG_BS, c0, c1, e0, e1, win_entry<false>(P, Q, e0 + lane, e1, k, c0, c1), ct[0],
+    win_task<WIN_HEAVY_PART>(P, Q, S, row / TSG_BS, row % TSG_BS, c0, c1, e0, e1, win_entry<WIN_HEAVY_PART>(P, Q, e0 + lane, e1, k, c0, c1), ct[0],
              ct[1], lane);
 }
 
@@ -417,18 +486,73 @@ __device__ __forceinline__ void win_claim_rows(const ProdView &P, const WinPlan 
     int k1 = col(0);
     int k2 = col(1);
     int e0 = __shfl_sync(TSG_FULL_MASK, e, 0), e1 = __shfl_sync(TSG_FULL_MASK, e, 1);
-    WinEntry E = win_entry<true>(P, Q, e0 + lane, e1, k1, c0, c1);
+    WinEntry E = win_entry<WIN_WINDOW>(P, Q, e0 + lane, e1, k1, c0, c1);
 #pragma unroll 1
     for (int i = 0; i < WIN_ROWS; i++)
     {
         const int e2 = __shfl_sync(TSG_FULL_MASK, e, min(i + 2, WIN_ROWS));
-        const WinEntry nxt = win_entry<true>(P, Q, e1 + lane, e2, k2, c0, c1);
+        const WinEntry nxt = win_entry<WIN_WINDOW>(P, Q, e1 + lane, e2, k2, c0, c1);
         k2 = col(i + 2);
         if (e0 < e1 && e1 - e0 < Q.heavy_min)
-            win_task<true>(P, Q, S, I, r0 + i, c0, c1, e0, e1, E, t0, t1, lane);
+            win_task<WIN_WINDOW>(P, Q, S, I, r0 + i, c0, c1, e0, e1, E, t0, t1, lane);
         e0 = e1;
         e1 = e2;
         E = nxt;
     }
 }
 
+// claim c of the tile rows from row0 on: NAR_ROWS rows of a tile row.  A wide
+// row (kind: the row kinds of the fused step 1/2 pass, or null) is left.
+#define NAR_PER (TSG_BS / NAR_ROWS)
+__device__ __forceinline__ void nar_claim(const ProdView &P, const WinPlan &Q, NarTask &S, int row0, unsigned c,
+                                          const int *__restrict__ kind, int *__restrict__ left, int lane)
+{
+    const int I = row0 + (int)(c / NAR_PER), r0 = (int)(c % NAR_PER) * NAR_ROWS;
+    const int t0 = P.C_ptr[I], t1 = P.C_ptr[I + 1];
+    const int ends = Q.A_rptr[min(I * TSG_BS + r0 + min(lane, NAR_ROWS), Q.mA)];
+    if (t0 == t1)
+        return;
+    if (kind ? kind[I] != 0 : t1 - t0 > S12_MAXT)
+    {
+        if (r0 == 0 && lane == 0)
+        {
+            left[I] = 1;
+            atomicAdd(&left[P.tilemA], 1);
+        }
+        return;
+    }
+    const int all0 = __shfl_sync(TSG_FULL_MASK, ends, 0), all1 = __shfl_sync(TSG_FULL_MASK, ends, NAR_ROWS);
+    if (all0 == all1)
+        return;
+    // the first rows' entries and the C tiles at once
+    int k = all0 + lane < all1 ? Q.A_rcol[all0 + lane] : 0;
+    for (int ta = t0; ta < t1;)
+    {
+        const int J0 = P.C_col[ta];
+        const int j0 = ta + lane < t1 ? P.C_col[ta + lane] - J0 : NAR_SPAN;
+        const int j1 = ta + 32 + lane < t1 ? P.C_col[ta + 32 + lane] - J0 : NAR_SPAN;
+        const bool in0 = j0 < NAR_SPAN, in1 = j1 < NAR_SPAN;
+        const int nt = __popc(__ballot_sync(TSG_FULL_MASK, in0)) + __popc(__ballot_sync(TSG_FULL_MASK, in1));
+        const int span = 1 + __reduce_max_sync(TSG_FULL_MASK, in1 ? j1 : in0 ? j0 : 0);
+        if (in0)
+            S.map[j0] = (unsigned char)lane;
+        if (in1)
+            S.map[j1] = (unsigned char)(lane + 32);
+        __syncwarp();
+        const int rows = nt <= NAR_TILES / 4 ? 4 : nt <= NAR_TILES / 2 ? 2 : 1;
+#pragma unroll 1
+        for (int r = 0; r < NAR_ROWS; r += rows)
+        {
+            const int e0 = __shfl_sync(TSG_FULL_MASK, ends, r), e1 = __shfl_sync(TSG_FULL_MASK, ends, r + rows);
+            const int mine = __shfl_sync(TSG_FULL_MASK, ends, min(r + lane, NAR_ROWS));
+            if (r > 0 || ta > t0)
+                k = e0 + lane < e1 ? Q.A_rcol[e0 + lane] : 0;
+            if (e0 < e1)
+                win_task<WIN_WHOLE_ROWS>(P, Q, S, I, r0 + r, J0, span, e0, e1,
+                                         win_entry<WIN_WHOLE_ROWS>(P, Q, e0 + lane, e1, k, 0, 0), ta, ta + nt, lane, rows,
+                                         mine);
+        }
+        __syncwarp();
+        ta += nt;
+    }
+}
