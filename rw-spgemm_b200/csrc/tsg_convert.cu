@@ -16,11 +16,15 @@
 
 #define HW_MASK(tid) (0xFFFFu << ((tid) & 16))
 
-// Tile rows of at least this many entries are listed (heavy[0] of them) and
-// done by a CTA each: the half-warp's merge takes one tile after another, a
-// chain of loads as long as the tile row.  An R-MAT matrix
-// of 16,384 rows, column view included: 1.65 -> 0.42 ms.
+// Tile rows of at least HEAVY_ENTRIES entries, or more than HEAVY_TILES tiles, are
+// listed (heavy[0] of them) and done by a CTA each: the half-warp's merge takes
+// one tile after another, a chain of loads as long as the tile row.  With column
+// view on a B200: R-MAT of 16,384 rows 1.65 -> 0.25 ms (entries alone 0.42),
+// 20,000 rows of 8 random entries 0.254 -> 0.161 (128 tiles a row), a band of 81
+// (6 tiles, 1,296 entries a row) 0.178 -> 0.123; a 48^3 grid's matrix, 22 tiles
+// and 432 entries a row, 0.199, 0.268 by CTAs.
 #define HEAVY_ENTRIES 512
+#define HEAVY_TILES 32
 #define HEAVY_THREADS 256
 
 // ---------------------------------------------------------------------------
@@ -56,7 +60,8 @@ __global__ void k_tile_count(int m, int tilem, const int *__restrict__ rowptr,
         const int jm = __reduce_min_sync(hmask, cur);
         if (jm == INT_MAX)
             break;
-        cnt++;
+        if (++cnt > HEAVY_TILES)
+            break;
         if (cur == jm)
         {
             do
@@ -67,7 +72,11 @@ __global__ void k_tile_count(int m, int tilem, const int *__restrict__ rowptr,
         }
     }
     if (lane == 0)
+    {
         tile_cnt[tr] = cnt;
+        if (cnt > HEAVY_TILES)
+            heavy[1 + atomicAdd(&heavy[0], 1)] = tr;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -94,7 +103,7 @@ __global__ void k_tile_fill(int m, int tilem, const int *__restrict__ rowptr,
         p = rowptr[r];
         e = rowptr[r + 1];
     }
-    if (__reduce_add_sync(hmask, e - p) >= HEAVY_ENTRIES)
+    if (tile_ptr[tr + 1] - tile_ptr[tr] > HEAVY_TILES || __reduce_add_sync(hmask, e - p) >= HEAVY_ENTRIES)
         return; // by k_tile_fill_cta
     // value offset of the tile row's first tile: the row's first CSR entry
     int run = __shfl_sync(hmask, p, 0, 16);
@@ -394,7 +403,7 @@ extern "C" int tsg_csr_to_tiled(tsg_context *ctx, int m, int n, int nnz, const i
     TSG_TRY(tsg_alloc(ctx, &out->tile_ptr, (size_t)tilem + 1));
     long long T = 0;
     int *heavy = nullptr;
-    const int most = std::min(tilem, nnz / HEAVY_ENTRIES); // tile rows that can be heavy
+    const int most = std::min(tilem, nnz / std::min(HEAVY_ENTRIES, HEAVY_TILES + 1)); // tile rows that can be heavy
     TSG_TRY(tsg_alloc(ctx, &heavy, (size_t)most + 1));
     TSG_CUDA(cudaMemsetAsync(heavy, 0, sizeof(int), ctx->stream));
     if (tilem > 0)

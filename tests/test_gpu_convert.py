@@ -31,6 +31,7 @@ SHAPES = [
     ("each", 16, 16 * 1100000, 80000), # one tile row of > 2048 steps: the 16-bit sums are emptied
     ("each", 48, 900, 31), ("each", 48, 900, 32), ("each", 37, 16 * 1024 + 5, 33),  # around 512 entries a tile row
     ("full", 37, 700, 0),              # a CTA each, full tiles, ragged
+    ("each", 69, 16 * 4000, 2), ("each", 69, 16 * 4000, 3),  # on both sides of 32 tiles a tile row
 ]
 
 
