@@ -21,6 +21,13 @@ extern "C" const char *tsg_last_error(void) { return g_last_error; }
 
 // ---------------------------------------------------------------------------
 // Exclusive scan: reduce-then-scan over blocks of SCAN_ITEMS * SCAN_THREADS.
+//
+// Bound: bytes (an int read twice and written once) for millions of items,
+// launches below.  A thread's items are two 16-byte words (item by item, a
+// load touched 32 sectors), and up to 8.4 M items every block adds up the sums
+// of those before it, without a launch that scans them.  Step 2 of a product,
+// whose last part is the scan of C's tile counts, on a B200: 16.4 M tiles 0.540
+// -> 0.479 ms, 1.4 M 0.039 -> 0.026, 21 K 0.031 -> 0.022.
 // ---------------------------------------------------------------------------
 #define SCAN_THREADS 1024
 #define SCAN_ITEMS 8
@@ -64,53 +71,94 @@ __device__ __forceinline__ T block_excl_scan(T v, T *s_warp, T *block_total)
     return res;
 }
 
+// a thread's SCAN_ITEMS consecutive items from i on (0 past n), by 16-byte
+// loads where they are ints on a 16-byte boundary
+template <typename TIn>
+__device__ __forceinline__ void scan_load(const TIn *in, long long i, long long n, bool wide, long long *v)
+{
+    if (sizeof(TIn) == 4 && wide && i + SCAN_ITEMS <= n)
+    {
+#pragma unroll
+        for (int q = 0; q < SCAN_ITEMS / 4; q++)
+        {
+            const int4 x = reinterpret_cast<const int4 *>(in + i)[q];
+            v[4 * q] = x.x;
+            v[4 * q + 1] = x.y;
+            v[4 * q + 2] = x.z;
+            v[4 * q + 3] = x.w;
+        }
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < SCAN_ITEMS; k++)
+        v[k] = i + k < n ? (long long)in[i + k] : 0;
+}
+
 template <typename TIn>
 __global__ void k_scan_reduce(const TIn *__restrict__ in, long long n, long long *__restrict__ partial)
 {
     __shared__ long long s_warp[33];
     long long base = (long long)blockIdx.x * SCAN_TILE;
+    long long v[SCAN_ITEMS];
+    scan_load(in, base + (long long)threadIdx.x * SCAN_ITEMS, n, ((uintptr_t)in & 15) == 0, v);
     long long sum = 0;
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; k++)
-    {
-        long long i = base + (long long)threadIdx.x * SCAN_ITEMS + k;
-        if (i < n)
-            sum += (long long)in[i];
-    }
+        sum += v[k];
     long long tot;
     block_excl_scan<long long>(sum, s_warp, &tot);
     if (threadIdx.x == 0)
         partial[blockIdx.x] = tot;
 }
 
-// Exclusive scan of each tile; offset[blockIdx] added (nullptr = 0).  Writes
-// out[n] = grand total from the last block.  in/out may alias.
-template <typename TIn, typename TOut>
+// Exclusive scan of each tile, offset by the tiles before: offset[blockIdx]
+// (nullptr = 0), or with SUMS the sum of offset[0..blockIdx), a word a thread.
+// Writes out[n] = grand total from the last block.  in/out may alias.
+template <typename TIn, typename TOut, bool SUMS = false>
 __global__ void k_scan_apply(const TIn *in, long long n, const long long *__restrict__ offset,
                              TOut *out, long long *total_out)
 {
     __shared__ long long s_warp[33];
     long long base = (long long)blockIdx.x * SCAN_TILE;
     long long v[SCAN_ITEMS];
+    const bool wide = (((uintptr_t)in | (uintptr_t)out) & 15) == 0;
+    const long long i = base + (long long)threadIdx.x * SCAN_ITEMS;
+    scan_load(in, i, n, wide, v);
     long long sum = 0;
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; k++)
-    {
-        long long i = base + (long long)threadIdx.x * SCAN_ITEMS + k;
-        v[k] = i < n ? (long long)in[i] : 0;
         sum += v[k];
-    }
     long long tot;
     long long run = block_excl_scan<long long>(sum, s_warp, &tot);
-    long long off = offset ? offset[blockIdx.x] : 0;
+    long long off = 0;
+    if (SUMS)
+        block_excl_scan<long long>(threadIdx.x < blockIdx.x ? offset[threadIdx.x] : 0, s_warp, &off);
+    else if (offset)
+        off = offset[blockIdx.x];
     run += off;
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; k++)
+    if (sizeof(TOut) == 4 && wide && i + SCAN_ITEMS <= n)
     {
-        long long i = base + (long long)threadIdx.x * SCAN_ITEMS + k;
-        if (i < n)
-            out[i] = (TOut)run;
-        run += v[k];
+#pragma unroll
+        for (int q = 0; q < SCAN_ITEMS / 4; q++)
+        {
+            int4 x;
+            x.x = (int)run;
+            x.y = (int)(run += v[4 * q]);
+            x.z = (int)(run += v[4 * q + 1]);
+            x.w = (int)(run += v[4 * q + 2]);
+            run += v[4 * q + 3];
+            reinterpret_cast<int4 *>(out + i)[q] = x;
+        }
+    }
+    else
+    {
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS; k++)
+        {
+            if (i + k < n)
+                out[i + k] = (TOut)run;
+            run += v[k];
+        }
     }
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == SCAN_THREADS - 1)
     {
@@ -157,8 +205,13 @@ int tsg_scan_counts(tsg_context *ctx, const int *in, int *out, long long n, long
         TSG_TRY(tsg_alloc(ctx, &partial, (size_t)nb + 1));
         k_scan_reduce<int><<<(unsigned)nb, SCAN_THREADS, 0, ctx->stream>>>(in, n, partial);
         TSG_LAUNCH_CHECK();
-        TSG_TRY(scan_partials(ctx, partial, nb));
-        k_scan_apply<int, int><<<(unsigned)nb, SCAN_THREADS, 0, ctx->stream>>>(in, n, partial, out, d_total);
+        if (nb <= SCAN_THREADS)
+            k_scan_apply<int, int, true><<<(unsigned)nb, SCAN_THREADS, 0, ctx->stream>>>(in, n, partial, out, d_total);
+        else
+        {
+            TSG_TRY(scan_partials(ctx, partial, nb));
+            k_scan_apply<int, int><<<(unsigned)nb, SCAN_THREADS, 0, ctx->stream>>>(in, n, partial, out, d_total);
+        }
         TSG_LAUNCH_CHECK();
         tsg_release(ctx, partial);
     }
