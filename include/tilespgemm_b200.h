@@ -304,7 +304,7 @@ typedef struct
 
 /* tsg_spgemm_info.step3_kernel */
 #define TSG_STEP3_NONE 0   /* C has no nonzeros                               */
-#define TSG_STEP3_TILES 1  /* k_step3: half-warp per C tile                   */
+#define TSG_STEP3_TILES 1  /* k_step3: half-warp per C tile, a lane per column */
 #define TSG_STEP3_ELEMS 2  /* k_step3_elems: warp per C tile, per element     */
 #define TSG_STEP3_ROWS 3   /* k_step3_rows: half-warp per run of C tiles      */
 #define TSG_STEP3_FLAT 4   /* k_step3_spa<flat>: SPA, CTA per C tile block    */
@@ -314,6 +314,8 @@ typedef struct
 #define TSG_STEP3_WINDOWS 7 /* k_step3_win: warp per C row and column window */
 #define TSG_STEP3_NARROW 8 /* k_step3_nar: warp per C rows of few tiles, then
                               k_step3_rest                                   */
+#define TSG_STEP3_TILE_ROWS 9 /* k_step3_tile_rows: half-warp per C tile, a lane
+                               * per row: A tiles of few values              */
 
 const char *tsg_status_string(int status);
 /* Message describing the last failure on the calling thread. */

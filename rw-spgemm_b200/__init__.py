@@ -67,7 +67,8 @@ class TsgTiled(ctypes.Structure):
 
 
 STEP3_KERNELS = {0: "none", 1: "k_step3", 2: "k_step3_elems", 3: "k_step3_rows", 4: "k_step3_spa<flat>",
-                 5: "k_step3_spa", 6: "k_step3_stg + k_step3_rest", 7: "k_step3_win", 8: "k_step3_nar"}
+                 5: "k_step3_spa", 6: "k_step3_stg + k_step3_rest", 7: "k_step3_win", 8: "k_step3_nar",
+                 9: "k_step3_tile_rows"}
 
 
 class TsgInfo(ctypes.Structure):

@@ -78,7 +78,8 @@ struct tsg_batch
     long long *d_s1off, *d_winoff;
     int4 *d_wlist, *d_hlist; // wide units of step 2; heavy rows' parts of the window step 3
     int *win_tables;
-    long long *d_denseoff;      // C tiles of the products with dense tiles, prefix
+    long long *d_denseoff;      // C tiles of the products with dense tiles, prefixes (rows form, columns form)
+    int rows_form, cols_form;   // products of either form of the tile kernel
     cudaStream_t side[2];       // step 3's kernels run beside one another
     cudaEvent_t fork, join[2];
     int split;   // A entries of a unit of step 2's wide rows
@@ -558,19 +559,24 @@ __global__ void __launch_bounds__(NT)
     // k_batch_spa3 and k_batch_dense3, each at its own occupancy)
     if (SCHED == 3)
     {
-        // C tiles of the products that take the tile kernel, prefix
+        // C tiles of the products that take the tile kernel by rows, prefix,
+        // and by columns
         if (blockIdx.x == 0)
-        {
-            for (int p = threadIdx.x; p < count; p += NT)
+            for (int cols = 0; cols < 2; cols++)
             {
-                const BatchProd &bp = prods[p];
-                denseoff[p] = !bp.status && bp.numC > 0 && bp.nnzC >= (long long)dense * bp.numC ? bp.numC : 0;
+                long long *off = denseoff + cols * ((long long)count + 1);
+                for (int p = threadIdx.x; p < count; p += NT)
+                {
+                    const BatchProd &bp = prods[p];
+                    off[p] = bp.P.cols == cols && !bp.status && bp.numC > 0 && bp.nnzC >= (long long)dense * bp.numC
+                                 ? bp.numC
+                                 : 0;
+                }
+                __syncthreads();
+                const long long all = block_scan_ll<NT>(off, count, s_tmp);
+                if (threadIdx.x == 0)
+                    off[count] = all;
             }
-            __syncthreads();
-            const long long all = block_scan_ll<NT>(denseoff, count, s_tmp);
-            if (threadIdx.x == 0)
-                denseoff[count] = all;
-        }
         return;
     }
     if (SCHED == 2)
@@ -588,6 +594,7 @@ __global__ void __launch_bounds__(NT)
     else
     {
         double *tA = reinterpret_cast<double *>(s_raw) + hw * S3T_WORDS;
+        bool clear = false; // tA is all zero, as step3_tile_rows takes and leaves it
         const long long total_items = itemoff[count];
         for (long long h = (long long)blockIdx.x * (NT / 16) + hw; h < total_items; h += nhw)
         {
@@ -598,8 +605,18 @@ __global__ void __launch_bounds__(NT)
             const long long item = h - itemoff[p];
             if (SCHED == 1)
                 step3_rows_item<W, CAP>(P, item, hmask, lane, reinterpret_cast<S3RowsSmem<W, CAP> *>(s_raw)[hw]);
+            else if (SCHED == 0 && P.cols)
+            {
+                step3_tile_cols(P, (int)item, hmask, lane, tA);
+                clear = false;
+            }
             else
-                step3_tile(P, (int)item, hmask, lane, tA);
+            {
+                if (!clear)
+                    step3_tile_clear(tA, hmask, lane);
+                step3_tile_rows(P, (int)item, hmask, lane, tA);
+                clear = true;
+            }
         }
     }
     __syncthreads();
@@ -777,11 +794,12 @@ __global__ void __launch_bounds__(WIN_THREADS, WIN_CTAS)
 }
 
 // ... and products with dense C tiles (>= the batch's threshold of values per
-// tile on average): the tile kernel, a half-warp per C tile of theirs
-// (denseoff: their tiles, prefix; walked among the tiles of all products,
-// finding out cost four times the work).
+// tile on average): the tile kernel in the form of their A tiles (P.cols), a
+// half-warp per C tile of theirs (denseoff: their tiles, prefix; walked among
+// the tiles of all products, finding out cost four times the work).
 #define DENSE3_THREADS 128
-__global__ void __launch_bounds__(DENSE3_THREADS, 4)
+template <bool COLS>
+__global__ void __launch_bounds__(DENSE3_THREADS, COLS ? 4 : 8)
     k_batch_dense3(BatchProd *prods, int count, const long long *__restrict__ denseoff, const long long *__restrict__ itemoff,
                    const int *err)
 {
@@ -793,11 +811,16 @@ __global__ void __launch_bounds__(DENSE3_THREADS, 4)
     const long long total_items = denseoff[count];
     if (total_items == 0)
         return;
+    if (!COLS)
+        step3_tile_clear(s_A[hw], hmask, lane);
     const long long nhw = (long long)gridDim.x * (DENSE3_THREADS / 16);
     for (long long h = (long long)blockIdx.x * (DENSE3_THREADS / 16) + hw; h < total_items; h += nhw)
     {
         const int p = find_product(denseoff, count, h);
-        step3_tile(prods[p].P, (int)(h - denseoff[p]), hmask, lane, s_A[hw]);
+        if (COLS)
+            step3_tile_cols(prods[p].P, (int)(h - denseoff[p]), hmask, lane, s_A[hw]);
+        else
+            step3_tile_rows(prods[p].P, (int)(h - denseoff[p]), hmask, lane, s_A[hw]);
     }
     __syncthreads();
     if (threadIdx.x == 0)
@@ -928,8 +951,10 @@ extern "C" int tsg_product_bounds(tsg_context *ctx, const tsg_tiled *A, const ts
 typedef void (*batch_kernel_t)(BatchProd *, int, const long long *, const long long *, int4 *, int, long long *,
                                int, long long *, unsigned *, int *, int *);
 
-// Kernel, dynamic shared memory and block size of a batch schedule.
-static batch_kernel_t pick_kernel(const tsg_batch_params &p, size_t *smem, int *threads)
+// Kernel, dynamic shared memory and block size of a batch schedule.  cols:
+// some product takes the columns form of the tile kernel, whose registers would
+// halve the blocks of a batch that has none (SCHED 4).
+static batch_kernel_t pick_kernel(const tsg_batch_params &p, bool cols, size_t *smem, int *threads)
 {
     *threads = BATCH_THREADS;
     const size_t s1a = (size_t)(BATCH_THREADS / 32) * S1_WORDS * 4;
@@ -953,7 +978,7 @@ static batch_kernel_t pick_kernel(const tsg_batch_params &p, size_t *smem, int *
     {
         const size_t s3 = (size_t)(BATCH_THREADS / 16) * S3T_WORDS * 8;
         *smem = s1 > s3 ? s1 : s3;
-        return k_batch<0, 8, 256, BATCH_THREADS>;
+        return cols ? k_batch<0, 8, 256, BATCH_THREADS> : k_batch<4, 8, 256, BATCH_THREADS>;
     }
 #define TSG_PICK(w, c)                                                                          \
     if (p.seg_tiles == w && p.acc_cap == c)                                                     \
@@ -975,7 +1000,7 @@ static int record_run(tsg_batch *b, cudaStream_t st)
 {
     size_t smem;
     int threads;
-    batch_kernel_t kern = pick_kernel(b->params, &smem, &threads);
+    batch_kernel_t kern = pick_kernel(b->params, b->cols_form > 0, &smem, &threads);
     TSG_CUDA(cudaMemsetAsync(b->d_err, 0, sizeof(int), st));
     TSG_CUDA(cudaMemsetAsync(b->d_bar, 0, sizeof(unsigned), st));
     // phase stamps (after the two item prefixes): [7] is a running maximum
@@ -1016,9 +1041,18 @@ static int record_run(tsg_batch *b, cudaStream_t st)
     k_batch_spa3<<<b->grid3, SPA_THREADS, sizeof(SpaSmem), b->side[0]>>>(b->d_prod, b->count, b->d_itemoff, b->d_bar,
                                                                        b->d_err, b->dense);
     TSG_CUDA(cudaGetLastError());
-    k_batch_dense3<<<b->ctx->num_sms * 4, DENSE3_THREADS, 0, b->side[1]>>>(b->d_prod, b->count, b->d_denseoff,
-                                                                         b->d_itemoff, b->d_err);
-    TSG_CUDA(cudaGetLastError());
+    if (b->rows_form)
+    {
+        k_batch_dense3<false><<<b->ctx->num_sms * 8, DENSE3_THREADS, 0, b->side[1]>>>(b->d_prod, b->count, b->d_denseoff,
+                                                                                    b->d_itemoff, b->d_err);
+        TSG_CUDA(cudaGetLastError());
+    }
+    if (b->cols_form)
+    {
+        k_batch_dense3<true><<<b->ctx->num_sms * 4, DENSE3_THREADS, 0, b->side[1]>>>(
+            b->d_prod, b->count, b->d_denseoff + b->count + 1, b->d_itemoff, b->d_err);
+        TSG_CUDA(cudaGetLastError());
+    }
     for (int q = 0; q < 2; q++)
     {
         TSG_CUDA(cudaEventRecord(b->join[q], b->side[q]));
@@ -1051,7 +1085,10 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
         return tsg_set_error(TSG_ERR_INVALID, "dense threshold %d outside [0, 257]", prm.dense_threshold);
     size_t smem;
     int threads;
-    batch_kernel_t kern = pick_kernel(prm, &smem, &threads);
+    int cols_form = 0;
+    for (int p = 0; p < count; p++)
+        cols_form += step3_by_columns(&A[p]);
+    batch_kernel_t kern = pick_kernel(prm, cols_form > 0, &smem, &threads);
     if (!kern)
         return tsg_set_error(TSG_ERR_INVALID, "unsupported batch schedule (%d, %d, %d)", prm.schedule, prm.seg_tiles,
                              prm.acc_cap);
@@ -1075,6 +1112,8 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
     b->n.resize(count);
     b->tilen.resize(count);
     b->launches = 0;
+    b->cols_form = cols_form;
+    b->rows_form = count - cols_form;
     // bounds and arena layout
     size_t bytes = 0;
     std::vector<size_t> off(count);
@@ -1185,7 +1224,7 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
         tsg_batch_destroy(b);
         return tsg_set_error(TSG_ERR_CUDA, "batch streams: %s", cudaGetErrorString(se));
     }
-    if ((st = tsg_alloc(ctx, &b->d_denseoff, (size_t)count + 1)) != TSG_OK ||
+    if ((st = tsg_alloc(ctx, &b->d_denseoff, 2 * ((size_t)count + 1))) != TSG_OK ||
         (b->wins && ((st = tsg_alloc(ctx, &b->win_tables, (size_t)table_words)) != TSG_OK ||
                      (st = tsg_alloc(ctx, &b->d_hlist, (size_t)hparts)) != TSG_OK ||
                      (st = tsg_alloc(ctx, &b->d_winoff, b->winoff.size())) != TSG_OK)) ||
@@ -1235,6 +1274,7 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
         P.mB = B[p].m;
         P.nB = B[p].n;
         P.browB = B[p].m > 0 ? (int)(B[p].nnz / B[p].m) : 0;
+        P.cols = step3_by_columns(&A[p]);
         P.tilenB = B[p].tilen;
         P.C_ptr = (int *)take(((size_t)A[p].tilem + 1) * 4);
         h.wide = (int *)take((size_t)A[p].tilem * 4);

@@ -38,6 +38,7 @@ struct ProdView
     const double *A_rval;
     int mA, mB, nB;
     int browB; // mean entries per row of B (rounded down)
+    int cols;  // the tile kernel holds C by columns (S3T_MEAN)
     int tilenB;
     int *C_ptr, *C_col, *C_row, *C_tnnz;
     unsigned short *C_mask;
@@ -666,8 +667,9 @@ __device__ __forceinline__ void step2_tile(const ProdView &P, int t, unsigned hm
     step2_store(P, t, hmask, lane, acc, s_bins);
 }
 
-// Step 3 of one C tile by a half-warp: lane c holds column c of the C tile,
-// its 16 rows in registers.  For every matched pair, k ascending:
+// Step 3 of one C tile by a half-warp, for products of dense A tiles: lane c
+// holds column c of the C tile, its 16 rows in registers.  For every matched
+// pair, k ascending:
 //  - an A tile of at least S3T_DENSE values is spread into shared memory
 //    (column by column, zeros where it has no entry) and B's column c into
 //    registers, and the pair is one 16x16x16 product without any index: 8
@@ -682,14 +684,14 @@ __device__ __forceinline__ void step2_tile(const ProdView &P, int t, unsigned hm
 //
 // Bound: the FP64 pipe on dense tiles (32 instructions per k and two tiles).
 // Before, lane r walked row r's entries through a shared-memory row: a
-// load-add-store and a column byte per product.: a band of 81 times a band of
-// 81, 16,384 rows (107 M products), 0.345 -> 0.123 ms on a B200.
+// load-add-store and a column byte per product (step3_tile_rows): a band of 81
+// times a band of 81, 16,384 rows (107 M products), 0.345 -> 0.123 ms on a B200.
 #define S3T_DENSE 64
 #define S3T_STRIDE 18 // doubles per column of the spread A tile: 16-byte loads, stores spread over the banks
 #define S3T_WORDS (TSG_BS * S3T_STRIDE)
 
 // sA: S3T_WORDS doubles of this half-warp, 16-byte aligned
-__device__ __forceinline__ void step3_tile(const ProdView &P, int t, unsigned hmask, int lane, double *sA)
+__device__ __forceinline__ void step3_tile_cols(const ProdView &P, int t, unsigned hmask, int lane, double *sA)
 {
     const int cb = P.C_tnnz[t];
     if (P.C_tnnz[t + 1] == cb)
@@ -772,6 +774,93 @@ __device__ __forceinline__ void step3_tile(const ProdView &P, int t, unsigned hm
             P.C_Colb[p] = (unsigned char)lane;
         }
     }
+}
+
+// ... and for products of sparser A tiles: lane r walks row r's entries through
+// the row of the C tile it holds in shared memory, the 16 rows of an A tile at
+// once.  Entry by entry, all lanes to one entry, the columns form takes 2 to 5
+// times as long: 64^3 stencil 3.13 and 15.8 ms, a 512^2 grid 0.187 and 0.79,
+// 4,096 random rows of 16 entries 0.72 and 3.5 (B200, tile schedule).
+//
+// S3T_MEAN: values of A per tile, on average, from which a product takes the
+// columns form.  Tile-tridiagonal A of 65,536 rows, rows form and columns form:
+// 48 values in every tile 0.069 and 0.144 ms, 64 0.088 and 0.065, 96 0.127 and
+// 0.069; bands, where some tiles are below S3T_DENSE: 13 wide (69 on average)
+// 0.102 and 0.090, 21 wide 0.156 and 0.149, 25 wide 0.188 and 0.066.
+#define S3T_MEAN 64
+static inline int step3_by_columns(const tsg_tiled *A)
+{
+    return A->nnz >= (long long)S3T_MEAN * A->numtile;
+}
+
+#define S3R_STRIDE 17
+static_assert(TSG_BS * S3R_STRIDE <= S3T_WORDS, "one half-warp's words hold either form");
+
+// acc: 16 x S3R_STRIDE doubles of this half-warp, all zero on entry and on exit
+__device__ __forceinline__ void step3_tile_rows(const ProdView &P, int t, unsigned hmask, int lane, double *acc)
+{
+    const int cb = P.C_tnnz[t], cn = P.C_tnnz[t + 1] - cb;
+    if (cn == 0)
+        return;
+    const int i = P.C_row[t], j = P.C_col[t];
+    const int abase = P.A_ptr[i], la = P.A_ptr[i + 1] - abase;
+    const int bbase = P.B_cptr[j], lb = P.B_cptr[j + 1] - bbase;
+    double *myrow = acc + lane * S3R_STRIDE;
+    intersect_tiles(hmask, lane, P.A_col, abase, la, P.B_crow, P.B_cpos, bbase, lb, [&](int posA, int posB) {
+        const int a0 = P.A_tnnz[posA], na = P.A_tnnz[posA + 1] - a0;
+        const int sa = P.A_Ptr[(long long)posA * TSG_BS + lane];
+        const int ea = lane == TSG_BS - 1 ? na : P.A_Ptr[(long long)posA * TSG_BS + lane + 1];
+        const int b0 = P.B_tnnz[posB], nb = P.B_tnnz[posB + 1] - b0;
+        const unsigned char *bp = P.B_Ptr + (long long)posB * TSG_BS;
+        for (int x = sa; x < ea; x++)
+        {
+            const int ca = P.A_Colb[a0 + x] & 15;
+            const double a = P.A_Val[a0 + x];
+            const int sb = bp[ca];
+            const int eb = ca == TSG_BS - 1 ? nb : bp[ca + 1];
+            for (int y = sb; y < eb; y++)
+            {
+                const int c = P.B_Colb[b0 + y] & 15;
+                myrow[c] = __dadd_rn(myrow[c], __dmul_rn(a, P.B_Val[b0 + y]));
+            }
+        }
+    });
+    __syncwarp(hmask);
+    const int excl = P.C_Ptr[(long long)t * TSG_BS + lane];
+    const unsigned mrev = __brev((unsigned)P.C_mask[(long long)t * TSG_BS + lane]) >> 16;
+    // every lane runs the same trip count so the shuffles see all 16 lanes
+    for (int pb = 0; pb < cn; pb += 16)
+    {
+        const int p = pb + lane;
+        int r = 0;
+#pragma unroll
+        for (int s = 8; s >= 1; s >>= 1)
+        {
+            const int v = __shfl_sync(hmask, excl, r + s, 16);
+            if (v <= p)
+                r += s;
+        }
+        const unsigned mr = __shfl_sync(hmask, mrev, r, 16);
+        const int rank = p - __shfl_sync(hmask, excl, r, 16);
+        if (p < cn)
+        {
+            const int c = (int)__fns(mr, 0, rank + 1) & 15;
+            double *cell = acc + r * S3R_STRIDE + c;
+            P.C_Colb[cb + p] = (unsigned char)c;
+            P.C_Val[cb + p] = *cell;
+            *cell = 0.0;
+        }
+    }
+    __syncwarp(hmask);
+}
+
+// acc: S3T_WORDS doubles of this half-warp
+__device__ __forceinline__ void step3_tile_clear(double *acc, unsigned hmask, int lane)
+{
+    __syncwarp(hmask);
+    for (int q = lane; q < TSG_BS * S3R_STRIDE; q += 16)
+        acc[q] = 0.0;
+    __syncwarp(hmask);
 }
 
 // ---------------------------------------------------------------------------

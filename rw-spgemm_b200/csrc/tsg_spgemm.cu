@@ -177,7 +177,21 @@ __global__ void __launch_bounds__(S3_THREADS, 4) k_step3(ProdView P)
     __shared__ __align__(16) double s_A[S3_HW][S3T_WORDS];
     const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
     if (t < P.numC)
-        step3_tile(P, (int)t, TSG_HW_MASK(threadIdx.x), threadIdx.x & 15, s_A[threadIdx.x >> 4]);
+        step3_tile_cols(P, (int)t, TSG_HW_MASK(threadIdx.x), threadIdx.x & 15, s_A[threadIdx.x >> 4]);
+}
+
+#define S3R_THREADS 256
+
+__global__ void __launch_bounds__(S3R_THREADS) k_step3_tile_rows(ProdView P)
+{
+    __shared__ double s_acc[S3R_THREADS / 16][TSG_BS * S3R_STRIDE];
+    const int lane = threadIdx.x & 15;
+    const unsigned hmask = TSG_HW_MASK(threadIdx.x);
+    double *acc = s_acc[threadIdx.x >> 4];
+    step3_tile_clear(acc, hmask, lane);
+    const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
+    if (t < P.numC)
+        step3_tile_rows(P, (int)t, hmask, lane, acc);
 }
 
 __global__ void __launch_bounds__(256) k_step3_elems(ProdView P)
@@ -455,6 +469,7 @@ static ProdView make_view(const tsg_tiled *A, const tsg_tiled *B, tsg_tiled *C)
     P.mB = B->m;
     P.nB = B->n;
     P.browB = B->m > 0 ? (int)(B->nnz / B->m) : 0;
+    P.cols = step3_by_columns(A);
     P.tilenB = B->tilen;
     P.C_ptr = C->tile_ptr;
     P.C_col = C->tile_columnidx;
@@ -813,8 +828,11 @@ static int launch_step3(tsg_context *ctx, const ProdView &P, const tsg_tiled *A,
         TSG_LAUNCH_CHECK();
         return TSG_OK;
     }
-    ctx->last_step3 = TSG_STEP3_TILES;
-    k_step3<<<tsg_blocks((long long)P.numC * 16, S3_THREADS), S3_THREADS, 0, ctx->stream>>>(P);
+    ctx->last_step3 = P.cols ? TSG_STEP3_TILES : TSG_STEP3_TILE_ROWS;
+    if (P.cols)
+        k_step3<<<tsg_blocks((long long)P.numC * 16, S3_THREADS), S3_THREADS, 0, ctx->stream>>>(P);
+    else
+        k_step3_tile_rows<<<tsg_blocks((long long)P.numC * 16, S3R_THREADS), S3R_THREADS, 0, ctx->stream>>>(P);
     TSG_LAUNCH_CHECK();
     return TSG_OK;
 }
