@@ -41,6 +41,8 @@ enum
     TSG_OCC_WIN = 14,
     TSG_OCC_NAR,
     TSG_OCC_HYPER,
+    TSG_OCC_WIDE, // + 1,024 threads
+    TSG_OCC_WIDE_WIDER,
     TSG_OCC_COUNT
 };
 

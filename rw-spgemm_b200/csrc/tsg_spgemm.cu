@@ -554,16 +554,21 @@ static int clear_counters(tsg_context *ctx, int row0, int first, int count)
     return TSG_OK;
 }
 
-// step 2 for the rows k_step12 listed, through B's row view
+// step 2 for the rows k_step12 listed, through B's row view.  span: at most
+// WIDE_NARROW tile columns (512 threads) or WIDE_SPAN (1,024).  The kernel's
+// shared-memory limit belongs to the function on the device, not to the launch:
+// it is set to the largest size only, since a context on another host thread
+// that set a smaller one between this one's set and launch would make the
+// launch fail.
+#define WIDE_NARROW 512
 template <int NT>
 static int launch_step2_cta(tsg_context *ctx, const ProdView &P, int span, const int *d_wide, int *d_bins)
 {
-    const int smem = (int)wide_smem<NT>(span);
-    TSG_CUDA(cudaFuncSetAttribute(k_step2_cta<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     int per_sm = 0;
-    TSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step2_cta<NT>, NT, smem));
-    const int grid = std::min(P.tilemA, ctx->num_sms * std::max(per_sm, 1));
-    k_step2_cta<NT><<<grid, NT, smem, ctx->stream>>>(P, span, d_wide, &ctx->d_ctl->ctr[TSG_CTR_STEP2], d_bins);
+    TSG_TRY(resident_ctas(ctx, NT == 512 ? TSG_OCC_WIDE : TSG_OCC_WIDE_WIDER, k_step2_cta<NT>, NT,
+                          (int)wide_smem<NT>(NT == 512 ? WIDE_NARROW : WIDE_SPAN), &per_sm));
+    const int grid = std::min(P.tilemA, ctx->num_sms * per_sm);
+    k_step2_cta<NT><<<grid, NT, wide_smem<NT>(span), ctx->stream>>>(P, span, d_wide, &ctx->d_ctl->ctr[TSG_CTR_STEP2], d_bins);
     TSG_LAUNCH_CHECK();
     return TSG_OK;
 }
@@ -575,8 +580,8 @@ static int launch_step2_wide(tsg_context *ctx, const ProdView &P, int widest, co
     // 0.073 ms, 0.083 with 1,024 threads; 16,384 columns of R-MAT 14: 0.45 and
     // 0.38)
     const int span = std::max(1, std::min(widest, WIDE_SPAN));
-    return span <= 512 ? launch_step2_cta<512>(ctx, P, span, d_wide, d_bins)
-                       : launch_step2_cta<1024>(ctx, P, span, d_wide, d_bins);
+    return span <= WIDE_NARROW ? launch_step2_cta<512>(ctx, P, span, d_wide, d_bins)
+                               : launch_step2_cta<1024>(ctx, P, span, d_wide, d_bins);
 }
 
 // What the window form of step 3 keeps for a product.
