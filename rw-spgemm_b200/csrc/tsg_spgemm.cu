@@ -562,26 +562,29 @@ static int clear_counters(tsg_context *ctx, int row0, int first, int count)
 // launch fail.
 #define WIDE_NARROW 512
 template <int NT>
-static int launch_step2_cta(tsg_context *ctx, const ProdView &P, int span, const int *d_wide, int *d_bins)
+static int launch_step2_cta(tsg_context *ctx, const ProdView &P, int span, size_t units, const int *d_wide, int *d_bins)
 {
     int per_sm = 0;
     TSG_TRY(resident_ctas(ctx, NT == 512 ? TSG_OCC_WIDE : TSG_OCC_WIDE_WIDER, k_step2_cta<NT>, NT,
                           (int)wide_smem<NT>(NT == 512 ? WIDE_NARROW : WIDE_SPAN), &per_sm));
-    const int grid = std::min(P.tilemA, ctx->num_sms * per_sm);
+    // units, not tile rows: few rows of A may be many parts of rows (64 rows of
+    // 1,000 entries times 1 M rows: 4.0 ms on 4 CTAs, 0.33 on 64)
+    const int grid = (int)std::min(units, (size_t)ctx->num_sms * per_sm);
     k_step2_cta<NT><<<grid, NT, wide_smem<NT>(span), ctx->stream>>>(P, span, d_wide, &ctx->d_ctl->ctr[TSG_CTR_STEP2], d_bins);
     TSG_LAUNCH_CHECK();
     return TSG_OK;
 }
 
-static int launch_step2_wide(tsg_context *ctx, const ProdView &P, int widest, const int *d_wide, int *d_bins)
+static int launch_step2_wide(tsg_context *ctx, const ProdView &P, int widest, size_t units, const int *d_wide,
+                             int *d_bins)
 {
     // the widest row of C, or as many columns as a CTA's shared memory holds;
     // narrow C leaves room for four CTAs of 512 threads on an SM (8,192 columns:
     // 0.073 ms, 0.083 with 1,024 threads; 16,384 columns of R-MAT 14: 0.45 and
     // 0.38)
     const int span = std::max(1, std::min(widest, WIDE_SPAN));
-    return span <= WIDE_NARROW ? launch_step2_cta<512>(ctx, P, span, d_wide, d_bins)
-                               : launch_step2_cta<1024>(ctx, P, span, d_wide, d_bins);
+    return span <= WIDE_NARROW ? launch_step2_cta<512>(ctx, P, span, units, d_wide, d_bins)
+                               : launch_step2_cta<1024>(ctx, P, span, units, d_wide, d_bins);
 }
 
 // What the window form of step 3 keeps for a product.
@@ -846,6 +849,7 @@ static int launch_step3(tsg_context *ctx, const ProdView &P, const tsg_tiled *A,
 struct SpgemmRun
 {
     int *d_wide; // row kinds of the fused pass, or null
+    size_t units;     // units of the wide step 2 at most
     int widest;       // widest window of a C tile row, in tile columns
     StepOneBits bits; // step 1's bitmaps, until the emit pass has read them
     WinScratch win;
@@ -913,7 +917,8 @@ static int spgemm_structure(tsg_context *ctx, const tsg_tiled *A, const tsg_tile
         if (fused)
         {
             const int split = wide_split(A->nnz, ctx->num_sms);
-            TSG_TRY(tsg_alloc(ctx, &R.d_wide, (size_t)tilem + 3 + 2 * wide_units(tilem, A->nnz, split)));
+            R.units = wide_units(tilem, A->nnz, split);
+            TSG_TRY(tsg_alloc(ctx, &R.d_wide, (size_t)tilem + 3 + 2 * R.units));
             TSG_CUDA(cudaMemsetAsync(R.d_wide + tilem, 0, 2 * sizeof(int), st));
             k_step12<<<tsg_blocks(tilem, S12_WARPS), S12_WARPS * 32, 0, st>>>(P, R.bits, split, R.d_wide, d_bins);
             TSG_LAUNCH_CHECK();
@@ -934,7 +939,7 @@ static int spgemm_structure(tsg_context *ctx, const tsg_tiled *A, const tsg_tile
     {
         ProdView P = make_view(A, B, C);
         if (fused && P.B_rptr)
-            TSG_TRY(launch_step2_wide(ctx, P, R.widest, R.d_wide, d_bins));
+            TSG_TRY(launch_step2_wide(ctx, P, R.widest, R.units, R.d_wide, d_bins));
         else if (fused)
         {
             k_step2_wide<<<tsg_blocks(numC * 16, 256), 256, 0, st>>>(P, R.d_wide, d_bins);

@@ -1,0 +1,39 @@
+"""Products and conversions whose time must not depend on what their data does
+not hold: the best of a few runs against a bound several times the measured
+time (B200) and well below what the fault took that each stands for."""
+import numpy as np
+import pytest
+
+from test_gpu_unstructured import _tiled
+
+pytestmark = pytest.mark.gpu
+
+
+def _fixed(m, n, e, seed):
+    """m rows of about e entries spread over all n columns."""
+    rng = np.random.default_rng(seed)
+    c = np.sort(rng.integers(0, n, (m, e)), axis=1)
+    keep = np.ones((m, e), bool)
+    keep[:, 1:] = c[:, 1:] != c[:, :-1]
+    rp = np.concatenate([[0], np.cumsum(keep.sum(1))]).astype(np.int32)
+    return m, n, rp, c[keep].astype(np.int32), rng.uniform(-1, 1, int(keep.sum()))
+
+
+def _best_steps(tsg, A, B, runs=4):
+    ctx = tsg.Context(0, timing=True)
+    tA, tB = _tiled(tsg, ctx, A, tsg.TSG_TILED_CSC_VIEW), _tiled(tsg, ctx, B, tsg.TSG_TILED_CSC_VIEW)
+    best = [1e9] * 3
+    for _ in range(runs):
+        C, info = tsg.spgemm(ctx, tA, tB)
+        C.free()
+        best = [min(b, info[f"ms_step{q + 1}"]) for q, b in enumerate(best)]
+    for t in (tA, tB):
+        t.free()
+    ctx.close()
+    return best
+
+
+def test_few_rows_of_a_split_over_the_gpu(tsg):
+    """64 rows of 1,000 entries are 64 parts of wide rows: 4.2 ms on a CTA per
+    tile row."""
+    assert _best_steps(tsg, _fixed(64, 1 << 19, 1000, 1), _fixed(1 << 19, 1 << 19, 16, 2))[1] < 2.0
