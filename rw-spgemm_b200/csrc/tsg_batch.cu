@@ -312,7 +312,7 @@ __device__ __forceinline__ unsigned long long gtimer() { return batch_clock_ns()
 template <int SCHED, int W, int CAP, int NT>
 __global__ void __launch_bounds__(NT)
     k_batch(BatchProd *prods, int count, const long long *__restrict__ rowoff, const long long *__restrict__ s1off,
-            int4 *wlist, int split, long long *denseoff, int dense, long long *itemoff, unsigned *bar, int *err, int *bins)
+            int4 *wlist, int split, int per_pair, long long *denseoff, int dense, long long *itemoff, unsigned *bar, int *err, int *bins)
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
     __shared__ long long s_tmp[NT / 32 + 1];
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(NT)
                 step1_row<true>(prods[p].P, i, bm, lane32, nullptr);
             else
             {
-                const int done = step12_row(prods[p].P, i, *s12, lane32, s_bins, prods[p].K);
+                const int done = step12_row(prods[p].P, i, *s12, lane32, s_bins, SCHED == 3 ? per_pair : 0, prods[p].K);
                 int kind = 0;
                 if (!done)
                 {
@@ -948,7 +948,7 @@ extern "C" int tsg_product_bounds(tsg_context *ctx, const tsg_tiled *A, const ts
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-typedef void (*batch_kernel_t)(BatchProd *, int, const long long *, const long long *, int4 *, int, long long *,
+typedef void (*batch_kernel_t)(BatchProd *, int, const long long *, const long long *, int4 *, int, int, long long *,
                                int, long long *, unsigned *, int *, int *);
 
 // Kernel, dynamic shared memory and block size of a batch schedule.  cols:
@@ -1016,7 +1016,8 @@ static int record_run(tsg_batch *b, cudaStream_t st)
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     TSG_CUDA(cudaLaunchKernelEx(&cfg, kern, b->d_prod, b->count, (const long long *)b->d_rowoff,
-                                (const long long *)b->d_s1off, b->d_wlist, b->split, b->d_denseoff, b->dense,
+                                (const long long *)b->d_s1off, b->d_wlist, b->split,
+                                s12_per_pair(b->rowoff[b->count], b->ctx->num_sms), b->d_denseoff, b->dense,
                                 b->d_itemoff,
                                 b->d_bar, b->d_err, b->d_bins));
     if (b->params.schedule != TSG_SCHED_SPA)

@@ -269,9 +269,22 @@ __device__ __forceinline__ int nnz_bin(int total);
 // ---------------------------------------------------------------------------
 #define S12_WORDS 256
 #define S12_MAXT 128
-// tile pairs from which a row is wide whatever its tiles: the warp takes them
-// 32 at a time (1,500 x 1,300 random, 3,775 pairs and 980 products a tile row)
+// Tile pairs from which a row with few products for them is left to the CTA that
+// takes the wide rows: the warp takes pairs 32 at a time, about 100 ns each, the
+// CTA scalar products, all its warps at once, about 0.35 ns each.  Fewer than
+// s12_per_pair products a pair: what a CTA an SM does while the warps of 28 tile
+// rows an SM take their pairs.  Steps 1 and 2 on a B200, by warps and by CTAs:
+// 100,000 x 1,100 x 1,300 random, 4 entries a row (4,096 pairs and 256 products a
+// tile row) 0.32 and 0.22 ms, 1,500 rows of 8 entries 0.23 and 0.071; random bands
+// of 3,700 pairs a tile row, 65,536 rows 4 products a pair 0.48 and 0.30, 18 a pair
+// 0.59 and 0.66, 70 a pair 0.84 and 1.7, 8,192 rows 70 a pair 0.51 and 0.32; full
+// matrix of 1,000 rows (4,096 a pair) 0.45 and 5.7.
 #define S12_MAXP 1024
+static inline int s12_per_pair(long long tile_rows, int num_sms)
+{
+    const long long n = 256LL * num_sms / (tile_rows > 0 ? tile_rows : 1);
+    return (int)(n < 16 ? 16 : n > 256 ? 256 : n);
+}
 
 struct S12Smem
 {
@@ -281,7 +294,7 @@ struct S12Smem
     unsigned b[8][32];                    // [two rows][lane]: the lane's B tile
 };
 
-__device__ __forceinline__ int step12_row(const ProdView &P, int i, S12Smem &sm, int lane, int *s_bins,
+__device__ __forceinline__ int step12_row(const ProdView &P, int i, S12Smem &sm, int lane, int *s_bins, int per_pair,
                                           const StepOneBits &K = {nullptr, nullptr, 0, nullptr})
 {
     const int a0 = P.A_ptr[i], a1 = P.A_ptr[i + 1];
@@ -291,11 +304,27 @@ __device__ __forceinline__ int step12_row(const ProdView &P, int i, S12Smem &sm,
         return 1;
     if (ntiles > S12_MAXT)
         return 0; // wide row: the caller emits it and runs step 2 on it
-    int pairs = 0;
-    for (int pa = a0 + lane; pa < a1; pa += 32)
-        pairs += P.B_ptr[P.A_col[pa] + 1] - P.B_ptr[P.A_col[pa]];
-    if (__reduce_add_sync(TSG_FULL_MASK, pairs) > S12_MAXP)
-        return 0;
+    if (per_pair) // the caller has a CTA for wide rows
+    {
+        // products: as if the entries of a B tile row were spread evenly over its 16 rows
+        int pairs = 0;
+        float products = 0.f;
+        for (int pa = a0 + lane; pa < a1; pa += 32)
+        {
+            const int b0 = P.B_ptr[P.A_col[pa]], b1 = P.B_ptr[P.A_col[pa] + 1];
+            pairs += b1 - b0;
+            products += (float)(P.A_tnnz[pa + 1] - P.A_tnnz[pa]) * (float)(P.B_tnnz[b1] - P.B_tnnz[b0]) / TSG_BS;
+        }
+        pairs = __reduce_add_sync(TSG_FULL_MASK, pairs);
+        if (pairs > S12_MAXP)
+        {
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1)
+                products += __shfl_xor_sync(TSG_FULL_MASK, products, d);
+            if (products < (float)per_pair * (float)pairs)
+                return 0;
+        }
+    }
     int c0, nw;
     const int2 kept = K.words ? K.span[i] : make_int2(0, 0);
     if (kept.y)

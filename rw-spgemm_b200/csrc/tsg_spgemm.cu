@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(S1_WARPS * 32) k_step1_total(ProdView P, unsig
 // alone and left to the wide-row step 2: wide[i] says 1, or 2 when the row is
 // hypersparse (0 otherwise), and wide[tilemA ...] lists their units (wide_list).
 #define S12_WARPS 4
-__global__ void __launch_bounds__(S12_WARPS * 32) k_step12(ProdView P, StepOneBits K, int split, int *__restrict__ wide,
+__global__ void __launch_bounds__(S12_WARPS * 32) k_step12(ProdView P, StepOneBits K, int split, int per_pair, int *__restrict__ wide,
                                                 int *__restrict__ bins)
 {
     __shared__ S12Smem sm[S12_WARPS];
@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(S12_WARPS * 32) k_step12(ProdView P, StepOneBi
     const int i = blockIdx.x * S12_WARPS + warp;
     if (i < P.tilemA)
     {
-        const int done = step12_row(P, i, sm[warp], lane, s_bins, K);
+        const int done = step12_row(P, i, sm[warp], lane, s_bins, per_pair, K);
         int kind = 0;
         if (!done)
         {
@@ -920,7 +920,8 @@ static int spgemm_structure(tsg_context *ctx, const tsg_tiled *A, const tsg_tile
             R.units = wide_units(tilem, A->nnz, split);
             TSG_TRY(tsg_alloc(ctx, &R.d_wide, (size_t)tilem + 3 + 2 * R.units));
             TSG_CUDA(cudaMemsetAsync(R.d_wide + tilem, 0, 2 * sizeof(int), st));
-            k_step12<<<tsg_blocks(tilem, S12_WARPS), S12_WARPS * 32, 0, st>>>(P, R.bits, split, R.d_wide, d_bins);
+            k_step12<<<tsg_blocks(tilem, S12_WARPS), S12_WARPS * 32, 0, st>>>(
+                P, R.bits, split, P.B_rptr ? s12_per_pair(tilem, ctx->num_sms) : 0, R.d_wide, d_bins);
             TSG_LAUNCH_CHECK();
         }
         else

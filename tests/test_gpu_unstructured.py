@@ -126,3 +126,24 @@ def test_dense_tiles_with_values_that_zero_does_not_absorb(tsg, ctx, oracle, gen
         _check(tsg, ctx, oracle, A, B, tsg.TSG_TILED_CSC_VIEW)
     finally:
         ctx.set_schedule("spa", dense=0)
+
+
+@pytest.mark.parametrize("n,entries", [(520, 520), (600, 600), (530, 40), (530, 8)])
+def test_rows_of_many_tile_pairs(tsg, ctx, oracle, n, entries):
+    """33 and 38 tiles a row on both sides (1,089 and 1,444 pairs, at most 128 C
+    tiles): full rows, whose masks a warp makes pair by pair, and sparse ones,
+    left to the CTA of wide rows."""
+    A, B = _rows(n, n, [entries] * n, 1), _rows(n, n, [entries] * n, 2)
+    for fused in (True, False):
+        ctx.set_fusion(fused)
+        try:
+            _check(tsg, ctx, oracle, A, B, tsg.TSG_TILED_CSC_VIEW)
+        finally:
+            ctx.set_fusion(True)
+    pairs = [tuple(_tiled(tsg, ctx, x, tsg.TSG_TILED_CSC_VIEW) for x in (A, B))]
+    for sched in ("spa", "tiles", "elems"):
+        batch = tsg.Batch(ctx, pairs, sched)
+        batch.run()
+        batch.sync()
+        _same([x.cpu().numpy() for x in tsg.tiled_to_csr(ctx, batch.product(0))], oracle.gustavson(A, B, nthreads=8))
+        batch.close()
