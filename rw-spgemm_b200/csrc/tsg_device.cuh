@@ -1092,6 +1092,11 @@ __device__ __forceinline__ void step3_rows_item(const ProdView &P, long long ite
 #define SPA_CMS (SPA_SEGT + 1) // row stride of the [row][tile] words: a tile's 16 rows in 16 banks
 #define SPA_WIN 2048
 #define SPA_STAGE 64
+// entries after the first that a batch adds entry by entry: finding the columns
+// that meet is dearer where most of them do (16 products of a 60^2 grid in a
+// batch, step 3: 0.319 ms always by columns, 0.284 from 4, 6, 8 or 10 entries on;
+// rows meeting few columns twice, no difference)
+#define SPA_ROUNDS 6
 #define SPA_DENSE TSG_SPA_DENSE_DEFAULT
 #define SPA_FLAT 16  // B rows averaging fewer entries (inside a segment) have their products flattened
 
@@ -1223,7 +1228,7 @@ __host__ __device__ __forceinline__ bool spa_wants_flat(int browB, long long num
 // bl (cut to the segment) and values a, in k order -- to the row's
 // accumulator run.  FLATTEN: when their B rows hold fewer than SPA_FLAT
 // entries on average, the products are flattened, 32 per batch in k order;
-// lanes of a batch meeting the same slot add one after another in lane order
+// lanes of a batch meeting the same slot add one after another in k order
 // and batches follow one another behind warp barriers, so every
 // slot still sums its products in k order.  Otherwise (or !FLATTEN) a warp
 // pass per entry streams its B row, the next row's first 32 entries
@@ -1273,8 +1278,13 @@ __device__ __forceinline__ void spa_apply_stage(const ProdView &P, SpaSmem &S, c
                     if (pos >= 0)
                         prod = __dmul_rn(a[ent], P.B_rval[bi]);
                 }
-                int last;
-                const int rank = same_key_rank(pos, pos >= 0, S.tag[threadIdx.x >> 5], lane, last);
+                // products of one entry meet distinct columns: those of a few
+                // entries add entry by entry, others in lane order where
+                // columns meet
+                int rank = ent - __shfl_sync(TSG_FULL_MASK, ent, 0);
+                int last = __reduce_max_sync(TSG_FULL_MASK, item < ni ? rank : 0);
+                if (last > SPA_ROUNDS)
+                    rank = same_key_rank(pos, pos >= 0, S.tag[threadIdx.x >> 5], lane, last);
                 for (int q = 0; q <= last; q++)
                 {
                     if (pos >= 0 && rank == q)

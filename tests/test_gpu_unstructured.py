@@ -147,3 +147,17 @@ def test_rows_of_many_tile_pairs(tsg, ctx, oracle, n, entries):
         batch.sync()
         _same([x.cpu().numpy() for x in tsg.tiled_to_csr(ctx, batch.product(0))], oracle.gustavson(A, B, nthreads=8))
         batch.close()
+
+
+@pytest.mark.parametrize("entries", [1, 4, 5, 6, 12])
+def test_spa_rows_whose_products_meet(tsg, ctx, oracle, entries):
+    """B rows of a few entries in 60 columns far apart, so that a batch of
+    products meets most columns several times: batches of few entries (added
+    entry by entry) and of many."""
+    rng = np.random.default_rng(entries)
+    hubs = np.sort(rng.choice(2500, 60, replace=False)) * 16 + 5
+    A = _rows(70, 500, [40] * 70, 1)
+    rows = [np.sort(rng.choice(hubs, entries if i % 7 else 1, replace=False)) for i in range(500)]
+    rp = np.concatenate([[0], np.cumsum([r.size for r in rows])]).astype(np.int32)
+    B = 500, 40000, rp, np.concatenate(rows).astype(np.int32), rng.uniform(-1, 1, rp[-1])
+    assert _check(tsg, ctx, oracle, A, B, tsg.TSG_TILED_CSC_VIEW)["step3_name"] == "k_step3_spa<flat>"
