@@ -95,6 +95,18 @@ extern "C" int tsg_context_destroy(tsg_context *ctx)
         cudaStreamDestroy(ctx->copy_stream);
         cudaEventDestroy(ctx->copy_ev);
     }
+    for (int q = 0; q < TSG_SIDE_STREAMS; q++)
+    {
+        if (ctx->side[q])
+        {
+            cudaStreamSynchronize(ctx->side[q]);
+            cudaStreamDestroy(ctx->side[q]);
+        }
+        if (ctx->side_join[q])
+            cudaEventDestroy(ctx->side_join[q]);
+    }
+    if (ctx->side_fork)
+        cudaEventDestroy(ctx->side_fork);
     if (ctx->own_stream)
         cudaStreamDestroy(ctx->stream);
     cudaFreeHost(ctx->h_pinned);
@@ -929,6 +941,33 @@ int tsg_copy_stream(tsg_context *ctx)
         cudaEventDestroy(ctx->copy_ev);
         ctx->copy_stream = nullptr;
         return tsg_set_error(TSG_ERR_CUDA, "copy stream creation failed: %s", cudaGetErrorString(e));
+    }
+    return TSG_OK;
+}
+
+int tsg_fork(tsg_context *ctx, cudaStream_t st, int n)
+{
+    if (!ctx->side_fork)
+        TSG_CUDA(cudaEventCreateWithFlags(&ctx->side_fork, cudaEventDisableTiming));
+    for (int q = 0; q < n; q++)
+    {
+        if (!ctx->side_join[q])
+            TSG_CUDA(cudaEventCreateWithFlags(&ctx->side_join[q], cudaEventDisableTiming));
+        if (!ctx->side[q])
+            TSG_CUDA(cudaStreamCreateWithFlags(&ctx->side[q], cudaStreamNonBlocking));
+    }
+    TSG_CUDA(cudaEventRecord(ctx->side_fork, st));
+    for (int q = 0; q < n; q++)
+        TSG_CUDA(cudaStreamWaitEvent(ctx->side[q], ctx->side_fork, 0));
+    return TSG_OK;
+}
+
+int tsg_join(tsg_context *ctx, cudaStream_t st, int n)
+{
+    for (int q = 0; q < n; q++)
+    {
+        TSG_CUDA(cudaEventRecord(ctx->side_join[q], ctx->side[q]));
+        TSG_CUDA(cudaStreamWaitEvent(st, ctx->side_join[q], 0));
     }
     return TSG_OK;
 }

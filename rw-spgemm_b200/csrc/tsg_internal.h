@@ -46,6 +46,8 @@ enum
     TSG_OCC_COUNT
 };
 
+#define TSG_SIDE_STREAMS 3
+
 struct tsg_context
 {
     int device;
@@ -62,6 +64,8 @@ struct tsg_context
     int fuse12;          // step-1 emit fused with step 2 for narrow tile rows
     cudaStream_t copy_stream; // device-to-host copies overlapping compute (created on first use)
     cudaEvent_t copy_ev;      // orders a chunk's copy after its fill
+    cudaStream_t side[TSG_SIDE_STREAMS]; // kernels beside those of the context's stream (tsg_fork, tsg_join)
+    cudaEvent_t side_fork, side_join[TSG_SIDE_STREAMS];
     TsgControl *d_ctl;        // device block of counters and the error word
     int *d_status;            // its error word, 0 when clear
     int occ[TSG_OCC_COUNT];   // resident CTAs per SM, 0: not asked yet
@@ -80,6 +84,13 @@ int tsg_check_device_status(tsg_context *ctx, int code);
 // least TSG_CHUNK_NNZ nonzeros (tsg_spgemm_to_host).
 #define TSG_MAX_CHUNKS 8
 #define TSG_CHUNK_NNZ (1LL << 20)
+
+// What is queued on the context's side streams [0, n) between the two calls
+// runs after what stream st holds at the first and before what it gets after
+// the second.  The streams are made on first use and kept: a batch that made its
+// own took 0.2 ms longer to create.
+int tsg_fork(tsg_context *ctx, cudaStream_t st, int n);
+int tsg_join(tsg_context *ctx, cudaStream_t st, int n);
 
 // Creates the context's copy stream and event if needed.
 int tsg_copy_stream(tsg_context *ctx);

@@ -169,6 +169,9 @@ __global__ void __launch_bounds__(256) k_step2(ProdView P, int *__restrict__ bin
         atomicAdd(&bins[threadIdx.x], s_bins[threadIdx.x]);
 }
 
+// fewest C tiles of a product that runs its hypersparse rows beside the others
+#define HYP_APART (1 << 17)
+
 #define S3_THREADS 128
 #define S3_HW (S3_THREADS / 16)
 
@@ -267,7 +270,11 @@ __global__ void __launch_bounds__(SPA_THREADS, 3) k_step3_spa(ProdView P, const 
 // The hypersparse rows of tile rows [row0, row1), a CTA each, from step 2's
 // list of wide rows.  Found through the blocks of C tiles they took longer to
 // find than to compute: 65,536 rows of 64 products, 16 blocks to a tile row,
-// 0.759 -> 0.391 ms.
+// 0.759 -> 0.391 ms.  Runs beside k_step3_spa, which takes the other rows: one
+// after the other, each waited for the other's longest row (65,536 rows of
+// uneven length times a band, step 3: 1.91 ms, 1.19 side by side; R-MAT 17 of 4
+// edges a row 6.9 and 5.8; the two in one kernel spill, 65,536 random rows 0.38
+// and 0.53).  k_step3_spa goes first, its rows being the longer ones.
 __global__ void __launch_bounds__(SPA_THREADS, 3) k_step3_hyper(ProdView P, const int *__restrict__ wide, int row0,
                                                                 int row1, unsigned *__restrict__ ctr)
 {
@@ -699,17 +706,18 @@ static int launch_step3_spa(tsg_context *ctx, const ProdView &P0, const int *d_k
                           k_step3_spa<FLAT, RANGED, BLK>, SPA_THREADS, smem, &per_sm));
     TSG_TRY(clear_counters(ctx, row0, TSG_CTR_STEP3, 2));
     if (hyper_apart)
-    {
-        int hper_sm = 0;
-        TSG_TRY(resident_ctas(ctx, TSG_OCC_HYPER, k_step3_hyper, SPA_THREADS, (int)sizeof(HypSmem), &hper_sm));
-        k_step3_hyper<<<ctx->num_sms * hper_sm, SPA_THREADS, sizeof(HypSmem), ctx->stream>>>(
-            P, d_kind, RANGED ? row0 : 0, RANGED ? row1 : P.tilemA, &ctr[TSG_CTR_REST]);
-        TSG_LAUNCH_CHECK();
-    }
+        TSG_TRY(tsg_fork(ctx, ctx->stream, 1));
     k_step3_spa<FLAT, RANGED, BLK><<<ctx->num_sms * per_sm, SPA_THREADS, smem, ctx->stream>>>(
         P, d_kind, !hyper_apart, row0, row1, &ctr[TSG_CTR_STEP3]);
     TSG_LAUNCH_CHECK();
-    return TSG_OK;
+    if (!hyper_apart)
+        return TSG_OK;
+    int hper_sm = 0;
+    TSG_TRY(resident_ctas(ctx, TSG_OCC_HYPER, k_step3_hyper, SPA_THREADS, (int)sizeof(HypSmem), &hper_sm));
+    k_step3_hyper<<<ctx->num_sms * hper_sm, SPA_THREADS, sizeof(HypSmem), ctx->side[0]>>>(
+        P, d_kind, RANGED ? row0 : 0, RANGED ? row1 : P.tilemA, &ctr[TSG_CTR_REST]);
+    TSG_LAUNCH_CHECK();
+    return tsg_join(ctx, ctx->stream, 1);
 }
 
 // the staged numeric step for tile rows [row0, row1), then the SPA kernel
@@ -797,8 +805,11 @@ static int launch_step3_spa_rows(tsg_context *ctx, const ProdView &P, const tsg_
     if (flat && nnzC >= (long long)SPA_BLK_NARROW_VALUES * P.numC)
         return whole ? launch_step3_spa<true, false, SPA_BLK_NARROW>(ctx, P, d_kind, false, 0, 0)
                      : launch_step3_spa<true, true, SPA_BLK_NARROW>(ctx, P, d_kind, false, row0, row1);
-    // mostly hypersparse rows (few values in many tiles): those by themselves
-    const bool hyper = d_kind && nnzC < (long long)HYP_RATIO * P.numC && P.numC > (long long)S12_MAXT * P.tilemA;
+    // mostly hypersparse rows (few values in many tiles): those by themselves,
+    // unless the second stream costs more (4,096 random rows of 4, 65 K tiles:
+    // 0.036 ms, 0.027 without)
+    const bool hyper = d_kind && nnzC < (long long)HYP_RATIO * P.numC && P.numC > (long long)S12_MAXT * P.tilemA &&
+                       P.numC >= HYP_APART;
     if (flat)
         return whole ? launch_step3_spa<true, false>(ctx, P, d_kind, hyper, 0, 0)
                      : launch_step3_spa<true, true>(ctx, P, d_kind, hyper, row0, row1);

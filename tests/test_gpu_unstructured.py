@@ -161,3 +161,37 @@ def test_spa_rows_whose_products_meet(tsg, ctx, oracle, entries):
     rp = np.concatenate([[0], np.cumsum([r.size for r in rows])]).astype(np.int32)
     B = 500, 40000, rp, np.concatenate(rows).astype(np.int32), rng.uniform(-1, 1, rp[-1])
     assert _check(tsg, ctx, oracle, A, B, tsg.TSG_TILED_CSC_VIEW)["step3_name"] == "k_step3_spa<flat>"
+
+
+def _mixed(tile_rows, seed):
+    """Wide C tile rows, one in six with several values a tile and the others
+    hypersparse, too few values a window for the window step."""
+    m = 16 * tile_rows - 11
+    A = _rows(m, 4000, [300 if i // 16 % 6 == 1 else 3 for i in range(m)], seed)
+    return A, _rows(4000, 64000, [4] * 4000, seed + 1)
+
+
+@pytest.mark.parametrize("dense", [257, 0])
+def test_hypersparse_rows_among_others(tsg, ctx, oracle, dense):
+    A, B = _mixed(14, 1)
+    ctx.set_schedule("spa", dense=dense)
+    try:
+        info = _check(tsg, ctx, oracle, A, B, tsg.TSG_TILED_CSC_VIEW)
+    finally:
+        ctx.set_schedule("spa", dense=0)
+    assert info["step3_name"] == "k_step3_spa<flat>"
+    batch = tsg.Batch(ctx, [tuple(_tiled(tsg, ctx, x, tsg.TSG_TILED_CSC_VIEW) for x in (A, B))] * 2)
+    for _ in range(2):
+        batch.run()
+        batch.sync()
+        for p in range(2):
+            _same([x.cpu().numpy() for x in tsg.tiled_to_csr(ctx, batch.product(p))], oracle.gustavson(A, B, nthreads=8))
+    batch.close()
+
+
+def test_hypersparse_rows_among_others_on_tile_row_ranges(tsg, ctx, oracle):
+    A, B = _mixed(640, 3)
+    out = tsg.HostResultBuffers(A[0], 1 << 22)
+    got, info = tsg.spgemm_csr_host_overlap(ctx, A, B, out)
+    assert info["nnz_C"] > 2 << 20 and info["step3_name"] == "k_step3_spa<flat>"
+    _same(got[2:], oracle.gustavson(A, B, nthreads=8))
