@@ -306,24 +306,15 @@ __device__ __forceinline__ int step12_row(const ProdView &P, int i, S12Smem &sm,
         return 0; // wide row: the caller emits it and runs step 2 on it
     if (per_pair) // the caller has a CTA for wide rows
     {
-        // products: as if the entries of a B tile row were spread evenly over its 16 rows
         int pairs = 0;
-        float products = 0.f;
         for (int pa = a0 + lane; pa < a1; pa += 32)
-        {
-            const int b0 = P.B_ptr[P.A_col[pa]], b1 = P.B_ptr[P.A_col[pa] + 1];
-            pairs += b1 - b0;
-            products += (float)(P.A_tnnz[pa + 1] - P.A_tnnz[pa]) * (float)(P.B_tnnz[b1] - P.B_tnnz[b0]) / TSG_BS;
-        }
+            pairs += P.B_ptr[P.A_col[pa] + 1] - P.B_ptr[P.A_col[pa]];
         pairs = __reduce_add_sync(TSG_FULL_MASK, pairs);
-        if (pairs > S12_MAXP)
-        {
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1)
-                products += __shfl_xor_sync(TSG_FULL_MASK, products, d);
-            if (products < (float)per_pair * (float)pairs)
-                return 0;
-        }
+        // products: A's entries times B's mean row (a hub's are more, but its row
+        // is the better one to leave)
+        const float products = (float)(P.A_tnnz[a1] - P.A_tnnz[a0]) * (float)(P.browB + 1);
+        if (pairs > S12_MAXP && products < (float)per_pair * (float)pairs)
+            return 0;
     }
     int c0, nw;
     const int2 kept = K.words ? K.span[i] : make_int2(0, 0);
