@@ -1172,7 +1172,7 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
         if (prm.schedule == TSG_SCHED_SPA && A[p].row_ptr && A[p].m > 0 && B[p].n > 0)
         {
             const long long windows = (B[p].n + WIN_COLS - 1LL) / WIN_COLS;
-            const long long parts = (long long)(A[p].nnz / win_heavy(A[p].nnz)) * ((B[p].n + WIN_PART - 1) / WIN_PART);
+            const long long parts = (long long)(A[p].nnz / win_heavy(A[p].nnz, A[p].m)) * ((B[p].n + WIN_PART - 1) / WIN_PART);
             const long long claims = (long long)A[p].tilem * windows * WIN_PER, centries = A[p].tilem * (windows + 1);
             int bits, blocks;
             if (prods >= BATCH_WIN_MIN * windows * A[p].m &&
@@ -1184,7 +1184,7 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
                 h.Q.bits = bits;
                 h.Q.blocks = blocks;
                 h.Q.mA = A[p].m;
-                h.Q.heavy_min = win_heavy(A[p].nnz);
+                h.Q.heavy_min = win_heavy(A[p].nnz, A[p].m);
                 hparts += parts;
                 tables[p] = (blocks + 1LL) * B[p].m + centries + 2 * windows * B[p].m + 1;
                 words += (blocks + 1LL + 2 * windows) * B[p].m;

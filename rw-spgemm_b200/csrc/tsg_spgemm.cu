@@ -600,13 +600,20 @@ struct WinScratch
     WinPlan Q;
     int *rptr, *rcol; // A's row view, when A has none
     double *rval;
-    bool ready;
+    bool ready;  // the tables are made
+    bool failed; // no memory for them
 };
 
-// Whether a product runs step 3 by windows, and their table's shape
-static bool win_shape(const ProdView &P, long long nnzA, long long nnzC, WinPlan &Q)
+// Whether wtab is made: B's rows times the windows
+static bool win_has_wtab(const ProdView &P, const WinPlan &Q)
 {
-    if (!P.B_rptr || P.nB < 1 || P.mA < 1)
+    return (long long)P.mB * Q.windows <= WIN_TABLE_WORDS / 2;
+}
+
+// Whether a product runs step 3 by windows, and their table's shape
+static bool win_shape(const ProdView &P, long long nnzA, long long nnzB, long long nnzC, WinPlan &Q)
+{
+    if (!P.B_rptr || P.nB < 1 || P.mA < 1 || P.mB < 1)
         return false;
     const long long windows = (P.nB + WIN_COLS - 1LL) / WIN_COLS;
     // claims of every row as if it were heavy: 32-bit
@@ -616,8 +623,10 @@ static bool win_shape(const ProdView &P, long long nnzA, long long nnzC, WinPlan
         return false;
     Q.windows = (int)windows;
     Q.mA = P.mA;
-    Q.heavy_min = win_heavy(nnzA);
-    return true;
+    Q.heavy_min = win_heavy(nnzA, P.mA);
+    const long long tables = (Q.blocks + 1LL + (win_has_wtab(P, Q) ? 2 * windows : 0)) * P.mB;
+    return win_worth(nnzC, (long long)((double)nnzA * (double)nnzB / P.mB), nnzA, P.numC, P.tilemA,
+                     P.tilenB, windows, tables);
 }
 
 static void win_release(tsg_context *ctx, WinScratch &W)
@@ -666,7 +675,7 @@ static int win_prepare(tsg_context *ctx, const ProdView &P, const tsg_tiled *A, 
     WinPlan &Q = W.Q;
     TSG_TRY(tsg_alloc(ctx, &Q.btab, (size_t)P.mB * (Q.blocks + 1)));
     Q.wtab = nullptr;
-    if ((long long)P.mB * Q.windows <= WIN_TABLE_WORDS / 2)
+    if (win_has_wtab(P, Q))
         TSG_TRY(tsg_alloc(ctx, &Q.wtab, (size_t)P.mB * Q.windows));
     TSG_TRY(tsg_alloc(ctx, &Q.ctab, (size_t)P.tilemA * (Q.windows + 1)));
     TSG_TRY(tsg_alloc(ctx, &Q.heavy, (size_t)P.mA));
@@ -785,16 +794,24 @@ static bool step3_by_spa(const tsg_context *ctx, const ProdView &P, long long nn
 }
 
 // the SPA numeric step for tile rows [row0, row1)
-static int launch_step3_spa_rows(tsg_context *ctx, const ProdView &P, const tsg_tiled *A, long long nnzC,
+static int launch_step3_spa_rows(tsg_context *ctx, const ProdView &P, const tsg_tiled *A, long long nnzB, long long nnzC,
                                  const int *d_kind, WinScratch &W, int row0, int row1)
 {
     const bool flat = spa_wants_flat(P.browB, P.numC, nnzC, P.tilemA);
     const bool whole = row0 == 0 && row1 == P.tilemA;
     ctx->last_step3 = flat ? TSG_STEP3_FLAT : P.padded ? TSG_STEP3_STAGED : TSG_STEP3_SPA;
-    if (flat && win_shape(P, A->nnz, nnzC, W.Q))
+    if (flat && !W.failed && win_shape(P, A->nnz, nnzB, nnzC, W.Q))
     {
+        const int kernel = ctx->last_step3;
         ctx->last_step3 = TSG_STEP3_WINDOWS;
-        return launch_step3_win(ctx, P, A, W, row0, row1);
+        const int status = launch_step3_win(ctx, P, A, W, row0, row1);
+        if (status != TSG_ERR_OOM || W.ready)
+            return status;
+        // no room for the tables, which the other kernels do without
+        cudaGetLastError();
+        win_release(ctx, W);
+        W.failed = true;
+        ctx->last_step3 = kernel;
     }
     if (flat && P.numC <= (long long)NAR_MEAN * P.tilemA)
     {
@@ -822,11 +839,11 @@ static int launch_step3_spa_rows(tsg_context *ctx, const ProdView &P, const tsg_
 
 // d_kind: the row kinds of the fused step 1/2 pass (0 narrow, 1 wide,
 // 2 hypersparse), or null
-static int launch_step3(tsg_context *ctx, const ProdView &P, const tsg_tiled *A, long long nnzC, const int *d_kind,
-                        WinScratch &W)
+static int launch_step3(tsg_context *ctx, const ProdView &P, const tsg_tiled *A, long long nnzB, long long nnzC,
+                        const int *d_kind, WinScratch &W)
 {
     if (step3_by_spa(ctx, P, nnzC))
-        return launch_step3_spa_rows(ctx, P, A, nnzC, d_kind, W, 0, P.tilemA);
+        return launch_step3_spa_rows(ctx, P, A, nnzB, nnzC, d_kind, W, 0, P.tilemA);
     if (ctx->sched == TSG_SCHED_ROWS)
     {
         const int W = ctx->seg_tiles, cap = ctx->acc_cap;
@@ -1015,7 +1032,7 @@ extern "C" int tsg_spgemm(tsg_context *ctx, const tsg_tiled *A, const tsg_tiled 
     TSG_TRY(spgemm_structure(ctx, A, B, C, R));
     // step 3: numeric
     if (R.nnzC > 0)
-        TSG_TRY(launch_step3(ctx, make_view(A, B, C), A, R.nnzC, R.d_wide, R.win));
+        TSG_TRY(launch_step3(ctx, make_view(A, B, C), A, B->nnz, R.nnzC, R.d_wide, R.win));
     if (ctx->timing)
         TSG_CUDA(cudaEventRecord(ctx->ev[3], ctx->stream));
     return spgemm_finish(ctx, R, info);
@@ -1068,7 +1085,7 @@ int tsg_spgemm_to_host(tsg_context *ctx, const tsg_tiled *A, const tsg_tiled *B,
             const ProdView P = make_view(A, B, &C);
             const bool spa = step3_by_spa(ctx, P, R.nnzC);
             if (!spa)
-                TSG_TRY(launch_step3(ctx, P, A, R.nnzC, R.d_wide, R.win));
+                TSG_TRY(launch_step3(ctx, P, A, B->nnz, R.nnzC, R.d_wide, R.win));
             // chunks of about equal nonzeros (>= TSG_CHUNK_NNZ each, at most TSG_MAX_CHUNKS)
             const long long nch = std::max(1LL, std::min((long long)TSG_MAX_CHUNKS, R.nnzC / TSG_CHUNK_NNZ));
             int r0 = 0;
@@ -1093,7 +1110,7 @@ int tsg_spgemm_to_host(tsg_context *ctx, const tsg_tiled *A, const tsg_tiled *B,
                 if (r1 <= r0)
                     continue;
                 if (spa)
-                    TSG_TRY(launch_step3_spa_rows(ctx, P, A, R.nnzC, R.d_wide, R.win, r0, r1));
+                    TSG_TRY(launch_step3_spa_rows(ctx, P, A, B->nnz, R.nnzC, R.d_wide, R.win, r0, r1));
                 TSG_TRY(tsg_t2c_fill(ctx, &C, r0, r1, d_rp, d_ci, d_v));
                 TSG_CUDA(cudaEventRecord(ctx->copy_ev, st));
                 TSG_CUDA(cudaStreamWaitEvent(ctx->copy_stream, ctx->copy_ev, 0));

@@ -37,6 +37,7 @@
 #define WIN_PART_BITS 8
 #define WIN_HEAVY 256 // fewest A entries that make a row heavy
 #define WIN_HEAVY_SHARE 2048 // and the share of A's entries
+#define WIN_HEAVY_MEANS 4    // and how many mean rows
 #define WIN_ROWS 2 // rows per claim
 #define WIN_CTAS 3
 #define WIN_TILES (WIN_COLS / TSG_BS)
@@ -46,9 +47,31 @@
 #define WIN_THREADS (WIN_WARPS * 32)
 #define WIN_FEW 3 // values of a tile's row up to which a lane stores its tile's own
 #define WIN_ROUNDS 6 // entries after the first that a batch adds entry by entry
-// a product takes the windows when C holds at least this many values per (row, window)
+// When a product takes the windows (win_worth).  A task costs its entries of A
+// and its C tiles whatever the products in the window, the tables cost every row
+// of B: C has to hold WIN_MIN_VALUES values (a batch, that knows no values:
+// BATCH_WIN_MIN products) per (row, window) and WIN_MIN_TILES tiles per (tile
+// row, window), and the tables may take WIN_TABLE_SHARE words per value of C, or
+// WIN_TABLE_FREE.  What the windows are for is uneven work: where C has WIN_SKEW
+// times the products that A's entries and B's mean row give, that is all.
+// Elsewhere C's tiles have to hold WIN_TILE_VALUES values on average -- below,
+// k_step3_spa's hypersparse form keeps up -- or C one value for every entry of A
+// and window.  Step 3, k_step3_spa<flat> and windows, B200:
+//   uneven: R-MAT 13 2.2 and 0.40 ms, a 64th of R-MAT 16's rows 4.7 and 1.0
+//   values a tile: 16,384 random rows of 11 (2) 0.125 and 0.244, 65,536 of 128
+//     times 4 (2) 2.0 and 8.0, of 25 (2.4) 3.7 and 4.1, of 32 (4) 7.1 and 4.8;
+//     4,096 rows of 256 times 65,536 of 16 (16) 2.6 and 1.3
+//   words of table a value: rows of 60 times 100,000 x 40,000 of 12, 4,000 rows
+//     (8) 0.53 and 0.35, 1,000 rows (33) 0.199 and 0.169, 256 rows (130) 0.078
+//     and 0.124; 64 rows of 64 times 1 M x 16,384 (1,600) 0.067 and 0.25
+//   tiles a window: batch of 24^3 grids (3) 0.35 and 0.51
 #define WIN_MIN_VALUES 8
-#define WIN_TABLE_WORDS (1LL << 26) // most words of the table of B's row pointers
+#define WIN_MIN_TILES 8
+#define WIN_SKEW 2
+#define WIN_TILE_VALUES 3
+#define WIN_TABLE_FREE (1LL << 21)
+#define WIN_TABLE_SHARE 32
+#define WIN_TABLE_WORDS (1LL << 26) // most words of the table of B's row pointers, and twice those of wtab
 
 struct WinTask
 {
@@ -98,11 +121,26 @@ struct WinPlan
 // A row is heavy when it would hold up the others: a task of 256 columns
 // meets shorter parts of B's rows, so only then is it worth cutting.  R-MAT 14
 // (228 K entries of A): 0.72 ms from 256 entries on, 0.81 from 512; R-MAT 16
-// (955 K): 5.99 and 5.52 ms.
-static inline int win_heavy(long long nnzA)
+// (955 K): 5.99 and 5.52 ms.  Rows of about the same length hold up none: 1,024
+// rows of 256 entries times 65,536 of 16, 1.10 ms as heavy rows, 0.45 as others.
+static inline int win_heavy(long long nnzA, long long rows)
 {
-    const long long share = nnzA / WIN_HEAVY_SHARE;
-    return share < WIN_HEAVY ? WIN_HEAVY : (int)share;
+    long long least = nnzA / WIN_HEAVY_SHARE;
+    if (least < WIN_HEAVY)
+        least = WIN_HEAVY;
+    const long long mean = nnzA / (rows > 0 ? rows : 1);
+    return (int)(least < WIN_HEAVY_MEANS * mean ? WIN_HEAVY_MEANS * mean : least);
+}
+
+// values: nnz(C), or a bound of it; products: the products of A's entries with
+// B's mean row; tables: words of the tables
+static inline bool win_worth(long long values, long long products, long long nnzA, long long tilesC, long long tile_rows,
+                             long long tilen, long long windows, long long tables)
+{
+    const long long least = WIN_MIN_TILES * windows < tilen ? WIN_MIN_TILES * windows : tilen;
+    if (tilesC < least * tile_rows || (tables > WIN_TABLE_FREE && tables > WIN_TABLE_SHARE * values))
+        return false;
+    return values >= WIN_SKEW * products || values >= WIN_TILE_VALUES * tilesC || values >= nnzA * windows;
 }
 
 // B row w's entry offset at every block boundary, by a warp

@@ -48,6 +48,19 @@ def test_narrow_rows(tsg, ctx, oracle, seed, view):
     assert info["step3_name"] == "k_step3_nar"
 
 
+def test_narrow_rows_without_the_fused_pass(tsg, ctx, oracle):
+    """No row kinds: rows of more than 128 tiles are told by their tiles alone."""
+    A, B = _operands(3)
+    ctx.set_schedule("spa", dense=257)
+    ctx.set_fusion(False)
+    try:
+        info = _check(tsg, ctx, oracle, A, B, tsg.TSG_TILED_CSC_VIEW)
+    finally:
+        ctx.set_fusion(True)
+        ctx.set_schedule("spa", dense=0)
+    assert info["step3_name"] == "k_step3_nar"
+
+
 def test_narrow_rows_on_tile_row_ranges(tsg, ctx, oracle, gen):
     """The host call computes a band times a band in ranges of tile rows."""
     mat = gen.banded(120000, 5, seed=5)
@@ -58,4 +71,5 @@ def test_narrow_rows_on_tile_row_ranges(tsg, ctx, oracle, gen):
     finally:
         ctx.set_schedule("spa", dense=0)
     assert info["nnz_C"] > 2 << 20  # more than one chunk
+    assert info["step3_name"] == "k_step3_nar"
     _same(got[2:], oracle.gustavson(mat, mat, nthreads=8))

@@ -62,17 +62,26 @@ def _case(name):
     if name == "heavy":  # rows around WIN_HEAVY entries among light ones, every B row holding column 0
         counts = [255, 0, 257, 3, 256, 40, 700, 1, 2, 5, 0, 258, 9, 9, 9, 9, 600, 4]
         return _rows(18, 1500, counts, 3), _rows(1500, 1300, rng.integers(0, 30, 1500), 4, hub=1)
+    if name == "heavy among light":  # ... where the mean row is short
+        counts = [255, 0, 257, 3, 256, 40, 700, 1, 2, 5, 0, 258, 9, 9, 9, 9, 600, 4] + [2] * 300
+        return _rows(318, 1500, counts, 3), _rows(1500, 1300, rng.integers(0, 30, 1500), 4, hub=1)
     if name == "parts":  # tile rows of 1, 2 and 5 parts
         counts = [63] * 16 + [64] * 16 + [65] * 16 + [257] * 16 + [3] * 5
         return _rows(69, 4000, counts, 5), _rows(4000, 5000, rng.integers(0, 12, 4000), 6)
     if name == "coarse table":  # 70,000 x 300,000: a table block wider than a heavy row's part; step 2 in passes
-        return _rows(40, 70000, [200] * 39 + [600], 8), _rows(70000, 300000, np.full(70000, 20), 9)
+        long = [40 * i for i in range(400)]
+        counts = np.zeros(70000, int)
+        counts[long] = 2500  # rows of B that all of A meets
+        rows = [np.sort(rng.choice(long, k, replace=False)) for k in [30] * 39 + [390]]
+        rp = np.concatenate([[0], np.cumsum([r.size for r in rows])]).astype(np.int32)
+        A = 40, 70000, rp, np.concatenate(rows).astype(np.int32), rng.uniform(-1, 1, rp[-1])
+        return A, _rows(70000, 300000, counts, 9)
     assert name == "step 1 in passes"
     return _rows(33, 400, rng.integers(1, 40, 33), 10), _rows(400, 1100000, np.full(400, 300), 11)
 
 
 @pytest.mark.parametrize("name", ["cols15", "cols255", "cols256", "cols257", "cols1024", "cols1025", "cols2000", "heavy",
-                                  "parts", "coarse table", "step 1 in passes"])
+                                  "heavy among light", "parts", "coarse table", "step 1 in passes"])
 @pytest.mark.parametrize("view", [True, False])
 def test_uneven_products(tsg, ctx, oracle, name, view):
     A, B = _case(name)
@@ -91,6 +100,7 @@ def test_window_step_on_tile_row_ranges(tsg, ctx, oracle, gen):
     out = tsg.HostResultBuffers(mat[0], 1 << 24)
     got, info = tsg.spgemm_csr_host_overlap(ctx, mat, None, out)
     assert info["nnz_C"] > 2 << 20  # more than one chunk
+    assert info["step3_name"] == "k_step3_win"
     _same(got[2:], oracle.gustavson(mat, mat, nthreads=8))
 
 
@@ -195,3 +205,16 @@ def test_hypersparse_rows_among_others_on_tile_row_ranges(tsg, ctx, oracle):
     got, info = tsg.spgemm_csr_host_overlap(ctx, A, B, out)
     assert info["nnz_C"] > 2 << 20 and info["step3_name"] == "k_step3_spa<flat>"
     _same(got[2:], oracle.gustavson(A, B, nthreads=8))
+
+
+@pytest.mark.parametrize("m,e,wins", [(300, 60, False), (2000, 60, True)])
+def test_few_rows_of_a_do_not_pay_for_tables_of_a_large_b(tsg, ctx, oracle, m, e, wins):
+    """The windows' tables cost every row of B: 130 words of them a value of C
+    are too many, 20 are not."""
+    A, B = _rows(m, 100000, [e] * m, 1), _rows(100000, 40000, [12] * 100000, 2)
+    ctx.synchronize()
+    used = ctx.pool_used()
+    info = _check(tsg, ctx, oracle, A, B, tsg.TSG_TILED_CSC_VIEW)
+    assert (info["step3_name"] == "k_step3_win") == wins
+    ctx.synchronize()
+    assert ctx.pool_used() <= used
