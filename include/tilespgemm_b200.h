@@ -571,6 +571,12 @@ int tsg_batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const tsg_
 int tsg_batch_create_bounded(tsg_context *ctx, int count, const tsg_tiled *A, const tsg_tiled *B,
                              const tsg_batch_params *params, const long long *products,
                              const long long *c_tiles, tsg_batch **out);
+/* Device bytes that product A*B with these bounds adds to a batch of the
+ * schedule (TSG_SCHED_*), at most: a batch's arena_bytes (tsg_batch_info) is no
+ * more than its products' sum.  For admission control (no reference
+ * counterpart); host arithmetic only. */
+int tsg_batch_product_bytes(tsg_context *ctx, const tsg_tiled *A, const tsg_tiled *B, int schedule,
+                            long long products, long long c_tiles, long long *bytes);
 /* Queues one execution of the whole batch on the context's stream. */
 int tsg_batch_run(tsg_batch *b);
 /* Waits for the last run and reads per-product sizes; reports a device wait

@@ -719,6 +719,8 @@ def _declare_batch(L):
     L.tsg_batch_create_bounded.argtypes = [vp, ip, ctypes.POINTER(TsgTiled), ctypes.POINTER(TsgTiled),
                                            ctypes.POINTER(BatchParams), ctypes.POINTER(ctypes.c_longlong),
                                            ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(vp)]
+    L.tsg_batch_product_bytes.argtypes = [vp, ctypes.POINTER(TsgTiled), ctypes.POINTER(TsgTiled), ip,
+                                          ctypes.c_longlong, ctypes.c_longlong, ctypes.POINTER(ctypes.c_longlong)]
     L.tsg_batch_run.argtypes = [vp]
     L.tsg_batch_sync.argtypes = [vp, ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_longlong)]
     L.tsg_batch_product.argtypes = [vp, ip, ctypes.POINTER(TsgTiled)]
@@ -764,6 +766,15 @@ def product_bounds_many(ctx: Context, pairs, c_tiles: bool = False):
     if c_tiles:
         return [(pr[i], tp[i], ct[i]) for i in range(n)]
     return [(pr[i], tp[i]) for i in range(n)]
+
+
+def batch_product_bytes(ctx: Context, A: Tiled, B: Tiled, products: int, c_tiles: int, schedule: str = "spa") -> int:
+    """Device bytes that A*B with these bounds adds to a batch, at most
+    (tsg_batch_product_bytes)."""
+    out = ctypes.c_longlong(0)
+    check(lib().tsg_batch_product_bytes(ctx.handle, ctypes.byref(A.s), ctypes.byref(B.s), SCHEDULE_IDS[schedule],
+                                        int(products), int(c_tiles), ctypes.byref(out)))
+    return out.value
 
 
 class Batch:

@@ -90,10 +90,11 @@ struct tsg_batch
 
 #define BATCH_THREADS 128
 #define BATCH_SPAN 3072 // tile columns of step 2's wide rows in a CTA's shared memory (two CTAs an SM)
-// step 3 by windows: products with this many scalar products per (row,
-// window), up to this many words of table each and in all
+// step 3 by windows: products with this many scalar products per (row, window)
+// (win_worth says the rest), whose tables and lists together take up to this
+// many words each and in all
 #define BATCH_WIN_MIN 16
-#define BATCH_WIN_WORDS (1LL << 22) // (btab; wtab holds two words a window beside it)
+#define BATCH_WIN_WORDS (1LL << 23)
 #define BATCH_WIN_TOTAL (1LL << 26)
 // a barrier wait gives up after this floor plus a share of the batch's work
 // (a B200 does well over 10 scalar products per ns, so the bound is loose)
@@ -1062,6 +1063,76 @@ static int record_run(tsg_batch *b, cudaStream_t st)
     return TSG_OK;
 }
 
+// A product's share of a batch, from its bounds: what batch_create lays out and
+// tsg_batch_product_bytes predicts.
+struct BatchShare
+{
+    long long capN;                        // values of C at most
+    size_t arena;                          // C's arrays, tile rows' counts and kinds
+    long long units, chunks;               // of step 2's wide rows; of the tile-count scan
+    int win, windows, bits, blocks;        // step 3 by windows
+    long long centries, claims, parts, words; // ctab's entries, claims, heavy rows' parts, words of all tables
+    int heavy_min;
+    bool wtab;
+};
+
+// win_words: table words that the batch has left
+static BatchShare batch_share(const tsg_tiled *A, const tsg_tiled *B, int schedule, long long prods, long long capT,
+                              int split, long long win_words)
+{
+    BatchShare S = {};
+    S.capN = std::min(prods, 256 * capT);
+    S.arena = align256(((size_t)A->tilem + 1) * 4) + align256((size_t)A->tilem * 4) + 2 * align256((size_t)capT * 4) +
+              align256(((size_t)capT + 1) * 4) + align256((size_t)capT * 32) + align256((size_t)capT * 16) +
+              align256((size_t)S.capN) + align256((size_t)S.capN * 8);
+    S.units = (long long)wide_units(A->tilem, A->nnz, split);
+    S.chunks = (capT + SCAN_CHUNK - 1) / SCAN_CHUNK;
+    if (schedule != TSG_SCHED_SPA || !A->row_ptr || A->m < 1 || B->m < 1 || B->n < 1)
+        return S;
+    const long long windows = (B->n + WIN_COLS - 1LL) / WIN_COLS;
+    if (prods < BATCH_WIN_MIN * windows * A->m)
+        return S;
+    S.heavy_min = win_heavy(A->nnz, A->m);
+    S.centries = A->tilem * (windows + 1);
+    S.claims = (long long)A->tilem * windows * WIN_PER;
+    S.parts = std::min((long long)A->m, (long long)A->nnz / S.heavy_min) * ((B->n + WIN_PART - 1LL) / WIN_PART);
+    // all that the windows take: btab (coarser blocks when it is large), wtab
+    // unless it alone is too much, ctab and the list of heavy rows' parts
+    const long long rest = S.centries + 4 * S.parts + 2;
+    S.wtab = 2 * windows * B->m + rest <= BATCH_WIN_WORDS / 2;
+    const long long fixed = rest + (S.wtab ? 2 * windows * B->m : 0);
+    if (fixed >= BATCH_WIN_WORDS || !win_table(B->m, B->n, BATCH_WIN_WORDS - fixed, S.bits, S.blocks))
+        return S;
+    S.words = fixed + (S.blocks + 1LL) * B->m;
+    S.windows = (int)windows;
+    S.win = S.words <= win_words && win_worth(S.capN, (long long)((double)A->nnz * (double)B->nnz / B->m), A->nnz, capT,
+                                              A->tilem, B->tilen, windows, S.words);
+    return S;
+}
+
+// Bytes of a batch beside its arena and tables, and of a product in them (rounded up)
+#define BATCH_FIXED_BYTES 2048
+#define BATCH_PRODUCT_BYTES (sizeof(BatchProd) + 128)
+
+static size_t batch_share_bytes(const BatchShare &S, long long tilem)
+{
+    return S.arena + BATCH_PRODUCT_BYTES + 8 * (size_t)S.chunks + sizeof(int4) * (size_t)S.units +
+           (S.win ? 4 * (size_t)S.words : 0);
+}
+
+extern "C" int tsg_batch_product_bytes(tsg_context *ctx, const tsg_tiled *A, const tsg_tiled *B, int schedule,
+                                       long long products, long long c_tiles, long long *bytes)
+{
+    if (!ctx || !A || !B || !bytes || products < 0 || c_tiles < 0)
+        return tsg_set_error(TSG_ERR_INVALID, "bad arguments");
+    // alone in its batch a product has the largest share: the whole of the
+    // table words, rows in the most parts
+    const int split = wide_split(A->nnz, ctx->num_sms);
+    *bytes = BATCH_FIXED_BYTES +
+             (long long)batch_share_bytes(batch_share(A, B, schedule, products, c_tiles, split, BATCH_WIN_TOTAL), A->tilem);
+    return TSG_OK;
+}
+
 // products / c_tiles: the bounds of every product when the caller has them
 // (tsg_product_bounds_many), else null and computed here
 static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const tsg_tiled *B,
@@ -1144,72 +1215,61 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
     }
     b->s1off.assign(2 * ((size_t)count + 1), 0);
     b->winoff.assign(4 * ((size_t)count + 1), 0);
-    std::vector<long long> tables(count, 0); // words of each product's window tables
+    std::vector<BatchShare> share(count);
     long long wunits = 0, hparts = 0, words = 0, entries = 0;
     for (int p = 0; p < count; p++)
         entries += A[p].nnz;
     b->split = wide_split(entries, ctx->num_sms);
+    b->arena_bytes = BATCH_FIXED_BYTES;
     for (int p = 0; p < count; p++)
     {
         const long long prods = v_prods[p], capT = v_tiles[p];
         const bool cta = step1_by_cta(&A[p], &B[p]);
         b->s1off[p + 1] = b->s1off[p] + (cta ? A[p].tilem : 0);
         b->s1off[count + 2 + p] = b->s1off[count + 1 + p] + (cta ? 0 : A[p].tilem);
-        wunits += (long long)wide_units(A[p].tilem, A[p].nnz, b->split);
         total_prods += prods;
-        long long capN = prods < 256 * capT ? prods : 256 * capT;
-        if (capN > 2147483647LL || capT > 2147483647LL / 16)
+        if (std::min(prods, 256 * capT) > 2147483647LL || capT > 2147483647LL / 16)
         {
             delete b;
             return tsg_set_error(TSG_ERR_OVERFLOW, "product %d exceeds 32-bit offsets", p);
         }
+        BatchShare &S = share[p] = batch_share(&A[p], &B[p], prm.schedule, prods, capT, b->split, BATCH_WIN_TOTAL - words);
+        if (S.win && b->winoff[3 * ((size_t)count + 1) + p] + S.claims + hparts + S.parts >= 2147483647LL)
+            S.win = 0;
+        b->arena_bytes += batch_share_bytes(S, A[p].tilem);
+        wunits += S.units;
+        chunk_cap += S.chunks;
         BatchProd &h = b->host[p];
         memset(&h, 0, sizeof(h));
         h.capT = capT;
-        h.capN = capN;
-        chunk_cap += (capT + SCAN_CHUNK - 1) / SCAN_CHUNK;
+        h.capN = S.capN;
         h.tilemA = A[p].tilem;
-        if (prm.schedule == TSG_SCHED_SPA && A[p].row_ptr && A[p].m > 0 && B[p].n > 0)
+        if (S.win)
         {
-            const long long windows = (B[p].n + WIN_COLS - 1LL) / WIN_COLS;
-            const long long parts = (long long)(A[p].nnz / win_heavy(A[p].nnz, A[p].m)) * ((B[p].n + WIN_PART - 1) / WIN_PART);
-            const long long claims = (long long)A[p].tilem * windows * WIN_PER, centries = A[p].tilem * (windows + 1);
-            int bits, blocks;
-            if (prods >= BATCH_WIN_MIN * windows * A[p].m &&
-                win_table(B[p].m, B[p].n, std::min(BATCH_WIN_WORDS, BATCH_WIN_TOTAL - words), bits, blocks) &&
-                b->winoff[3 * ((size_t)count + 1) + p] + claims + hparts + parts < 2147483647LL)
-            {
-                h.win = 1;
-                h.Q.windows = (int)windows;
-                h.Q.bits = bits;
-                h.Q.blocks = blocks;
-                h.Q.mA = A[p].m;
-                h.Q.heavy_min = win_heavy(A[p].nnz, A[p].m);
-                hparts += parts;
-                tables[p] = (blocks + 1LL) * B[p].m + centries + 2 * windows * B[p].m + 1;
-                words += (blocks + 1LL + 2 * windows) * B[p].m;
-                b->wins++;
-            }
-            const long long add[4] = {B[p].m, centries, A[p].m, claims};
-            for (int q = 0; q < 4; q++)
-                b->winoff[q * ((size_t)count + 1) + p + 1] = b->winoff[q * ((size_t)count + 1) + p] + (h.win ? add[q] : 0);
+            h.win = 1;
+            h.Q.windows = S.windows;
+            h.Q.bits = S.bits;
+            h.Q.blocks = S.blocks;
+            h.Q.mA = A[p].m;
+            h.Q.heavy_min = S.heavy_min;
+            hparts += S.parts;
+            words += S.words;
+            b->wins++;
         }
+        const long long add[4] = {B[p].m, S.centries, A[p].m, S.claims};
+        for (int q = 0; q < 4; q++)
+            b->winoff[q * ((size_t)count + 1) + p + 1] = b->winoff[q * ((size_t)count + 1) + p] + (h.win ? add[q] : 0);
         b->rowoff[p] = run;
         run += A[p].tilem;
         b->m[p] = A[p].m;
         b->n[p] = B[p].n;
         b->tilen[p] = B[p].tilen;
         off[p] = bytes;
-        bytes += align256(((size_t)A[p].tilem + 1) * 4) + align256((size_t)A[p].tilem * 4) + 2 * align256((size_t)capT * 4) +
-                 align256(((size_t)capT + 1) * 4) +
-                 align256((size_t)capT * 32) + align256((size_t)capT * 16) + align256((size_t)capN) +
-                 align256((size_t)capN * 8);
+        bytes += S.arena;
     }
     b->rowoff[count] = run;
-    long long table_words = 0;
-    for (long long t : tables)
-        table_words += t;
-    b->arena_bytes = bytes + (b->wins ? 4 * (size_t)table_words + sizeof(int4) * (size_t)hparts : 0);
+    // the tables' words without the lists of heavy rows' parts
+    const long long table_words = words - 4 * hparts;
     int st = TSG_OK;
     if ((st = tsg_alloc(ctx, (char **)&b->arena, bytes ? bytes : 256)) != TSG_OK)
     {
@@ -1225,17 +1285,32 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
         tsg_batch_destroy(b);
         return tsg_set_error(TSG_ERR_CUDA, "batch streams: %s", cudaGetErrorString(se));
     }
+    if (b->wins && ((st = tsg_alloc(ctx, &b->win_tables, (size_t)table_words)) != TSG_OK ||
+                    (st = tsg_alloc(ctx, &b->d_hlist, (size_t)hparts)) != TSG_OK ||
+                    (st = tsg_alloc(ctx, &b->d_winoff, b->winoff.size())) != TSG_OK))
+    {
+        if (st != TSG_ERR_OOM)
+        {
+            tsg_batch_destroy(b);
+            return st;
+        }
+        // no room for the tables, which the SPA kernel does without
+        cudaGetLastError();
+        tsg_release(ctx, b->win_tables);
+        tsg_release(ctx, b->d_hlist);
+        for (BatchProd &h : b->host)
+            h.win = 0;
+        b->wins = 0;
+        b->arena_bytes -= 4 * (size_t)words;
+    }
     if ((st = tsg_alloc(ctx, &b->d_denseoff, 2 * ((size_t)count + 1))) != TSG_OK ||
-        (b->wins && ((st = tsg_alloc(ctx, &b->win_tables, (size_t)table_words)) != TSG_OK ||
-                     (st = tsg_alloc(ctx, &b->d_hlist, (size_t)hparts)) != TSG_OK ||
-                     (st = tsg_alloc(ctx, &b->d_winoff, b->winoff.size())) != TSG_OK)) ||
         (st = tsg_alloc(ctx, &b->d_s1off, b->s1off.size())) != TSG_OK ||
         (st = tsg_alloc(ctx, &b->d_wlist, (size_t)wunits)) != TSG_OK)
     {
         tsg_batch_destroy(b);
         return st;
     }
-    table_words = 0;
+    long long table = 0;
     for (int p = 0; p < count; p++)
     {
         BatchProd &h = b->host[p];
@@ -1303,10 +1378,11 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
             h.Q.A_rptr = P.A_rptr;
             h.Q.A_rcol = P.A_rcol;
             h.Q.A_rval = P.A_rval;
-            h.Q.wtab = (int2 *)(b->win_tables + ((table_words + 1) & ~1LL));
-            h.Q.btab = (int *)(h.Q.wtab + (long long)h.Q.windows * P.mB);
+            table = (table + 1) & ~1LL; // wtab holds pairs
+            h.Q.wtab = share[p].wtab ? (int2 *)(b->win_tables + table) : nullptr;
+            h.Q.btab = b->win_tables + table + (share[p].wtab ? 2LL * h.Q.windows * P.mB : 0);
             h.Q.ctab = h.Q.btab + (h.Q.blocks + 1LL) * P.mB;
-            table_words += tables[p];
+            table += share[p].words - 4 * share[p].parts;
         }
     }
     if ((st = tsg_alloc(ctx, &b->d_prod, (size_t)count)) != TSG_OK || (st = tsg_alloc(ctx, &b->d_rowoff, (size_t)count + 1)) ||

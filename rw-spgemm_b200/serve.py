@@ -34,7 +34,7 @@ from concurrent.futures import Future
 
 import numpy as np
 
-from . import (TSG_TILED_CSC_VIEW, Batch, Context, check, csr_host_to_tiled, lib, product_bounds,
+from . import (TSG_TILED_CSC_VIEW, Batch, Context, batch_product_bytes, check, csr_host_to_tiled, lib, product_bounds,
                product_bounds_many)
 
 
@@ -274,23 +274,13 @@ class SpGEMMServer:
     def _in_use(self):
         return self.cache.bytes + sum(s.arena for s in self.slots if s.batch is not None)
 
-    @staticmethod
-    def _arena_of(A, prods, ctiles):
-        """Device bytes of a product's share of the batch arena, laid out as
-        tsg_batch_create does (row offsets and flags per A tile row, C's tile
-        arrays for ctiles tiles, min(products, 256 ctiles) values; every
-        array 256-byte aligned)."""
-        def al(x):
-            return (x + 255) & ~255
-        tm = A.s.tilem
-        vals = min(prods, 256 * ctiles)
-        return (al((tm + 1) * 4) + al(tm * 4) + 2 * al(ctiles * 4) + al((ctiles + 1) * 4) + al(ctiles * 32) +
-                al(ctiles * 16) + al(vals) + al(vals * 8))
-
     def _predict_many(self, ops):
         """(arena bytes, scalar products, C tiles) of each (A, B), with one
-        synchronisation (step 1's exact C-tile count)."""
-        return [(self._arena_of(A, prods, ctiles), prods, ctiles)
+        synchronisation (step 1's exact C-tile count).  The bytes are the
+        library's own bound of the product's share of a batch; the SPA
+        schedule's, which has the largest, unless the server keeps to another."""
+        sched = "spa" if self.schedule == "auto" else self.schedule[0]
+        return [(batch_product_bytes(self.cache.ctx, A, B, prods, ctiles, sched), prods, ctiles)
                 for (A, B), (prods, _, ctiles) in zip(ops, product_bounds_many(self.cache.ctx, ops, c_tiles=True))]
 
     def _predict(self, A, B):

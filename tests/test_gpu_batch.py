@@ -170,3 +170,50 @@ def test_batch_barrier_bound_gives_up_and_the_batch_recovers(tsg, ctx, oracle, g
             np.testing.assert_array_equal(np.asarray(got[k]).view(np.uint8), np.asarray(want[k]).view(np.uint8),
                                           err_msg=f"product {p} {k}")
     batch.close()
+
+
+def _fixed(m, n, e, seed):
+    """m rows of about e entries spread over all n columns."""
+    rng = np.random.default_rng(seed)
+    c = np.sort(rng.integers(0, n, (m, e)), axis=1)
+    keep = np.ones((m, e), bool)
+    keep[:, 1:] = c[:, 1:] != c[:, :-1]
+    rp = np.concatenate([[0], np.cumsum(keep.sum(1))]).astype(np.int32)
+    return m, n, rp, c[keep].astype(np.int32), rng.uniform(-1, 1, int(keep.sum()))
+
+
+@pytest.mark.parametrize("sched", ["spa", "rows", "tiles"])
+def test_predicted_bytes_hold_the_batch(tsg, ctx, gen, sched):
+    """A batch takes no more memory than it says, and it says no more than its
+    products' predictions: windows with heavy rows, hypersparse rows, dense
+    tiles, empty and tiny products."""
+    mats = _pairs(gen) + [(gen.rmat(12, 16, seed=5), gen.rmat(12, 16, seed=6)), (gen.rmat(13, 12, seed=7),) * 2,
+                          (_fixed(300, 5000, 700, 1), _fixed(5000, 9000, 12, 2))]
+    for some in (mats, mats[-3:], mats[-2:-1], mats[:1]):
+        pairs = [(_tiled(tsg, ctx, a, tsg.TSG_TILED_CSC_VIEW), _tiled(tsg, ctx, b, tsg.TSG_TILED_CSC_VIEW)) for a, b in some]
+        bounds = tsg.product_bounds_many(ctx, pairs, c_tiles=True)
+        ctx.synchronize()
+        used = ctx.pool_used()
+        batch = tsg.Batch(ctx, pairs, sched, 8, 512)
+        held = ctx.pool_used() - used
+        said = batch.info()["arena_bytes"]
+        predicted = sum(tsg.batch_product_bytes(ctx, a, b, pr, ct, sched) for (a, b), (pr, _, ct) in zip(pairs, bounds))
+        batch.close()
+        assert held <= said <= predicted
+        assert predicted - said < 4096 * len(pairs) + sum(a.nnz for a, _ in pairs)  # no wide margin either
+
+
+def test_batch_of_few_rows_times_a_wide_matrix_takes_no_tables(tsg, ctx, oracle):
+    """64 rows times 400,000 x 400,000: tables of the windows over all of B's
+    rows would be 1.25 GB for half a million products."""
+    A, B = _fixed(64, 400000, 2000, 1), _fixed(400000, 400000, 4, 2)
+    pair = _tiled(tsg, ctx, A, tsg.TSG_TILED_CSC_VIEW), _tiled(tsg, ctx, B, tsg.TSG_TILED_CSC_VIEW)
+    batch = tsg.Batch(ctx, [pair])
+    arena = batch.info()["arena_bytes"]
+    batch.run()
+    batch.sync()
+    got = [x.cpu().numpy() for x in tsg.tiled_to_csr(ctx, batch.product(0))]
+    batch.close()
+    want = oracle.gustavson(A, B, nthreads=8)
+    assert arena < 100 << 20
+    assert all(np.array_equal(g.view(np.uint8), w.view(np.uint8)) for g, w in zip(got, want[2:]))
