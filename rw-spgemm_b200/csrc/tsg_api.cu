@@ -945,7 +945,7 @@ int tsg_copy_stream(tsg_context *ctx)
     return TSG_OK;
 }
 
-int tsg_fork(tsg_context *ctx, cudaStream_t st, int n)
+int tsg_side_streams(tsg_context *ctx, int n)
 {
     if (!ctx->side_fork)
         TSG_CUDA(cudaEventCreateWithFlags(&ctx->side_fork, cudaEventDisableTiming));
@@ -956,6 +956,12 @@ int tsg_fork(tsg_context *ctx, cudaStream_t st, int n)
         if (!ctx->side[q])
             TSG_CUDA(cudaStreamCreateWithFlags(&ctx->side[q], cudaStreamNonBlocking));
     }
+    return TSG_OK;
+}
+
+int tsg_fork(tsg_context *ctx, cudaStream_t st, int n)
+{
+    TSG_TRY(tsg_side_streams(ctx, n));
     TSG_CUDA(cudaEventRecord(ctx->side_fork, st));
     for (int q = 0; q < n; q++)
         TSG_CUDA(cudaStreamWaitEvent(ctx->side[q], ctx->side_fork, 0));

@@ -80,8 +80,6 @@ struct tsg_batch
     int *win_tables;
     long long *d_denseoff;      // C tiles of the products with dense tiles, prefixes (rows form, columns form)
     int rows_form, cols_form;   // products of either form of the tile kernel
-    cudaStream_t side[2];       // step 3's kernels run beside one another
-    cudaEvent_t fork, join[2];
     int split;   // A entries of a unit of step 2's wide rows
     int wins;    // products that take the windows
     int gridw;   // persistent grid of k_batch_win
@@ -678,7 +676,8 @@ __global__ void __launch_bounds__(SPA_THREADS, 3)
 
 // ... the hypersparse rows of those products, a CTA each, from step 2's list ...
 __global__ void __launch_bounds__(SPA_THREADS, 3)
-    k_batch_hyper(const BatchProd *prods, const int4 *__restrict__ wlist, unsigned *bar, const int *err, int dense)
+    k_batch_hyper(const BatchProd *prods, int count, const long long *itemoff, const int4 *__restrict__ wlist,
+                  unsigned *bar, const int *err, int dense)
 {
     if (*(volatile const int *)err)
         return;
@@ -705,6 +704,11 @@ __global__ void __launch_bounds__(SPA_THREADS, 3)
         if ((u.z & 0xFFFF) == 0 && b.wide[u.y] == 2 && !b.win && !b.status && b.nnzC < (long long)dense * b.numC)
             step3_hyper_row(b.P, S, u.y);
     }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        atomicMax(reinterpret_cast<unsigned long long *>(const_cast<long long *>(itemoff)) + 2 * ((long long)count + 1) +
+                      7,
+                  gtimer());
 }
 
 // ... the tables of the products that take the windows (prefixes over the
@@ -1024,10 +1028,11 @@ static int record_run(tsg_batch *b, cudaStream_t st)
     if (b->params.schedule != TSG_SCHED_SPA)
         return TSG_OK;
     // step 3's kernels share no product: side by side, so that none waits for
-    // another's last rows
-    TSG_CUDA(cudaEventRecord(b->fork, st));
-    for (int q = 0; q < 2; q++)
-        TSG_CUDA(cudaStreamWaitEvent(b->side[q], b->fork, 0));
+    // another's last rows.  k_batch_hyper and k_batch_spa3, of the same products,
+    // stay in order: a branch more costs every batch (64 tiny products, step 3 0.039
+    // ms, 0.080 with a third).
+    TSG_TRY(tsg_fork(b->ctx, st, TSG_SIDE_STREAMS));
+    cudaStream_t *side = b->ctx->side;
     if (b->wins)
     {
         k_batch_wtab<<<b->ctx->num_sms * 8, 256, 0, st>>>(b->d_prod, b->count, b->d_winoff, b->d_hlist, b->d_bar, b->d_err,
@@ -1037,29 +1042,25 @@ static int record_run(tsg_batch *b, cudaStream_t st)
             b->d_prod, b->count, b->d_winoff, b->d_hlist, b->d_itemoff, b->d_bar, b->d_err, b->dense);
         TSG_CUDA(cudaGetLastError());
     }
-    k_batch_hyper<<<b->gridh, SPA_THREADS, sizeof(HypSmem), b->side[0]>>>(b->d_prod, b->d_wlist, b->d_bar, b->d_err,
-                                                                        b->dense);
+    k_batch_hyper<<<b->gridh, SPA_THREADS, sizeof(HypSmem), side[0]>>>(b->d_prod, b->count, b->d_itemoff, b->d_wlist,
+                                                                     b->d_bar, b->d_err, b->dense);
     TSG_CUDA(cudaGetLastError());
-    k_batch_spa3<<<b->grid3, SPA_THREADS, sizeof(SpaSmem), b->side[0]>>>(b->d_prod, b->count, b->d_itemoff, b->d_bar,
-                                                                       b->d_err, b->dense);
+    k_batch_spa3<<<b->grid3, SPA_THREADS, sizeof(SpaSmem), side[0]>>>(b->d_prod, b->count, b->d_itemoff, b->d_bar, b->d_err,
+                                                                    b->dense);
     TSG_CUDA(cudaGetLastError());
     if (b->rows_form)
     {
-        k_batch_dense3<false><<<b->ctx->num_sms * 8, DENSE3_THREADS, 0, b->side[1]>>>(b->d_prod, b->count, b->d_denseoff,
-                                                                                    b->d_itemoff, b->d_err);
+        k_batch_dense3<false><<<b->ctx->num_sms * 8, DENSE3_THREADS, 0, side[1]>>>(b->d_prod, b->count, b->d_denseoff,
+                                                                                 b->d_itemoff, b->d_err);
         TSG_CUDA(cudaGetLastError());
     }
     if (b->cols_form)
     {
-        k_batch_dense3<true><<<b->ctx->num_sms * 4, DENSE3_THREADS, 0, b->side[1]>>>(
+        k_batch_dense3<true><<<b->ctx->num_sms * 4, DENSE3_THREADS, 0, side[1]>>>(
             b->d_prod, b->count, b->d_denseoff + b->count + 1, b->d_itemoff, b->d_err);
         TSG_CUDA(cudaGetLastError());
     }
-    for (int q = 0; q < 2; q++)
-    {
-        TSG_CUDA(cudaEventRecord(b->join[q], b->side[q]));
-        TSG_CUDA(cudaStreamWaitEvent(st, b->join[q], 0));
-    }
+    TSG_TRY(tsg_join(b->ctx, st, TSG_SIDE_STREAMS));
     return TSG_OK;
 }
 
@@ -1276,14 +1277,10 @@ static int batch_create(tsg_context *ctx, int count, const tsg_tiled *A, const t
         delete b;
         return st;
     }
-    cudaError_t se = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
-    for (int q = 0; q < 2 && se == cudaSuccess; q++)
-        if ((se = cudaEventCreateWithFlags(&b->join[q], cudaEventDisableTiming)) == cudaSuccess)
-            se = cudaStreamCreateWithFlags(&b->side[q], cudaStreamNonBlocking);
-    if (se != cudaSuccess)
+    if (prm.schedule == TSG_SCHED_SPA && (st = tsg_side_streams(ctx, TSG_SIDE_STREAMS)) != TSG_OK)
     {
         tsg_batch_destroy(b);
-        return tsg_set_error(TSG_ERR_CUDA, "batch streams: %s", cudaGetErrorString(se));
+        return st;
     }
     if (b->wins && ((st = tsg_alloc(ctx, &b->win_tables, (size_t)table_words)) != TSG_OK ||
                     (st = tsg_alloc(ctx, &b->d_hlist, (size_t)hparts)) != TSG_OK ||
@@ -1635,16 +1632,6 @@ extern "C" int tsg_batch_destroy(tsg_batch *b)
     tsg_release(ctx, b->win_tables);
     char *a = (char *)b->arena;
     tsg_release(ctx, a);
-    cudaStreamSynchronize(ctx->stream);
-    for (int q = 0; q < 2; q++)
-    {
-        if (b->side[q])
-            cudaStreamDestroy(b->side[q]);
-        if (b->join[q])
-            cudaEventDestroy(b->join[q]);
-    }
-    if (b->fork)
-        cudaEventDestroy(b->fork);
     delete b;
     return TSG_OK;
 }

@@ -217,3 +217,43 @@ def test_batch_of_few_rows_times_a_wide_matrix_takes_no_tables(tsg, ctx, oracle)
     want = oracle.gustavson(A, B, nthreads=8)
     assert arena < 100 << 20
     assert all(np.array_equal(g.view(np.uint8), w.view(np.uint8)) for g, w in zip(got, want[2:]))
+
+
+def test_batches_of_one_context_share_its_streams(tsg, ctx, oracle, gen):
+    """Batches of one context, captured and not, run in turn and are destroyed
+    while others live: their step 3 uses the same side streams."""
+    mats = _pairs(gen)[-4:]
+    pairs = [(_tiled(tsg, ctx, a, tsg.TSG_TILED_CSC_VIEW), _tiled(tsg, ctx, b, tsg.TSG_TILED_CSC_VIEW)) for a, b in mats]
+    batches = [tsg.Batch(ctx, pairs, graph=g) for g in (True, False, True)]
+    for k in (0, 1, 2, 1):
+        batches[k].run()
+    batches.pop(0).close()
+    more = tsg.Batch(ctx, pairs[:2], graph=True)
+    for b in batches + [more]:
+        b.run()
+    for b, some in [(b, mats) for b in batches] + [(more, mats[:2])]:
+        b.sync()
+        for p, (x, y) in enumerate(some):
+            got = [t.cpu().numpy() for t in tsg.tiled_to_csr(ctx, b.product(p))]
+            want = oracle.gustavson(x, y, nthreads=8)
+            assert all(np.array_equal(g.view(np.uint8), w.view(np.uint8)) for g, w in zip(got, want[2:]))
+        b.close()
+
+
+def test_phase_times_hold_a_hypersparse_step_3(tsg, ctx, gen):
+    """The end stamp is the last kernel's, also when that takes the hypersparse
+    rows alone."""
+    import torch
+    pairs = [(_tiled(tsg, ctx, gen.random_poisson(32768, 32768, 8.0, seed=1), 2),
+              _tiled(tsg, ctx, gen.random_poisson(32768, 32768, 8.0, seed=2), 2))]
+    batch = tsg.Batch(ctx, pairs, graph=False)
+    events = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+    ratio = []
+    for _ in range(5):
+        events[0].record()
+        batch.run()
+        events[1].record()
+        batch.sync()
+        ratio.append(sum(batch.phase_ms().values()) / events[0].elapsed_time(events[1]))
+    batch.close()
+    assert max(ratio) > 0.8
