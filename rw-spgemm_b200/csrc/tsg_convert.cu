@@ -804,15 +804,15 @@ struct T2cSmem
     int len[TSG_BS], off[TSG_BS];    // row lengths; next output position of each row
 };
 
+// tile row tr, by the CTA (NT threads)
 template <int NT, int MODE>
-__global__ void __launch_bounds__(NT, 2048 / NT)
-    k_t2c(int m, int tr0, int tilem, const int *__restrict__ tile_ptr, const int *__restrict__ tile_col,
-          const int *__restrict__ tnnz, const unsigned char *__restrict__ Ptr, const unsigned char *__restrict__ Col,
-          const double *__restrict__ Val, int *__restrict__ rowptr, int *__restrict__ ccol, double *__restrict__ cval, int colmask)
+__device__ __forceinline__ void t2c_row(T2cSmem<NT> &S, int tr, int m, int tilem, const int *__restrict__ tile_ptr,
+                                        const int *__restrict__ tile_col, const int *__restrict__ tnnz,
+                                        const unsigned char *__restrict__ Ptr, const unsigned char *__restrict__ Col,
+                                        const double *__restrict__ Val, int *__restrict__ rowptr, int *__restrict__ ccol,
+                                        double *__restrict__ cval, int colmask)
 {
-    __shared__ T2cSmem<NT> S;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int tr = tr0 + blockIdx.x;
     const int rows = tr == tilem - 1 ? m - (tilem - 1) * TSG_BS : TSG_BS;
     const int t0 = tile_ptr[tr], t1 = tile_ptr[tr + 1];
     const bool aligned = ((uintptr_t)Ptr & 15) == 0;
@@ -999,15 +999,103 @@ __global__ void __launch_bounds__(NT, 2048 / NT)
     }
 }
 
+template <int NT, int MODE>
+__global__ void __launch_bounds__(NT, 2048 / NT)
+    k_t2c(int m, int tr0, int tilem, const int *__restrict__ tile_ptr, const int *__restrict__ tile_col,
+          const int *__restrict__ tnnz, const unsigned char *__restrict__ Ptr, const unsigned char *__restrict__ Col,
+          const double *__restrict__ Val, int *__restrict__ rowptr, int *__restrict__ ccol, double *__restrict__ cval, int colmask)
+{
+    __shared__ T2cSmem<NT> S;
+    t2c_row<NT, MODE>(S, tr0 + blockIdx.x, m, tilem, tile_ptr, tile_col, tnnz, Ptr, Col, Val, rowptr, ccol, cval, colmask);
+}
+
+// ... and a half-warp per tile row, lane = row, where a tile row holds few values:
+// a CTA's barriers and its 16 rows' lists are more than their own work.  A tile
+// row of more than T2C_LONG tiles among them is left to the CTA.
+#define T2C_HALVES 16 // tile rows of a CTA
+#define T2C_LONG 64
+template <int MODE>
+__global__ void __launch_bounds__(T2C_HALVES * 16)
+    k_t2c_few(int m, int tr0, int tr1, int tilem, const int *__restrict__ tile_ptr, const int *__restrict__ tile_col,
+              const int *__restrict__ tnnz, const unsigned char *__restrict__ Ptr, const unsigned char *__restrict__ Col,
+              const double *__restrict__ Val, int *__restrict__ rowptr, int *__restrict__ ccol, double *__restrict__ cval,
+              int colmask)
+{
+    __shared__ T2cSmem<T2C_HALVES * 16> S;
+    const int lane = threadIdx.x & 15;
+    const unsigned hmask = HW_MASK(threadIdx.x);
+    const int first = tr0 + blockIdx.x * T2C_HALVES, tr = first + (threadIdx.x >> 4);
+    const int t0 = tr < tr1 ? tile_ptr[tr] : 0, t1 = tr < tr1 ? tile_ptr[tr + 1] : 0;
+    const bool mine = tr < tr1 && t1 - t0 <= T2C_LONG;
+    if (mine)
+    {
+        const int rows = tr == tilem - 1 ? m - (tilem - 1) * TSG_BS : TSG_BS;
+        auto start = [&](int t) { return (int)Ptr[(long long)t * TSG_BS + lane]; };
+        auto end = [&](int t) {
+            return lane == rows - 1 ? tnnz[t + 1] - tnnz[t] : (int)Ptr[(long long)t * TSG_BS + lane + 1];
+        };
+        int off = 0;
+        if (MODE != T2C_FILL)
+        {
+            int n = 0;
+            if (lane < rows)
+                for (int t = t0; t < t1; t++)
+                    n += end(t) - start(t);
+            int incl = n;
+#pragma unroll
+            for (int d = 1; d < TSG_BS; d <<= 1)
+            {
+                const int o = __shfl_up_sync(hmask, incl, d, 16);
+                if (lane >= d)
+                    incl += o;
+            }
+            off = tnnz[t0] + incl - n;
+            if (lane < rows)
+                rowptr[tr * TSG_BS + lane] = off;
+            if (tr == tilem - 1 && lane == rows - 1)
+                rowptr[m] = off + n;
+        }
+        else if (lane < rows)
+            off = rowptr[tr * TSG_BS + lane];
+        if (MODE != T2C_ROWS && lane < rows)
+            for (int t = t0; t < t1; t++)
+            {
+                const int base = tnnz[t], cb = tile_col[t] * TSG_BS, e = end(t);
+                for (int q = start(t); q < e; q++, off++)
+                {
+                    ccol[off] = cb + (Col[base + q] & colmask);
+                    cval[off] = Val[base + q];
+                }
+            }
+    }
+    if (!__syncthreads_or(tr < tr1 && !mine))
+        return;
+    for (int q = first; q < min(first + T2C_HALVES, tr1); q++)
+        if (tile_ptr[q + 1] - tile_ptr[q] > T2C_LONG)
+        {
+            t2c_row<T2C_HALVES * 16, MODE>(S, q, m, tilem, tile_ptr, tile_col, tnnz, Ptr, Col, Val, rowptr, ccol, cval,
+                                           colmask);
+            __syncthreads();
+        }
+}
+
 // Row pointers and / or entries of tile rows [tr0, tr1) of C; nothing is
 // allocated.  512 threads for wide tile rows (R-MAT 16, 3,075 tiles a row:
 // 1.47 ms, 1.80 with 256, 2.89 with 128; 8,192 rows of 366 tiles: 0.049, 0.052
 // and 0.079 ms).  For narrow ones the step's barriers cost more than its width
 // gives, so CTAs are small once there are enough of them to fill the GPU (64^3
 // stencil, 16,384 rows of 84 tiles: 0.196 ms with 128, 0.224 with 256, 0.297
-// with 512; 21^3, 579 rows of 36: 0.0215, 0.0177, 0.0176 ms).
-#define T2C_WIDE 256    // mean tiles per tile row
-#define T2C_MANY (148 * 16) // tile rows that fill every SM with 128-thread CTAs
+// with 512; 21^3, 579 rows of 36: 0.0215, 0.0177, 0.0176 ms).  Tile rows of few
+// values are a half-warp's (half-warp and CTA: 31,250 tile rows of 48 values 0.017
+// and 0.154 ms, 62,500 of 47 0.031 and 0.283, 12,500 of 188 0.037 and 0.079, 6,912 of
+// 414 0.041 and 0.051, 3,125 of 496 0.033 and 0.025, of 976 0.060 and 0.032; few
+// tile rows: 1,250 of 48 0.011 and 0.018, 625 of 96 0.020 and 0.014, 579 of 394
+// 0.018 and 0.015).
+#define T2C_WIDE 256       // mean tiles per tile row
+#define T2C_FEW 64         // mean values per tile row up to which a tile row is a half-warp's,
+#define T2C_FEW_OF_MANY 448 // also with T2C_MANY tile rows,
+#define T2C_FEW_TILES 32   // in as many tiles at most (6,250 of 128 in 128: 0.106 and 0.067)
+#define T2C_MANY 16        // tile rows per SM that fill it with 128-thread CTAs
 template <int MODE>
 static int t2c_launch(tsg_context *ctx, const tsg_tiled *C, int tr0, int tr1, int *rowptr, int *colidx, double *val,
                       int colmask = 0xFF)
@@ -1015,7 +1103,16 @@ static int t2c_launch(tsg_context *ctx, const tsg_tiled *C, int tr0, int tr1, in
     if (tr1 <= tr0)
         return TSG_OK;
     const unsigned grid = (unsigned)(tr1 - tr0);
-    const int nt = C->numtile / C->tilem >= T2C_WIDE ? 512 : tr1 - tr0 >= T2C_MANY ? 128 : 256;
+    const bool many = tr1 - tr0 >= T2C_MANY * ctx->num_sms;
+    if (C->nnz / C->tilem <= (many ? T2C_FEW_OF_MANY : T2C_FEW) && C->numtile / C->tilem <= T2C_FEW_TILES)
+    {
+        k_t2c_few<MODE><<<tsg_blocks(grid, T2C_HALVES), T2C_HALVES * 16, 0, ctx->stream>>>(
+            C->m, tr0, tr1, C->tilem, C->tile_ptr, C->tile_columnidx, C->tile_nnz, C->tile_csr_Ptr, C->tile_csr_Col,
+            C->tile_csr_Value, rowptr, colidx, val, colmask);
+        TSG_LAUNCH_CHECK();
+        return TSG_OK;
+    }
+    const int nt = C->numtile / C->tilem >= T2C_WIDE ? 512 : many ? 128 : 256;
 #define T2C_GO(NT)                                                                                                  \
     k_t2c<NT, MODE><<<grid, NT, 0, ctx->stream>>>(C->m, tr0, C->tilem, C->tile_ptr, C->tile_columnidx, C->tile_nnz, \
                                                   C->tile_csr_Ptr, C->tile_csr_Col, C->tile_csr_Value, rowptr, colidx, val, colmask)

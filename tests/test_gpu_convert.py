@@ -17,6 +17,8 @@ def _matrix(kind, m, n, per_row, seed=3):
         counts = np.where(rng.random(m) < 0.3, 0, rng.integers(0, min(n, per_row) + 1, m))
     else:
         counts = np.full(m, min(n, per_row))
+        if kind == "hubs":  # rows of n / 20 entries in every 40th tile row and the last row
+            counts[7::640] = counts[-1] = n // 20
     cols = [np.sort(rng.choice(n, c, replace=False)) if c < n else np.arange(n) for c in counts]
     rp = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
     ci = np.concatenate(cols).astype(np.int32) if rp[-1] else np.zeros(0, np.int32)
@@ -25,8 +27,13 @@ def _matrix(kind, m, n, per_row, seed=3):
 
 SHAPES = [
     ("full", 1, 1, 0), ("full", 17, 33, 0), ("full", 47, 16, 0), ("some", 31, 700, 40),
-    ("some", 5000, 600, 9),            # narrow tile rows, 256 threads
-    ("some", 16 * 2400 + 5, 300, 3),   # narrow and many, 128 threads
+    ("some", 5000, 600, 9),            # few values a tile row: a half-warp each
+    ("some", 16 * 2400 + 5, 300, 3),
+    ("each", 600, 600, 4), ("each", 600, 600, 5),  # on both sides of 64 values a tile row
+    ("each", 5000, 600, 9),            # narrow tile rows, 256 threads
+    ("each", 16 * 2400 + 5, 600, 28),  # many of 448 values, a half-warp each ...
+    ("each", 16 * 2400 + 5, 600, 29),  # ... and of 464, 128 threads
+    ("hubs", 16 * 2400 + 5, 16 * 300, 2),  # long tile rows among them, the last too
     ("each", 33, 16 * 900, 400),       # wide, several steps of 512 tiles, most tiles empty in a row
     ("each", 16, 16 * 1100000, 80000), # one tile row of > 2048 steps: the 16-bit sums are emptied
     ("each", 48, 900, 31), ("each", 48, 900, 32), ("each", 37, 16 * 1024 + 5, 33),  # around 512 entries a tile row
