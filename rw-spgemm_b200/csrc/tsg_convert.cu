@@ -16,23 +16,50 @@
 
 #define HW_MASK(tid) (0xFFFFu << ((tid) & 16))
 
-// Tile rows of at least HEAVY_ENTRIES entries, or more than HEAVY_TILES tiles, are
-// listed (heavy[0] of them) and done by a CTA each: the half-warp's merge takes
-// one tile after another, a chain of loads as long as the tile row.  With column
-// view on a B200: R-MAT of 16,384 rows 1.65 -> 0.25 ms (entries alone 0.42),
-// 20,000 rows of 8 random entries 0.254 -> 0.161 (128 tiles a row), a band of 81
-// (6 tiles, 1,296 entries a row) 0.178 -> 0.123; a 48^3 grid's matrix, 22 tiles
-// and 432 entries a row, 0.199, 0.268 by CTAs.
-#define HEAVY_ENTRIES 512
-#define HEAVY_TILES 32
+// Heavy tile rows are listed (heavy[0] of them) and done by a CTA each: the
+// half-warp's merge takes one tile after another, a chain of loads as long as the
+// tile row.  A CTA takes about 4 us for every HEAVY_SPAN tile columns that the row
+// spans, but only three run on an SM at a time, where the half-warps of thousands
+// of tile rows hide each other's loads: so a row is heavy from `entries` entries or
+// `tiles` tiles on, if it holds `per_pass` entries for every HEAVY_SPAN columns, and
+// all three grow with the rounds of CTAs that all rows would take.  Conversion on a
+// B200, half-warps and CTAs:
+//   8 random entries a row (128 tiles a tile row): 20,000 rows (64 entries a pass)
+//     0.18 and 0.10 ms, 50,000 (32) 0.203 and 0.221, 100,000 (18) 0.22 and 0.57
+//   40 entries a row over 1 M columns (10 a pass): 64 rows 0.64 and 0.27; 20 entries,
+//     20,000 rows (5) 0.37 and 0.88
+//   200,000 rows of 41 in 5 tiles 0.26 and 0.33, 50,000 of 61 in 5 0.144 and 0.127;
+//     100,000 rows of 30 in 33 tiles 0.151 and 0.210, 1,000 rows of 1,000 in 63 0.69
+//     and 0.13; R-MAT 16 of 8 edges a row 3.2 and 0.25
+#define HEAVY_SPAN 1024
 #define HEAVY_THREADS 256
+struct HeavyRule
+{
+    int entries, tiles, per_pass;
+};
+
+static HeavyRule heavy_rule(const tsg_context *ctx, int tilem)
+{
+    const int rounds = std::max(1, tilem / (3 * ctx->num_sms));
+    return HeavyRule{std::max(512, 48 * rounds), std::min(256, std::max(32, 8 * rounds)),
+                     std::min(64, std::max(4, 3 * rounds))};
+}
+
+// entries a tile row of at least one needs to be heavy; lo: its first tile column,
+// lane r of the half-warp holds row r's entries [p, e), or what is left of them
+__device__ __forceinline__ int heavy_least(unsigned hmask, const HeavyRule &H, const int *__restrict__ col, int lo, int p,
+                                           int e)
+{
+    const int hi = __reduce_max_sync(hmask, p < e ? col[e - 1] >> 4 : lo);
+    return ((hi - lo) / HEAVY_SPAN + 1) * H.per_pass;
+}
 
 // ---------------------------------------------------------------------------
 // Pass 1: number of non-empty tiles in each tile row (half-warp per row).
 // ---------------------------------------------------------------------------
 __global__ void k_tile_count(int m, int tilem, const int *__restrict__ rowptr,
-                             const int *__restrict__ col, const int *__restrict__ err, int *__restrict__ tile_cnt,
-                             int *__restrict__ heavy)
+                             const int *__restrict__ col, const int *__restrict__ err, HeavyRule H,
+                             int *__restrict__ tile_cnt, int *__restrict__ heavy)
 {
     const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int tr = (int)(gid >> 4);
@@ -47,21 +74,21 @@ __global__ void k_tile_count(int m, int tilem, const int *__restrict__ rowptr,
         p = rowptr[r];
         e = rowptr[r + 1];
     }
-    if (__reduce_add_sync(hmask, e - p) >= HEAVY_ENTRIES)
-    {
-        if (lane == 0)
-            heavy[1 + atomicAdd(&heavy[0], 1)] = tr;
-        return;
-    }
+    const int entries = __reduce_add_sync(hmask, e - p);
     int cur = p < e ? (col[p] >> 4) : INT_MAX;
+    const int first = __reduce_min_sync(hmask, cur);
+    bool heavy_row = entries >= H.entries && entries >= heavy_least(hmask, H, col, first, p, e);
     int cnt = 0;
-    while (true)
+    while (!heavy_row)
     {
         const int jm = __reduce_min_sync(hmask, cur);
         if (jm == INT_MAX)
             break;
-        if (++cnt > HEAVY_TILES)
+        if (++cnt == H.tiles + 1 && entries >= heavy_least(hmask, H, col, first, p, e))
+        {
+            heavy_row = true;
             break;
+        }
         if (cur == jm)
         {
             do
@@ -73,8 +100,8 @@ __global__ void k_tile_count(int m, int tilem, const int *__restrict__ rowptr,
     }
     if (lane == 0)
     {
-        tile_cnt[tr] = cnt;
-        if (cnt > HEAVY_TILES)
+        tile_cnt[tr] = cnt; // of a heavy row k_tile_count_cta's
+        if (heavy_row)
             heavy[1 + atomicAdd(&heavy[0], 1)] = tr;
     }
 }
@@ -84,7 +111,7 @@ __global__ void k_tile_count(int m, int tilem, const int *__restrict__ rowptr,
 // ---------------------------------------------------------------------------
 __global__ void k_tile_fill(int m, int tilem, const int *__restrict__ rowptr,
                             const int *__restrict__ col, const double *__restrict__ val,
-                            const int *__restrict__ tile_ptr, int packed,
+                            const int *__restrict__ tile_ptr, int packed, HeavyRule H,
                             int *__restrict__ tile_columnidx, int *__restrict__ tile_rowidx,
                             int *__restrict__ tile_nnz, unsigned char *__restrict__ tPtr,
                             unsigned char *__restrict__ tCol, double *__restrict__ tVal,
@@ -103,7 +130,9 @@ __global__ void k_tile_fill(int m, int tilem, const int *__restrict__ rowptr,
         p = rowptr[r];
         e = rowptr[r + 1];
     }
-    if (tile_ptr[tr + 1] - tile_ptr[tr] > HEAVY_TILES || __reduce_add_sync(hmask, e - p) >= HEAVY_ENTRIES)
+    const int entries = __reduce_add_sync(hmask, e - p);
+    if ((tile_ptr[tr + 1] - tile_ptr[tr] > H.tiles || entries >= H.entries) &&
+        entries >= heavy_least(hmask, H, col, __reduce_min_sync(hmask, p < e ? col[p] >> 4 : INT_MAX), p, e))
         return; // by k_tile_fill_cta
     // value offset of the tile row's first tile: the row's first CSR entry
     int run = __shfl_sync(hmask, p, 0, 16);
@@ -251,14 +280,15 @@ __global__ void __launch_bounds__(HEAVY_THREADS)
 // entries set their bits in the tiles' row masks; a thread per tile column
 // numbers the tiles there are and writes their structure; the entries again
 // find their place: the tile's first value, its row's offset, and the bits of
-// the row's mask before their own.
-#define HEAVY_SPAN 1024
+// the row's mask before their own.  A pass takes its part of every row, the rows
+// being in order of columns, and begins at the first column that is left.
 struct HeavyFill
 {
     unsigned mask[HEAVY_SPAN][9];       // [tile column][two rows a word]; 9: a stride of its own bank
     unsigned char off[HEAVY_SPAN][TSG_BS + 4]; // row offsets in the tile
     int base[HEAVY_SPAN];               // the tile's first value
-    int rp[TSG_BS + 1];
+    int cur[TSG_BS], end[TSG_BS];       // what is left of the rows
+    int seg[TSG_BS + 1];                // the pass's entries, row by row
     int sum[HEAVY_THREADS / 32];
 };
 
@@ -275,31 +305,59 @@ __global__ void __launch_bounds__(HEAVY_THREADS)
     for (int l = blockIdx.x; l < heavy[0]; l += gridDim.x)
     {
         const int tr = heavy[1 + l];
-        if (tid <= TSG_BS)
-            S.rp[tid] = rowptr[min(m, tr * TSG_BS + tid)];
-        const int2 span = heavy_span(m, tr, rowptr, col);
+        if (tid < TSG_BS)
+        {
+            S.cur[tid] = rowptr[min(m, tr * TSG_BS + tid)];
+            S.end[tid] = rowptr[min(m, tr * TSG_BS + tid + 1)];
+        }
         __syncthreads();
-        const int e0 = S.rp[0], e1 = S.rp[TSG_BS];
-        auto row_of = [&](int e) {
-            int r = 0;
+        // the pass's entry x: its row, and its place in the matrix
+        auto entry = [&](int x, int &r) {
+            r = 0;
 #pragma unroll
             for (int h = 8; h > 0; h >>= 1)
-                r += S.rp[r + h] <= e ? h : 0;
-            return r;
+                r += S.seg[r + h] <= x ? h : 0;
+            return S.cur[r] + x - S.seg[r];
         };
-        int t = tile_ptr[tr], v = e0; // tiles and values before this pass
-        for (int c0 = span.x; c0 <= span.y; c0 += HEAVY_SPAN)
+        int t = tile_ptr[tr], v = S.cur[0]; // tiles and values before this pass
+        for (;;)
         {
-            const int cols = min(HEAVY_SPAN, span.y - c0 + 1);
+            // every warp for itself: the first column left, and the rows' ends in the pass
+            const int row = tid & 15, p = S.cur[row], e = S.end[row];
+            const int c0 = __reduce_min_sync(0xffffffffu, p < e ? col[p] >> 4 : INT_MAX);
+            if (c0 == INT_MAX)
+                break;
+            const int c1 = __reduce_max_sync(0xffffffffu, p < e ? col[e - 1] >> 4 : -1);
+            const int cols = min(HEAVY_SPAN, c1 - c0 + 1);
+            int lo = c1 - c0 < HEAVY_SPAN ? e : p, hi = e; // the first entry past the pass
+            while (lo < hi)
+            {
+                const int mid = (lo + hi) >> 1;
+                if ((col[mid] >> 4) - c0 < cols)
+                    lo = mid + 1;
+                else
+                    hi = mid;
+            }
+            int incl = lo - p;
+#pragma unroll
+            for (int d = 1; d < TSG_BS; d <<= 1)
+            {
+                const int o = __shfl_up_sync(0xffffffffu, incl, d, 16);
+                if ((tid & 15) >= d)
+                    incl += o;
+            }
+            if (tid < TSG_BS)
+                S.seg[tid + 1] = incl;
+            if (tid == 0)
+                S.seg[0] = 0;
             for (int q = tid; q < cols * 9; q += HEAVY_THREADS)
                 (&S.mask[0][0])[q] = 0u;
             __syncthreads();
-            for (int e = e0 + tid; e < e1; e += HEAVY_THREADS)
+            const int n = S.seg[TSG_BS];
+            for (int x = tid; x < n; x += HEAVY_THREADS)
             {
-                const int c = col[e], w = (c >> 4) - c0;
-                if (w < 0 || w >= cols)
-                    continue;
-                const int r = row_of(e);
+                int r;
+                const int c = col[entry(x, r)], w = (c >> 4) - c0;
                 atomicOr(&S.mask[w][r >> 1], 0x8000u >> (c & 15) << ((r & 1) * 16));
             }
             __syncthreads();
@@ -341,21 +399,25 @@ __global__ void __launch_bounds__(HEAVY_THREADS)
                 v += values;
             }
             __syncthreads();
-            for (int e = e0 + tid; e < e1; e += HEAVY_THREADS)
+            for (int x = tid; x < n; x += HEAVY_THREADS)
             {
-                const int c = col[e], w = (c >> 4) - c0;
-                if (w < 0 || w >= cols)
-                    continue;
-                const int r = row_of(e);
+                int r;
+                const int e = entry(x, r), c = col[e], w = (c >> 4) - c0;
                 const unsigned mr = (S.mask[w][r >> 1] >> ((r & 1) * 16)) & 0xFFFFu;
                 const int at = S.base[w] + S.off[w][r] + __popc(mr >> (16 - (c & 15)));
                 tCol[at] = (unsigned char)(packed ? ((r << 4) | (c & 15)) : (c & 15));
                 tVal[at] = val[e];
             }
             __syncthreads();
+            if (c1 - c0 < HEAVY_SPAN) // the rows' ends
+                break;
+            if (tid < TSG_BS)
+                S.cur[tid] = lo;
+            __syncthreads();
         }
         if (tr == tilem - 1 && tid == 0)
             tile_nnz[t] = v; // tile_nnz[numtile] = nnz
+        __syncthreads();
     }
 }
 
@@ -403,13 +465,14 @@ extern "C" int tsg_csr_to_tiled(tsg_context *ctx, int m, int n, int nnz, const i
     TSG_TRY(tsg_alloc(ctx, &out->tile_ptr, (size_t)tilem + 1));
     long long T = 0;
     int *heavy = nullptr;
-    const int most = std::min(tilem, nnz / std::min(HEAVY_ENTRIES, HEAVY_TILES + 1)); // tile rows that can be heavy
+    const HeavyRule H = heavy_rule(ctx, tilem);
+    const int most = std::min(tilem, nnz / std::min(H.entries, H.tiles + 1)); // tile rows that can be heavy
     TSG_TRY(tsg_alloc(ctx, &heavy, (size_t)most + 1));
     TSG_CUDA(cudaMemsetAsync(heavy, 0, sizeof(int), ctx->stream));
     if (tilem > 0)
     {
         k_tile_count<<<tsg_blocks((long long)tilem * 16, 256), 256, 0, ctx->stream>>>(
-            m, tilem, d_rowptr, d_colidx, d_err, out->tile_ptr, heavy);
+            m, tilem, d_rowptr, d_colidx, d_err, H, out->tile_ptr, heavy);
         TSG_LAUNCH_CHECK();
         if (most > 0)
         {
@@ -437,7 +500,7 @@ extern "C" int tsg_csr_to_tiled(tsg_context *ctx, int m, int n, int nnz, const i
     if (tilem > 0)
     {
         k_tile_fill<<<tsg_blocks((long long)tilem * 16, 256), 256, 0, ctx->stream>>>(
-            m, tilem, d_rowptr, d_colidx, d_val, out->tile_ptr, out->col_packed, out->tile_columnidx,
+            m, tilem, d_rowptr, d_colidx, d_val, out->tile_ptr, out->col_packed, H, out->tile_columnidx,
             out->tile_rowidx, out->tile_nnz, out->tile_csr_Ptr, out->tile_csr_Col, out->tile_csr_Value,
             out->mask);
         TSG_LAUNCH_CHECK();

@@ -39,6 +39,8 @@ SHAPES = [
     ("each", 48, 900, 31), ("each", 48, 900, 32), ("each", 37, 16 * 1024 + 5, 33),  # around 512 entries a tile row
     ("full", 37, 700, 0),              # a CTA each, full tiles, ragged
     ("each", 69, 16 * 4000, 2), ("each", 69, 16 * 4000, 3),  # on both sides of 32 tiles a tile row
+    ("each", 27, 16 * 300000, 74), ("each", 27, 16 * 300000, 78),  # and of 4 entries for every 1,024 tile columns
+    ("hubs", 33, 16 * 70000, 1),       # rows of very different length, passes with gaps between them
 ]
 
 
