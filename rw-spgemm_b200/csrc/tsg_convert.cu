@@ -547,8 +547,15 @@ extern "C" int tsg_csr_to_tiled(tsg_context *ctx, int m, int n, int nnz, const i
 // to a CTA that marks its rows in a bitmap, a tile's place being the number of
 // marks before its own.  A radix sort of all tiles took two to three passes
 // and as many launches again, whatever the size.  A 256^2 grid's
-// matrix, conversion with column view: 0.16 -> 0.107 ms.
+// matrix, conversion with column view: 0.16 -> 0.107 ms.  The sort stays where
+// there are few, long columns, whose tiles wait for one another at the columns'
+// counters and for the few CTAs that order them (column view alone, counted and
+// sorted: 62,500 tile rows times 4 columns 0.346 and 0.130 ms, times 40 1.03 and
+// 0.255, 18,750 times 800, 1,100 tiles a column, 0.232 and 0.154; 1,875 times 40,
+// 1,300 a column, 0.064 and 0.067, times 10 0.047 and 0.060).
 // ---------------------------------------------------------------------------
+#define CSC_SORTED 1024       // mean tiles per tile column from which they are sorted,
+#define CSC_SORTED_LEAST 24576 // if there are this many
 #define CSC_COL 256
 #define CSC_WARPS 8
 #define CSC_WORDS 8192 // bitmap words of a pass: 262,144 tile rows
@@ -689,6 +696,51 @@ __global__ void __launch_bounds__(CSC_LONG_THREADS)
     }
 }
 
+__global__ void k_csc_keys(int T, const int *__restrict__ tile_col, unsigned int *__restrict__ keys,
+                           int *__restrict__ vals)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < T)
+    {
+        keys[t] = (unsigned int)tile_col[t];
+        vals[t] = t;
+    }
+}
+
+// from the sorted keys: every column's first tile, and the tiles' rows
+__global__ void k_csc_rows(int T, int tilen, const unsigned int *__restrict__ keys, const int *__restrict__ pos,
+                           const int *__restrict__ tile_row, int *__restrict__ ptr, int *__restrict__ row)
+{
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= T)
+        return;
+    row[q] = tile_row[pos[q]];
+    const int c = (int)keys[q];
+    for (int j = q > 0 ? (int)keys[q - 1] + 1 : 0; j <= c; j++)
+        ptr[j] = q;
+    if (q == T - 1)
+        for (int j = c + 1; j <= tilen; j++)
+            ptr[j] = T;
+}
+
+static int csc_by_sort(tsg_context *ctx, tsg_tiled *mat)
+{
+    const int T = mat->numtile;
+    unsigned int *keys;
+    TSG_TRY(tsg_alloc(ctx, &keys, (size_t)T));
+    k_csc_keys<<<tsg_blocks(T, 256), 256, 0, ctx->stream>>>(T, mat->tile_columnidx, keys, mat->csc_tile_pos);
+    TSG_LAUNCH_CHECK();
+    int bits = 1;
+    while ((1LL << bits) < mat->tilen)
+        bits++;
+    TSG_TRY(tsg_sort_pairs_u32(ctx, keys, mat->csc_tile_pos, T, bits));
+    k_csc_rows<<<tsg_blocks(T, 256), 256, 0, ctx->stream>>>(T, mat->tilen, keys, mat->csc_tile_pos, mat->tile_rowidx,
+                                                           mat->csc_tile_ptr, mat->csc_tile_rowidx);
+    TSG_LAUNCH_CHECK();
+    tsg_release(ctx, keys);
+    return TSG_OK;
+}
+
 int tsg_build_mask_t(tsg_context *ctx, tsg_tiled *mat, int *hist)
 {
     const int T = mat->numtile;
@@ -722,11 +774,14 @@ int tsg_build_csc_view(tsg_context *ctx, tsg_tiled *mat)
         TSG_TRY(tsg_alloc(ctx, &mat->csc_tile_pos, (size_t)T));
     }
     TSG_CUDA(cudaMemsetAsync(mat->csc_tile_ptr, 0, ((size_t)tilen + 1) * sizeof(int), st));
-    TSG_TRY(tsg_build_mask_t(ctx, mat, mat->csc_tile_ptr));
+    const bool sorted = T >= CSC_SORTED_LEAST && T >= (long long)CSC_SORTED * tilen;
+    TSG_TRY(tsg_build_mask_t(ctx, mat, sorted ? nullptr : mat->csc_tile_ptr));
     if (!mat->row_ptr)
         TSG_TRY(tsg_build_row_view(ctx, mat));
     if (T == 0)
         return TSG_OK;
+    if (sorted)
+        return csc_by_sort(ctx, mat);
     TSG_TRY(tsg_scan_counts(ctx, mat->csc_tile_ptr, mat->csc_tile_ptr, tilen, nullptr));
     int *count, *any, *longs; // count: then longs, cleared together
     const int most = T / CSC_COL;

@@ -72,11 +72,13 @@ def test_tiles_and_back(tsg, ctx, oracle, shape, off_boundary):
 
 
 @pytest.mark.parametrize("m,n,tiles", [(16 * 300, 70, 255), (16 * 300, 70, 256), (16 * 300, 70, 257),
-                                       (16 * 5000 + 3, 40, 4000), (16 * 262150, 33, 262149)])
+                                       (16 * 5000 + 3, 40, 4000), (16 * 262150, 33, 262149),
+                                       (16 * 262150, 32000, 262149),
+                                       (16 * 45000 + 3, 100, 40000)])
 def test_column_view_of_columns_short_and_long(tsg, ctx, m, n, tiles):
     """Tile columns around the 256 tiles that a warp ranks, past them, and over
-    more tile rows (262,144) than one bitmap pass: tiles ascending by row in
-    every column."""
+    more tile rows (262,144) than one bitmap pass, and few columns of many
+    (sorted from 1,024 tiles a column on): tiles ascending by row in every column."""
     import torch
     rng = np.random.default_rng(tiles)
     rows = 16 * np.sort(rng.choice((m + 15) // 16, tiles, replace=False)).astype(np.int64)  # one entry a tile row
