@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(NT)
             if (u >= (int)*(volatile unsigned *)&bar[6])
                 break;
             const int4 w = __ldcg(wlist + u);
-            step2_wide_row<NT>(prods[w.x].P, S2, BATCH_SPAN, w.y, w.z, s_bins);
+            step2_wide_row<NT, false>(prods[w.x].P, S2, BATCH_SPAN, w.y, w.z, s_bins);
         }
     }
     else

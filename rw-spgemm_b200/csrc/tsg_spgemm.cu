@@ -149,7 +149,8 @@ __global__ void __launch_bounds__(NT, 1) k_step2_cta(ProdView P, int span, const
         if (q >= units)
             break;
         const int2 u = wide_units_of(P, wide)[q];
-        step2_wide_row<NT>(P, S, span, u.x, u.y, s_bins);
+        // with 512 threads the span is the widest row
+        step2_wide_row<NT, NT == 512>(P, S, span, u.x, u.y, s_bins);
     }
     if (threadIdx.x < 4 && s_bins[threadIdx.x])
         atomicAdd(&bins[threadIdx.x], s_bins[threadIdx.x]);

@@ -218,3 +218,16 @@ def test_few_rows_of_a_do_not_pay_for_tables_of_a_large_b(tsg, ctx, oracle, m, e
     assert (info["step3_name"] == "k_step3_win") == wins
     ctx.synchronize()
     assert ctx.pool_used() <= used
+
+
+@pytest.mark.parametrize("entries,n", [(1, 98304), (1, 98320), (1, 300000), (3, 300000), (40, 300000), (200, 300000)])
+def test_few_tiles_over_many_columns(tsg, ctx, oracle, entries, n):
+    """Wide rows of few C tiles on both sides of what a pass of step 2 holds by
+    columns (98,304), by a slot per tile, and of too many for that."""
+    A, B = _rows(70, 2000, [entries] * 69 + [60], 1), _rows(2000, n, [1 + entries % 7] * 2000, 2)
+    _check(tsg, ctx, oracle, A, B, tsg.TSG_TILED_CSC_VIEW)
+    batch = tsg.Batch(ctx, [tuple(_tiled(tsg, ctx, x, tsg.TSG_TILED_CSC_VIEW) for x in (A, B))])
+    batch.run()
+    batch.sync()
+    _same([x.cpu().numpy() for x in tsg.tiled_to_csr(ctx, batch.product(0))], oracle.gustavson(A, B, nthreads=8))
+    batch.close()
