@@ -258,57 +258,72 @@ __global__ void k_sym_edges(int n, const int *__restrict__ rowptr, const int *__
     }
 }
 
+// Rows of the matrix, a warp each, f(row, first entry, its end, step between the
+// lane's entries); rows of RCM_LONG_ROW entries and more by the whole block (256
+// threads), which all its threads call.
+#define RCM_LONG_ROW 1024
+template <typename F>
+__device__ __forceinline__ void rcm_rows(int n, const int *__restrict__ rowptr, F f)
+{
+    const long long first = (long long)blockIdx.x * (blockDim.x >> 5), r = first + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    const int s = r < n ? rowptr[r] : 0, e = r < n ? rowptr[r + 1] : 0;
+    const bool is_long = e - s >= RCM_LONG_ROW;
+    if (!is_long)
+        f((int)r, s + lane, e, 32);
+    if (!__syncthreads_or(is_long))
+        return;
+    for (long long q = first; q < min((long long)n, first + (blockDim.x >> 5)); q++)
+        if (rowptr[q + 1] - rowptr[q] >= RCM_LONG_ROW)
+            f((int)q, rowptr[q] + (int)threadIdx.x, rowptr[q + 1], (int)blockDim.x);
+}
+
 // *odd becomes nonzero unless the matrix is square-symmetric in its pattern
 // with rows strictly increasing: the off-diagonal entries of every row are
 // then its neighbours as they stand
 __global__ void k_sym_check(int n, const int *__restrict__ rowptr, const int *__restrict__ col, int *__restrict__ odd)
 {
-    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (w >= n)
-        return;
-    const int r = (int)w, s = rowptr[r], e = rowptr[r + 1];
-    bool bad = false;
-    for (int p = s + lane; p < e && !bad; p += 32)
-    {
-        const int j = col[p];
-        bad = j < 0 || j >= n || (p + 1 < e && col[p + 1] <= j);
-        if (bad || j == r)
-            continue;
-        int lo = rowptr[j], hi = rowptr[j + 1]; // r among row j's columns
-        const int end = hi;
-        while (lo < hi)
+    rcm_rows(n, rowptr, [&](int r, int first, int e, int step) {
+        bool bad = false;
+        for (int p = first; p < e && !bad; p += step)
         {
-            const int mid = (lo + hi) >> 1;
-            if (col[mid] < r)
-                lo = mid + 1;
-            else
-                hi = mid;
+            const int j = col[p];
+            bad = j < 0 || j >= n || (p + 1 < e && col[p + 1] <= j);
+            if (bad || j == r)
+                continue;
+            int lo = rowptr[j], hi = rowptr[j + 1]; // r among row j's columns
+            const int end = hi;
+            while (lo < hi)
+            {
+                const int mid = (lo + hi) >> 1;
+                if (col[mid] < r)
+                    lo = mid + 1;
+                else
+                    hi = mid;
+            }
+            bad = lo >= end || col[lo] != r;
         }
-        bad = lo >= end || col[lo] != r;
-    }
-    if (bad)
-        *odd = 1;
+        if (bad)
+            *odd = 1;
+    });
 }
 
-// warp per row: its off-diagonal columns, in order, to adj + offs[row]
+// The off-diagonal columns of every row, in order, to adj + offs[row], rows
+// strictly increasing: past the diagonal entry, if there is one, a place earlier
 __global__ void k_offdiag_copy(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
                                const int *__restrict__ offs, int *__restrict__ adj)
 {
-    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (w >= n)
-        return;
-    const int r = (int)w, s = rowptr[r], e = rowptr[r + 1];
-    int base = offs[r];
-    for (int p0 = s; p0 < e; p0 += 32)
-    {
-        const int j = p0 + lane < e ? col[p0 + lane] : r;
-        const unsigned bal = __ballot_sync(0xffffffffu, j != r);
-        if (j != r)
-            adj[base + __popc(bal & ((1u << lane) - 1u))] = j;
-        base += __popc(bal);
-    }
+    rcm_rows(n, rowptr, [&](int r, int first, int e, int step) {
+        if (first >= e)
+            return;
+        const int s = rowptr[r], base = offs[r], diagonal = (e - s) - (offs[r + 1] - base);
+        for (int p = first; p < e; p += step)
+        {
+            const int j = col[p];
+            if (j != r)
+                adj[base + (p - s) - (j > r ? diagonal : 0)] = j;
+        }
+    });
 }
 
 __global__ void k_uniq_flags(long long ne, const unsigned long long *__restrict__ keys, int *__restrict__ rowlen,
@@ -351,7 +366,12 @@ __global__ void k_uniq_scatter(long long ne, const unsigned long long *__restric
 // ---------------------------------------------------------------------------
 #define RCM_THREADS 512
 #define RCM_BUCKET 2048
-#define RCM_WAIT_NS 2000000000ULL // bound of every barrier wait
+// Neighbours from which a vertex is expanded by many warps: one warp took a hub's
+// 32 at a time (a star of 100,000 leaves, the whole ordering: 7.7 ms, 0.95).
+#define RCM_LONG 1024
+// bound of every barrier wait: a floor, and a share of the vertices and edges
+#define RCM_WAIT_NS 2000000000ULL
+#define RCM_WAIT_NS_PER_ITEM 100ULL
 
 struct RcmRun
 {
@@ -360,14 +380,19 @@ struct RcmRun
     int cnt;
     int err;
     int maxb;     // largest bucket of the level
-    int found[3]; // new vertices, a level's counter cleared two levels before
+    int2 found[3]; // new vertices, and the frontier's of many neighbours (listed in tmp);
+                   // a level's counters are cleared in the level before
     unsigned bar[2];
+    unsigned long long wait_ns; // bound of a barrier wait
 };
 
-// All blocks are resident (cooperative launch); false when the wait ran out.
+// All blocks are resident (cooperative launch); false when the block's wait ran
+// out or another's had: it does not arrive again, so that every block's next
+// wait ends too.
 __device__ __forceinline__ bool rcm_barrier(RcmRun *R)
 {
     __syncthreads();
+    bool left = false; // thread 0
     if (threadIdx.x == 0)
     {
         volatile unsigned *gen = &R->bar[1];
@@ -386,17 +411,17 @@ __device__ __forceinline__ bool rcm_barrier(RcmRun *R)
             while (*gen == g)
             {
                 asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-                if (*(volatile int *)&R->err || t - t0 > RCM_WAIT_NS)
+                if (*(volatile int *)&R->err || t - t0 > R->wait_ns)
                 {
                     atomicCAS(&R->err, 0, TSG_ERR_TIMEOUT);
+                    left = true;
                     break;
                 }
             }
         }
         __threadfence();
     }
-    __syncthreads();
-    return *(volatile int *)&R->err == 0;
+    return !__syncthreads_or(left);
 }
 
 // What other blocks write during the launch is read past L1 (__ldcg).
@@ -411,12 +436,10 @@ __global__ void __launch_bounds__(RCM_THREADS)
     int lo = R->lo, hi = R->hi;
     for (int level = 0;; level++)
     {
-        int *found = &R->found[level % 3];
-        for (int p = lo + gw; p < hi; p += nw)
-        {
-            const int v = __ldcg(order + p);
-            const int q1 = gptr[v + 1];
-            for (int q = gptr[v]; q < q1; q += 32)
+        int *found = &R->found[level % 3].x, *longs = &R->found[level % 3].y;
+        // neighbours [q0, q1) of the vertex at position p, 32 at every `step`-th
+        auto expand = [&](int p, int q0, int q1, int step) {
+            for (int q = q0; q < q1; q += step)
             {
                 int u = -1;
                 bool first = false;
@@ -440,10 +463,34 @@ __global__ void __launch_bounds__(RCM_THREADS)
                         next[at + __popc(b & ((1u << lane) - 1u))] = u;
                 }
             }
+        };
+        for (int p = lo + gw; p < hi; p += nw)
+        {
+            const int v = __ldcg(order + p);
+            const int q0 = gptr[v], q1 = gptr[v + 1];
+            if (q1 - q0 < RCM_LONG)
+                expand(p, q0, q1, 32);
+            else if (lane == 0)
+                tmp[atomicAdd(longs, 1)] = p;
         }
         if (!rcm_barrier(R))
             return;
-        const int c = __ldcg(found);
+        const int2 counts = __ldcg(&R->found[level % 3]);
+        const int nlong = counts.y;
+        int c = counts.x;
+        if (nlong > 0)
+        {
+            // the warps in groups, a vertex of the list to a group at a time
+            const int group = max(1, nw / nlong), groups = nw / group;
+            for (int l = gw / group; l < nlong && gw < groups * group; l += groups)
+            {
+                const int p = __ldcg(tmp + l), v = __ldcg(order + p);
+                expand(p, gptr[v] + gw % group * 32, gptr[v + 1], group * 32);
+            }
+            if (!rcm_barrier(R))
+                return;
+            c = __ldcg(found);
+        }
         if (c == 0)
         {
             if (gt == 0)
@@ -499,7 +546,7 @@ __global__ void __launch_bounds__(RCM_THREADS)
             {
                 boff[hi - lo] = run;
                 R->maxb = s_max;
-                R->found[(level + 1) % 3] = 0;
+                R->found[(level + 1) % 3] = make_int2(0, 0);
             }
         }
         if (!rcm_barrier(R))
@@ -600,17 +647,30 @@ __global__ void k_reverse(int n, const int *__restrict__ in, int *__restrict__ o
         out[i] = in[n - 1 - i];
 }
 
-static int rcm_order(tsg_context *ctx, int n, const int *rowptr, const int *col, int *d_order)
+// What rcm_order allocates; released whichever way it returns.
+struct RcmScratch
 {
+    int *offs, *gptr, *odd, *adj, *idx, *keep, *seeds, *pos, *parent, *order, *next, *cnt, *best, *tmp, *bcnt, *boff;
+    unsigned int *dk, *ik;
+    unsigned long long *keys, *lk;
+    RcmRun *run;
+};
+
+static int rcm_order_in(tsg_context *ctx, int n, const int *rowptr, const int *col, int *d_order, RcmScratch &W)
+{
+    int *&offs = W.offs, *&gptr = W.gptr, *&odd = W.odd, *&adj = W.adj, *&idx = W.idx, *&keep = W.keep, *&seeds = W.seeds,
+        *&pos = W.pos, *&parent = W.parent, *&order = W.order, *&next = W.next, *&cnt = W.cnt, *&best = W.best,
+        *&tmp = W.tmp, *&bcnt = W.bcnt, *&boff = W.boff;
+    unsigned int *&dk = W.dk, *&ik = W.ik;
+    unsigned long long *&keys = W.keys, *&lk = W.lk;
+    RcmRun *&run = W.run;
     cudaStream_t st = ctx->stream;
     const unsigned gw = tsg_blocks((long long)n * 32, 256), g1 = tsg_blocks(n, 256);
     // symmetrised off-diagonal graph: gptr / adj (sorted, duplicate-free)
-    int *offs, *gptr;
     TSG_TRY(tsg_alloc(ctx, &offs, (size_t)n + 1));
     TSG_TRY(tsg_alloc(ctx, &gptr, (size_t)n + 1));
     // A grid's or graph's matrix has its neighbours in order already; only a
     // pattern that does not is symmetrised by a sort (of twice its entries)
-    int *odd;
     TSG_TRY(tsg_alloc(ctx, &odd, 1));
     TSG_CUDA(cudaMemsetAsync(odd, 0, sizeof(int), st));
     k_sym_check<<<gw, 256, 0, st>>>(n, rowptr, col, odd);
@@ -621,8 +681,8 @@ static int rcm_order(tsg_context *ctx, int n, const int *rowptr, const int *col,
     long long half = 0;
     TSG_TRY(tsg_scan_counts(ctx, offs, offs, n, &half));
     const bool symmetric = *(const int *)(ctx->h_pinned + 1) == 0;
+    const long long edges = symmetric ? half : 2 * half;
     tsg_release(ctx, odd);
-    int *adj;
     if (symmetric)
     {
         TSG_TRY(tsg_alloc(ctx, &adj, (size_t)half));
@@ -633,8 +693,6 @@ static int rcm_order(tsg_context *ctx, int n, const int *rowptr, const int *col,
     else
     {
         const long long ne = 2 * half;
-        unsigned long long *keys;
-        int *idx, *keep;
         TSG_TRY(tsg_alloc(ctx, &keys, (size_t)ne));
         TSG_TRY(tsg_alloc(ctx, &idx, (size_t)ne));
         TSG_TRY(tsg_alloc(ctx, &keep, (size_t)ne + 1));
@@ -665,12 +723,6 @@ static int rcm_order(tsg_context *ctx, int n, const int *rowptr, const int *col,
     tsg_release(ctx, offs);
 
     // seeds in (degree, id) order; isolated vertices are the leading seeds
-    unsigned int *dk;
-    int *seeds, *pos, *parent, *order, *next, *cnt, *best;
-    unsigned long long *lk;
-    unsigned int *ik;
-    int *tmp, *bcnt, *boff;
-    RcmRun *run;
     static_assert(sizeof(RcmRun) <= 32 * sizeof(long long), "read-back buffer");
     TSG_TRY(tsg_alloc(ctx, &tmp, (size_t)n));
     TSG_TRY(tsg_alloc(ctx, &bcnt, (size_t)n + 1));
@@ -717,6 +769,7 @@ static int rcm_order(tsg_context *ctx, int n, const int *rowptr, const int *col,
     if (per_sm < 1)
         return tsg_set_error(TSG_ERR_CUDA, "the RCM level kernel cannot be resident");
     const unsigned grid = (unsigned)ctx->num_sms;
+    const unsigned long long wait_ns = RCM_WAIT_NS + RCM_WAIT_NS_PER_ITEM * (unsigned long long)(n + edges);
     while (placed < n)
     {
         TSG_CUDA(cudaMemcpyAsync(best, &n, sizeof(int), cudaMemcpyHostToDevice, st));
@@ -734,6 +787,7 @@ static int rcm_order(tsg_context *ctx, int n, const int *rowptr, const int *col,
         memset(hr, 0, sizeof(RcmRun));
         hr->lo = placed;
         hr->hi = placed + 1;
+        hr->wait_ns = wait_ns;
         for (;;)
         {
             TSG_CUDA(cudaMemcpyAsync(run, hr, sizeof(RcmRun), cudaMemcpyHostToDevice, st));
@@ -762,28 +816,29 @@ static int rcm_order(tsg_context *ctx, int n, const int *rowptr, const int *col,
             memset(hr, 0, sizeof(RcmRun));
             hr->lo = hi;
             hr->hi = hi + c;
+            hr->wait_ns = wait_ns;
         }
         placed = hr->hi;
     }
     k_reverse<<<g1, 256, 0, st>>>(n, order, d_order);
     TSG_LAUNCH_CHECK();
-    tsg_release(ctx, dk);
-    tsg_release(ctx, seeds);
-    tsg_release(ctx, pos);
-    tsg_release(ctx, parent);
-    tsg_release(ctx, order);
-    tsg_release(ctx, next);
-    tsg_release(ctx, lk);
-    tsg_release(ctx, ik);
-    tsg_release(ctx, tmp);
-    tsg_release(ctx, bcnt);
-    tsg_release(ctx, boff);
-    tsg_release(ctx, run);
-    tsg_release(ctx, cnt);
-    tsg_release(ctx, best);
-    tsg_release(ctx, gptr);
-    tsg_release(ctx, adj);
     return TSG_OK;
+}
+
+static int rcm_order(tsg_context *ctx, int n, const int *rowptr, const int *col, int *d_order)
+{
+    RcmScratch W = {};
+    const int status = rcm_order_in(ctx, n, rowptr, col, d_order, W);
+    int **ints[] = {&W.offs, &W.gptr, &W.odd, &W.adj, &W.idx, &W.keep, &W.seeds, &W.pos,
+                    &W.parent, &W.order, &W.next, &W.cnt, &W.best, &W.tmp, &W.bcnt, &W.boff};
+    for (int **p : ints)
+        tsg_release(ctx, *p);
+    tsg_release(ctx, W.dk);
+    tsg_release(ctx, W.ik);
+    tsg_release(ctx, W.keys);
+    tsg_release(ctx, W.lk);
+    tsg_release(ctx, W.run);
+    return status;
 }
 
 extern "C" int tsg_order(tsg_context *ctx, int kind, int m, int n, int nnz, const int *d_rowptr, const int *d_col,

@@ -232,3 +232,30 @@ def test_rcm_of_patterns_that_are_not_symmetric_or_not_in_order(tsg, ctx, oracle
     ci3 = ci.copy()
     ci3[rp[50]:rp[51]] = ci3[rp[50]:rp[51]][::-1]
     assert np.array_equal(rcm(rp, ci3), want)
+
+
+@pytest.mark.parametrize("hubs,leaves", [(1, 1023), (1, 1024), (7, 1500), (40, 1100), (2, 60000)])
+def test_rcm_of_vertices_with_many_neighbours(tsg, ctx, oracle, hubs, leaves):
+    """Hubs around the number of neighbours that one warp expands, several in a
+    level and one of most vertices, each joined to the first; leaves of two hubs
+    among them; rows that a block checks and copies as a whole."""
+    import torch
+    rng = np.random.default_rng(hubs)
+    n = 1 + hubs * (leaves + 1)
+    first = 1 + np.arange(hubs) * (leaves + 1)
+    edges = [np.stack([np.zeros(hubs, np.int64), first])]
+    edges += [np.stack([np.full(leaves, h), h + 1 + np.arange(leaves)]) for h in first]
+    if hubs > 1:
+        edges.append(np.stack([rng.choice(first, 300), rng.integers(1, n, 300)]))
+    a, b = np.concatenate(edges, axis=1)
+    a, b = a[a != b], b[a != b]
+    diag = rng.choice(n, n // 3, replace=False)  # some diagonal entries
+    key = np.unique(np.concatenate([a * n + b, b * n + a, diag * n + diag]))
+    rp = np.searchsorted(key // n, np.arange(n + 1)).astype(np.int32)
+    ci = (key % n).astype(np.int32)
+    d = torch.device("cuda", torch.cuda.current_device())
+    used = ctx.pool_used()
+    got = tsg.order(ctx, "rcm", n, n, torch.from_numpy(rp).to(d), torch.from_numpy(ci).to(d)).cpu().numpy()
+    assert np.array_equal(got, oracle.order("rcm", (n, n, rp, ci, np.ones(ci.size))))
+    ctx.synchronize()
+    assert ctx.pool_used() <= used
