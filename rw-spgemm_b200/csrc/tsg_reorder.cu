@@ -902,7 +902,7 @@ extern "C" int tsg_order(tsg_context *ctx, int kind, int m, int n, int nnz, cons
 // bipermutation of a device CSR
 // ---------------------------------------------------------------------------
 __global__ void k_perm_rowlen(int m, const int *__restrict__ rowptr, const int *__restrict__ row_old,
-                              int *__restrict__ cnt, int *__restrict__ longest)
+                              int *__restrict__ cnt, int *__restrict__ longest) // longest: may be null
 {
     int most = 0;
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < m; r += gridDim.x * blockDim.x)
@@ -912,7 +912,7 @@ __global__ void k_perm_rowlen(int m, const int *__restrict__ rowptr, const int *
         most = max(most, cnt[r]);
     }
     most = __reduce_max_sync(0xffffffffu, most);
-    if ((threadIdx.x & 31) == 0 && most > *(volatile int *)longest)
+    if (longest && (threadIdx.x & 31) == 0 && most > *(volatile int *)longest)
         atomicMax(longest, most);
 }
 
@@ -987,14 +987,23 @@ extern "C" int tsg_permute_csr(tsg_context *ctx, int m, int n, int nnz, const in
         TSG_CUDA(cudaMemsetAsync(d_out_rowptr, 0, sizeof(int), st));
         return TSG_OK;
     }
-    int *longest;
-    TSG_TRY(tsg_alloc(ctx, &longest, 1));
-    TSG_CUDA(cudaMemsetAsync(longest, 0, sizeof(int), st));
+    // The longest row is read back, except where that is not needed (some row has
+    // to be longer than PERM_ROW) or not allowed: a stream that is being captured
+    // takes the sort, which any matrix may.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    TSG_CUDA(cudaStreamIsCapturing(st, &capture));
+    const bool sorted = capture != cudaStreamCaptureStatusNone || nnz > (long long)PERM_ROW * m;
+    int *longest = nullptr;
+    if (!sorted)
+    {
+        TSG_TRY(tsg_alloc(ctx, &longest, 1));
+        TSG_CUDA(cudaMemsetAsync(longest, 0, sizeof(int), st));
+    }
     k_perm_rowlen<<<tsg_blocks(m, 256), 256, 0, st>>>(m, d_rowptr, d_row_old, d_out_rowptr, longest);
     TSG_LAUNCH_CHECK();
-    long long most = 0;
+    long long most = PERM_ROW + 1;
     TSG_TRY(tsg_scan_counts(ctx, d_out_rowptr, d_out_rowptr, m, nullptr));
-    if (nnz > 0)
+    if (nnz > 0 && longest)
         TSG_TRY(tsg_read_int(ctx, longest, &most));
     tsg_release(ctx, longest);
     if (nnz == 0)

@@ -259,3 +259,38 @@ def test_rcm_of_vertices_with_many_neighbours(tsg, ctx, oracle, hubs, leaves):
     assert np.array_equal(got, oracle.order("rcm", (n, n, rp, ci, np.ones(ci.size))))
     ctx.synchronize()
     assert ctx.pool_used() <= used
+
+
+@pytest.mark.parametrize("longest", [30, 900])
+def test_permute_csr_in_a_captured_graph(tsg, oracle, gen, longest):
+    """The C call may be captured: the graph's replay permutes what its inputs
+    hold then."""
+    import ctypes
+    import torch
+    rng = np.random.default_rng(longest)
+    m, n = 300, 1000
+    counts = rng.integers(0, 31, m)
+    counts[5] = longest
+    rp = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    ci = np.concatenate([np.sort(rng.choice(n, c, replace=False)) for c in counts]).astype(np.int32)
+    d = torch.device("cuda", 0)
+    row_old, col_new = rng.permutation(m).astype(np.int32), rng.permutation(n).astype(np.int32)
+    dev = [torch.from_numpy(x).to(d) for x in (rp, ci, np.zeros(ci.size), row_old, col_new)]
+    out = [torch.empty(m + 1, dtype=torch.int32, device=d), torch.empty(ci.size, dtype=torch.int32, device=d),
+           torch.empty(ci.size, dtype=torch.float64, device=d)]
+    stream = torch.cuda.Stream()
+    ctx = tsg.Context(0, stream=stream.cuda_stream)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        tsg.check(tsg.lib().tsg_permute_csr(ctx.handle, m, n, ci.size, *[ctypes.c_void_p(t.data_ptr()) for t in dev + out]))
+    for seed in (1, 2):
+        v = np.random.default_rng(seed).uniform(-1, 1, ci.size)
+        dev[2].copy_(torch.from_numpy(v))
+        graph.replay()
+        torch.cuda.synchronize()
+        want = oracle.apply_bipermutation((m, n, rp, ci, v), row_old, col_new)
+        for got, w in zip(out, want[2:]):
+            np.testing.assert_array_equal(got.cpu().numpy(), w)
+    del graph
+    ctx.close()
