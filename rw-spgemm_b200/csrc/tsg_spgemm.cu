@@ -1023,6 +1023,15 @@ static int spgemm_finish(tsg_context *ctx, SpgemmRun &R, tsg_spgemm_info *info)
     return TSG_OK;
 }
 
+// the scratch of a product that failed
+static void spgemm_drop(tsg_context *ctx, SpgemmRun &R)
+{
+    tsg_release(ctx, R.bits.words);
+    tsg_release(ctx, R.bits.span);
+    tsg_release(ctx, R.d_wide);
+    win_release(ctx, R.win);
+}
+
 extern "C" int tsg_spgemm(tsg_context *ctx, const tsg_tiled *A, const tsg_tiled *B, tsg_tiled *C,
                           tsg_spgemm_info *info)
 {
@@ -1030,10 +1039,15 @@ extern "C" int tsg_spgemm(tsg_context *ctx, const tsg_tiled *A, const tsg_tiled 
         return tsg_set_error(TSG_ERR_INVALID, "null argument");
     TSG_TRY(validate_operands(A, B));
     SpgemmRun R;
-    TSG_TRY(spgemm_structure(ctx, A, B, C, R));
+    int status = spgemm_structure(ctx, A, B, C, R);
     // step 3: numeric
-    if (R.nnzC > 0)
-        TSG_TRY(launch_step3(ctx, make_view(A, B, C), A, B->nnz, R.nnzC, R.d_wide, R.win));
+    if (status == TSG_OK && R.nnzC > 0)
+        status = launch_step3(ctx, make_view(A, B, C), A, B->nnz, R.nnzC, R.d_wide, R.win);
+    if (status != TSG_OK)
+    {
+        spgemm_drop(ctx, R);
+        return status;
+    }
     if (ctx->timing)
         TSG_CUDA(cudaEventRecord(ctx->ev[3], ctx->stream));
     return spgemm_finish(ctx, R, info);
@@ -1139,10 +1153,7 @@ int tsg_spgemm_to_host(tsg_context *ctx, const tsg_tiled *A, const tsg_tiled *B,
     if (status == TSG_OK)
         status = spgemm_finish(ctx, R, info);
     else
-    {
-        tsg_release(ctx, R.d_wide);
-        win_release(ctx, R.win);
-    }
+        spgemm_drop(ctx, R);
     tsg_tiled_free(ctx, &C);
     if (status == TSG_OK)
         TSG_CUDA(cudaStreamSynchronize(st));

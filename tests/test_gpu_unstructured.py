@@ -231,3 +231,24 @@ def test_few_tiles_over_many_columns(tsg, ctx, oracle, entries, n):
     batch.sync()
     _same([x.cpu().numpy() for x in tsg.tiled_to_csr(ctx, batch.product(0))], oracle.gustavson(A, B, nthreads=8))
     batch.close()
+
+
+def test_products_that_fail_leave_no_scratch(tsg, ctx):
+    """C past 32-bit offsets is refused after steps 1 and 2, whose scratch goes."""
+    n = 50000
+    A = n, 16, np.arange(n + 1, dtype=np.int32), np.zeros(n, np.int32), np.ones(n)
+    B = 16, n, np.array([0] + [n] * 16, np.int32), np.arange(n, dtype=np.int32), np.ones(n)
+    tA, tB = _tiled(tsg, ctx, A, tsg.TSG_TILED_CSC_VIEW), _tiled(tsg, ctx, B, tsg.TSG_TILED_CSC_VIEW)
+    ctx.synchronize()
+    used = ctx.pool_used()
+    for _ in range(2):
+        with pytest.raises(tsg.TsgError) as e:
+            tsg.spgemm(ctx, tA, tB)
+        assert e.value.status == tsg.TSG_ERR_OVERFLOW
+        del e
+    import gc
+    gc.collect()
+    ctx.synchronize()
+    assert ctx.pool_used() <= used
+    for t in (tA, tB):
+        t.free()
