@@ -522,10 +522,13 @@ extern "C" int tsg_csr_to_tiled(tsg_context *ctx, int m, int n, int nnz, const i
     tsg_release(ctx, heavy);
     if (flags & TSG_TILED_CSC_VIEW)
     {
-        // the row view is the input itself
+        // the row view is the input itself (of a matrix without rows nothing is read)
         TSG_TRY(alloc_row_view(ctx, out));
-        TSG_CUDA(cudaMemcpyAsync(out->row_ptr, d_rowptr, ((size_t)m + 1) * sizeof(int), cudaMemcpyDeviceToDevice,
-                                 ctx->stream));
+        if (m > 0)
+            TSG_CUDA(cudaMemcpyAsync(out->row_ptr, d_rowptr, ((size_t)m + 1) * sizeof(int), cudaMemcpyDeviceToDevice,
+                                     ctx->stream));
+        else
+            TSG_CUDA(cudaMemsetAsync(out->row_ptr, 0, sizeof(int), ctx->stream));
         if (nnz > 0)
         {
             TSG_CUDA(cudaMemcpyAsync(out->row_col, d_colidx, (size_t)nnz * sizeof(int), cudaMemcpyDeviceToDevice,

@@ -95,3 +95,13 @@ def test_column_view_of_columns_short_and_long(tsg, ctx, m, n, tiles):
     tc = np.unique((ci // 16).astype(np.int64) * ((m + 15) // 16) + r // 16)  # (tile column, tile row)
     np.testing.assert_array_equal(got["csc_tile_rowidx"], tc % ((m + 15) // 16))
     np.testing.assert_array_equal(np.diff(got["csc_tile_ptr"]), np.bincount(tc // ((m + 15) // 16), minlength=(n + 15) // 16))
+
+
+@pytest.mark.parametrize("flags", [0, 1, 2, 3])
+def test_a_matrix_without_rows_needs_no_arrays(tsg, ctx, flags):
+    import ctypes
+    T = tsg.Tiled(ctx)
+    tsg.check(tsg.lib().tsg_csr_to_tiled(ctx.handle, 0, 40, 0, None, None, None, flags, ctypes.byref(T.s)))
+    got = [x.cpu().numpy() for x in tsg.tiled_to_csr(ctx, T)]
+    assert T.numtile == 0 and np.array_equal(got[0], [0]) and got[1].size == 0
+    T.free()
