@@ -1048,16 +1048,17 @@ static int record_run(tsg_batch *b, cudaStream_t st)
     k_batch_spa3<<<b->grid3, SPA_THREADS, sizeof(SpaSmem), side[0]>>>(b->d_prod, b->count, b->d_itemoff, b->d_bar, b->d_err,
                                                                     b->dense);
     TSG_CUDA(cudaGetLastError());
-    if (b->rows_form)
-    {
-        k_batch_dense3<false><<<b->ctx->num_sms * 8, DENSE3_THREADS, 0, side[1]>>>(b->d_prod, b->count, b->d_denseoff,
-                                                                                 b->d_itemoff, b->d_err);
-        TSG_CUDA(cudaGetLastError());
-    }
+    // dense A tiles first, before the windows' CTAs hold the SMs' shared memory
     if (b->cols_form)
     {
         k_batch_dense3<true><<<b->ctx->num_sms * 4, DENSE3_THREADS, 0, side[1]>>>(
             b->d_prod, b->count, b->d_denseoff + b->count + 1, b->d_itemoff, b->d_err);
+        TSG_CUDA(cudaGetLastError());
+    }
+    if (b->rows_form)
+    {
+        k_batch_dense3<false><<<b->ctx->num_sms * 8, DENSE3_THREADS, 0, side[1]>>>(b->d_prod, b->count, b->d_denseoff,
+                                                                                 b->d_itemoff, b->d_err);
         TSG_CUDA(cudaGetLastError());
     }
     TSG_TRY(tsg_join(b->ctx, st, TSG_SIDE_STREAMS));
