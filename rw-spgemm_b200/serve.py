@@ -209,7 +209,8 @@ class SpGEMMServer:
         of a queued or running job cannot be replaced."""
         if key in self.matrices and self.matrices[key] is not mat:
             keys = {key, (key, "T")}
-            busy = [j for j in self.queue] + [j for sl in self.slots for j in sl.jobs]
+            with self.lock:
+                busy = list(self.queue) + [j for sl in self.slots for j in sl.jobs]
             if any(j.a_key in keys or j.b_key in keys for j in busy):
                 raise RuntimeError(f"operand {key!r} is in use by a queued or running job")
             self.matrices.pop((key, "T"), None)
@@ -305,8 +306,10 @@ class SpGEMMServer:
         """Predicts the queued jobs of the first job's class within the
         lookahead (as many as a batch holds) whose operands are resident,
         with at most one synchronisation."""
-        cls = self.queue[0].cls if self.queue else 0
-        todo = [j for j in itertools.islice(self.queue, self.lookahead) if j.cls == cls and j.pred_prods < 0 and
+        with self.lock:  # submit appends from other threads
+            head = list(itertools.islice(self.queue, self.lookahead))
+        cls = head[0].cls if head else 0
+        todo = [j for j in head if j.cls == cls and j.pred_prods < 0 and
                 j.a_key in self.cache.tiles and j.b_key in self.cache.tiles][:self.max_batch]
         if todo:
             self._predict_jobs(todo, [(self.cache.tiles[j.a_key], self.cache.tiles[j.b_key]) for j in todo])

@@ -294,3 +294,22 @@ def test_host_delivery_copies_every_result_out_of_the_staging_buffer(serve_mod, 
         assert np.array_equal(got[4].view(np.uint64), v.view(np.uint64))
     assert slot.pending is None and slot.batch is None
     srv._pool.shutdown()
+
+
+def test_jobs_may_arrive_while_the_queue_is_looked_through(serve_mod, monkeypatch):
+    """submit appends to the queue from other threads at any time, also while
+    the dispatcher looks through it for jobs to predict."""
+    predict = {("a", "b"): (10, 1), ("c", "d"): (10, 1)}
+    srv = make_server(serve_mod, monkeypatch, 10_000, 1e9, {k: 1 for k in "abcd"}, predict)
+
+    class Tiles(collections.OrderedDict):
+        def __contains__(self, key):
+            if srv.next_id < 6:
+                srv.submit("AB", "c", "d")
+            return super().__contains__(key)
+
+    srv.cache.tiles = Tiles()
+    for _ in range(2):
+        srv.submit("AB", "a", "b")
+    assert srv._form_batch(srv.slots[0])
+    assert len(srv.slots[0].jobs) + len(srv.queue) == srv.next_id == 6
