@@ -31,6 +31,8 @@
 // 0.72 ms, a band of 65 times 8,192 random rows (4.2 M) 0.169 -> 0.136 ms.
 #pragma once
 
+#include <algorithm>
+
 #include "tsg_device.cuh"
 
 #define WIN_COLS 1024 // (512: as many warps again, R-MAT 16 no faster)
@@ -52,9 +54,12 @@
 // of B: C has to hold WIN_MIN_VALUES values (a batch, that knows no values:
 // BATCH_WIN_MIN products) per (row, window) and WIN_MIN_TILES tiles per (tile
 // row, window), and the tables may take WIN_TABLE_SHARE words per value of C, or
-// WIN_TABLE_FREE.  What the windows are for is uneven work: where C has WIN_SKEW
-// times the products that A's entries and B's mean row give, that is all.
-// Elsewhere C's tiles have to hold WIN_TILE_VALUES values on average -- below,
+// WIN_TABLE_FREE.  What the windows are for is uneven work -- where C has WIN_SKEW
+// times the products that A's entries and B's mean row give -- and A rows of few
+// entries, WIN_VISIT_VALUES values of C for each and window: that is all there.
+// Elsewhere C has to fill the windows, WIN_EVEN_TILES of 64 tiles or all there
+// are -- k_step3_spa walks A's entries once for 256 tiles of C, however far apart
+// -- and its tiles have to hold WIN_TILE_VALUES values on average -- below,
 // k_step3_spa's hypersparse form keeps up -- or C one value for every entry of A
 // and window.  Step 3, k_step3_spa<flat> and windows, B200:
 //   uneven: R-MAT 13 2.2 and 0.40 ms, a 64th of R-MAT 16's rows 4.7 and 1.0
@@ -64,9 +69,15 @@
 //   words of table a value: rows of 60 times 100,000 x 40,000 of 12, 4,000 rows
 //     (8) 0.53 and 0.35, 1,000 rows (33) 0.199 and 0.169, 256 rows (130) 0.078
 //     and 0.124; 64 rows of 64 times 1 M x 16,384 (1,600) 0.067 and 0.25
-//   tiles a window: batch of 24^3 grids (3) 0.35 and 0.51
+//   tiles a window: batch of 24^3 grids (3) 0.35 and 0.51; a band of 129 times
+//     random rows of 8, 65,536 rows (18) 3.2 and 7.5, 32,768 (31) 1.5 and 2.1, of 65
+//     16,384 rows (36) 0.33 and 0.38, 8,192 (50) 0.169 and 0.136
+//   values a visit: random rows of 8 times a band, 16,384 rows, 97 wide (6) 0.41
+//     and 0.28, 17 (1) 0.19 and 0.20; 32,768, 33 (1) 0.43 and 0.63
 #define WIN_MIN_VALUES 8
 #define WIN_MIN_TILES 8
+#define WIN_EVEN_TILES 38
+#define WIN_VISIT_VALUES 2
 #define WIN_SKEW 2
 #define WIN_TILE_VALUES 3
 #define WIN_TABLE_FREE (1LL << 21)
@@ -137,10 +148,12 @@ static inline int win_heavy(long long nnzA, long long rows)
 static inline bool win_worth(long long values, long long products, long long nnzA, long long tilesC, long long tile_rows,
                              long long tilen, long long windows, long long tables)
 {
-    const long long least = WIN_MIN_TILES * windows < tilen ? WIN_MIN_TILES * windows : tilen;
-    if (tilesC < least * tile_rows || (tables > WIN_TABLE_FREE && tables > WIN_TABLE_SHARE * values))
+    const auto fills = [&](long long tiles) { return tilesC >= std::min(tiles * windows, tilen) * tile_rows; };
+    if (!fills(WIN_MIN_TILES) || (tables > WIN_TABLE_FREE && tables > WIN_TABLE_SHARE * values))
         return false;
-    return values >= WIN_SKEW * products || values >= WIN_TILE_VALUES * tilesC || values >= nnzA * windows;
+    const long long visits = nnzA * windows;
+    return values >= WIN_SKEW * products || values >= WIN_VISIT_VALUES * visits ||
+           (fills(WIN_EVEN_TILES) && (values >= WIN_TILE_VALUES * tilesC || values >= visits));
 }
 
 // B row w's entry offset at every block boundary, by a warp

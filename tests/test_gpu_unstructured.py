@@ -252,3 +252,12 @@ def test_products_that_fail_leave_no_scratch(tsg, ctx):
     assert ctx.pool_used() <= used
     for t in (tA, tB):
         t.free()
+
+
+@pytest.mark.parametrize("n,wins", [(20000, False), (2000, True)])
+def test_windows_that_c_does_not_fill(tsg, ctx, oracle, gen, n, wins):
+    """A band times random rows: each C tile row meets about 230 tile columns,
+    12 of a window's 64 over 20,000 columns and all of them over 2,000."""
+    A, B = gen.banded(n, 16, seed=1), gen.random_poisson(n, n, 8.0, seed=2)
+    info = _check(tsg, ctx, oracle, A, B, tsg.TSG_TILED_CSC_VIEW)
+    assert (info["step3_name"] == "k_step3_win") == wins
