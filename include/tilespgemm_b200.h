@@ -265,7 +265,9 @@ typedef struct tsg_context tsg_context;
  * (csc_tile_rowidx) and the row-major tile index (csc_tile_pos) of each tile.
  * Matrices converted for the B role (TSG_TILED_CSC_VIEW) also carry a row
  * view: the same matrix as scalar CSR (row_ptr[m+1], row_col[nnz],
- * row_val[nnz]), read by the numeric step of TSG_SCHED_SPA.
+ * row_val[nnz]), read by the symbolic and numeric steps of TSG_SCHED_SPA: of B
+ * always, of A by some of its numeric kernels.  A caller that changes a
+ * matrix's entries changes them in both forms.
  * All pointers are device pointers owned by the library. */
 typedef struct
 {
@@ -284,7 +286,7 @@ typedef struct
     int *csc_tile_rowidx;
     int *csc_tile_pos;
     unsigned short *mask_t; /* B operand: per tile column masks, bit (15-row) */
-    int *row_ptr;           /* B operand: row view (scalar CSR)             */
+    int *row_ptr;           /* row view (scalar CSR)                        */
     int *row_col;
     double *row_val;
     void *_alloc;           /* internal: non-NULL marks a borrowed view      */
@@ -342,11 +344,11 @@ int tsg_context_set_stream(tsg_context *ctx, void *cuda_stream);
  *                  through A's row masks and B's column masks (register
  *                  accumulator, no shared-memory scatter). */
 #define TSG_SCHED_ELEMS 2
-/* TSG_SCHED_SPA    step 2 as TILES; step 3 as a row Gustavson over B's row
- *                  view (scalar CSR): a CTA per run of C tiles of one tile
- *                  row, a warp per C row, products accumulated in shared
- *                  memory in C's tiled layout.  B without a row view runs
- *                  TSG_SCHED_TILES. */
+/* TSG_SCHED_SPA    step 2 row by row (see tsg_context_set_fusion), wide tile
+ *                  rows over B's row view; step 3 as a row Gustavson over B's
+ *                  row view (scalar CSR), a warp per C row or part of one,
+ *                  products accumulated in shared memory.  B without a row
+ *                  view runs TSG_SCHED_TILES. */
 #define TSG_SCHED_SPA 3
 int tsg_context_set_schedule(tsg_context *ctx, int schedule, int seg_tiles, int acc_cap);
 /* TSG_SCHED_SPA: a product whose C tiles hold at least values_per_tile
@@ -355,8 +357,11 @@ int tsg_context_set_schedule(tsg_context *ctx, int schedule, int seg_tiles, int 
  * the default (64); 257 never switches.  Results are identical either way. */
 int tsg_context_set_dense_threshold(tsg_context *ctx, int values_per_tile);
 /* 1 (default): step-1 emit and step 2 run as one row-wise pass for tile rows
- * with at most 128 C tiles (others fall back to step 2 per tile); 0: separate
- * step 2 of the schedule.  Results are identical. */
+ * with at most 128 C tiles in a window of 8,192 tile columns (TSG_SCHED_SPA
+ * sends the others, and rows of more than 1,024 tile pairs with few scalar
+ * products in each, to a step 2 of its own for wide rows; the other schedules
+ * do step 2 per tile there); 0: separate step 2 of the schedule.  Results are
+ * identical. */
 int tsg_context_set_fusion(tsg_context *ctx, int fuse_step12);
 /* 0 when all work queued on the context's stream has finished, 1 while
  * some is pending, a negative status on error (non-blocking). */

@@ -1,16 +1,24 @@
 // Batched tiled SpGEMM: many independent products C_p = A_p * B_p of uneven
-// size in ONE persistent, cooperatively launched kernel, captured once in a
-// CUDA graph and replayed by tsg_batch_run.
+// size in ONE persistent, cooperatively launched kernel (and, for the SPA
+// schedule, step 3's kernels after it), captured once in a CUDA graph and
+// replayed by tsg_batch_run.
 //
-// The kernel runs seven phases separated by a grid barrier; in each phase the
+// The kernel runs its phases separated by a grid barrier; in each phase the
 // work of all products is one flattened index space (product found by binary
 // search over a prefix array), so small products do not leave the GPU idle:
-//   1 step-1 counts (warp per A tile row)        2 per-product scan of them
-//   3 item prefix over products (block 0)        4 step-1 emit
-//   5 step 2 (half-warp per item)                6 per-product scan of tile nnz
-//   7 step 3 (half-warp per item)
-// An item is one C tile (tile schedule) or seg_tiles C tiles (row schedule);
-// the per-item code is tsg_device.cuh's, identical to the one-product path.
+//   1 step-1 counts: tile rows of products with many tile pairs a CTA each, the
+//     others' a warp each                  2 per-product scan of them
+//   3 item prefix over products (block 0)  4 step-1 emit, fused with step 2 for
+//     narrow rows unless the row schedule runs its own
+//   5 step 2 of the rest: units of wide rows, a CTA each (SPA), or a half-warp
+//     per item                             6 per-product scan of tile nnz
+//   7 step 3, a half-warp or warp per item; the SPA schedule leaves it to up to
+//     six kernels: k_batch_wtab and k_batch_win (windows), k_batch_hyper and
+//     k_batch_spa3 (the other sparse C tiles) and k_batch_dense3 in one or both of
+//     its forms (dense C tiles), side by side on the context's streams
+// An item is one C tile (tile and element schedules) or seg_tiles C tiles (row
+// schedule); the per-item code is tsg_device.cuh's, identical to the one-product
+// path.
 //
 // Memory: one arena per batch, sized at creation from per-product upper
 // bounds computed on the device (C tiles <= matched tile pairs, C nonzeros <=
@@ -89,8 +97,10 @@ struct tsg_batch
 #define BATCH_THREADS 128
 #define BATCH_SPAN 3072 // tile columns of step 2's wide rows in a CTA's shared memory (two CTAs an SM)
 // step 3 by windows: products with this many scalar products per (row, window)
-// (win_worth says the rest), whose tables and lists together take up to this
-// many words each and in all
+// (win_worth says the rest; 4 products of 4,096 random rows, step 3 by
+// k_batch_spa3 and by windows, with 8 products a (row, window) 0.066 and 0.086 ms,
+// with 16 0.110 and 0.096), whose tables and lists together take up to this many
+// words each and in all
 #define BATCH_WIN_MIN 16
 #define BATCH_WIN_WORDS (1LL << 23)
 #define BATCH_WIN_TOTAL (1LL << 26)
@@ -554,8 +564,8 @@ __global__ void __launch_bounds__(NT)
     if (!grid_barrier(bar, err))
         return;
     BATCH_STAMP(6)
-    // phase 7: step 3 (the SPA schedule runs it as two kernels after this one:
-    // k_batch_spa3 and k_batch_dense3, each at its own occupancy)
+    // phase 7: step 3 (the SPA schedule's kernels follow this one, each at its own
+    // occupancy; they get the prefix of the dense products' tiles)
     if (SCHED == 3)
     {
         // C tiles of the products that take the tile kernel by rows, prefix,

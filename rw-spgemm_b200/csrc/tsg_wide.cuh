@@ -18,8 +18,10 @@
 // bitmap words are kept (`words`, see StepOneBits) for the emit pass.
 // ---------------------------------------------------------------------------
 #define S1C_WORDS 2048
-// a CTA per tile row from this many tile pairs per row (mean tiles per row of
-// A times B's): below it a warp per row keeps up
+// A CTA per tile row from this many tile pairs per row (mean tiles per row of
+// A times B's).  Step 1 by warps and by CTAs, random rows: 262,144 rows, 256 pairs
+// 0.250 and 0.264 ms, 502 0.326 and 0.339, 1,024 0.423 and 0.417; 32,768 rows, 125
+// 0.073 and 0.075, 502 0.071 and 0.058; 64^3 stencil (484) 0.384 and 0.411.
 #define S1_CTA_PAIRS 512
 // a row's words are kept up to this many (16,384 tile columns)
 #define S1_KEEP_WORDS 512
@@ -198,12 +200,13 @@ __device__ __forceinline__ int step1_row_cta(const ProdView &P, int i, S1cSmem<N
 // unless it is set already.  A thread per C tile then writes its masks, row
 // offsets and count.  A tile row is walked once per WD tile columns, where
 // segments of 1,024 tiles walked (and cut B's rows) four times as often at
-// 65,536 columns, and a hypersparse row is no special case.
+// 65,536 columns; a hypersparse row is a special case only where its few tiles
+// lie in more columns than that.
 //
 // Bound: instructions of the walk and, for hypersparse rows, the 52 bytes
 // written per C tile.  On a B200, with the scan of the counts: R-MAT 16 (402 M
 // products) 3.09 -> 1.51 ms, R-MAT 14 (53 M) 1.03 -> 0.295 ms, 65,536 random rows
-// (16.4 M C tiles, 4.2 M products) 0.875 -> 0.545 ms.
+// (16.4 M C tiles, 4.2 M products) 0.875 -> 0.480 ms.
 // ---------------------------------------------------------------------------
 #define WIDE_UNROLL 4
 #define WIDE_SPARSE 4 // products a C tile up to which a row may take a slot per tile
