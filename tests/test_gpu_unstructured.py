@@ -105,8 +105,8 @@ def test_window_step_on_tile_row_ranges(tsg, ctx, oracle, gen):
 
 
 def test_batch_of_uneven_products(tsg, ctx, oracle, gen):
-    """All routes of a batch's steps in one: windows with heavy rows, the SPA
-    kernel, hypersparse rows, dense tiles, an empty product."""
+    """Windows with heavy rows, hypersparse rows, dense tiles and an empty product
+    in one batch (the SPA kernel's rows in a batch: test_hypersparse_rows_among_others)."""
     empty = (20, 300, np.zeros(21, np.int32), np.zeros(0, np.int32), np.zeros(0))
     mats = [_case("heavy"), _case("cols257"), _case("parts"), (gen.rmat(11, 12, seed=2), gen.rmat(11, 12, seed=3)),
             (gen.random_poisson(8192, 8192, 4.0, seed=10), gen.random_poisson(8192, 8192, 4.0, seed=11)),
@@ -173,11 +173,11 @@ def test_spa_rows_whose_products_meet(tsg, ctx, oracle, entries):
     assert _check(tsg, ctx, oracle, A, B, tsg.TSG_TILED_CSC_VIEW)["step3_name"] == "k_step3_spa<flat>"
 
 
-def _mixed(tile_rows, seed):
-    """Wide C tile rows, one in six with several values a tile and the others
+def _mixed(tile_rows, seed, every=6):
+    """Wide C tile rows, one in `every` with several values a tile and the others
     hypersparse, too few values a window for the window step."""
     m = 16 * tile_rows - 11
-    A = _rows(m, 4000, [300 if i // 16 % 6 == 1 else 3 for i in range(m)], seed)
+    A = _rows(m, 4000, [300 if i // 16 % every == 1 else 3 for i in range(m)], seed)
     return A, _rows(4000, 64000, [4] * 4000, seed + 1)
 
 
@@ -200,10 +200,12 @@ def test_hypersparse_rows_among_others(tsg, ctx, oracle, dense):
 
 
 def test_hypersparse_rows_among_others_on_tile_row_ranges(tsg, ctx, oracle):
-    A, B = _mixed(640, 3)
+    A, B = _mixed(1100, 3, every=9)
     out = tsg.HostResultBuffers(A[0], 1 << 22)
     got, info = tsg.spgemm_csr_host_overlap(ctx, A, B, out)
     assert info["nnz_C"] > 2 << 20 and info["step3_name"] == "k_step3_spa<flat>"
+    # a kernel of its own takes the hypersparse rows: enough tiles, few values in them
+    assert info["numtile_C"] >= 1 << 17 and info["nnz_C"] < 4 * info["numtile_C"]
     _same(got[2:], oracle.gustavson(A, B, nthreads=8))
 
 
